@@ -70,5 +70,9 @@ __device__ __forceinline__ uint2 pack8(const int (&q)[8]) {
 __device__ __forceinline__ float swiglu(float g, float u) {
   return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf_exact(-g))), u);
 }
+// The same bits with the branch-free exponential (expf_exact.cuh says which kernels take which).
+__device__ __forceinline__ float swiglu_flat(float g, float u) {
+  return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf_exact_flat(-g))), u);
+}
 
 }  // namespace cmld

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(1024 / W) attn_prompt_kernel(AttnArgs a, float
 #pragma unroll
     for (int j = 0; j < 4; ++j) e[j] = sc[(int64_t)min(p + j * PS, own - 1) * PITCH + m];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) e[j] = expf_exact(__fsub_rn(e[j], top));
+    for (int j = 0; j < 4; ++j) e[j] = expf_exact_flat(__fsub_rn(e[j], top));
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (p + j * PS < own) sc[(int64_t)(p + j * PS) * PITCH + m] = e[j];

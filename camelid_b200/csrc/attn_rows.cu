@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kRowsThreads) attn_rows_kernel(AttnArgs a, int
   __syncthreads();
   for (int i = tid; i < G * n_pos; i += kRowsThreads) {
     const int g = i / n_pos, p = i % n_pos;
-    sc[(int64_t)g * cap + p] = expf_exact(__fsub_rn(sc[(int64_t)g * cap + p], s_head[g][0]));
+    sc[(int64_t)g * cap + p] = expf_exact_flat(__fsub_rn(sc[(int64_t)g * cap + p], s_head[g][0]));
   }
   __syncthreads();
   if (tid < G) {

@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kExactAttnThreads) attn_exact_kernel(AttnArgs 
   __syncthreads();
   m = s_bcast[0];
   for (int p = threadIdx.x; p < n_pos; p += blockDim.x)
-    if (live(p)) s_sc[p] = expf_exact(__fsub_rn(s_sc[p], m));
+    if (live(p)) s_sc[p] = expf_exact_flat(__fsub_rn(s_sc[p], m));
   __syncthreads();
   if (threadIdx.x == 0) {
     float sum = 0.0f;

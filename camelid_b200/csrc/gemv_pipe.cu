@@ -907,7 +907,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) gemv_pipe_kernel(const PipeAr
           for (int k = 0; k < B; ++k) {
             int r, b;
             if (chain_slot<B>(J.qt, rpw, k, lane, r, b) && wge * rpw + r < nrows)
-              a.job[0].y[(int64_t)b * a.job[0].y_stride + row0 + wge * rpw + r] = swiglu(res[k], buf[(wg * rpw + r) * B + b]);
+              a.job[0].y[(int64_t)b * a.job[0].y_stride + row0 + wge * rpw + r] = swiglu_flat(res[k], buf[(wg * rpw + r) * B + b]);
           }
         }
         ++done_pairs;

@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kQ8AttnThreads) attn_q8_kernel(AttnArgs a, con
   }
   __syncthreads();
   m = s_bcast[0];
-  for (int p = threadIdx.x; p < n_pos; p += blockDim.x) s_sc[p] = expf_exact(__fsub_rn(s_sc[p], m));
+  for (int p = threadIdx.x; p < n_pos; p += blockDim.x) s_sc[p] = expf_exact_flat(__fsub_rn(s_sc[p], m));
   __syncthreads();
   if (threadIdx.x == 0) {
     float sum = 0.0f;

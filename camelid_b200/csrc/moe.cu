@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float *__restrict_
   float sum = 0.0f;
   for (int s = 0; s < k; ++s) {
     const float v = logits[idx[s]];
-    w[s] = isfinite(v) ? expf_exact(__fsub_rn(v, mx)) : 0.0f;
+    w[s] = isfinite(v) ? expf_exact_flat(__fsub_rn(v, mx)) : 0.0f;
     sum = __fadd_rn(sum, w[s]);
   }
   for (int s = 0; s < k; ++s) w[s] = sum > 0.0f ? __fdiv_rn(w[s], sum) : __fdiv_rn(1.0f, (float)k);
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(256) moe_quant3_kernel(const Quant3Args a) {
         }
       }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = swiglu(g[i], u[i]);
+      for (int i = 0; i < 8; ++i) v[i] = swiglu_flat(g[i], u[i]);
     }
 #pragma unroll
     for (int p3 = 0; p3 < 3; ++p3) {

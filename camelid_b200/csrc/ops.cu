@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kNormThreads) norm_quant_kernel(NormQuantArgs 
         if (MODE == 1) t = __fmul_rn(__fmul_rn(x[e], scale), a.weight[e]);
         else if (MODE == 2) {
           const float g = x[e];
-          t = swiglu(g, x2[e]);
+          t = swiglu_flat(g, x2[e]);
         } else t = x[e];
         if (a.out) a.out[(int64_t)b * a.cols + e] = t;
       }

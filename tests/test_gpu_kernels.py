@@ -331,6 +331,40 @@ def test_rms_norm_and_swiglu(cm, orc, cols, batch):
     assert np.array_equal(out.view(np.uint32), ref.view(np.uint32))  # expf restated from glibc: the same bits
 
 
+# Both forms of the restated expf outside its range: the branch-free one in the separate SwiGLU kernel, the branching one in the
+# staged matvec's prologue (one argument per call, so that the sum is its value).
+def test_silu_mul_beyond_the_range_of_expf(cm, orc):
+    from camelid_b200.engine import DeviceBuffer
+    from camelid_b200._lib import check
+
+    g = np.zeros(256, np.float32)
+    g[:20] = [88.7, 88.73, 89.0, -88.7, -88.73, -89.0, 103.9, 104.0, 110.0, -103.9, -104.0, -110.0, 3e38, -3e38, 0.0, -0.0, 1e-40, -1e-40, 200.0, -200.0]
+    u = np.ones(256, np.float32)
+    gd, ud, od = DeviceBuffer.from_numpy(g), DeviceBuffer.from_numpy(u), DeviceBuffer(g.nbytes)
+    check(cm.lib().cmld_silu_mul(gd.ptr, ud.ptr, 256, 1, od.ptr, 0, None))
+    want = orc.silu_mul(g, u)
+    assert np.array_equal(od.to_numpy(np.float32).view(np.uint32), want.view(np.uint32))
+    special = g.copy()
+    special[:3] = [np.inf, -np.inf, np.nan]
+    sd = DeviceBuffer.from_numpy(special)
+    check(cm.lib().cmld_silu_mul(sd.ptr, ud.ptr, 256, 1, od.ptr, 0, None))
+    with np.errstate(all="ignore"):
+        want = orc.silu_mul(special, u)
+    assert np.array_equal(od.to_numpy(np.float32), want, equal_nan=True)
+    wire = orc.quantize(8, np.ones((4, 256), np.float32))
+    w = cm.Weight.from_wire(8, 4, 256, wire)
+    y = DeviceBuffer(16)
+    for v in (88.7, -88.7, 104.0, -104.0, 3e34, -3e38, 200.0, -200.0):
+        x = np.zeros((1, 256), np.float32)
+        x[0, 5] = v
+        xd = DeviceBuffer.from_numpy(x)
+        check(cm.lib().cmld_gemv_fused(w._h, 3, xd.ptr, ud.ptr, ud.ptr, 1e-5, 1, y.ptr, None))
+        f = orc.silu_mul(x[0], u)
+        codes, scales = orc.quantize_act_q8_0(f)
+        ref = orc.matvec_quantised(8, wire, 4, 256, codes, scales)
+        assert np.array_equal(y.to_numpy(np.float32).view(np.uint32), ref.view(np.uint32)), v
+
+
 # The sum of squares is evaluated in parallel with the sequential sum's bits (runs of additions inside one binade
 # applied as integer steps, ties and binade crossings replayed): rows built to hit the replay paths.
 @pytest.mark.parametrize("cols", [4096, 8192, 1024])
