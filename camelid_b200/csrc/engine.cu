@@ -166,7 +166,7 @@ int32_t init_rows(cmld_engine *e, int64_t rows, int64_t logit_rows, int64_t voca
 static int32_t prompt_rows(const cmld_engine *e) {
   const cmld_config &c = e->cfg;
   const uint32_t other = CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV | CMLD_FLAG_TENSOR_BATCH | CMLD_FLAG_FAST_ORDER | CMLD_FLAG_KV_Q8_0;
-  if (((uint32_t)c.flags & other) || c.hidden % 256 || c.ffn_dim % 256 || (c.n_heads * c.head_dim) % 256) return 32;
+  if (((uint32_t)c.flags & other) || c.hidden % 256 || c.ffn_dim % 256 || (c.n_heads * c.head_dim) % 256) return kShortRows;
   return (int32_t)std::min<int64_t>(512, ((int64_t)c.max_pos + 31) / 32 * 32);
 }
 
@@ -174,7 +174,7 @@ static int32_t engine_init(cmld_engine *e) {
   const cmld_config &c = e->cfg;
   CMLD_TRY(engine_open(e, e->device));
   const int seqs = std::max(1, c.max_seqs);
-  const int64_t L = std::max(seqs, 32);  // rows of a step that the caller lists one by one, and of the logits
+  const int64_t L = std::max(seqs, kShortRows);  // rows of a step that the caller lists one by one, and of the logits
   e->chunk_rows = prompt_rows(e);
   const int64_t R = std::max<int64_t>(L, e->chunk_rows);
   CMLD_TRY(init_rows(e, R, L, e->vocab_local));
@@ -755,8 +755,9 @@ static int32_t engine_step(cmld_engine *e, const StepOpts &o) {
   if (sharded && !e->comm)
     return fail(CMLD_ERR_STATE, "this sharded engine has no communicator (cmld_engine_comm_init not called, or aborted after a peer stopped answering)");
   const bool lead = e->shard_rank == 0;  // the rank whose partial sums carry the residual
-  if (B < 1 || B > std::max(e->max_rows, e->chunk_rows) || (B > e->max_rows && (o.logits || o.taps)))
-    return fail(CMLD_ERR_INVALID, "step of %d rows exceeds the engine's %d", B, e->max_rows);
+  const int32_t most = o.prompt_end ? e->chunk_rows : e->max_rows;
+  if (B < 1 || B > most) return fail(CMLD_ERR_INVALID, "step of %d rows exceeds the engine's %d", B, most);
+  if (o.prompt_end && (o.logits || o.taps)) return fail(CMLD_ERR_INVALID, "a prompt's long step has its logits formed row by row");
   if (o.from_tokens) {
     if (!e->has_embd) return fail(CMLD_ERR_STATE, "token embedding table not set");
     CMLD_TRY(launch_embed_gather(e->token_embd, e->d_tokens, B, e->h, e->stream));
@@ -839,7 +840,7 @@ static int32_t engine_step(cmld_engine *e, const StepOpts &o) {
       const bool rows = !fast && !(c.flags & CMLD_FLAG_EXACT_ORDER) && B >= 3 && o.attn_cap > 0 && !o.tree_mask &&
                         attention_rows_fits(c.n_heads, c.n_kv_heads, c.head_dim, o.attn_cap);
       // a prompt's long steps (never captured: their context is exact): neighbouring rows share a CTA
-      const bool prompt = rows && B > e->max_rows && attention_prompt_fits(c.n_heads, c.n_kv_heads, c.head_dim, B, o.prompt_end);
+      const bool prompt = rows && o.prompt_end && attention_prompt_fits(c.n_heads, c.n_kv_heads, c.head_dim, B, o.prompt_end);
       const bool ordered = !rows && !fast && !(c.flags & CMLD_FLAG_EXACT_ORDER) && o.attn_cap > 0 && !o.tree_mask &&
                            attention_ordered_fits(c.n_heads, c.n_kv_heads, c.head_dim, o.attn_cap);
       const bool fuse = !o.shared_slots && (fast || ordered);
@@ -974,7 +975,7 @@ static int32_t engine_step(cmld_engine *e, const StepOpts &o) {
 int32_t run_step(cmld_engine *e, const StepOpts &o) {
   // (a layered design's portion of one sequence has launch shapes that depend on its place: no graph)
   // (nor of a llama-shaped prompt's long steps: their kernels outlast their launches, and every length is another shape)
-  if ((e->cfg.flags & CMLD_FLAG_NO_GRAPH) || e->graphs_off || o.tree_mask || (e->lay && o.shared_slots) || o.batch > e->max_rows) return engine_step(e, o);
+  if ((e->cfg.flags & CMLD_FLAG_NO_GRAPH) || e->graphs_off || o.tree_mask || (e->lay && o.shared_slots) || o.prompt_end) return engine_step(e, o);
   uint32_t bits = (o.from_tokens ? 1u : 0u) | (o.rope_by_position ? 2u : 0u) | (o.logits ? 4u : 0u) | (o.argmax ? 8u : 0u) |
                   (o.feed_back ? 16u : 0u) | (o.taps ? 32u : 0u) | (o.shared_slots ? 64u : 0u) | (o.attn_cluster ? 128u : 0u) | ((uint32_t)(o.layer_begin & 0xfff) << 8) | ((uint32_t)((o.layer_end + 1) & 0xfff) << 20);
   uint32_t scale_bits;
@@ -1097,7 +1098,7 @@ static int32_t context_bucket(const cmld_engine *e, int64_t max_position) {
 // One sequence-0 row fed by an embedding vector: the forward_token family.
 static int32_t forward_embedding_rows(cmld_engine *e, const float *embeddings, const float *cosv, const float *sinv,
                                       int64_t position0, int32_t n_rows, float scale, bool logits, bool argmax, bool taps,
-                                      int32_t layer_begin = 0, int32_t layer_end = -1) {
+                                      int32_t layer_begin = 0, int32_t layer_end = -1, bool prompt = false) {
   const cmld_config &c = e->cfg;
   CMLD_TRY(llama_only(e));
   if (!embeddings || !cosv || !sinv) return fail(CMLD_ERR_INVALID, "embedding / cos / sin pointer is null");
@@ -1125,7 +1126,7 @@ static int32_t forward_embedding_rows(cmld_engine *e, const float *embeddings, c
   o.layer_end = layer_end;
   o.attn_cluster = use_attn_cluster(n_rows, position0 + n_rows - 1);
   o.attn_cap = attn_cap_for(position0 + n_rows - 1);
-  o.prompt_end = position0 + n_rows;
+  o.prompt_end = prompt && n_rows > kShortRows ? position0 + n_rows : 0;
   return run_step(e, o);
 }
 
@@ -1638,12 +1639,12 @@ int32_t cmld_engine_prefill_from(cmld_engine *e, const float *embeddings, const 
   CMLD_ENGINE_ENTER(e);
   if (n < 0 || start < 0 || start > n) return fail(CMLD_ERR_INVALID, "prefill: start=%lld exceeds n=%lld", (long long)start, (long long)n);
   const int half = e->cfg.rope_dim / 2;
-  // up to 8 rows go through the row kernel (bit-identical to serial calls); longer prompts chunk_rows at a time
+  // up to 8 rows are one short step; longer prompts go in chunk_rows at a time
   const int chunk = (n - start > 8 && !(e->cfg.flags & CMLD_FLAG_EXACT_ORDER)) ? e->chunk_rows : 8;
   for (int64_t i = start; i < n; i += chunk) {
     const int rows = (int)std::min<int64_t>(chunk, n - i);
     CMLD_TRY(forward_embedding_rows(e, embeddings + i * e->cfg.hidden, cos_all + i * half, sin_all + i * half, i, rows, scale,
-                                    false, false, false));
+                                    false, false, false, 0, -1, true));
   }
   return finish(e, "prefill");
 }
@@ -1891,7 +1892,7 @@ static int32_t llama_extend(cmld_engine *e, int32_t seq, const int32_t *tokens, 
     }
     CMLD_TRY(stage_rows(e, rows, tokens + i, pos32.data(), seqs.data()));
     const bool wanted = w < n_want && want[w] < i + rows, last = i + chunk >= n;
-    const bool by_row = rows > e->max_rows;  // logits of the rows that are asked for only
+    const bool by_row = rows > kShortRows;  // a long step: logits of the rows that are asked for only
     StepOpts o;
     o.batch = rows;
     o.shared_slots = rows > 1;
@@ -1900,7 +1901,7 @@ static int32_t llama_extend(cmld_engine *e, int32_t seq, const int32_t *tokens, 
     o.logits = o.argmax = !by_row && (last || wanted);
     o.attn_cluster = use_attn_cluster(rows, start_pos + i + rows - 1);
     o.attn_cap = attn_cap_for(start_pos + i + rows - 1);
-    o.prompt_end = start_pos + i + rows;
+    o.prompt_end = by_row ? start_pos + i + rows : 0;
     CMLD_TRY(run_step(e, o));
     if (by_row) {
       std::vector<int32_t> places;

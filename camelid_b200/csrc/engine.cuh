@@ -57,8 +57,8 @@ struct cmld_engine {
   int device = 0;
   cudaStream_t stream = nullptr;
   int32_t max_rows = 0;    // most rows of a step that the caller lists (sequences per step)
-  int32_t chunk_rows = 0;  // llama-shaped: rows of one step of a prompt
-  int32_t *d_rows = nullptr;  // rows of such a step whose logits are asked for
+  int32_t chunk_rows = 0;  // llama-shaped: most rows of one step of a prompt
+  int32_t *d_rows = nullptr;  // rows of a long step whose logits are asked for
   int32_t n_splits = 1, sm_count = 148;
   int32_t q_width = 0, kv_width = 0;
   std::vector<LayerW> layers;
@@ -136,6 +136,8 @@ inline int32_t dev_alloc(cmld_engine *e, T **p, int64_t count, bool zero = true)
   return CMLD_OK;
 }
 
+constexpr int32_t kShortRows = 32;  // llama shapes: portions of a prompt up to here are ordinary steps
+
 struct StepOpts {
   int32_t batch = 1;
   bool from_tokens = false;    // gather embeddings of d_tokens, else h holds them
@@ -152,7 +154,8 @@ struct StepOpts {
   int32_t tree_base = 0, tree_words = 0;
   bool shared_slots = false;  // several rows of this step belong to one sequence (prefill, verify): row b
                               // reads K/V that rows < b write, so the KV append must be a kernel of its own
-  int64_t prompt_end = 0;     // llama shapes, rows that are consecutive tokens of one sequence: the position after the last
+  int64_t prompt_end = 0;     // llama shapes, a long step (more than kShortRows consecutive tokens of one prompt): the position
+                              // after its last row; 0 for every other step
   // layered designs, rows that are consecutive tokens of one sequence (shared_slots):
   int64_t seq_start = 0;      // position of row 0
   int32_t seq_slot = 0;

@@ -281,6 +281,27 @@ def test_long_prompt_steps_equal_the_serial_path(cm, orc, heads, kv, hd, first, 
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), hidden_gate(got, want)
 
 
+@pytest.mark.parametrize("slots", [40, 64, 512])
+def test_prompts_take_the_same_steps_whatever_the_number_of_slots(cm, orc, slots):
+    """A prompt's steps are chosen by its rows: an engine of many slots launches what an engine of one launches (no logits of
+    rows that nobody asked for) and gives its bits, the second time as the first (long steps are not captured)."""
+    from camelid_b200 import synth
+
+    def engine(n_slots):
+        cfg = cm.EngineConfig(n_layers=2, n_heads=8, n_kv_heads=4, head_dim=64, hidden=512, ffn_dim=512, vocab=512, max_pos=704, max_seqs=n_slots)
+        return synth.build_engine(cfg, "q4_k_m", 5)
+
+    one, many = engine(1), engine(slots)
+    for n in (40, 200, 600):
+        prompt = orc.synth_tokens(3, 1, n, 512)
+        for want in ([], [], [], [0, n // 2, n - 2]):  # a step was captured at its second call and replayed from the third on
+            t1, l1 = one.extend(0, prompt, 0, want=want)
+            launches = one.last_timing()[1]
+            t2, l2 = many.extend(slots - 1, prompt, 0, want=want)
+            assert t1 == t2 and np.array_equal(l1.view(np.uint32), l2.view(np.uint32)), (n, want)
+            assert many.last_timing()[1] == launches, (n, want)
+
+
 def test_tensor_batch_flag_moves_small_batches_to_the_tensor_core_kernel(cm, orc):
     """CMLD_FLAG_TENSOR_BATCH (64): steps of 5..32 rows use the int8 mma.sync matvec.  Same integers, f32 terms
     added in another order: logits within the acceptance gate of the default engine's, and the rows of such a
