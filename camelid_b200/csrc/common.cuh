@@ -84,6 +84,7 @@ struct Weight {
   int64_t rows = 0, cols = 0, stride = 0;
   uint8_t *data = nullptr;  // device
   bool owned = true;
+  bool inf_scale = false;  // Q4_K experts: some superblock's scale is infinite (moe_find_inf_scale)
 };
 
 }  // namespace cmld

@@ -565,6 +565,7 @@ int32_t moe_combine3(float *h, const float *y3, const float *sel_w, const int32_
 int32_t moe_expert_gemv(const Weight &slab, int64_t rows_per_expert, int n_local_experts, int first_expert, int expert_step,
                         const float *x, int64_t x_stride, int x_div, float *y, const int32_t *counts, const int32_t *lists,
                         int n_assign, cudaStream_t s);
+int32_t moe_find_inf_scale(Weight &slab, cudaStream_t s);
 int32_t moe_expert_gemv_ordered(const Weight &slab, int64_t rows_per_expert, int n_experts, int used, int n_local_experts, int first_expert, int expert_step,
                                 const float *x, int64_t x_stride, int x_div, float *y, const int32_t *counts, const int32_t *lists,
                                 int n_assign, cudaStream_t s, const Weight *slab2 = nullptr, float *y2 = nullptr);
@@ -1394,6 +1395,7 @@ int32_t cmld_engine_set_layer_moe(cmld_engine *e, int32_t layer, const float *ro
     if (ts[i]->qtype != CMLD_Q4_K && ts[i]->qtype != CMLD_Q6_K)
       return fail(CMLD_ERR_UNSUPPORTED, "set_layer_moe: expert tensors must be Q4_K or Q6_K (got type %d)", ts[i]->qtype);
     CMLD_TRY(weight_upload(L.exps[i], ts[i]->qtype, shapes[i][0], shapes[i][1], ts[i]->data, ts[i]->nbytes, e->stream));
+    CMLD_TRY(moe_find_inf_scale(L.exps[i], e->stream));
   }
   CMLD_TRY(upload_f32(&L.router, router, (int64_t)c.n_experts * c.hidden, e->stream));
   L.moe_set = true;
@@ -1488,7 +1490,10 @@ int32_t cmld_engine_adopt_layer_moe(cmld_engine *e, int32_t layer, cmld_weight *
   for (int i = 0; i < 3; ++i)
     if (ts[i]->rows != shapes[i][0] || ts[i]->cols != shapes[i][1] || (ts[i]->qt != CMLD_Q4_K && ts[i]->qt != CMLD_Q6_K))
       return fail(CMLD_ERR_SHAPE, "adopt_layer_moe: expert tensor %d has the wrong shape or type", i);
-  for (int i = 0; i < 3; ++i) CMLD_TRY(adopt(L.exps[i], ts[i], shapes[i][0], shapes[i][1], "adopt_layer_moe"));
+  for (int i = 0; i < 3; ++i) {
+    CMLD_TRY(adopt(L.exps[i], ts[i], shapes[i][0], shapes[i][1], "adopt_layer_moe"));
+    CMLD_TRY(moe_find_inf_scale(L.exps[i], e->stream));
+  }
   cudaFree(L.router);
   L.router = reinterpret_cast<float *>(router_f32->data);
   router_f32->data = nullptr;

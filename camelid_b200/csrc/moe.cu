@@ -507,7 +507,8 @@ __device__ __forceinline__ void ord_pass(const MoeGemvArgs &a, float *yout, int 
           int sc, m;
           q4k_scale_min(2 * p + hl, meta.y, meta.z, meta.w, sc, m);
           const float dsc = __fmul_rn(d, (float)sc), dm = __fmul_rn(dmin, (float)m);
-          // round(dsc * q) as dsc * (2^23 + q) - dsc * 2^23 with one rounding (the second product is exact)
+          // round(dsc * q) as dsc * (2^23 + q) - dsc * 2^23 with one rounding (the second product is exact; a finite dsc is
+          // below 65504 * 63, so that no term overflows; slabs with an infinite scale take the tiled product)
           const uint64_t dsc2 = both(dsc), base2 = both(__fmul_rn(dsc, -8388608.0f)), dm2 = both(-dm);
           const int xo = 64 * p + 32 * hl;
 #pragma unroll
@@ -844,6 +845,33 @@ int32_t moe_expert_gemv(const Weight &slab, int64_t rows_per_expert, int n_local
   return CMLD_OK;
 }
 
+__global__ void moe_find_inf_kernel(const uint8_t *w, int64_t rows, int64_t stride, int nsb, int32_t *found) {
+  bool inf = false;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < rows * nsb; i += (int64_t)gridDim.x * blockDim.x)
+    inf |= isinf(f16_bits_to_f32(*reinterpret_cast<const uint16_t *>(w + i / nsb * stride + i % nsb * 144)));
+  if (inf) *found = 1;
+}
+
+// Looks for an infinite superblock scale in an expert slab, once when the engine gets it: moe_gemv_ordered_kernel's
+// dequantisation is for finite ones (handled inside that kernel, a decode step of two Mixtral-8x7B layers was 0.4 to 0.9 % slower).
+int32_t moe_find_inf_scale(Weight &slab, cudaStream_t s) {
+  slab.inf_scale = false;
+  if (slab.qt != CMLD_Q4_K) return CMLD_OK;
+  int32_t *found = nullptr, host = 0;
+  CMLD_CUDA(cudaMalloc(&found, 4));
+  cudaError_t ce = cudaMemsetAsync(found, 0, 4, s);
+  if (ce == cudaSuccess) {
+    moe_find_inf_kernel<<<1184, 256, 0, s>>>(slab.data, slab.rows, slab.stride, (int)(slab.cols >> 8), found);
+    ce = cudaGetLastError();
+  }
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(&host, found, 4, cudaMemcpyDeviceToHost, s);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+  cudaFree(found);
+  if (ce != cudaSuccess) return fail(CMLD_ERR_CUDA, "expert scales: %s", cudaGetErrorString(ce));
+  slab.inf_scale = host != 0;
+  return CMLD_OK;
+}
+
 // Which of the two ordered kernels: the tiles pay once an expert has five assignments on average.  A step of one Mixtral-8x7B
 // layer (two of eight experts) with 12 | 16 | 24 | 32 rows: 1509 | 1874 | 2407 | 3180 us by rows, 1832 | 1948 | 2084 | 2236 us by tiles.
 static bool moe_ordered_tile(int n_assign, int n_experts, const float *x, int64_t x_stride) {
@@ -862,7 +890,7 @@ int32_t moe_expert_gemv_ordered(const Weight &slab, int64_t rows_per_expert, int
   }
   if (slab.cols % 256) return fail(CMLD_ERR_SHAPE, "expert tensor width %lld is not a multiple of 256", (long long)slab.cols);
   if (slab.qt != CMLD_Q4_K && slab.qt != CMLD_Q6_K) return fail(CMLD_ERR_UNSUPPORTED, "expert tensors must be Q4_K or Q6_K");
-  if (moe_ordered_tile(n_assign, n_experts, x, x_stride)) {
+  if (slab.inf_scale || (slab2 && slab2->inf_scale) || moe_ordered_tile(n_assign, n_experts, x, x_stride)) {
     const int slabs = slab2 ? 2 : 1, expect = (n_assign + n_experts - 1) / n_experts;
     const int64_t tiles = (rows_per_expert + kTileRows - 1) / kTileRows;
     // as many assignments per pass as leave about four CTAs for every SM, but 16: below that the unpacking dominates

@@ -258,6 +258,37 @@ def test_moe_prompts_equal_the_serial_path(cm, orc, qt, n):
     assert token == orc.argmax(want)
 
 
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 10])  # ten rows give every expert enough assignments for the tiled product
+def test_infinite_superblock_scales_give_the_cpus_infinities(cm, orc, rows):
+    """Q4_K experts with an infinite scale: a code above 0 stands for an infinity, a code of 0 for NaN, in both expert
+    products.  The activations of the down projection are made equal, so that the infinities of a row have one sign."""
+    from camelid_b200 import synth
+
+    cfg = cm.EngineConfig(n_layers=1, n_heads=4, n_kv_heads=2, head_dim=64, hidden=256, ffn_dim=512, vocab=256, max_pos=32, n_experts=4,
+                          n_experts_used=2, max_seqs=rows)
+    pair = ModelPair(cfg, "q4_k_m", seed=3)
+    eng, ref = pair.engine, pair.oracle
+    rng = np.random.default_rng(0)
+    router = rng.normal(0, 0.1, (4, 256)).astype(np.float32)
+    gate, up = (np.tile(orc.synth_tensor(12, 41, i, 1, 256, 0.02), 4 * 512) for i in range(2))
+    down = orc.synth_tensor(12, 41, 2, 4 * 256, 512, 0.02).copy()
+    blocks = down.reshape(4, 256, 2, 144)
+    blocks[:, 3:6, 1, 4:16] = 0x11   # scales and mins above 0
+    blocks[:, 3:6, 1, 16:] |= 0x11   # codes above 0
+    blocks[:, 3, 1, 0:2] = [0, 0x7C]  # +inf
+    blocks[:, 4, 1, 0:2] = [0, 0xFC]  # -inf
+    blocks[:, 5, 1, 0:2] = [0, 0x7C]
+    blocks[:, 5, 1, 77] = 0x10
+    for m in (eng.set_layer_moe, ref.set_moe):
+        m(0, router, (12, gate), (12, up), (12, down))
+    with np.errstate(all="ignore"):
+        _, want, _ = ref.forward(ref.embedding(7), 0)
+    assert np.isinf(want[3]) and want[4] == -want[3] and np.isnan(want[5]) and np.isfinite(np.delete(want, [3, 4, 5])).all()
+    _, _, hidden = eng.step_batch(list(range(rows)), [7] * rows, [0] * rows, want_hidden=True)
+    for got in hidden:
+        assert np.array_equal(got, want, equal_nan=True), (got[3:6], want[3:6])
+
+
 @pytest.mark.parametrize("heads,kv,hd,first,n", [(16, 16, 64, 0, 150), (16, 8, 64, 3, 150), (8, 4, 128, 0, 300), (12, 4, 64, 0, 301), (12, 4, 64, 900, 301),
                                                   (12, 4, 128, 30, 299), (32, 8, 64, 5, 77), (16, 4, 64, 1400, 150), (16, 4, 128, 0, 161), (32, 4, 64, 100, 75),
                                                   (16, 2, 128, 0, 149), (16, 4, 128, 10, 40)])
