@@ -71,16 +71,22 @@ static int g_gemv_kernel_choice = 0;  // 0 auto (staged when the shape fits), 1 
 static int g_gemv_mma_min_batch = 1 << 30;  // rows from which the int8 mma.sync kernel is used (opt-in: bit 3 of the choice from 9 rows, bit 2 from 1)
 static int g_gemv_tc5_min_batch = 9;        // rows from which the tcgen05 kernel is used (bit 4 of the choice: never; bit 5: from 1 row)
 
+constexpr int32_t kOpTc5Rows = 2048;  // rows per pass of the tcgen05 kernel: bounds its scratch and its grids
+
 // One matvec launch on the default stream: staged kernel if it takes the shape, else the generic one.
 static int32_t gemv_launch(const cmld_weight *w, const uint8_t *act, int32_t batch, float *y, const float *residual,
                            cudaStream_t stream = nullptr, bool pdl = false) {
   GemvJob probe{w->data, w->qt, w->rows, w->cols, w->stride, y, residual, w->rows};
   if (g_gemv_kernel_choice == 0 && batch >= g_gemv_tc5_min_batch && batch < g_gemv_mma_min_batch && gemv_tc5_fits(&probe, 1, batch)) {
-    // several rows: one pass over the weights on the tcgen05 tensor cores, same bits as the one-row kernels
-    const int64_t need = gemv_tc5_pack_bytes(w->cols, batch);
+    // several rows: one pass over the weights per 2048 rows on the tcgen05 tensor cores, same bits as the one-row kernels
+    const int64_t need = std::max(gemv_tc5_pack_bytes(w->cols, std::min(batch, kOpTc5Rows)), gemv_tc5_pack_bytes(w->cols, 32));
     uint8_t *pack = reinterpret_cast<uint8_t *>(op_scratch((need + 3) / 4));
     if (!pack) return fail(CMLD_ERR_OOM, "gemv: no room for %lld bytes of packed activations", (long long)need);
-    return launch_gemv_tc5(&probe, 1, act, batch, pack, need, op_status(), stream, nullptr);
+    for (int32_t b0 = 0; b0 < batch; b0 += kOpTc5Rows) {
+      const GemvJob j{w->data, w->qt, w->rows, w->cols, w->stride, y + (int64_t)b0 * w->rows, residual ? residual + (int64_t)b0 * w->rows : nullptr, w->rows};
+      CMLD_TRY(launch_gemv_tc5(&j, 1, act + (int64_t)b0 * act_row_stride(w->cols), std::min(batch - b0, kOpTc5Rows), pack, need, op_status(), stream, nullptr));
+    }
+    return CMLD_OK;
   }
   if (g_gemv_kernel_choice == 0 && batch >= g_gemv_mma_min_batch && batch <= 32) {
     // more than 8 rows: one pass over the weights on the tensor cores

@@ -266,6 +266,26 @@ def test_gemv_tcgen05_row_tiles(cm, orc, name, rows, cols, batch):
         assert np.array_equal(y_res[b], (res[b] + y[b]).astype(np.float32))
 
 
+@pytest.mark.parametrize("batch", [2048, 2049, 2048 + 33, 4096 + 130, 65535 * 8 + 1])
+def test_gemv_of_many_rows_goes_in_passes(cm, orc, batch):
+    """Any number of activation rows: passes of 2048, the last one full, of one row, of a short tile, of more; and more rows
+    than one launch's grid could take."""
+    from camelid_b200.engine import quantize_activation, export_activation, DeviceBuffer
+
+    rows, cols, n = 3, 256, 1024
+    wire = orc.synth_tensor(12, 3, 1, rows, cols, 0.02)
+    w = cm.Weight.from_wire(12, rows, cols, wire)
+    act = quantize_activation(cm.ACT_Q8_K, np.random.default_rng(batch).standard_normal((n, cols)).astype(np.float32))
+    codes, scales = export_activation(cm.ACT_Q8_K, act, cols, n)
+    want = np.stack([orc.matvec_quantised(12, wire, rows, cols, codes[b], scales[b]) for b in range(n)])
+    row_bytes = act.to_numpy(np.uint8).reshape(n, -1)
+    which = np.arange(batch) * 7 % n
+    many = DeviceBuffer.from_numpy(row_bytes[which])
+    res = np.arange(batch * rows, dtype=np.float32).reshape(batch, rows)
+    assert np.array_equal(w.gemv(many, batch), want[which])
+    assert np.array_equal(w.gemv(many, batch, DeviceBuffer.from_numpy(res)), res + want[which])
+
+
 @pytest.mark.parametrize("name,rows,cols,batch", [
     ("Q4_K", 128 * 40 + 17, 512, 32), ("Q4_K", 128 * 170, 256, 32), ("Q4_K", 128 * 170, 256, 16),
     ("Q6_K", 128 * 90 + 5, 512, 32), ("Q6_K", 128 * 170, 256, 11), ("Q8_0", 128 * 40, 768, 24), ("Q8_0", 128 * 170 + 64, 256, 32)])
