@@ -48,51 +48,45 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float *__restrict_
   for (int e = warp; e < n_exp; e += 8) {
     const float *r = router + (int64_t)e * hidden;
     float s = 0.0f;
-    if ((hidden & 1023) == 0) {
-      float4 xv[8], rv[8];
-      auto load = [&](int i0) {
+    float4 xv[8], rv[8];
+    // (the last chunk may be short: products behind the row are +0, which leave a sum that started at +0 as it is)
+    auto load = [&](int i0) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          xv[j] = __ldg(reinterpret_cast<const float4 *>(xr + i0 + lane * 4 + 128 * j));
-          rv[j] = __ldg(reinterpret_cast<const float4 *>(r + i0 + lane * 4 + 128 * j));
+      for (int j = 0; j < 8; ++j) {
+        const int i = i0 + lane * 4 + 128 * j;
+        xv[j] = rv[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < hidden) {
+          xv[j] = __ldg(reinterpret_cast<const float4 *>(xr + i));
+          rv[j] = __ldg(reinterpret_cast<const float4 *>(r + i));
         }
-      };
-      load(0);
-      for (int i0 = 0; i0 < hidden; i0 += 1024) {
-        float4 *p4 = reinterpret_cast<float4 *>(prod[warp]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          p4[lane + 32 * j] = make_float4(__fmul_rn(xv[j].x, rv[j].x), __fmul_rn(xv[j].y, rv[j].y), __fmul_rn(xv[j].z, rv[j].z), __fmul_rn(xv[j].w, rv[j].w));
-        __syncwarp();
-        if (i0 + 1024 < hidden) load(i0 + 1024);
-        float4 v[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = p4[j];
-        for (int i = 0; i < 256; i += 4) {
-          float4 next[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) next[j] = p4[min(i + 4 + j, 255)];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            s = __fadd_rn(s, v[j].x);
-            s = __fadd_rn(s, v[j].y);
-            s = __fadd_rn(s, v[j].z);
-            s = __fadd_rn(s, v[j].w);
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) v[j] = next[j];
-        }
-        __syncwarp();
       }
-      if (lane == 0) logits[e] = s;
-      continue;
-    }
+    };
+    load(0);
     for (int i0 = 0; i0 < hidden; i0 += 1024) {
-      const int cnt = min(1024, hidden - i0);
-      for (int i = lane; i < cnt; i += 32) prod[warp][i] = __fmul_rn(xr[i0 + i], r[i0 + i]);
+      float4 *p4 = reinterpret_cast<float4 *>(prod[warp]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        p4[lane + 32 * j] = make_float4(__fmul_rn(xv[j].x, rv[j].x), __fmul_rn(xv[j].y, rv[j].y), __fmul_rn(xv[j].z, rv[j].z), __fmul_rn(xv[j].w, rv[j].w));
       __syncwarp();
-      if (lane == 0)
-        for (int i = 0; i < cnt; ++i) s = __fadd_rn(s, prod[warp][i]);
+      if (i0 + 1024 < hidden) load(i0 + 1024);
+      float4 v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = p4[j];
+      const int n4 = min(256, (hidden - i0 + 15) / 16 * 4);
+      for (int i = 0; i < n4; i += 4) {
+        float4 next[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) next[j] = p4[min(i + 4 + j, 255)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s = __fadd_rn(s, v[j].x);
+          s = __fadd_rn(s, v[j].y);
+          s = __fadd_rn(s, v[j].z);
+          s = __fadd_rn(s, v[j].w);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = next[j];
+      }
       __syncwarp();
     }
     if (lane == 0) logits[e] = s;
@@ -825,6 +819,7 @@ namespace cmld {
 int32_t moe_route(const float *normed, const float *router, int hidden, int n_exp, int k, int batch, int32_t *sel_idx,
                   float *sel_w, int32_t *counts, int32_t *lists, cudaStream_t s, int32_t *pos) {
   if (n_exp > kMaxExperts) return fail(CMLD_ERR_SHAPE, "more than %d experts", kMaxExperts);
+  if (hidden % 4) return fail(CMLD_ERR_SHAPE, "router: width %d is not a multiple of 4", hidden);  // (expert matrices: of 256)
   moe_route_kernel<<<batch, 256, 0, s>>>(normed, router, hidden, n_exp, k, sel_idx, sel_w);
   CMLD_CUDA(cudaGetLastError());
   moe_group_kernel<<<1, std::min(32, n_exp) * 32, 0, s>>>(sel_idx, batch * k, n_exp, counts, lists, pos);

@@ -258,6 +258,28 @@ def test_moe_prompts_equal_the_serial_path(cm, orc, qt, n):
     assert token == orc.argmax(want)
 
 
+@pytest.mark.parametrize("qt", [12, 14])  # Q4_K, Q6_K experts
+def test_moe_prompts_on_a_wide_shape(cm, orc, qt):
+    """Enough row tiles that gate and up keep the largest passes: prompts whose experts have about 6 to 60 assignments go through
+    every number of assignments per thread (1 to 6) and through passes that split an expert's.  The width leaves the router a
+    short last chunk."""
+    cfg = cm.EngineConfig(n_layers=1, n_heads=4, n_kv_heads=2, head_dim=64, hidden=1280, ffn_dim=4864, vocab=256, max_pos=256, n_experts=8, n_experts_used=2)
+    pair = ModelPair(cfg, "q4_k_m", seed=33)
+    eng, ref = pair.engine, pair.oracle
+    router = np.random.default_rng(0).normal(0, 0.1, (cfg.n_experts, cfg.hidden)).astype(np.float32)
+    exps = [(qt, orc.synth_tensor(qt, 41, i, cfg.n_experts * r, c, 0.02))
+            for i, (r, c) in enumerate([(cfg.ffn_dim, cfg.hidden), (cfg.ffn_dim, cfg.hidden), (cfg.hidden, cfg.ffn_dim)])]
+    eng.set_layer_moe(0, router, *exps)
+    ref.set_moe(0, router, *exps)
+    prompt = orc.synth_tokens(8, 1, 200, cfg.vocab)
+    want = np.stack([ref.forward(ref.embedding(int(t)), pos)[0] for pos, t in enumerate(prompt)])
+    for n in (3, 24, 45, 66, 97, 130, 163, 200):
+        token, logits = eng.extend(0, prompt[:n], 0, want=list(range(n)))
+        bad = np.nonzero((logits.view(np.uint32) != want[:n].view(np.uint32)).any(axis=1))[0]
+        assert bad.size == 0, (n, bad, hidden_gate(logits, want[:n]))
+        assert token == orc.argmax(want[n - 1])
+
+
 @pytest.mark.parametrize("rows", [1, 2, 3, 4, 10])  # ten rows give every expert enough assignments for the tiled product
 def test_infinite_superblock_scales_give_the_cpus_infinities(cm, orc, rows):
     """Q4_K experts with an infinite scale: a code above 0 stands for an infinity, a code of 0 for NaN, in both expert
