@@ -357,12 +357,9 @@ static int32_t launch_gp(const AttnArgs &a, cudaStream_t s) {
   }
   cfg.attrs = attr;
   cfg.numAttrs = n_attr;
-  static bool carveout_set = false;
-  if (!carveout_set) {
-    prefer_max_smem_carveout(attn_decode_kernel<G, PER, false>);
-    prefer_max_smem_carveout(attn_decode_kernel<G, PER, true>);
-    carveout_set = true;
-  }
+  static SmemLimit limit[2];
+  CMLD_TRY(prefer_max_smem_carveout(limit[0], attn_decode_kernel<G, PER, false>));
+  CMLD_TRY(prefer_max_smem_carveout(limit[1], attn_decode_kernel<G, PER, true>));
   if (a.cluster) CMLD_CUDA(cudaLaunchKernelEx(&cfg, attn_decode_kernel<G, PER, true>, a));
   else CMLD_CUDA(cudaLaunchKernelEx(&cfg, attn_decode_kernel<G, PER, false>, a));
   return CMLD_OK;

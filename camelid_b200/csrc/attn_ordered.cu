@@ -551,11 +551,8 @@ __global__ void __launch_bounds__(kOaThreads, 1) attn_ordered_kernel(AttnArgs a,
 template <int G, int HD, int VD>
 static int32_t launch_oa_vd(const AttnArgs &a, int64_t cap, cudaStream_t s) {
   const OaLayout L = oa_layout(G, HD, cap);
-  static int configured = 0;
-  if (L.total > configured) {
-    CMLD_CUDA(cudaFuncSetAttribute(attn_ordered_kernel<G, HD, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total));
-    configured = L.total;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, attn_ordered_kernel<G, HD, VD>, L.total));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(kOaCluster, (unsigned)a.n_kv_heads, (unsigned)a.batch);
   cfg.blockDim = dim3(kOaThreads);

@@ -286,11 +286,8 @@ template <int G, int HD, int A, int W>
 int32_t launch_prompt(const AttnArgs &a, int64_t n_pos, cudaStream_t s) {
   constexpr int R = 8 * A / G;
   const size_t smem = prompt_smem_bytes(HD, A, n_pos);
-  static size_t configured = 0;
-  if (smem > configured) {
-    CMLD_CUDA(cudaFuncSetAttribute(attn_prompt_kernel<G, HD, A, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, attn_prompt_kernel<G, HD, A, W>, smem));
   dim3 grid((unsigned)a.n_kv_heads, (unsigned)((a.batch + R - 1) / R));
   attn_prompt_kernel<G, HD, A, W><<<grid, 1024 / W, smem, s>>>(a, -0.0f);
   CMLD_CUDA(cudaGetLastError());

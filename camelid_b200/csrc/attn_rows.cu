@@ -172,11 +172,8 @@ size_t rows_smem_bytes(int G, int HD, int cap) { return (size_t)G * (HD + 4) * 4
 template <int G, int HD>
 int32_t launch_rows(const AttnArgs &a, int cap, cudaStream_t s) {
   const size_t smem = rows_smem_bytes(G, HD, cap);
-  static size_t configured = 0;
-  if (smem > configured) {
-    CMLD_CUDA(cudaFuncSetAttribute(attn_rows_kernel<G, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, attn_rows_kernel<G, HD>, smem));
   dim3 grid((unsigned)a.n_kv_heads, (unsigned)a.batch);
   attn_rows_kernel<G, HD><<<grid, kRowsThreads, smem, s>>>(a, cap);
   CMLD_CUDA(cudaGetLastError());

@@ -12,6 +12,7 @@
 #include <cstring>
 
 #include "../../include/camelid_b200.h"
+#include "smem_limit.h"
 
 namespace cmld {
 
@@ -175,11 +176,30 @@ __device__ __forceinline__ uint4 ld_stream16(const void *p) {
 
 #endif  // __CUDACC__
 
+// Before a launch with more than the usual 48 KB: the kernel's limit on the current device, at least `bytes`.  `limit` is the
+// kernel's own; `carveout`: with the largest shared-memory share of the L1.
+template <typename K>
+inline int32_t allow_smem(SmemLimit &limit, K kernel, size_t bytes, bool carveout = false) {
+  int dev = 0;
+  CMLD_CUDA(cudaGetDevice(&dev));
+  return limit.raise(dev, (int)bytes, [&](int n) {
+    CMLD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, n));
+    if (carveout) CMLD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    return (int32_t)CMLD_OK;
+  });
+}
+
 // Every kernel of the decode step asks for the same (maximum) shared-memory carve-out as the
 // staged matvec: an SM whose L1/shared split has to change between two kernels drains first.
+// (A preference of the device's, like the limit above: `limit` counts 1 once it is set.)
 template <typename K>
-inline void prefer_max_smem_carveout(K kernel) {
-  cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+inline int32_t prefer_max_smem_carveout(SmemLimit &limit, K kernel) {
+  int dev = 0;
+  CMLD_CUDA(cudaGetDevice(&dev));
+  return limit.raise(dev, 1, [&](int) {
+    CMLD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    return (int32_t)CMLD_OK;
+  });
 }
 
 // ------------------------------------------------------------------ kernel launchers (host)

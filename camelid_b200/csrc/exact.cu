@@ -220,12 +220,9 @@ __global__ void __launch_bounds__(kExactAttnThreads) attn_exact_kernel(AttnArgs 
 int32_t launch_attention_exact(const AttnArgs &a, cudaStream_t s) {
   if (a.head_dim > 128) return fail(CMLD_ERR_SHAPE, "attention (reference order): head_dim %d > 128", a.head_dim);
   const size_t smem = (size_t)a.max_pos * 4;
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    CMLD_CUDA(cudaFuncSetAttribute(attn_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(smem, 200 * 1024)));
-    configured = smem;
-  }
+  static SmemLimit limit;
   if (smem > 200 * 1024) return fail(CMLD_ERR_SHAPE, "attention (reference order): max_pos %lld too large", (long long)a.max_pos);
+  if (smem > 48 * 1024) CMLD_TRY(allow_smem(limit, attn_exact_kernel, smem));
   dim3 grid((unsigned)a.n_heads, (unsigned)a.batch);
   attn_exact_kernel<<<grid, kExactAttnThreads, smem, s>>>(a);
   CMLD_CUDA(cudaGetLastError());

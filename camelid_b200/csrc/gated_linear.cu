@@ -464,11 +464,8 @@ __global__ void __launch_bounds__(kScanThreads) gated_scan_kernel(const Lightnin
 
 template <int MT>
 int32_t scan(const LightningArgs &a, const uint8_t *scratch, bool pdl, cudaStream_t s) {
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(gated_scan_kernel<MT>, Scan<MT>::kSmem));
-    ready = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, gated_scan_kernel<MT>, Scan<MT>::kSmem));
   return launch_kernel(gated_scan_kernel<MT>, dim3(a.heads, (a.vdim + kCols - 1) / kCols), dim3(kScanThreads), Scan<MT>::kSmem, pdl, s, a, scratch);
 }
 
@@ -481,11 +478,8 @@ int64_t gated_scratch_bytes(int32_t heads, int32_t dim, int32_t vdim, int64_t ro
 }
 
 int32_t launch_gated_chunks(const LightningArgs &a, void *scratch, bool pdl, cudaStream_t s) {
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(gated_prep_kernel, 227 * 1024));
-    ready = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, gated_prep_kernel, 227 * 1024));
   if (a.half || !a.one_sequence || !gated_chunk_fits(a.dim, a.channel.w.cols)) return fail(CMLD_ERR_SHAPE, "gated linear attention: the chunked form does not take this");
   uint8_t *buf = static_cast<uint8_t *>(scratch);
   CMLD_TRY(launch_kernel(gated_prep_kernel, dim3(a.heads, (a.rows + kC - 1) / kC), dim3(kPrepThreads), prep_smem(a.dim, a.channel.w.cols), pdl, s, a, buf));

@@ -461,7 +461,6 @@ struct MmaPlan {
 };
 
 int g_mma_sms = 0;
-bool g_mma_attr[5] = {false, false, false, false, false};
 
 bool plan_mma(const GemvJob *jobs, int n_jobs, int32_t batch, MmaPlan &p) {
   if (n_jobs < 1 || n_jobs > 3 || batch < 1 || batch > 32) return false;
@@ -523,10 +522,8 @@ bool plan_mma(const GemvJob *jobs, int n_jobs, int32_t batch, MmaPlan &p) {
 
 template <int NT>
 int32_t launch_nt(const MmaPlan &p, cudaStream_t s, bool pdl) {
-  if (!g_mma_attr[NT]) {
-    CMLD_CUDA(cudaFuncSetAttribute(gemv_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    g_mma_attr[NT] = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, gemv_mma_kernel<NT>, 227 * 1024));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)p.grid, (unsigned)p.grid_y, (unsigned)p.grid_z);
   cfg.blockDim = dim3((unsigned)(p.args.n_warps * 32));

@@ -964,15 +964,12 @@ struct PipePlan {
 };
 
 static int g_sm_count = 0;
-static bool g_attr_set[9] = {false};
 
 template <int B>
 static int32_t launch_pipe_b(const PipePlan &p, int grid, cudaStream_t s, bool pdl) {
-  if (!g_attr_set[B]) {
-    CMLD_CUDA(cudaFuncSetAttribute(gemv_pipe_kernel<B, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    CMLD_CUDA(cudaFuncSetAttribute(gemv_pipe_kernel<B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    g_attr_set[B] = true;
-  }
+  static SmemLimit limit[2];
+  CMLD_TRY(allow_smem(limit[0], gemv_pipe_kernel<B, false>, 227 * 1024));
+  CMLD_TRY(allow_smem(limit[1], gemv_pipe_kernel<B, true>, 227 * 1024));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(kPipeThreads);

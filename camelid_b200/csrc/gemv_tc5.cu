@@ -787,11 +787,8 @@ bool gemv_tc5_fits(const GemvJob *jobs, int n_jobs, int32_t batch) {
 
 template <int QT, int NW, int MR>
 static int32_t launch_tc(TcArgs &a, const GemvJob *jobs, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    CMLD_CUDA(cudaFuncSetAttribute(gemv_tc5_kernel<QT, NW, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    attr = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, gemv_tc5_kernel<QT, NW, MR>, 227 * 1024));
   int tiles = 0;
   for (int i = 0; i < a.n_jobs; ++i) {
     TcJob &J = a.job[i];

@@ -173,12 +173,9 @@ int32_t launch_attention_q8(const AttnArgs &a, const uint8_t *kq, const uint8_t 
   if (a.head_dim > 128 || a.head_dim % 32) return fail(CMLD_ERR_SHAPE, "Q8_0 KV attention: head_dim %d", a.head_dim);
   if (a.tree_mask) return fail(CMLD_ERR_UNSUPPORTED, "tree verification over a Q8_0 KV cache is not supported");
   const size_t smem = (size_t)a.max_pos * 4;
-  static size_t configured = 0;
+  static SmemLimit limit;
   if (smem > 200 * 1024) return fail(CMLD_ERR_SHAPE, "Q8_0 KV attention: max_pos %lld too large", (long long)a.max_pos);
-  if (smem > 48 * 1024 && smem > configured) {
-    CMLD_CUDA(cudaFuncSetAttribute(attn_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  if (smem > 48 * 1024) CMLD_TRY(allow_smem(limit, attn_q8_kernel, smem));
   dim3 grid((unsigned)a.n_heads, (unsigned)a.batch);
   attn_q8_kernel<<<grid, kQ8AttnThreads, smem, s>>>(a, kq, vq);
   CMLD_CUDA(cudaGetLastError());

@@ -675,11 +675,8 @@ __global__ void __launch_bounds__(kPfThreads) latent_prefill_kernel(const Latent
 
 template <int DV>
 int32_t prefill(const LatentPrefillArgs &a, bool pdl, cudaStream_t s) {
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(latent_prefill_kernel<DV>, 227 * 1024));
-    ready = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, latent_prefill_kernel<DV>, 227 * 1024));
   return launch_kernel(latent_prefill_kernel<DV>, dim3((a.rows + kPfQ - 1) / kPfQ, a.m.heads), dim3(kPfThreads), pf_smem(pf_qd(a.m), DV), pdl, s, a);
 }
 
@@ -692,11 +689,8 @@ bool latent_shape_ok(const LatentShape &m) {
 
 template <int ROWS>
 int32_t prep(const LatentArgs &a, bool pdl, cudaStream_t s) {
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(latent_prep_kernel<ROWS>, 160 * 1024));
-    ready = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, latent_prep_kernel<ROWS>, 160 * 1024));
   const int slices = (a.m.rank + kPrepRanks - 1) / kPrepRanks, ys = a.m.heads * slices;
   const size_t smem = (size_t)(ROWS * ((a.m.dim + 3) & ~3) + 16 * ROWS * kPrepRanks) * 4;
   return launch_kernel(latent_prep_kernel<ROWS>, dim3((a.rows + ROWS - 1) / ROWS, ys + ROWS), dim3(kPrepThreads), smem, pdl, s, a, slices, ys);
@@ -715,16 +709,13 @@ int latent_attention_groups(const LatentArgs &a) {
 }
 
 int32_t launch_latent_attention(const LatentArgs &a, bool pdl, cudaStream_t s) {
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(latent_attn_kernel<1>, 227 * 1024));
-    CMLD_TRY(allow_smem(latent_attn_kernel<2>, 227 * 1024));
-    CMLD_TRY(allow_smem(latent_attn_mma_kernel<2, 2>, 227 * 1024));
-    CMLD_TRY(allow_smem(latent_attn_mma_kernel<4, 3>, 227 * 1024));
-    CMLD_TRY(allow_smem(latent_attn_mma_kernel<8, 5>, 227 * 1024));
-    CMLD_TRY(allow_smem(latent_attn_mma_kernel<16, 9>, 227 * 1024));
-    ready = true;
-  }
+  static SmemLimit limit[6];
+  CMLD_TRY(allow_smem(limit[0], latent_attn_kernel<1>, 227 * 1024));
+  CMLD_TRY(allow_smem(limit[1], latent_attn_kernel<2>, 227 * 1024));
+  CMLD_TRY(allow_smem(limit[2], latent_attn_mma_kernel<2, 2>, 227 * 1024));
+  CMLD_TRY(allow_smem(limit[3], latent_attn_mma_kernel<4, 3>, 227 * 1024));
+  CMLD_TRY(allow_smem(limit[4], latent_attn_mma_kernel<8, 5>, 227 * 1024));
+  CMLD_TRY(allow_smem(limit[5], latent_attn_mma_kernel<16, 9>, 227 * 1024));
   const dim3 grid(a.splits, latent_attention_groups(a), a.rows);
   const int D = a.m.rank + a.m.rot_dim;
   if (latent_attention_mma(a)) {

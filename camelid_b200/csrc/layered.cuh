@@ -248,12 +248,6 @@ inline int32_t launch_kernel(void (*k)(KA...), dim3 grid, dim3 block, size_t sme
   CMLD_CUDA(cudaLaunchKernelEx(&cfg, k, static_cast<KA>(args)...));
   return CMLD_OK;
 }
-// Once per kernel: full shared memory.
-template <typename K>
-inline int32_t allow_smem(K k, size_t bytes) {
-  CMLD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return CMLD_OK;
-}
 
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

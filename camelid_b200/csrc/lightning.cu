@@ -315,11 +315,8 @@ int32_t steps(const LightningArgs &a, bool pdl, cudaStream_t s) {
 template <int MT>
 int32_t chunks(const LightningArgs &a, bool pdl, cudaStream_t s) {
   const int smem = chunk_smem(64 * MT);
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(lightning_chunk_kernel<MT>, smem));
-    ready = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, lightning_chunk_kernel<MT>, smem));
   return launch_kernel(lightning_chunk_kernel<MT>, dim3(a.heads, (a.vdim + kChunkCols - 1) / kChunkCols), dim3(kChunkThreads), smem, pdl, s, a);
 }
 

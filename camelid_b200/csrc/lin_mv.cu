@@ -152,24 +152,16 @@ int mv_sms() {
 
 template <int R, int ROWS>
 int32_t mv_launch(const LinMvArgs &a, bool pdl, cudaStream_t s) {
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(lin_mv_kernel<R, ROWS>, kMvMaxSmem));
-    prefer_max_smem_carveout(lin_mv_kernel<R, ROWS>);
-    ready = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, lin_mv_kernel<R, ROWS>, kMvMaxSmem, true));
   const int groups = (a.w.rows + ROWS - 1) / ROWS;
   return launch_kernel(lin_mv_kernel<R, ROWS>, dim3(std::min(groups, mv_sms())), dim3(kMvThreads), mv_smem(a.w.cols, R), pdl, s, a);
 }
 
 template <int R, int ROWS>
 int32_t mv_launch_pair(const LinMvArgs &a, const LinMvArgs &b, bool pdl, cudaStream_t s) {
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(lin_mv_pair_kernel<R, ROWS>, kMvMaxSmem));
-    prefer_max_smem_carveout(lin_mv_pair_kernel<R, ROWS>);
-    ready = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, lin_mv_pair_kernel<R, ROWS>, kMvMaxSmem, true));
   const int sms = mv_sms();
   const double wa = (double)a.w.rows * a.w.ld, wb = (double)b.w.rows * b.w.ld;
   const int first = std::min(sms - 1, std::max(1, (int)(sms * wa / (wa + wb) + 0.5)));

@@ -312,12 +312,8 @@ int32_t make_map(CUtensorMap *map, const void *p, int64_t cols, int64_t rows, in
 
 template <int BN, typename OutT>
 int32_t launch_bn(const LinArgs &L, int32_t sms, int32_t *status, bool pdl, cudaStream_t s) {
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(lin_tc5_kernel<BN, OutT>, smem_bytes(BN)));
-    prefer_max_smem_carveout(lin_tc5_kernel<BN, OutT>);
-    ready = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, lin_tc5_kernel<BN, OutT>, smem_bytes(BN), true));
   CUtensorMap wmap, xmap;
   CMLD_TRY(make_map(&wmap, L.w.w, L.w.cols, L.w.rows, L.w.ld, kBM));
   CMLD_TRY(make_map(&xmap, L.x, L.w.cols, L.rows, L.x_ld, BN));

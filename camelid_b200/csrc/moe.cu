@@ -893,13 +893,10 @@ int32_t moe_expert_gemv_ordered(const Weight &slab, int64_t rows_per_expert, int
     while (max_a > 2 && tiles * n_local_experts * slabs * ((expect + 8 * max_a - 1) / (8 * max_a)) < 4 * 148) max_a = std::max(2, max_a / 2);
     const int z = std::max(1, std::min(8, (2 * expect + 8 * max_a - 1) / (8 * max_a)));
     dim3 grid((unsigned)tiles, (unsigned)n_local_experts, (unsigned)(z * slabs));
-    static bool attr[2] = {false, false};
+    static SmemLimit limit[2];
     const int smem = tile_smem(kTileMaxA), q6 = slab.qt == CMLD_Q6_K;
     const auto kernel = q6 ? moe_gemm_ordered_kernel<CMLD_Q6_K> : moe_gemm_ordered_kernel<CMLD_Q4_K>;
-    if (!attr[q6]) {
-      CMLD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      attr[q6] = true;
-    }
+    CMLD_TRY(allow_smem(limit[q6], kernel, smem));
     kernel<<<grid, kTileThreads, smem, s>>>(a, max_a, slabs);
     CMLD_CUDA(cudaGetLastError());
     return CMLD_OK;
@@ -909,11 +906,8 @@ int32_t moe_expert_gemv_ordered(const Weight &slab, int64_t rows_per_expert, int
   dim3 grid((unsigned)((rows_per_expert + kOrdThreads - 1) / kOrdThreads), (unsigned)n_local_experts, slab2 ? 2u : 1u);
   const int q6 = slab.qt == CMLD_Q6_K, sb_bytes = q6 ? 208 : 144;
   const auto kernel = q6 ? moe_gemv_ordered_kernel<CMLD_Q6_K> : moe_gemv_ordered_kernel<CMLD_Q4_K>;
-  static bool attr[2] = {false, false};
-  if (!attr[q6]) {
-    CMLD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdStages * ord_stage(sb_bytes, kOrdCols)));
-    attr[q6] = true;
-  }
+  static SmemLimit limit[2];
+  CMLD_TRY(allow_smem(limit[q6], kernel, kOrdStages * ord_stage(sb_bytes, kOrdCols)));
   kernel<<<grid, kOrdThreads, kOrdStages * ord_stage(sb_bytes, cols), s>>>(a, cols);
   CMLD_CUDA(cudaGetLastError());
   return CMLD_OK;

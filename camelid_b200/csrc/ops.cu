@@ -148,15 +148,10 @@ int32_t launch_norm_quant(const NormQuantArgs &a, cudaStream_t s) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = a.pdl ? 1 : 0;
-  static bool carveout_set = false;
-  if (!carveout_set) {
-    prefer_max_smem_carveout(norm_quant_kernel<0>);
-    prefer_max_smem_carveout(norm_quant_kernel<1>);
-    prefer_max_smem_carveout(norm_quant_kernel<2>);
-    CMLD_CUDA(cudaFuncSetAttribute(norm_quant_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   kNormMaxExact * 4 + xsum::workspace_bytes(kNormMaxExact)));
-    carveout_set = true;
-  }
+  static SmemLimit limit[3];
+  CMLD_TRY(prefer_max_smem_carveout(limit[0], norm_quant_kernel<0>));
+  CMLD_TRY(allow_smem(limit[1], norm_quant_kernel<1>, kNormMaxExact * 4 + xsum::workspace_bytes(kNormMaxExact), true));
+  CMLD_TRY(prefer_max_smem_carveout(limit[2], norm_quant_kernel<2>));
   if (mode == 0) CMLD_CUDA(cudaLaunchKernelEx(&cfg, norm_quant_kernel<0>, a));
   else if (mode == 1) CMLD_CUDA(cudaLaunchKernelEx(&cfg, norm_quant_kernel<1>, a));
   else CMLD_CUDA(cudaLaunchKernelEx(&cfg, norm_quant_kernel<2>, a));
@@ -312,12 +307,9 @@ __global__ void __launch_bounds__(kArgmaxThreads)
 int32_t launch_argmax(const float *x, int64_t n, int32_t batch, float *part_val, int32_t *part_idx, uint32_t *ticket,
                       int32_t *out_idx, int32_t *next_tokens, int32_t *positions, int32_t *history, cudaStream_t s,
                       unsigned long long *key_out, int32_t idx_offset) {
-  static bool carveout_set = false;
-  if (!carveout_set) {
-    prefer_max_smem_carveout(argmax_kernel);
-    prefer_max_smem_carveout(rope_kv_kernel);
-    carveout_set = true;
-  }
+  static SmemLimit limit[2];
+  CMLD_TRY(prefer_max_smem_carveout(limit[0], argmax_kernel));
+  CMLD_TRY(prefer_max_smem_carveout(limit[1], rope_kv_kernel));
   dim3 grid(kArgmaxBlocks, (unsigned)batch);
   argmax_kernel<<<grid, kArgmaxThreads, 0, s>>>(x, n, part_val, part_idx, ticket, out_idx, next_tokens, positions, history,
                                                 reinterpret_cast<int32_t *>(ticket) + batch, batch, key_out, idx_offset);
@@ -454,12 +446,8 @@ __global__ void __launch_bounds__(kNormThreads) exact_sum_selftest_kernel(const 
 int32_t launch_exact_sum_selftest(const float *terms, int32_t n, float *out, cudaStream_t s) {
   if (n <= 0 || n % 256 || n > kNormMaxExact) return fail(CMLD_ERR_SHAPE, "exact sum self-test: n must be a multiple of 256, at most %d", kNormMaxExact);
   const size_t smem = (size_t)n * 4 + xsum::workspace_bytes(n);
-  static bool configured = false;
-  if (!configured) {
-    CMLD_CUDA(cudaFuncSetAttribute(exact_sum_selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   kNormMaxExact * 4 + xsum::workspace_bytes(kNormMaxExact)));
-    configured = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, exact_sum_selftest_kernel, kNormMaxExact * 4 + xsum::workspace_bytes(kNormMaxExact)));
   exact_sum_selftest_kernel<<<1, kNormThreads, smem, s>>>(terms, n, out);
   CMLD_CUDA(cudaGetLastError());
   return CMLD_OK;

@@ -96,13 +96,15 @@ int32_t launch_stream_mix(const StreamMix &m, int32_t rows, ActBuf out, bool pdl
     return launch_kernel(post_norm_kernel<4>, dim3(rows), dim3(threads), 0, pdl, s, m, out);
   }
   const size_t smem = (size_t)m.width * 4;
-  if (smem > 48 * 1024) CMLD_TRY(allow_smem(stream_mix_kernel, smem));
+  static SmemLimit limit;
+  if (smem > 48 * 1024) CMLD_TRY(allow_smem(limit, stream_mix_kernel, smem));
   return launch_kernel(stream_mix_kernel, dim3(rows), dim3(mix_threads(rows)), smem, pdl, s, m, out);
 }
 
 int32_t launch_stream_tap(const StreamMix &m, int32_t rows, float *out, cudaStream_t s) {
   const size_t smem = (size_t)m.width * 4;
-  if (smem > 48 * 1024) CMLD_TRY(allow_smem(stream_tap_kernel, smem));
+  static SmemLimit limit;
+  if (smem > 48 * 1024) CMLD_TRY(allow_smem(limit, stream_tap_kernel, smem));
   return launch_kernel(stream_tap_kernel, dim3(rows), dim3(mix_threads(rows)), smem, false, s, m, out);
 }
 

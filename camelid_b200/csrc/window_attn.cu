@@ -516,11 +516,8 @@ int decode_stages(const WindowShape &m) {
 
 template <int VP>
 int32_t decode(const WindowArgs &a, bool pdl, cudaStream_t s) {
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(window_decode_kernel<VP>, kMaxSmem));
-    ready = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, window_decode_kernel<VP>, kMaxSmem));
   const int stages = decode_stages(a.m);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(a.splits, window_decode_groups(a), a.rows);
@@ -547,11 +544,8 @@ int32_t decode(const WindowArgs &a, bool pdl, cudaStream_t s) {
 
 template <int DV>
 int32_t prefill(const WindowArgs &a, bool pdl, cudaStream_t s) {
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(window_prefill_kernel<DV>, kMaxSmem));
-    ready = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, window_prefill_kernel<DV>, kMaxSmem));
   return launch_kernel(window_prefill_kernel<DV>, dim3(a.m.heads, (a.rows + kPfQ - 1) / kPfQ), dim3(kPfThreads), pf_smem(window_pad(a.m.dim), DV), pdl, s, a);
 }
 
@@ -559,11 +553,8 @@ size_t plain_smem(const WindowShape &m) { return (size_t)(m.dim + 8 * m.vdim) * 
 
 template <int NV>
 int32_t plain(const WindowArgs &a, bool pdl, cudaStream_t s) {
-  static bool ready = false;
-  if (!ready) {
-    CMLD_TRY(allow_smem(window_attn_kernel<NV>, 64 * 1024));
-    ready = true;
-  }
+  static SmemLimit limit;
+  CMLD_TRY(allow_smem(limit, window_attn_kernel<NV>, 64 * 1024));
   return launch_kernel(window_attn_kernel<NV>, dim3(a.rows, a.m.heads), dim3(256), plain_smem(a.m), pdl, s, a);
 }
 
