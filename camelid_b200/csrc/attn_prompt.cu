@@ -308,18 +308,18 @@ int32_t launch_prompt(const AttnArgs &a, int64_t n_pos, cudaStream_t s) {
 }  // namespace
 
 // n_pos: bound on positions[b] + 1 of every row; every row of the step belongs to one slot.
-bool attention_prompt_fits(int n_heads, int n_kv_heads, int head_dim, int batch, int64_t n_pos) {
+bool attention_prompt_fits(int n_heads, int n_kv_heads, int head_dim, int batch, int64_t n_pos, int sms) {
   if (n_kv_heads < 1 || n_heads % n_kv_heads) return false;
   const int G = n_heads / n_kv_heads;
   if (!(G == 1 || G == 2 || G == 3 || G == 4 || G == 8) || !(head_dim == 64 || head_dim == 128)) return false;
   // a CTA for every SM, or the row kernel's many small ones are faster (8B width: 36 rows at 700 positions 73 us against about
   // 50, 128 rows at 200 positions 47 us against 100)
   const int R = 8 * (G == 3 ? 3 : 2) / G;
-  return (batch + R - 1) / R * n_kv_heads >= 148 && n_pos > 0 && prompt_smem_bytes(head_dim, G == 3 ? 3 : 1, n_pos) <= kPromptOne;
+  return (batch + R - 1) / R * n_kv_heads >= sms && n_pos > 0 && prompt_smem_bytes(head_dim, G == 3 ? 3 : 1, n_pos) <= kPromptOne;
 }
 
-int32_t launch_attention_prompt(const AttnArgs &a, int64_t n_pos, cudaStream_t s) {
-  if (!attention_prompt_fits(a.n_heads, a.n_kv_heads, a.head_dim, a.batch, n_pos)) return CMLD_ERR_UNSUPPORTED;
+int32_t launch_attention_prompt(const AttnArgs &a, int64_t n_pos, int sms, cudaStream_t s) {
+  if (!attention_prompt_fits(a.n_heads, a.n_kv_heads, a.head_dim, a.batch, n_pos, sms)) return CMLD_ERR_UNSUPPORTED;
   if (a.tree_mask || a.fuse_rope) return fail(CMLD_ERR_INVALID, "attention (prompt): tree masks and fused RoPE are not supported here");
 #define CMLD_PROMPT(GG) \
   case GG: return a.head_dim == 128 ? launch_prompt<GG, 128>(a, n_pos, s) : launch_prompt<GG, 64>(a, n_pos, s);

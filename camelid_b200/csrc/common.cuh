@@ -370,8 +370,8 @@ bool attention_rows_fits(int n_heads, int n_kv_heads, int head_dim, int64_t cap)
 int32_t launch_attention_rows(const AttnArgs &a, int64_t cap, cudaStream_t s);
 
 // attn_prompt.cu: the reference-order attention for long steps of one sequence (n_pos: positions after the last row)
-bool attention_prompt_fits(int n_heads, int n_kv_heads, int head_dim, int batch, int64_t n_pos);
-int32_t launch_attention_prompt(const AttnArgs &a, int64_t n_pos, cudaStream_t s);
+bool attention_prompt_fits(int n_heads, int n_kv_heads, int head_dim, int batch, int64_t n_pos, int sms);
+int32_t launch_attention_prompt(const AttnArgs &a, int64_t n_pos, int sms, cudaStream_t s);
 
 // comm.cu: NCCL collectives of the sharded engine
 int32_t comm_unique_id(uint8_t *out128);

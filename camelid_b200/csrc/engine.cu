@@ -568,7 +568,7 @@ int32_t moe_expert_gemv(const Weight &slab, int64_t rows_per_expert, int n_local
 int32_t moe_find_inf_scale(Weight &slab, cudaStream_t s);
 int32_t moe_expert_gemv_ordered(const Weight &slab, int64_t rows_per_expert, int n_experts, int used, int n_local_experts, int first_expert, int expert_step,
                                 const float *x, int64_t x_stride, int x_div, float *y, const int32_t *counts, const int32_t *lists,
-                                int n_assign, cudaStream_t s, const Weight *slab2 = nullptr, float *y2 = nullptr);
+                                int n_assign, int sms, cudaStream_t s, const Weight *slab2 = nullptr, float *y2 = nullptr);
 int32_t moe_combine(float *h, const float *down, const float *sel_w, const int32_t *sel_idx, int hidden, int k, int batch,
                     int first_expert, int expert_step, bool add_residual, cudaStream_t s);
 
@@ -636,13 +636,13 @@ static int32_t moe_ffn_step(cmld_engine *e, LayerW &L, int32_t B) {
   if (pair) {
     // gate and up in one launch: the rows of the few active experts are too few to fill the machine on their own
     CMLD_TRY(moe_expert_gemv_ordered(L.exps[0], c.ffn_dim, c.n_experts, k, n_local, first, step, e->normed, c.hidden, k, e->moe_g, e->moe_counts,
-                                     e->moe_lists, na, e->stream, &L.exps[1], e->moe_u));
+                                     e->moe_lists, na, e->sm_count, e->stream, &L.exps[1], e->moe_u));
   } else if (fast) {
     CMLD_TRY(moe_expert_gemv(L.exps[0], c.ffn_dim, n_local, first, step, e->normed, c.hidden, k, e->moe_g, e->moe_counts, e->moe_lists, na, e->stream));
     CMLD_TRY(moe_expert_gemv(L.exps[1], c.ffn_dim, n_local, first, step, e->normed, c.hidden, k, e->moe_u, e->moe_counts, e->moe_lists, na, e->stream));
   } else {
-    CMLD_TRY(moe_expert_gemv_ordered(L.exps[0], c.ffn_dim, c.n_experts, k, n_local, first, step, e->normed, c.hidden, k, e->moe_g, e->moe_counts, e->moe_lists, na, e->stream));
-    CMLD_TRY(moe_expert_gemv_ordered(L.exps[1], c.ffn_dim, c.n_experts, k, n_local, first, step, e->normed, c.hidden, k, e->moe_u, e->moe_counts, e->moe_lists, na, e->stream));
+    CMLD_TRY(moe_expert_gemv_ordered(L.exps[0], c.ffn_dim, c.n_experts, k, n_local, first, step, e->normed, c.hidden, k, e->moe_g, e->moe_counts, e->moe_lists, na, e->sm_count, e->stream));
+    CMLD_TRY(moe_expert_gemv_ordered(L.exps[1], c.ffn_dim, c.n_experts, k, n_local, first, step, e->normed, c.hidden, k, e->moe_u, e->moe_counts, e->moe_lists, na, e->sm_count, e->stream));
   }
   NormQuantArgs a{};
   a.x = e->moe_g;
@@ -652,7 +652,7 @@ static int32_t moe_ffn_step(cmld_engine *e, LayerW &L, int32_t B) {
   a.out = e->moe_act;
   CMLD_TRY(launch_norm_quant(a, e->stream));
   if (fast) CMLD_TRY(moe_expert_gemv(L.exps[2], c.hidden, n_local, first, step, e->moe_act, c.ffn_dim, 1, e->moe_down, e->moe_counts, e->moe_lists, na, e->stream));
-  else CMLD_TRY(moe_expert_gemv_ordered(L.exps[2], c.hidden, c.n_experts, k, n_local, first, step, e->moe_act, c.ffn_dim, 1, e->moe_down, e->moe_counts, e->moe_lists, na, e->stream));
+  else CMLD_TRY(moe_expert_gemv_ordered(L.exps[2], c.hidden, c.n_experts, k, n_local, first, step, e->moe_act, c.ffn_dim, 1, e->moe_down, e->moe_counts, e->moe_lists, na, e->sm_count, e->stream));
   CMLD_TRY(moe_combine(e->h, e->moe_down, e->moe_sel_w, e->moe_sel_idx, c.hidden, k, B, first, step,
                        e->ep == 1 || e->shard_rank == 0, e->stream));
   e->launches += pair ? 6 : 7;
@@ -841,7 +841,7 @@ static int32_t engine_step(cmld_engine *e, const StepOpts &o) {
       const bool rows = !fast && !(c.flags & CMLD_FLAG_EXACT_ORDER) && B >= 3 && o.attn_cap > 0 && !o.tree_mask &&
                         attention_rows_fits(c.n_heads, c.n_kv_heads, c.head_dim, o.attn_cap);
       // a prompt's long steps (never captured: their context is exact): neighbouring rows share a CTA
-      const bool prompt = rows && o.prompt_end && attention_prompt_fits(c.n_heads, c.n_kv_heads, c.head_dim, B, o.prompt_end);
+      const bool prompt = rows && o.prompt_end && attention_prompt_fits(c.n_heads, c.n_kv_heads, c.head_dim, B, o.prompt_end, e->sm_count);
       const bool ordered = !rows && !fast && !(c.flags & CMLD_FLAG_EXACT_ORDER) && o.attn_cap > 0 && !o.tree_mask &&
                            attention_ordered_fits(c.n_heads, c.n_kv_heads, c.head_dim, o.attn_cap);
       const bool fuse = !o.shared_slots && (fast || ordered);
@@ -903,7 +903,7 @@ static int32_t engine_step(cmld_engine *e, const StepOpts &o) {
       a.tree_mask = o.tree_mask;
       a.tree_base = o.tree_base;
       a.tree_words = o.tree_words;
-      if (prompt) CMLD_TRY(launch_attention_prompt(a, o.prompt_end, e->stream));
+      if (prompt) CMLD_TRY(launch_attention_prompt(a, o.prompt_end, e->sm_count, e->stream));
       else if (rows) CMLD_TRY(launch_attention_rows(a, o.attn_cap, e->stream));
       else if (ordered) CMLD_TRY(launch_attention_ordered(a, o.attn_cap, e->stream));
       else if (fast) CMLD_TRY(launch_attention(a, e->stream));

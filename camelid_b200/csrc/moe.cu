@@ -875,7 +875,7 @@ static bool moe_ordered_tile(int n_assign, int n_experts, const float *x, int64_
 
 int32_t moe_expert_gemv_ordered(const Weight &slab, int64_t rows_per_expert, int n_experts, int used, int n_local_experts, int first_expert, int expert_step,
                                 const float *x, int64_t x_stride, int x_div, float *y, const int32_t *counts, const int32_t *lists,
-                                int n_assign, cudaStream_t s, const Weight *slab2, float *y2) {
+                                int n_assign, int sms, cudaStream_t s, const Weight *slab2, float *y2) {
   MoeGemvArgs a{slab.data, slab.qt, rows_per_expert, slab.cols, slab.stride, x, x_stride, x_div, y, counts, lists, n_assign,
                 first_expert, expert_step};
   if (slab2) {
@@ -890,7 +890,7 @@ int32_t moe_expert_gemv_ordered(const Weight &slab, int64_t rows_per_expert, int
     const int64_t tiles = (rows_per_expert + kTileRows - 1) / kTileRows;
     // as many assignments per pass as leave about four CTAs for every SM, but 16: below that the unpacking dominates
     int max_a = kTileMaxA;
-    while (max_a > 2 && tiles * n_local_experts * slabs * ((expect + 8 * max_a - 1) / (8 * max_a)) < 4 * 148) max_a = std::max(2, max_a / 2);
+    while (max_a > 2 && tiles * n_local_experts * slabs * ((expect + 8 * max_a - 1) / (8 * max_a)) < 4 * sms) max_a = std::max(2, max_a / 2);
     const int z = std::max(1, std::min(8, (2 * expect + 8 * max_a - 1) / (8 * max_a)));
     dim3 grid((unsigned)tiles, (unsigned)n_local_experts, (unsigned)(z * slabs));
     static SmemLimit limit[2];
