@@ -237,8 +237,8 @@ def test_mixtral_shaped_moe_parity(cm, orc):
 @pytest.mark.parametrize("qt", [12, 14])  # Q4_K, Q6_K experts
 @pytest.mark.parametrize("n", [9, 11, 37, 150, 301])
 def test_moe_prompts_equal_the_serial_path(cm, orc, qt, n):
-    """Prompts that give an expert 1 to 100 and more assignments: every number of them per thread of the tiled expert
-    product, its remainders, and passes that split an expert's assignments."""
+    """Prompts that give an expert 1 to 100 and more assignments, on a shape with few row tiles: the row product (9 tokens), and
+    one and two assignments per thread of the tiled product in many passes."""
     from camelid_b200 import synth
 
     cfg = synth.engine_config("tiny-moe", max_pos=352)
@@ -280,6 +280,43 @@ def test_moe_prompts_on_a_wide_shape(cm, orc, qt):
         assert token == orc.argmax(want[n - 1])
 
 
+@pytest.mark.parametrize("n", [150, 600])  # one long step; two, the first of 512 rows
+def test_logits_of_long_steps_by_row(cm, orc, n):
+    """The rows of a long step whose logits are asked for are gathered 32 at a time: more of them than one pass takes, lists with
+    and without the last token (whose greedy token is returned either way), none at all, places in two steps; and the draw from
+    the logits of the last token afterwards."""
+    cfg = cm.EngineConfig(n_layers=2, n_heads=8, n_kv_heads=4, head_dim=64, hidden=256, ffn_dim=512, vocab=512, max_pos=640)
+    pair = ModelPair(cfg, "q4_k_m", seed=61)
+    eng, ref = pair.engine, pair.oracle
+    prompt = orc.synth_tokens(9, 1, n, cfg.vocab)
+    all_logits = np.stack([ref.forward(ref.embedding(int(t)), pos)[0] for pos, t in enumerate(prompt)])
+    rng = np.random.default_rng(n)
+    some = lambda k: sorted(int(i) for i in rng.choice(n - 1, k, replace=False))
+    lists = [list(range(n)), list(range(n - 1)), some(32), some(33), some(31) + [n - 1], some(64), some(65), [0], [n - 1], [], list(range(n - 40, n - 1))]
+    for want in lists:
+        token, logits = eng.extend(0, prompt, 0, want=want)
+        assert np.array_equal(logits.view(np.uint32), all_logits[want].view(np.uint32)), want
+        assert token == orc.argmax(all_logits[n - 1]), want
+        assert eng.sample(1e-6, 7) == token, want  # so cold that the draw is the greedy token
+
+
+def test_long_prefill_from_embeddings_leaves_the_serial_kv(cm, orc):
+    """Embedding rows in, long steps of 512 and 88 rows and a start past row 0: the K/V rows are the checker's."""
+    cfg = cm.EngineConfig(n_layers=2, n_heads=8, n_kv_heads=4, head_dim=64, hidden=256, ffn_dim=512, vocab=512, max_pos=640)
+    pair = ModelPair(cfg, "q4_k_m", seed=62)
+    eng, ref = pair.engine, pair.oracle
+    prompt = orc.synth_tokens(9, 1, 600, cfg.vocab)
+    embs = np.stack([ref.embedding(int(t)) for t in prompt])
+    for pos in range(600):
+        ref.forward(embs[pos], pos, want_logits=False)
+    cos, sin = (np.stack(t) for t in zip(*[pair.rope(pos) for pos in range(600)]))
+    for start in (0, 3):
+        eng.prefill_from(embs, cos, sin, 600, pair.scale, start)
+        for layer in range(cfg.n_layers):
+            for got, want in zip(eng.read_kv_layer(layer, 600), ref.read_kv_layer(layer, 600)):
+                assert np.array_equal(got, want), (start, layer)
+
+
 @pytest.mark.parametrize("rows", [1, 2, 3, 4, 10])  # ten rows give every expert enough assignments for the tiled product
 def test_infinite_superblock_scales_give_the_cpus_infinities(cm, orc, rows):
     """Q4_K experts with an infinite scale: a code above 0 stands for an infinity, a code of 0 for NaN, in both expert
@@ -313,11 +350,13 @@ def test_infinite_superblock_scales_give_the_cpus_infinities(cm, orc, rows):
 
 @pytest.mark.parametrize("heads,kv,hd,first,n", [(16, 16, 64, 0, 150), (16, 8, 64, 3, 150), (8, 4, 128, 0, 300), (12, 4, 64, 0, 301), (12, 4, 64, 900, 301),
                                                   (12, 4, 128, 30, 299), (32, 8, 64, 5, 77), (16, 4, 64, 1400, 150), (16, 4, 128, 0, 161), (32, 4, 64, 100, 75),
-                                                  (16, 2, 128, 0, 149), (16, 4, 128, 10, 40)])
+                                                  (16, 2, 128, 0, 149), (16, 4, 128, 10, 40), (12, 4, 128, 800, 301), (16, 4, 128, 1300, 161),
+                                                  (32, 4, 64, 1300, 150), (32, 4, 128, 1300, 150), (8, 4, 64, 1200, 301), (16, 16, 64, 1300, 150)])
 def test_long_prompt_steps_equal_the_serial_path(cm, orc, heads, kv, hd, first, n):
     """Steps of more than 32 rows of one sequence, whose attention serves neighbouring rows together: every group size and
     head dimension, row counts that leave the last group short, contexts that end inside a tile, a start past position 0, long
-    contexts (fewer queries or outputs per thread), and a step too short for it."""
+    contexts (fewer queries per thread, or outputs with three heads per KV head, at both head dimensions), and a step too short
+    for it."""
     cfg = cm.EngineConfig(n_layers=2, n_heads=heads, n_kv_heads=kv, head_dim=hd, hidden=256, ffn_dim=512, vocab=512, max_pos=1600)
     pair = ModelPair(cfg, "q4_k_m", seed=61)
     eng, ref = pair.engine, pair.oracle
@@ -409,10 +448,9 @@ def test_steps_of_16_and_32_rows_equal_independent_sequences(cm, orc, shape, mix
     assert np.array_equal(lg2[::-1], lg)
 
 
-def test_prefill_chunk_of_32_rows_leaves_the_serial_kv(cm, orc):
+def test_prefill_of_40_rows_leaves_the_serial_kv(cm, orc):
     """prefill_then_decode_matches_sequential (src/cuda_resident/tests.rs:3143): a 40-token prompt ingested in
-    chunks of 32 rows leaves the KV rows, and gives the next token, of token-by-token steps — which are the
-    checker's."""
+    one step leaves the KV rows, and gives the next token, of token-by-token steps — which are the checker's."""
     from camelid_b200 import synth
 
     cfg = synth.engine_config("small", max_pos=64, max_seqs=2)

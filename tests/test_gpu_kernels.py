@@ -175,8 +175,8 @@ def test_fused_prologue_equals_separate_steps(cm, orc, name, rows, cols, mode, b
     assert np.array_equal(got, want)
 
 
-# More than 8 activation rows.  By default they take the tcgen05 kernel: the weights are read once for up to
-# 32 rows, the integer parts come from the tensor cores and the f32 terms are added in the CPU dot's order
+# More than 8 activation rows.  By default they take the tcgen05 kernel: the weights are read once for all
+# rows, the integer parts come from the tensor cores and the f32 terms are added in the CPU dot's order
 # (the checker's bits).  The older int8 mma.sync kernel adds the superblocks' f32 terms as a tree, so it is
 # opt-in and held to a tolerance.
 @pytest.mark.parametrize("name,rows,cols", [
