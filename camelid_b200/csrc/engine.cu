@@ -162,7 +162,8 @@ int32_t init_rows(cmld_engine *e, int64_t rows, int64_t logit_rows, int64_t voca
 // Rows of one step of a prompt.  The batched matrix product shares an unpacked weight among 128 rows and reads it once for
 // all rows of a step, so a prompt goes in by steps of up to 512 rows where that product takes the shapes (more rows fill the
 // last wave of its CTAs better; beyond 512 the scratch rows grow for little).  The experts of a Mixtral shape share an unpacked
-// weight among a step's rows likewise.  Everything else: 32 rows.
+// weight among a step's rows likewise.  Everything else: 32 rows, the rows of those modes' own products and attention (the
+// attention over a Q8_0 cache has a CTA for every row and head, the split-range one scratch for the rows of a listed step).
 static int32_t prompt_rows(const cmld_engine *e) {
   const cmld_config &c = e->cfg;
   const uint32_t other = CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV | CMLD_FLAG_TENSOR_BATCH | CMLD_FLAG_FAST_ORDER | CMLD_FLAG_KV_Q8_0;
@@ -450,11 +451,12 @@ constexpr int kFusedPrologueMaxBatch = 2;
 // different order from the CPU path, so it is opt-in (CMLD_FLAG_TENSOR_BATCH); by default every step
 // goes through the staged kernel, in passes of up to 8 rows.
 static int mma_min_rows(const cmld_engine *e) { return (e->cfg.flags & CMLD_FLAG_TENSOR_BATCH) ? 5 : (1 << 30); }
-// Steps of this many rows or more (and prompt chunks) take the tcgen05 batched matvec: one pass over the weights
-// for up to 128 rows, the same bits as the one-row kernels.  The staged kernel's time grows with the rows, this one's does not:
-// a step of 4 layers at 6 | 7 rows takes 1152 | 1364 us staged and 1213 | 1216 here (8B width, Q4_K_M), 646 | 737 and 696 | 697
-// (1B, Q4_K_M), 922 | 1020 and 809 | 835 (3B, Q4_K_M); Q8_0 matrices cross one row earlier, at 5 | 6 rows 663 | 712 and 669 | 671
-// (1B), 1447 | 1628 and 1282 | 1283 (8B).
+// Steps of this many rows or more (and prompts) take the tcgen05 batched matvec: one pass over the weights for all rows, the same
+// bits as the one-row kernels.  The staged kernel's time grows with the rows, this one's hardly does.  The line lies where no
+// measured width is slower for it; it is the 8B and 1B widths that set it for K-quants and the 1B width for Q8_0, while others
+// would gain from an earlier one.  A step of 4 layers, us, staged | here:
+//   Q4_K_M at 6 and 7 rows: 8B 1152 | 1213 and 1364 | 1216;  1B 646 | 696 and 737 | 697;  3B 922 | 809 and 1020 | 835
+//   Q8_0 at 5 and 6 rows: 1B 663 | 669 and 712 | 671;  8B 1447 | 1282 and 1628 | 1283
 static int tc5_min_rows(const cmld_engine *e, int32_t qt) {
   return (e->cfg.flags & (CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV | CMLD_FLAG_TENSOR_BATCH)) ? (1 << 30) : qt == CMLD_Q8_0 ? 6 : 7;
 }
