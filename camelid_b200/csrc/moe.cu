@@ -33,7 +33,9 @@ __device__ __forceinline__ int total_key(float f) {
   return b ^ (int)(((unsigned)(b >> 31)) >> 1);
 }
 
-// One CTA per token row: router logits, then top-k selection by thread 0.
+// One CTA per token row: router logits, then top-k selection by thread 0.  WHOLE: the width is a multiple of 1024 (the tests for a
+// short last chunk cost 2 of the 13 us below).
+template <bool WHOLE>
 __global__ void __launch_bounds__(256) moe_route_kernel(const float *__restrict__ x, const float *__restrict__ router, int hidden,
                                                         int n_exp, int k, int32_t *__restrict__ sel_idx, float *__restrict__ sel_w) {
   __shared__ float logits[kMaxExperts];
@@ -54,8 +56,8 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float *__restrict_
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int i = i0 + lane * 4 + 128 * j;
-        xv[j] = rv[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (i < hidden) {
+        if (!WHOLE) xv[j] = rv[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (WHOLE || i < hidden) {
           xv[j] = __ldg(reinterpret_cast<const float4 *>(xr + i));
           rv[j] = __ldg(reinterpret_cast<const float4 *>(r + i));
         }
@@ -72,7 +74,7 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float *__restrict_
       float4 v[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) v[j] = p4[j];
-      const int n4 = min(256, (hidden - i0 + 15) / 16 * 4);
+      const int n4 = WHOLE ? 256 : min(256, (hidden - i0 + 15) / 16 * 4);
       for (int i = 0; i < n4; i += 4) {
         float4 next[4];
 #pragma unroll
@@ -820,7 +822,8 @@ int32_t moe_route(const float *normed, const float *router, int hidden, int n_ex
                   float *sel_w, int32_t *counts, int32_t *lists, cudaStream_t s, int32_t *pos) {
   if (n_exp > kMaxExperts) return fail(CMLD_ERR_SHAPE, "more than %d experts", kMaxExperts);
   if (hidden % 4) return fail(CMLD_ERR_SHAPE, "router: width %d is not a multiple of 4", hidden);  // (expert matrices: of 256)
-  moe_route_kernel<<<batch, 256, 0, s>>>(normed, router, hidden, n_exp, k, sel_idx, sel_w);
+  if (hidden % 1024 == 0) moe_route_kernel<true><<<batch, 256, 0, s>>>(normed, router, hidden, n_exp, k, sel_idx, sel_w);
+  else moe_route_kernel<false><<<batch, 256, 0, s>>>(normed, router, hidden, n_exp, k, sel_idx, sel_w);
   CMLD_CUDA(cudaGetLastError());
   moe_group_kernel<<<1, std::min(32, n_exp) * 32, 0, s>>>(sel_idx, batch * k, n_exp, counts, lists, pos);
   CMLD_CUDA(cudaGetLastError());
