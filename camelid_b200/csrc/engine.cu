@@ -160,9 +160,10 @@ int32_t init_rows(cmld_engine *e, int64_t rows, int64_t logit_rows, int64_t voca
 }
 
 // Rows of one step of a prompt.  The batched matrix product shares an unpacked weight among 128 rows and reads it once for
-// all rows of a step, so a prompt goes in by steps of up to 512 rows where that product takes the shapes (more rows fill the
-// last wave of its CTAs better; beyond 512 the scratch rows grow for little).  The experts of a Mixtral shape share an unpacked
-// weight among a step's rows likewise.  Everything else: 32 rows, the rows of those modes' own products and attention (the
+// all rows of a step, so a prompt goes in by steps of up to 512 rows where that product takes the shapes.  Four layers, 1024 tokens
+// of the 8B width (Q4_K_M), in steps of 128 | 256 | 384 | 512 | 1024 rows: 14.2 | 11.8 | 11.3 | 10.1 | 9.4 ms; 1500 tokens of the 1B
+// width (Q8_0): 13.4 | 9.7 | 8.7 | 8.0 | 7.7 ms: each doubling gives less, while the scratch rows, which every engine holds, double
+// too.  The experts of a Mixtral shape share an unpacked weight among a step's rows likewise.  Everything else: 32 rows, the rows of those modes' own products and attention (the
 // attention over a Q8_0 cache has a CTA for every row and head, the split-range one scratch for the rows of a listed step).
 static int32_t prompt_rows(const cmld_engine *e) {
   const cmld_config &c = e->cfg;

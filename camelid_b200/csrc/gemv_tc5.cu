@@ -769,6 +769,8 @@ int g_tc_sms = 0;
 }  // namespace
 
 static bool tc5_qt_ok(int qt) { return qt == CMLD_Q4_K || qt == CMLD_Q6_K || qt == CMLD_Q8_0; }
+// Rows of an activation tile.  Up to 32 the MR = 32 form is a fifth to a third faster; from 33 on one 128-row tile is, against two passes
+// of it.  At 32 | 33 | 128 rows: Q4_K 28672 x 4096 68 | 83 | 89 us, Q6_K 4096 x 14336 81 | 107 | 107, Q8_0 16384 x 2048 35 | 46 | 48.
 static int tc5_mr(int32_t batch) { return batch <= 32 ? 32 : 128; }
 
 // Bytes of packed activation records a step of `batch` rows needs for `cols` columns of any type.
@@ -838,7 +840,10 @@ static int32_t launch_tc5_qt(const GemvJob *jobs, int n_jobs, const uint8_t *act
     default: tc5_pack_kernel<CMLD_Q8_0><<<pg, 128, 0, s>>>(act, cols, batch, mr, a.m_tiles, pack); break;
   }
   CMLD_CUDA(cudaGetLastError());
-  // Tiles of 64 weight rows, or of 32 where those leave the last wave of CTAs emptier.
+  // Tiles of 64 weight rows, or of 32 where those leave the last wave of CTAs emptier.  A tile of 32 takes about 0.6 of the time of
+  // one of 64 (it repeats the step's hand-offs for half of the rows), hence 3 rounds against 5.  Us with 32 | 64: Q4_K 28672 x 4096, 512
+  // rows, 383 | 276; Q4_K 4096 x 4096 67 | 48, and at 128 rows, one round either way, 21.8 | 26.9; Q8_0 2048 x 8192 at 512 rows 110 | 85,
+  // at 128 rows 58 | 84; Q8_0 3072 x 2048 at 512 rows 46.2 | 48.6.  The rule takes the faster one in each.
   auto rounds = [&](int nw) {
     int64_t t = 0;
     for (int i = 0; i < n_jobs; ++i) t += (jobs[i].rows + nw - 1) / nw;

@@ -46,7 +46,8 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float *__restrict_
   // src/inference.rs:29382-29409).  One warp per expert: the products of a 1024-value chunk are formed by all lanes
   // from coalesced loads (a product does not depend on the order), then added in index order while the next chunk's
   // values travel.  Bound by the latency of the additions (4 clocks each): sixteen products are in registers before
-  // they are needed.  One row of 4096 values, 8 experts: 34 -> 13 us.
+  // they are needed.  One row of 4096 values, 8 experts: 34 -> 13 us.  At a width of 3584 a layer of a small
+  // expert model went from 90 to 78 us a step when such widths took this form too.
   for (int e = warp; e < n_exp; e += 8) {
     const float *r = router + (int64_t)e * hidden;
     float s = 0.0f;
@@ -891,7 +892,9 @@ int32_t moe_expert_gemv_ordered(const Weight &slab, int64_t rows_per_expert, int
   if (slab.inf_scale || (slab2 && slab2->inf_scale) || moe_ordered_tile(n_assign, n_experts, x, x_stride)) {
     const int slabs = slab2 ? 2 : 1, expect = (n_assign + n_experts - 1) / n_experts;
     const int64_t tiles = (rows_per_expert + kTileRows - 1) / kTileRows;
-    // as many assignments per pass as leave about four CTAs for every SM, but 16: below that the unpacking dominates
+    // as many assignments per pass as leave about four CTAs for every SM, but 16: below that the unpacking dominates.  Two
+    // Mixtral-8x7B layers, a prompt of 130 tokens: 9.06 ms (48 for gate and up, 16 for down), with 16 | 24 | 32 | 48 for both 9.86 | 9.84 |
+    // 9.73 | 9.55
     int max_a = kTileMaxA;
     while (max_a > 2 && tiles * n_local_experts * slabs * ((expect + 8 * max_a - 1) / (8 * max_a)) < 4 * sms) max_a = std::max(2, max_a / 2);
     const int z = std::max(1, std::min(8, (2 * expect + 8 * max_a - 1) / (8 * max_a)));
