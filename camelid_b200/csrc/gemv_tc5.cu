@@ -769,7 +769,7 @@ int g_tc_sms = 0;
 }  // namespace
 
 static bool tc5_qt_ok(int qt) { return qt == CMLD_Q4_K || qt == CMLD_Q6_K || qt == CMLD_Q8_0; }
-// Rows of an activation tile.  Up to 32 the MR = 32 form is a fifth to a third faster; from 33 on one 128-row tile is, against two passes
+// Rows of an activation tile.  Up to 32 the MR = 32 form is up to a third faster; from 33 on one 128-row tile is faster than two passes
 // of it.  At 32 | 33 | 128 rows: Q4_K 28672 x 4096 68 | 83 | 89 us, Q6_K 4096 x 14336 81 | 107 | 107, Q8_0 16384 x 2048 35 | 46 | 48.
 static int tc5_mr(int32_t batch) { return batch <= 32 ? 32 : 128; }
 
