@@ -69,6 +69,7 @@ static int32_t check_op_status(const char *what) {
 static int g_gemv_pdl = 0;            // cmld_gemv_time: chain its launches with programmatic dependent launch
 static int g_gemv_kernel_choice = 0;  // 0 auto (staged when the shape fits), 1 generic kernel only
 static int g_gemv_mma_min_batch = 1 << 30;  // rows from which the int8 mma.sync kernel is used (opt-in: bit 3 of the choice from 9 rows, bit 2 from 1)
+static int g_gemv_rows_min_batch = 3;       // rows from which the row-batched kernel is used, up to 32 (any of bits 2 to 5 of the choice: never)
 static int g_gemv_tc5_min_batch = 9;        // rows from which the tcgen05 kernel is used (bit 4 of the choice: never; bit 5: from 1 row)
 
 constexpr int32_t kOpTc5Rows = 2048;  // rows per pass of the tcgen05 kernel: bounds its scratch and its grids
@@ -77,9 +78,16 @@ constexpr int32_t kOpTc5Rows = 2048;  // rows per pass of the tcgen05 kernel: bo
 static int32_t gemv_launch(const cmld_weight *w, const uint8_t *act, int32_t batch, float *y, const float *residual,
                            cudaStream_t stream = nullptr, bool pdl = false) {
   GemvJob probe{w->data, w->qt, w->rows, w->cols, w->stride, y, residual, w->rows};
+  if (g_gemv_kernel_choice == 0 && batch >= g_gemv_rows_min_batch && batch <= kRowsMaxBatch && gemv_rows_fits(&probe, 1, batch)) {
+    uint8_t *rec = reinterpret_cast<uint8_t *>(op_scratch((gemv_rows_rec_bytes(w->cols, batch) + 3) / 4));
+    if (!rec) return fail(CMLD_ERR_OOM, "gemv: no room for %lld bytes of activation records", (long long)gemv_rows_rec_bytes(w->cols, batch));
+    uint8_t *rec4 = w->qt == CMLD_Q4_K ? rec : nullptr, *rec6 = w->qt == CMLD_Q6_K ? rec : nullptr, *rec0 = w->qt == CMLD_Q8_0 ? rec : nullptr;
+    CMLD_TRY(launch_rows_pack(act, w->cols, batch, rec4, rec6, rec0, stream));
+    return launch_gemv_rows(&probe, 1, batch, rec4, rec6, rec0, op_status(), stream, pdl);
+  }
   if (g_gemv_kernel_choice == 0 && batch >= g_gemv_tc5_min_batch && batch < g_gemv_mma_min_batch && gemv_tc5_fits(&probe, 1, batch)) {
     // several rows: one pass over the weights per 2048 rows on the tcgen05 tensor cores, same bits as the one-row kernels
-    const int64_t need = std::max(gemv_tc5_pack_bytes(w->cols, std::min(batch, kOpTc5Rows)), gemv_tc5_pack_bytes(w->cols, 32));
+    const int64_t need = gemv_tc5_pack_bytes(w->cols, std::min(batch, kOpTc5Rows));
     uint8_t *pack = reinterpret_cast<uint8_t *>(op_scratch((need + 3) / 4));
     if (!pack) return fail(CMLD_ERR_OOM, "gemv: no room for %lld bytes of packed activations", (long long)need);
     for (int32_t b0 = 0; b0 < batch; b0 += kOpTc5Rows) {
@@ -385,6 +393,7 @@ int32_t cmld_gemv_select_kernel(int32_t choice) {
   g_gemv_kernel_choice = choice & 1;
   g_gemv_pdl = (choice >> 1) & 1;
   g_gemv_mma_min_batch = (choice & 4) ? 1 : ((choice & 8) ? 9 : (1 << 30));
+  g_gemv_rows_min_batch = (choice & 60) ? (1 << 30) : 3;
   g_gemv_tc5_min_batch = (choice & 16) ? (1 << 30) : ((choice & 32) ? 1 : 9);
   return CMLD_OK;
 }

@@ -288,6 +288,15 @@ bool gemv_tc5_fits(const GemvJob *jobs, int n_jobs, int32_t batch);
 int32_t launch_gemv_tc5(const GemvJob *jobs, int n_jobs, const uint8_t *act, int32_t batch, uint8_t *pack, int64_t pack_bytes,
                         int32_t *status, cudaStream_t s, int64_t *launches);
 
+// gemv_rows.cu: up to 32 activation rows, weights unpacked in the operand registers of mma.sync, the one-row kernels' bits.  The
+// activations come as records (rows_record.cuh), written by launch_norm_quant or rearranged from quantised rows.
+constexpr int32_t kRowsMaxBatch = 32;
+int64_t gemv_rows_rec_bytes(int64_t cols, int32_t batch);
+bool gemv_rows_fits(const GemvJob *jobs, int n_jobs, int32_t batch);
+int32_t launch_rows_pack(const uint8_t *act, int64_t cols, int32_t batch, uint8_t *rec4, uint8_t *rec6, uint8_t *rec0, cudaStream_t s);
+int32_t launch_gemv_rows(const GemvJob *jobs, int n_jobs, int32_t batch, const uint8_t *rec4, const uint8_t *rec6, const uint8_t *rec0,
+                         int32_t *status, cudaStream_t s, bool pdl);
+
 int64_t gemv_mma_expert_scratch_floats(const GemvJob *jobs, int n_jobs, int nt, int n_experts, int n_pass);
 int32_t launch_gemv_mma_experts(const GemvJob *jobs, int n_jobs, const uint8_t *act, int nt, int n_experts, int n_pass,
                                 const int32_t *counts, int first_expert, int expert_step, int cap, int count_mul, float *scratch,
@@ -305,6 +314,7 @@ struct NormQuantArgs {
   uint8_t *act;         // quantised result or null
   int32_t act_q8_0, act_q8_k;  // which formats to emit; both allowed: Q8_K at act, Q8_0 at act2
   uint8_t *act2;
+  uint8_t *rec4, *rec6, *rec0;  // records of the row-batched matvec instead of (or beside) the rows above; null = not wanted
   int32_t pdl;                 // launch with programmatic stream serialisation
   int32_t exact;               // RMSNorm: add the squares one after another like the CPU (slow)
 };

@@ -279,8 +279,9 @@ static int32_t engine_init(cmld_engine *e) {
   {
     const int64_t widest = std::max<int64_t>(std::max<int64_t>(c.hidden, c.ffn_dim), e->q_width);
     const int64_t wide = (widest + 255) / 256 * 256;
-    e->tc5_pack_bytes = std::max(gemv_tc5_pack_bytes(wide, 32), gemv_tc5_pack_bytes(wide, (int32_t)R));
+    e->tc5_pack_bytes = gemv_tc5_pack_bytes(wide, (int32_t)R);
     CMLD_TRY(dev_alloc(e, &e->tc5_pack, e->tc5_pack_bytes, false));
+    for (auto &rec : e->rows_rec) CMLD_TRY(dev_alloc(e, &rec, gemv_rows_rec_bytes(wide, kRowsMaxBatch), false));
   }
   if (const char *tp = getenv("CMLD_TRACE")) {
     e->trace_path = std::string(tp) + "." + std::to_string(e->shard_rank);
@@ -421,7 +422,8 @@ static int32_t run_gemv_group(cmld_engine *e, const Proj *p, int n, int32_t batc
 }
 
 static int32_t run_norm_quant(cmld_engine *e, const float *x, const float *x2, const float *weight, int64_t cols,
-                              int32_t batch, float *out, bool need_0, bool need_k) {
+                              int32_t batch, float *out, bool need_0, bool need_k, uint8_t *rec4 = nullptr, uint8_t *rec6 = nullptr,
+                              uint8_t *rec0 = nullptr) {
   NormQuantArgs a{};
   a.x = x;
   a.x2 = x2;
@@ -434,6 +436,9 @@ static int32_t run_norm_quant(cmld_engine *e, const float *x, const float *x2, c
   a.act_q8_k = need_k;
   a.act = need_k ? e->act_k : e->act_0;
   a.act2 = e->act_0;
+  a.rec4 = rec4;
+  a.rec6 = rec6;
+  a.rec0 = rec0;
   a.pdl = !(e->cfg.flags & CMLD_FLAG_NO_PDL);
   a.exact = (e->cfg.flags & CMLD_FLAG_EXACT_ORDER) != 0;
   CMLD_TRY(launch_norm_quant(a, e->stream));
@@ -452,14 +457,14 @@ constexpr int kFusedPrologueMaxBatch = 2;
 // different order from the CPU path, so it is opt-in (CMLD_FLAG_TENSOR_BATCH); by default every step
 // goes through the staged kernel, in passes of up to 8 rows.
 static int mma_min_rows(const cmld_engine *e) { return (e->cfg.flags & CMLD_FLAG_TENSOR_BATCH) ? 5 : (1 << 30); }
-// Steps of this many rows or more (and prompts) take the tcgen05 batched matvec: one pass over the weights for all rows, the same
-// bits as the one-row kernels.  The staged kernel's time grows with the rows, this one's hardly does.  The line lies where no
-// measured width is slower for it; it is the 8B and 1B widths that set it for K-quants and the 1B width for Q8_0, while others
-// would gain from an earlier one.  A step of 4 layers, us, staged | here:
-//   Q4_K_M at 6 and 7 rows: 8B 1152 | 1213 and 1364 | 1216;  1B 646 | 696 and 737 | 697;  3B 922 | 809 and 1020 | 835
-//   Q8_0 at 5 and 6 rows: 1B 663 | 669 and 712 | 671;  8B 1447 | 1282 and 1628 | 1283
-static int tc5_min_rows(const cmld_engine *e, int32_t qt) {
-  return (e->cfg.flags & (CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV | CMLD_FLAG_TENSOR_BATCH)) ? (1 << 30) : qt == CMLD_Q8_0 ? 6 : 7;
+// From this many rows on, and up to kRowsMaxBatch, a step's matvecs run on the row-batched kernel (gemv_rows.cu), longer steps of a
+// prompt on the tcgen05 one (gemv_tc5.cu): the same bits as the staged kernel's, whose time grows with the rows.  At one row the
+// staged kernel's fused prologue and its dp4a on the packed codes win for K-quants; Q8_0's codes are the tensor cores' operand as
+// they are.  Eight steps of 4 layers, us, staged | here:
+//   1 row: Q8_0 1B 2177 | 2023, 8B 4036 | 3557; Q4_K_M 1B 1844 | 2117, 8B 2843 | 3355
+//   2 rows: Q8_0 1B 2974 | 2269, 3B 3973 | 3183, 8B 5693 | 3947; Q4_K_M 1B 2514 | 2278, 3B 3260 | 2931, 8B 4096 | 3779
+static int rows_min_rows(const cmld_engine *e, int32_t qt) {
+  return (e->cfg.flags & (CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV | CMLD_FLAG_TENSOR_BATCH)) ? (1 << 30) : qt == CMLD_Q8_0 ? 1 : 2;
 }
 
 static int32_t gemv_fused(cmld_engine *e, const Proj *p, int n, int32_t batch, int mode, const float *x, const float *x2,
@@ -481,11 +486,22 @@ static int32_t gemv_fused(cmld_engine *e, const Proj *p, int n, int32_t batch, i
     }
     return CMLD_OK;
   }
-  if (batch >= tc5_min_rows(e, p[0].w->qt) && n <= 3 && !peer && !pair_swiglu && !(n0 && nk)) {
+  if (batch >= rows_min_rows(e, p[0].w->qt) && n <= 3 && !peer && !pair_swiglu && !(n0 && nk)) {
     GemvJob jobs[3];
-    for (int i = 0; i < n; ++i)
+    bool q4 = false, q6 = false;
+    for (int i = 0; i < n; ++i) {
       jobs[i] = GemvJob{p[i].w->data, p[i].w->qt, p[i].w->rows, p[i].w->cols, p[i].w->stride, p[i].y, p[i].residual, p[i].y_stride};
-    if (gemv_tc5_fits(jobs, n, batch) && gemv_tc5_pack_bytes(cols, batch) <= e->tc5_pack_bytes) {
+      q4 = q4 || jobs[i].qt == CMLD_Q4_K;
+      q6 = q6 || jobs[i].qt == CMLD_Q6_K;
+    }
+    if (batch <= kRowsMaxBatch && gemv_rows_fits(jobs, n, batch)) {
+      uint8_t *rec4 = q4 ? e->rows_rec[0] : nullptr, *rec6 = q6 ? e->rows_rec[1] : nullptr, *rec0 = n0 ? e->rows_rec[0] : nullptr;
+      CMLD_TRY(run_norm_quant(e, x, mode == 3 ? x2 : nullptr, mode == 1 ? norm_w : nullptr, cols, batch, nullptr, false, false, rec4, rec6, rec0));
+      CMLD_TRY(launch_gemv_rows(jobs, n, batch, rec4, rec6, rec0, e->d_status, e->stream, pdl));
+      e->launches += 1;
+      return CMLD_OK;
+    }
+    if (batch > kRowsMaxBatch && gemv_tc5_fits(jobs, n, batch) && gemv_tc5_pack_bytes(cols, batch) <= e->tc5_pack_bytes) {
       CMLD_TRY(run_norm_quant(e, x, mode == 3 ? x2 : nullptr, mode == 1 ? norm_w : nullptr, cols, batch, nullptr, n0, nk));
       return launch_gemv_tc5(jobs, n, n0 ? e->act_0 : e->act_k, batch, e->tc5_pack, e->tc5_pack_bytes, e->d_status, e->stream, &e->launches);
     }
@@ -935,7 +951,7 @@ static int32_t engine_step(cmld_engine *e, const StepOpts &o) {
       take_pending(g);
       // gate and up of equal type: the staged kernel pairs their tiles and writes SwiGLU(gate, up) itself,
       // so the down projection's operand is a plain quantisation of one vector
-      bool pair = !(c.flags & (CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV)) && L.proj[4].qt == L.proj[5].qt && B < mma_min_rows(e) && B < tc5_min_rows(e, L.proj[4].qt);
+      bool pair = !(c.flags & (CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV)) && L.proj[4].qt == L.proj[5].qt && B < mma_min_rows(e) && (use_peer || B < rows_min_rows(e, L.proj[4].qt));
       if (pair) {
         const GemvJob pj[2] = {{L.proj[4].data, L.proj[4].qt, L.proj[4].rows, L.proj[4].cols, L.proj[4].stride, nullptr, nullptr, 0},
                                {L.proj[5].data, L.proj[5].qt, L.proj[5].rows, L.proj[5].cols, L.proj[5].stride, nullptr, nullptr, 0}};

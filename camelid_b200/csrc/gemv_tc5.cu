@@ -16,25 +16,21 @@
 //     sc*(q-32) = 128*vh + vl (vh signed, vl in 0..127), and aux[l] = 128*D_hi + D_lo.
 //
 // The activation rows are operand A (M = 128), the weight rows operand B: a tile is 128 activation rows x NW weight rows, so
-// that unpacking a weight, the cost that dominates when few rows share it, is shared by 128 rows.  Steps of at most 32 rows
-// (MR = 32) put the same 32 rows into the four quarters of A, and each quarter's epilogue warp takes its own NW/4 weight
-// rows: the tensor cores repeat work they have time for, and every epilogue lane has a row.
+// that unpacking a weight is shared by 128 rows.  Steps of up to 32 rows have a kernel of their own (gemv_rows.cu).
 //
 // One CTA per SM, K step = 256 columns.  Warp roles (16 or 24 warps):
-//   epilogue    8 or 16 warps that share the weight rows, or 4 (MR = 32): tcgen05.ld, integer fix-up, f32 chains
-//   weights     4 warps, or 8 in two groups that take turns (MR = 32): cp.async of the raw wire bytes into a private ring,
-//               unpack into the K-major operand layout; Q8_0 codes are copied straight into that layout
+//   epilogue    8 or 16 warps that share the weight rows: tcgen05.ld, integer fix-up, f32 chains
+//   weights     4 warps: cp.async of the raw wire bytes into a ring, unpack into the K-major operand layout; Q8_0 codes are
+//               copied straight into that layout
 //   MMA         one lane issues the MMAs and commits them to the mbarriers
 //   activations one lane brings a step's packed record by bulk copies
 // Accumulators: Q4_K two slots of a whole step; Q6_K and Q8_0 four slots that each hold a quarter of a step (two classes,
 // two blocks), so that the tensor cores fill one while the epilogue reads another.
 // Why this split: with the weights as operand A (128 rows) and at most 32 activation rows per pass, unpacking (about 300
-// instructions of one thread per 64 Q6_K values) was repeated for every 8 to 32 activation rows and bound the launch: 105 us
-// for Q6_K 4096 x 14336 at 32 rows and 45 ms of a 1024-token prompt's 55.8 ms (4 layers of the 8B width).  With the
-// activations as A those launches take 81 us and 7.1 ms.
-// What bounds it now: at 512 rows the epilogue, then unpacking (Q6_K 4096 x 14336: 461 us, 301 without the f32 steps, 361 without
-// unpacking, 401 with half of the MMAs; Q4_K 28672 x 4096: 276, 229, 227, 266); at 32 rows no one stage (leaving any out gives
-// 5 to 12 %) but the chain of hand-offs of a step.
+// instructions of one thread per 64 Q6_K values) was repeated for every 8 to 32 activation rows and bound the launch: 45 ms of a
+// 1024-token prompt's 55.8 ms (4 layers of the 8B width).  With the activations as A those launches take 7.1 ms.
+// What bounds it now, at 512 rows: the epilogue, then unpacking (Q6_K 4096 x 14336: 461 us, 301 without the f32 steps, 361 without
+// unpacking, 401 with half of the MMAs; Q4_K 28672 x 4096: 276, 229, 227, 266).
 // Every wait is bounded: a wait that runs out sets the status word and an abort flag, all roles leave their loops, tensor
 // memory is freed and the kernel returns.
 #include "common.cuh"
@@ -46,32 +42,30 @@ namespace {
 constexpr int kTcMaxStages = 8;
 constexpr int kTcPrefetchAhead = 8;  // K steps by which a row's wire bytes are asked into L2 before they are copied
 constexpr uint32_t kTcSpin = 1u << 22;
+constexpr int kMR = 128;  // activation rows of a tile
 
 __host__ __device__ constexpr int kq_bytes(int qt) { return qt == CMLD_Q4_K ? 144 : qt == CMLD_Q6_K ? 208 : 256; }  // of a row per K step
 
-// packed activation record of one K step and one tile of MR rows: codes [row/8][k/16][row%8][16], (Q4_K) sums of 16 codes
-// as f16 [row/8][2][row%8][8], scales f32 [MR] (Q8_0: [8 blocks][MR])
-__host__ __device__ constexpr int rec_p(int qt, int mr) { return qt == CMLD_Q4_K ? mr * 32 : 0; }
-__host__ __device__ constexpr int rec_scales(int qt, int mr) { return (qt == CMLD_Q8_0 ? 8 : 1) * mr * 4; }
-__host__ __device__ constexpr int rec_bytes(int qt, int mr) { return mr * 256 + rec_p(qt, mr) + rec_scales(qt, mr); }
+// packed activation record of one K step and one tile of kMR rows: codes [row/8][k/16][row%8][16], (Q4_K) sums of 16 codes
+// as f16 [row/8][2][row%8][8], scales f32 [kMR] (Q8_0: [8 blocks][kMR])
+__host__ __device__ constexpr int rec_p(int qt) { return qt == CMLD_Q4_K ? kMR * 32 : 0; }
+__host__ __device__ constexpr int rec_scales(int qt) { return (qt == CMLD_Q8_0 ? 8 : 1) * kMR * 4; }
+__host__ __device__ constexpr int rec_bytes(int qt) { return kMR * 256 + rec_p(qt) + rec_scales(qt); }
 
-// shared memory of one stage (the record's codes and sums fill all 128 rows)
-__host__ __device__ constexpr int a_bytes(int qt, int mr) { return 128 * 256 + rec_p(qt, 128) + rec_scales(qt, mr); }
+// shared memory of one stage of weights
 __host__ __device__ constexpr int b_planes(int qt) { return qt == CMLD_Q8_0 ? 1 : 2; }
 __host__ __device__ constexpr int b_p(int qt, int nw) { return qt == CMLD_Q4_K ? nw * 32 : 0; }
 __host__ __device__ constexpr int b_scales(int qt, int nw) { return (qt == CMLD_Q8_0 ? 8 : qt == CMLD_Q4_K ? 2 : 1) * nw * 4; }
 __host__ __device__ constexpr int b_bytes(int qt, int nw) { return b_planes(qt) * nw * 256 + b_p(qt, nw) + b_scales(qt, nw); }
-// private ring of a weight group: wire bytes (Q6_K: and the words that hold the f16 scales), or the f16 scales of Q8_0
+// ring of the weight warps: wire bytes (Q6_K: and the words that hold the f16 scales), or the f16 scales of Q8_0
 __host__ __device__ constexpr int raw_bytes(int qt, int nw) { return qt == CMLD_Q8_0 ? nw * 16 : nw * (kq_bytes(qt) + (qt == CMLD_Q6_K ? 4 : 0)); }
 // Groups of four warps.  Q8_0's epilogue (16 waits for tensor memory a step, few registers) hides them behind one another with
 // twice the warps: 1B gate and up, 512 rows, 104 -> 93 us per launch on average; Q4_K does not gain (131 -> 147 us: its weight
 // path loses registers), Q6_K has none to spare.
-__host__ __device__ constexpr int epi_groups(int qt, int nw, int mr) { return mr == 32 ? 1 : qt == CMLD_Q8_0 && nw == 64 ? 4 : 2; }
-__host__ __device__ constexpr int weight_groups(int mr) { return mr == 32 ? 2 : 1; }
-__host__ __device__ constexpr int tc_threads(int qt, int nw, int mr) { return 128 * (epi_groups(qt, nw, mr) + weight_groups(mr) + 1); }
-// steps of its own by which a weight group's loads run ahead of their use; its ring holds one more
-__host__ __device__ constexpr int load_ahead(int qt, int nw, int mr) { return qt == CMLD_Q4_K && nw == 64 && mr == 32 ? 1 : 2; }
-__host__ __device__ constexpr int ring_bytes(int qt, int nw, int mr) { return weight_groups(mr) * (load_ahead(qt, nw, mr) + 1) * raw_bytes(qt, nw); }
+__host__ __device__ constexpr int epi_groups(int qt, int nw) { return qt == CMLD_Q8_0 && nw == 64 ? 4 : 2; }
+__host__ __device__ constexpr int tc_threads(int qt, int nw) { return 128 * (epi_groups(qt, nw) + 2); }
+constexpr int kLoadAhead = 2;  // steps by which the loads of weights run ahead of their use; their ring holds one more
+__host__ __device__ constexpr int ring_bytes(int qt, int nw) { return (kLoadAhead + 1) * raw_bytes(qt, nw); }
 
 __host__ __device__ constexpr int acc_groups(int qt) { return qt == CMLD_Q4_K ? 1 : 4; }  // accumulator slots filled per step
 __host__ __device__ constexpr int acc_slots(int qt) { return qt == CMLD_Q4_K ? 2 : 4; }
@@ -226,12 +220,12 @@ __device__ __forceinline__ int tc_tile_job(const TcArgs &a, int t) {
 // One CTA per (K step, eight rows): the quantised activation rows (global layout: codes | f32 scales | i16 sums of 16)
 // rearranged into the records the matrix product's CTAs fetch with bulk copies.  Rows past `batch` are zero.
 template <int QT>
-__global__ void __launch_bounds__(128) tc5_pack_kernel(const uint8_t *act, int64_t cols, int batch, int mr, int m_tiles, uint8_t *pack) {
+__global__ void __launch_bounds__(128) tc5_pack_kernel(const uint8_t *act, int64_t cols, int batch, int m_tiles, uint8_t *pack) {
   __shared__ uint4 codes[8][17];
-  const int ks = blockIdx.x, mt = blockIdx.y / (mr / 8), g = blockIdx.y % (mr / 8), tid = threadIdx.x;
+  const int ks = blockIdx.x, mt = blockIdx.y / (kMR / 8), g = blockIdx.y % (kMR / 8), tid = threadIdx.x;
   const int64_t astride = act_row_stride(cols);
-  const int n0 = mt * mr + g * 8;  // first row of the group
-  uint8_t *rec = pack + ((int64_t)ks * m_tiles + mt) * rec_bytes(QT, mr);
+  const int n0 = mt * kMR + g * 8;  // first row of the group
+  uint8_t *rec = pack + ((int64_t)ks * m_tiles + mt) * rec_bytes(QT);
   {
     const int i = tid >> 4, c = tid & 15;
     codes[i][c] = n0 + i < batch ? *reinterpret_cast<const uint4 *>(act + (n0 + i) * astride + (int64_t)ks * 256 + 16 * c) : make_uint4(0, 0, 0, 0);
@@ -260,13 +254,13 @@ __global__ void __launch_bounds__(128) tc5_pack_kernel(const uint8_t *act, int64
 #pragma unroll
       for (int x = 0; x < 4; ++x) s[x] = __halves2half2(__short2half_rn(b16[2 * x]), __short2half_rn(b16[2 * x + 1]));
     }
-    *reinterpret_cast<uint4 *>(rec + mr * 256 + g * 256 + ch * 128 + i * 16) = *reinterpret_cast<uint4 *>(s);
+    *reinterpret_cast<uint4 *>(rec + kMR * 256 + g * 256 + ch * 128 + i * 16) = *reinterpret_cast<uint4 *>(s);
   }
-  float *sc = reinterpret_cast<float *>(rec + mr * 256 + rec_p(QT, mr));
+  float *sc = reinterpret_cast<float *>(rec + kMR * 256 + rec_p(QT));
   if (tid < (QT == CMLD_Q8_0 ? 64 : 8)) {
     const int j = tid >> 3, i = tid & 7;
     const float *src = reinterpret_cast<const float *>(act + (n0 + i) * astride + act_scale_off(cols));
-    sc[j * mr + g * 8 + i] = n0 + i < batch ? src[QT == CMLD_Q8_0 ? ks * 8 + j : ks] : 0.0f;
+    sc[j * kMR + g * 8 + i] = n0 + i < batch ? src[QT == CMLD_Q8_0 ? ks * 8 + j : ks] : 0.0f;
   }
 }
 
@@ -387,13 +381,12 @@ __device__ __forceinline__ void unpack_q6k(const uint8_t *raw_stage, uint8_t *b,
 
 // ---------------------------------------------------------------- the kernel
 
-template <int QT, int NW, int MR>
-__global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(const TcArgs a) {
-  constexpr bool REP = MR == 32;
-  constexpr int EG = epi_groups(QT, NW, MR), EW = 4 * EG, NUG = weight_groups(MR);  // epilogue warps; groups of four weight warps
-  constexpr int CW = REP ? NW / 4 : NW / EG;            // weight rows of one epilogue thread
-  constexpr int MMA_WARP = EW + 4 * NUG, ACT_WARP = MMA_WARP + 1;
-  constexpr int REC = rec_bytes(QT, MR), AB = a_bytes(QT, MR), BB = b_bytes(QT, NW), RB = raw_bytes(QT, NW);
+template <int QT, int NW>
+__global__ void __launch_bounds__(tc_threads(QT, NW), 1) gemv_tc5_kernel(const TcArgs a) {
+  constexpr int EG = epi_groups(QT, NW), EW = 4 * EG;   // epilogue warps
+  constexpr int CW = NW / EG;                           // weight rows of one epilogue thread
+  constexpr int MMA_WARP = EW + 4, ACT_WARP = MMA_WARP + 1;
+  constexpr int REC = rec_bytes(QT), BB = b_bytes(QT, NW), RB = raw_bytes(QT, NW);
   constexpr int G = acc_groups(QT), NS = acc_slots(QT), SC = slot_cols(QT, NW);
   constexpr uint32_t TCOLS = tmem_cols(QT, NW);
   constexpr int PL = b_planes(QT) * NW * 256;  // bytes of the operand planes
@@ -433,9 +426,9 @@ __global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(con
   tc_fence_after();
   const uint32_t tbase = *tmem_slot;
 
-  // 128 rows: the epilogue threads hold up to 128 sums each and take registers from the other warpgroups
+  // The epilogue threads hold up to 128 sums each and take registers from the other warpgroups
   // (2 x 128 x 184 + 2 x 128 x 72 = the 512 x 128 of the launch).
-  if (!REP && tc_threads(QT, NW, MR) == 512) {
+  if (tc_threads(QT, NW) == 512) {
     if (warp < EW) asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
     else asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   }
@@ -443,8 +436,8 @@ __global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(con
   if (warp < EW) {
     // ------------------------------------------------ epilogue
     const int wg = warp >> 2, quarter = warp & 3;
-    const int m = REP ? lane : quarter * 32 + lane;         // row within the activation tile
-    const int col0 = REP ? quarter * CW : wg * CW;          // first weight row of this thread
+    const int m = quarter * 32 + lane;                      // row within the activation tile
+    const int col0 = wg * CW;                               // first weight row of this thread
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     int sa = 0, sb = 0, pa = 0, pb = 0, slot = 0, pc = 0;
     bool ok = true;
@@ -456,9 +449,9 @@ __global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(con
 #pragma unroll
         for (int l = 0; l < (QT == CMLD_Q6_K ? 8 : 1); ++l) acc[i][l] = 0.0f;
       for (int ks = 0; ks < nks; ++ks) {
-        const uint8_t *as = a_ring + sa * AB;
+        const uint8_t *as = a_ring + sa * REC;
         const uint8_t *bs = b_ring + sb * BB;
-        const float *xs = reinterpret_cast<const float *>(as + 128 * 256 + rec_p(QT, 128)) + m;
+        const float *xs = reinterpret_cast<const float *>(as + kMR * 256 + rec_p(QT)) + m;
         const float *ws = reinterpret_cast<const float *>(bs + PL + b_p(QT, NW)) + col0;
         // the record's bytes arrive through the async proxy and the scales of the weights through other warps: each reader
         // observes their barriers itself (both phases completed before the step's MMAs were issued, and neither is re-armed
@@ -517,7 +510,7 @@ __global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(con
               }
             }
           } else {
-            const float x0 = xs[(2 * g) * MR], x1 = xs[(2 * g + 1) * MR];
+            const float x0 = xs[(2 * g) * kMR], x1 = xs[(2 * g + 1) * kMR];
 #pragma unroll
             for (int u = 0; u < CW; u += 8) {
               int i0[8], i1[8];
@@ -557,7 +550,7 @@ __global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(con
       }
       if (!ok) break;
       const TcJob &J = a.job[tc_tile_job(a, wt)];
-      const int b = mt * MR + m, row0 = (wt - J.first_tile) * NW + col0;
+      const int b = mt * kMR + m, row0 = (wt - J.first_tile) * NW + col0;
       if (b < a.batch) {
         float *y = J.y + (int64_t)b * J.y_stride + row0;
         const float *res = J.residual ? J.residual + (int64_t)b * J.y_stride + row0 : nullptr;
@@ -590,13 +583,13 @@ __global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(con
     }
   } else if (warp < MMA_WARP) {
     // ------------------------------------------------ weight path
-    const int ug = (warp - EW) >> 2, tu = (tid - EW * 32) & 127, wu = tu >> 5;
+    const int tu = tid - EW * 32, wu = tu >> 5;
     constexpr int SEG = QT == CMLD_Q8_0 ? 1 : kq_bytes(QT) / 16;  // 16-byte pieces of a row (Q8_0: its scales of the step)
     constexpr int NP = (NW * SEG + 127) / 128;
-    constexpr int kAhead = load_ahead(QT, NW, MR), RS = kAhead + 1;
-    uint8_t *raw = smem + a.off_raw + ug * RS * RB;
+    constexpr int RS = kLoadAhead + 1;
+    uint8_t *raw = smem + a.off_raw;
     // state of the loads: the step they have reached, its tile, K step and raw stage
-    int lq = ug, l_it = ug / nks, l_ks = ug % nks, l_stage = 0;
+    int lq = 0, l_it = 0, l_ks = 0, l_stage = 0;
     const uint8_t *l_base = nullptr;
     int l_left = 0;
     int64_t l_stride = 0;
@@ -649,28 +642,27 @@ __global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(con
         }
       }
       cp_commit();
-      lq += NUG;
-      l_ks += NUG;
-      while (l_ks >= nks) {
-        l_ks -= nks;
+      ++lq;
+      if (++l_ks == nks) {
+        l_ks = 0;
         ++l_it;
         open_tile();
       }
       if (++l_stage == RS) l_stage = 0;
     };
-    for (int q = 0; q < kAhead; ++q) load_step();
-    int u_ks = ug % nks, stage = 0;
-    for (int q = ug; q < total_steps; q += NUG) {
+    for (int q = 0; q < kLoadAhead; ++q) load_step();
+    int u_ks = 0, stage = 0;
+    for (int q = 0; q < total_steps; ++q) {
       const int st = q % NB;
       uint8_t *b = b_ring + st * BB;
-      cp_wait<kAhead - 1>();  // this thread's pieces of step q have landed
+      cp_wait<kLoadAhead - 1>();  // this thread's pieces of step q have landed
       if (QT != CMLD_Q8_0 && q >= NB && ok) ok = bar_wait(&b_empty[st], (uint32_t)((q / NB - 1) & 1), abort_flag, a.status);
-      // One barrier per step over the group's 128 threads: everybody's pieces of step q are visible, everybody is done
+      // One barrier per step over the 128 threads: everybody's pieces of step q are visible, everybody is done
       // reading the stage that the next load overwrites, and the verdict of the bounded waits is shared.
       uint32_t all_ok;
       asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.and.pred p, %2, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                    : "=r"(all_ok)
-                   : "r"(ok ? 1u : 0u), "r"(1 + ug)
+                   : "r"(ok ? 1u : 0u), "r"(1)
                    : "memory");
       ok = all_ok != 0;
       if (!ok) break;
@@ -690,8 +682,7 @@ __global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(con
       __syncwarp();
       if (lane == 0) bar_arrive(&b_full[st]);
       if (++stage == RS) stage = 0;
-      u_ks += NUG;
-      while (u_ks >= nks) u_ks -= nks;
+      if (++u_ks == nks) u_ks = 0;
     }
     cp_wait<0>();
   } else if (warp == ACT_WARP) {
@@ -702,18 +693,8 @@ __global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(con
         if (q >= NA && !bar_wait(&a_empty[st], (uint32_t)((q / NA - 1) & 1), abort_flag, a.status)) break;
         const int mt = (cta + (q / nks) * n_ctas) % a.m_tiles;
         const uint8_t *src = a.pack + ((int64_t)(q % nks) * a.m_tiles + mt) * REC;
-        const uint32_t dst = s32(a_ring + st * AB);
-        bar_expect_tx(&a_full[st], (uint32_t)AB);
-        if (REP) {  // the 32 rows four times over
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            bulk_load(dst + c * (MR * 256), src, MR * 256, &a_full[st]);
-            if (QT == CMLD_Q4_K) bulk_load(dst + 128 * 256 + c * (MR * 32), src + MR * 256, MR * 32, &a_full[st]);
-          }
-          bulk_load(dst + 128 * 256 + rec_p(QT, 128), src + MR * 256 + rec_p(QT, MR), rec_scales(QT, MR), &a_full[st]);
-        } else {
-          bulk_load(dst, src, AB, &a_full[st]);
-        }
+        bar_expect_tx(&a_full[st], (uint32_t)REC);
+        bulk_load(s32(a_ring + st * REC), src, REC, &a_full[st]);
       }
     }
   } else if (warp == MMA_WARP) {
@@ -724,7 +705,7 @@ __global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(con
       for (int q = 0; q < total_steps && ok; ++q) {
         if (!bar_wait(&a_full[sa], (uint32_t)pa, abort_flag, a.status)) break;
         if (!bar_wait(&b_full[sb], (uint32_t)pb, abort_flag, a.status)) break;
-        const uint32_t a_addr = s32(a_ring + sa * AB), b_addr = s32(b_ring + sb * BB);
+        const uint32_t a_addr = s32(a_ring + sa * REC), b_addr = s32(b_ring + sb * BB);
         constexpr int BR = b_planes(QT) * NW;  // rows of the weight operand
 #pragma unroll
         for (int g = 0; g < G; ++g) {
@@ -739,7 +720,7 @@ __global__ void __launch_bounds__(tc_threads(QT, NW, MR), 1) gemv_tc5_kernel(con
 #pragma unroll
             for (int j = 0; j < 8; ++j)
               mma_i8(d0, smem_desc(a_addr + j * 256, 128, 2048), smem_desc(b_addr + j * 2 * (BR * 16), BR * 16, 128), idesc_i8(BR), j > 0);
-            mma_f16(d0 + 2 * NW, smem_desc(a_addr + 128 * 256, 128, 256), smem_desc(b_addr + PL, NW * 16, 128), idesc_f16(NW));
+            mma_f16(d0 + 2 * NW, smem_desc(a_addr + kMR * 256, 128, 256), smem_desc(b_addr + PL, NW * 16, 128), idesc_f16(NW));
           } else {
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
@@ -769,14 +750,9 @@ int g_tc_sms = 0;
 }  // namespace
 
 static bool tc5_qt_ok(int qt) { return qt == CMLD_Q4_K || qt == CMLD_Q6_K || qt == CMLD_Q8_0; }
-// Rows of an activation tile.  Up to 32 the MR = 32 form is up to a third faster; from 33 on one 128-row tile is faster than two passes
-// of it.  At 32 | 33 | 128 rows: Q4_K 28672 x 4096 68 | 83 | 89 us, Q6_K 4096 x 14336 81 | 107 | 107, Q8_0 16384 x 2048 35 | 46 | 48.
-static int tc5_mr(int32_t batch) { return batch <= 32 ? 32 : 128; }
-
 // Bytes of packed activation records a step of `batch` rows needs for `cols` columns of any type.
 int64_t gemv_tc5_pack_bytes(int64_t cols, int32_t batch) {
-  const int mr = tc5_mr(batch);
-  return cols / 256 * ((batch + mr - 1) / mr) * (int64_t)rec_bytes(CMLD_Q4_K, mr);
+  return cols / 256 * ((batch + kMR - 1) / kMR) * (int64_t)rec_bytes(CMLD_Q4_K);
 }
 
 bool gemv_tc5_fits(const GemvJob *jobs, int n_jobs, int32_t batch) {
@@ -787,10 +763,10 @@ bool gemv_tc5_fits(const GemvJob *jobs, int n_jobs, int32_t batch) {
   return true;
 }
 
-template <int QT, int NW, int MR>
+template <int QT, int NW>
 static int32_t launch_tc(TcArgs &a, const GemvJob *jobs, cudaStream_t s) {
   static SmemLimit limit;
-  CMLD_TRY(allow_smem(limit, gemv_tc5_kernel<QT, NW, MR>, 227 * 1024));
+  CMLD_TRY(allow_smem(limit, gemv_tc5_kernel<QT, NW>, 227 * 1024));
   int tiles = 0;
   for (int i = 0; i < a.n_jobs; ++i) {
     TcJob &J = a.job[i];
@@ -805,18 +781,18 @@ static int32_t launch_tc(TcArgs &a, const GemvJob *jobs, cudaStream_t s) {
   }
   a.w_tiles = tiles;
   constexpr int bar_bytes = 8 * (4 * kTcMaxStages + 8) + 16, a_stages = 3;
-  constexpr int left = 227 * 1024 - bar_bytes - a_stages * a_bytes(QT, MR) - ring_bytes(QT, NW, MR);
+  constexpr int left = 227 * 1024 - bar_bytes - a_stages * rec_bytes(QT) - ring_bytes(QT, NW);
   constexpr int b_stages = std::min(kTcMaxStages, left / b_bytes(QT, NW));
   // Q8_0 loads go straight into the operand ring: it must hold more than the steps that are loaded ahead, or a load would
   // wait for a step that is not yet complete.
-  static_assert(b_stages >= 2 && (QT != CMLD_Q8_0 || b_stages > load_ahead(QT, NW, MR) * weight_groups(MR)), "shared memory");
+  static_assert(b_stages >= 2 && (QT != CMLD_Q8_0 || b_stages > kLoadAhead), "shared memory");
   a.a_stages = a_stages;
   a.b_stages = b_stages;
-  a.off_b = a_stages * a_bytes(QT, MR);
+  a.off_b = a_stages * rec_bytes(QT);
   a.off_raw = a.off_b + b_stages * b_bytes(QT, NW);
-  a.off_bar = (a.off_raw + ring_bytes(QT, NW, MR) + 15) & ~15;
+  a.off_bar = (a.off_raw + ring_bytes(QT, NW) + 15) & ~15;
   const int grid = std::min(tiles * a.m_tiles, g_tc_sms);
-  gemv_tc5_kernel<QT, NW, MR><<<grid, tc_threads(QT, NW, MR), a.off_bar + bar_bytes, s>>>(a);
+  gemv_tc5_kernel<QT, NW><<<grid, tc_threads(QT, NW), a.off_bar + bar_bytes, s>>>(a);
   CMLD_CUDA(cudaGetLastError());
   return CMLD_OK;
 }
@@ -824,20 +800,20 @@ static int32_t launch_tc(TcArgs &a, const GemvJob *jobs, cudaStream_t s) {
 // Matrices of ONE type.  `pack`: room for gemv_tc5_pack_bytes(cols, batch).
 static int32_t launch_tc5_qt(const GemvJob *jobs, int n_jobs, const uint8_t *act, int32_t batch, uint8_t *pack, int32_t *status,
                              cudaStream_t s, int64_t *launches) {
-  const int qt = jobs[0].qt, mr = tc5_mr(batch);
+  const int qt = jobs[0].qt;
   const int64_t cols = jobs[0].cols;
   TcArgs a{};
   a.n_jobs = n_jobs;
   a.nks = (int32_t)(cols / 256);
   a.batch = batch;
-  a.m_tiles = (batch + mr - 1) / mr;
+  a.m_tiles = (batch + kMR - 1) / kMR;
   a.pack = pack;
   a.status = status;
-  const dim3 pg((unsigned)a.nks, (unsigned)(a.m_tiles * (mr / 8)));
+  const dim3 pg((unsigned)a.nks, (unsigned)(a.m_tiles * (kMR / 8)));
   switch (qt) {
-    case CMLD_Q4_K: tc5_pack_kernel<CMLD_Q4_K><<<pg, 128, 0, s>>>(act, cols, batch, mr, a.m_tiles, pack); break;
-    case CMLD_Q6_K: tc5_pack_kernel<CMLD_Q6_K><<<pg, 128, 0, s>>>(act, cols, batch, mr, a.m_tiles, pack); break;
-    default: tc5_pack_kernel<CMLD_Q8_0><<<pg, 128, 0, s>>>(act, cols, batch, mr, a.m_tiles, pack); break;
+    case CMLD_Q4_K: tc5_pack_kernel<CMLD_Q4_K><<<pg, 128, 0, s>>>(act, cols, batch, a.m_tiles, pack); break;
+    case CMLD_Q6_K: tc5_pack_kernel<CMLD_Q6_K><<<pg, 128, 0, s>>>(act, cols, batch, a.m_tiles, pack); break;
+    default: tc5_pack_kernel<CMLD_Q8_0><<<pg, 128, 0, s>>>(act, cols, batch, a.m_tiles, pack); break;
   }
   CMLD_CUDA(cudaGetLastError());
   // Tiles of 64 weight rows, or of 32 where those leave the last wave of CTAs emptier.  A tile of 32 takes about 0.6 of the time of
@@ -851,15 +827,9 @@ static int32_t launch_tc5_qt(const GemvJob *jobs, int n_jobs, const uint8_t *act
   };
   const bool wide = rounds(64) * 5 <= rounds(32) * 3;
   int32_t rc;
-  if (qt == CMLD_Q4_K) {
-    if (mr == 128) rc = wide ? launch_tc<CMLD_Q4_K, 64, 128>(a, jobs, s) : launch_tc<CMLD_Q4_K, 32, 128>(a, jobs, s);
-    else rc = wide ? launch_tc<CMLD_Q4_K, 64, 32>(a, jobs, s) : launch_tc<CMLD_Q4_K, 32, 32>(a, jobs, s);
-  } else if (qt == CMLD_Q6_K) {
-    rc = mr == 128 ? launch_tc<CMLD_Q6_K, 32, 128>(a, jobs, s) : launch_tc<CMLD_Q6_K, 32, 32>(a, jobs, s);
-  } else {
-    if (mr == 128) rc = wide ? launch_tc<CMLD_Q8_0, 64, 128>(a, jobs, s) : launch_tc<CMLD_Q8_0, 32, 128>(a, jobs, s);
-    else rc = wide ? launch_tc<CMLD_Q8_0, 64, 32>(a, jobs, s) : launch_tc<CMLD_Q8_0, 32, 32>(a, jobs, s);
-  }
+  if (qt == CMLD_Q4_K) rc = wide ? launch_tc<CMLD_Q4_K, 64>(a, jobs, s) : launch_tc<CMLD_Q4_K, 32>(a, jobs, s);
+  else if (qt == CMLD_Q6_K) rc = launch_tc<CMLD_Q6_K, 32>(a, jobs, s);
+  else rc = wide ? launch_tc<CMLD_Q8_0, 64>(a, jobs, s) : launch_tc<CMLD_Q8_0, 32>(a, jobs, s);
   CMLD_TRY(rc);
   if (launches) *launches += 2;
   return CMLD_OK;

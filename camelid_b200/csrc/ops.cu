@@ -2,6 +2,7 @@
 // RoPE fused with the f16 KV-cache write, and greedy argmax.
 #include "actquant.cuh"
 #include "exact_sum.cuh"
+#include "rows_record.cuh"
 
 namespace cmld {
 
@@ -65,67 +66,31 @@ __global__ void __launch_bounds__(kNormThreads) norm_quant_kernel(NormQuantArgs 
       }
       v[i] = t;
     }
-    if (a.act_q8_k && e0 < a.cols) {
-      uint8_t *act = a.act + b * astride;
-      float amax = 0.0f, mx = 0.0f;
-      int idx = 0;
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (fabsf(v[i]) > amax) {
-          amax = fabsf(v[i]);
-          mx = v[i];
-          idx = lane * 8 + i;
-        }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float oa = __shfl_xor_sync(0xffffffffu, amax, o);
-        const float om = __shfl_xor_sync(0xffffffffu, mx, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-        if (oa > amax || (oa == amax && oi < idx)) {
-          amax = oa;
-          mx = om;
-          idx = oi;
-        }
-      }
+    if ((a.act_q8_k || a.rec4 || a.rec6) && e0 < a.cols) {
       int q[8];
-      float d = 0.0f;
-      if (amax == 0.0f) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) q[i] = 0;
-      } else {
-        const float iscale = __fdiv_rn(-127.0f, mx);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) q[i] = min(127, __float2int_rn(__fmul_rn(iscale, v[i])));
-        d = __fdiv_rn(1.0f, iscale);
-      }
-      uint2 packed;
-      packed.x = (q[0] & 0xff) | ((q[1] & 0xff) << 8) | ((q[2] & 0xff) << 16) | ((q[3] & 0xff) << 24);
-      packed.y = (q[4] & 0xff) | ((q[5] & 0xff) << 8) | ((q[6] & 0xff) << 16) | ((q[7] & 0xff) << 24);
-      *reinterpret_cast<uint2 *>(act + e0) = packed;
-      int s = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      if ((lane & 1) == 0) reinterpret_cast<short *>(act + act_bsum_off(a.cols))[ch * 16 + (lane >> 1)] = (short)s;
-      if (lane == 0) reinterpret_cast<float *>(act + act_scale_off(a.cols))[ch] = d;
-    }
-    if (a.act_q8_0) {
-      uint8_t *act = (a.act_q8_k ? a.act2 : a.act) + b * astride;
-      float amax = 0.0f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-      const float du = __fdiv_rn(amax, 127.0f);
-      const float inv = du == 0.0f ? 0.0f : __fdiv_rn(1.0f, du);
-      if (e0 < a.cols) {
-        int q[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) q[i] = (int)fminf(fmaxf(roundf(__fmul_rn(v[i], inv)), -128.0f), 127.0f);
-        uint2 packed;
-        packed.x = (q[0] & 0xff) | ((q[1] & 0xff) << 8) | ((q[2] & 0xff) << 16) | ((q[3] & 0xff) << 24);
-        packed.y = (q[4] & 0xff) | ((q[5] & 0xff) << 8) | ((q[6] & 0xff) << 16) | ((q[7] & 0xff) << 24);
+      float d;
+      q8k_quantise_chunk(v, lane, q, d);
+      const uint2 packed = pack8(q);
+      if (a.rec4 || a.rec6) rows_store_k(packed, d, lane, b, ch, (a.batch + 7) >> 3, a.rec4, a.rec6);
+      if (a.act_q8_k) {
+        uint8_t *act = a.act + b * astride;
         *reinterpret_cast<uint2 *>(act + e0) = packed;
-        if ((lane & 3) == 0)
-          reinterpret_cast<float *>(act + act_scale_off(a.cols))[e0 >> 5] = f16_bits_to_f32(f32_to_f16_bits(du));
+        int s = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if ((lane & 1) == 0) reinterpret_cast<short *>(act + act_bsum_off(a.cols))[ch * 16 + (lane >> 1)] = (short)s;
+        if (lane == 0) reinterpret_cast<float *>(act + act_scale_off(a.cols))[ch] = d;
+      }
+    }
+    if (a.act_q8_0 || a.rec0) {
+      int q[8];
+      float scale;
+      q80_quantise_chunk(v, q, scale);
+      const uint2 packed = pack8(q);
+      if (a.rec0) rows_store_0(packed, scale, lane, b, ch, (a.batch + 7) >> 3, a.rec0);
+      if (a.act_q8_0 && e0 < a.cols) {
+        uint8_t *act = (a.act_q8_k ? a.act2 : a.act) + b * astride;
+        *reinterpret_cast<uint2 *>(act + e0) = packed;
+        if ((lane & 3) == 0) reinterpret_cast<float *>(act + act_scale_off(a.cols))[e0 >> 5] = scale;
       }
     }
   }
@@ -133,7 +98,7 @@ __global__ void __launch_bounds__(kNormThreads) norm_quant_kernel(NormQuantArgs 
 
 int32_t launch_norm_quant(const NormQuantArgs &a, cudaStream_t s) {
   if (a.cols % 32 != 0) return fail(CMLD_ERR_SHAPE, "activation width %lld is not a multiple of 32", (long long)a.cols);
-  if (a.act_q8_k && a.cols % 256 != 0)
+  if ((a.act_q8_k || a.rec4 || a.rec6 || a.rec0) && a.cols % 256 != 0)
     return fail(CMLD_ERR_SHAPE, "Q8_K activation width %lld is not a multiple of 256", (long long)a.cols);
   if (a.batch <= 0) return CMLD_OK;
   const int mode = a.x2 ? 2 : (a.weight ? 1 : 0);

@@ -398,8 +398,9 @@ CMLD_API int32_t cmld_sample_uniforms(uint64_t seed, int32_t n, float *out);
  * the CPU dot's bits); bit 1 set = cmld_gemv_time chains its launches with programmatic dependent
  * launch; bit 3 set = batches of 9..32 rows on the int8 mma.sync kernel (one pass over the weights,
  * tree sums: within tolerance, not the CPU's bits), bit 2 set = that kernel from 1 row.
- * Batches of 9 rows and more take the tcgen05 tensor-core kernel by default (one pass over the
- * weights per 2048 rows, the CPU dot's bits); bit 4 set = never, bit 5 set = from 1 row.
+ * By default batches of 3 to 32 rows take the row-batched tensor-core kernel and larger ones the
+ * tcgen05 kernel (one pass over the weights per 2048 rows), both with the CPU dot's bits; bit 4 set
+ * = neither, bit 5 set = the tcgen05 kernel from 1 row.
  * Process-wide; for A/B runs. */
 CMLD_API int32_t cmld_gemv_select_kernel(int32_t choice);
 /* Self-test of the bounded device-side wait of the peer-memory path (no reference counterpart): waits for an

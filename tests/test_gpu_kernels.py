@@ -142,6 +142,73 @@ def test_gemv_matches_checker(cm, orc, name, rows, cols, batch, kernel):
         check(cm.lib().cmld_gemv_select_kernel(0))
 
 
+# The row-batched kernel: both of its forms (a tile of weight rows per warp from five tiles per SM on, and for Q6_K up to eight
+# rows; else the units of a tile spread over the warps), at one unit per row, at units that do not fill a pass of the sixteen
+# warps, and at batches around its groups of eight rows.
+@pytest.mark.parametrize("name,rows,cols", [
+    ("Q8_0", 100, 256), ("Q8_0", 515, 2048), ("Q8_0", 70, 4352), ("Q8_0", 12003, 256),
+    ("Q4_K", 37, 256), ("Q4_K", 300, 3072), ("Q4_K", 64, 14336), ("Q4_K", 12003, 512),
+    ("Q6_K", 33, 256), ("Q6_K", 300, 1792), ("Q6_K", 2500, 4352), ("Q6_K", 12003, 512)])
+@pytest.mark.parametrize("batch", [3, 8, 9, 17, 25, 32])
+def test_gemv_rows_matches_checker(cm, orc, name, rows, cols, batch):
+    """Every output equals the checker's bit for bit, with and without a residual."""
+    from camelid_b200.engine import DeviceBuffer, export_activation, quantize_activation
+
+    qt = QT[name]
+    wire = orc.synth_tensor(qt, 12, rows * 5 + cols, rows, cols, 0.02)
+    w = cm.Weight.from_wire(qt, rows, cols, wire)
+    rng = np.random.default_rng(rows + cols + batch)
+    x = rng.standard_normal((batch, cols)).astype(np.float32)
+    kind = cm.ACT_Q8_0 if qt == 8 else cm.ACT_Q8_K
+    act = quantize_activation(kind, x)
+    codes, scales = export_activation(kind, act, cols, batch)
+    y = w.gemv(act, batch)
+    res = rng.standard_normal((batch, rows)).astype(np.float32)
+    y_res = w.gemv(act, batch, DeviceBuffer.from_numpy(res))
+    for b in range(batch) if rows * cols < 1 << 21 else {0, batch // 2, batch - 1}:
+        ref = orc.matvec_quantised(qt, wire, rows, cols, codes[b], scales[b])
+        bad = np.nonzero(y[b].view(np.uint32) != ref.view(np.uint32))[0]
+        assert bad.size == 0, (name, rows, cols, b, bad[:5], y[b][bad[:5]], ref[bad[:5]])
+        assert np.array_equal(y_res[b], (res[b] + ref).astype(np.float32))
+
+
+@pytest.mark.parametrize("name", ["Q8_0", "Q4_K", "Q6_K"])
+def test_gemv_rows_largest_sums(cm, orc, name):
+    """Codes and scales at the ends of their ranges: integer parts at their bounds (Q4_K: above 2^24, where the conversion rounds;
+    Q6_K: sc * (q - 32) = 4096), and infinite scales, against the checker."""
+    from camelid_b200.engine import export_activation, quantize_activation
+
+    qt, rows, cols = QT[name], 48, 1024
+    blk = {8: 34, 12: 144, 14: 210}[qt]
+    v = np.full((rows, cols // (32 if qt == 8 else 256), blk), 255, np.uint8)
+    scale_at = {8: [0], 12: [0, 2], 14: [208]}[qt]
+    for off in scale_at:
+        v[:, :, off:off + 2] = np.array([0x34, 0x2C], np.uint8)  # f16 0x2C34
+    if qt == 8:
+        v[:, :, 2:] = 0x80  # -128
+        v[1::3, :, 2:] = 0x7F
+    elif qt == 14:
+        v[:, :, :192] = 0  # q = 0
+        v[1::3, :, :192] = 255
+        v[:, :, 192:208] = 0x80  # scale -128
+        v[2::5, :, 192:208] = 0x7F
+    for off in scale_at:
+        v[7, 1, off:off + 2] = np.array([0x00, 0x7C], np.uint8)  # infinity
+    wire = v.reshape(-1)
+    w = cm.Weight.from_wire(qt, rows, cols, wire)
+    rng = np.random.default_rng(5)
+    x = np.where(rng.random((9, cols)) < 0.9, 1.0, -1.0).astype(np.float32)
+    x[3] = 1.0
+    kind = cm.ACT_Q8_0 if qt == 8 else cm.ACT_Q8_K
+    act = quantize_activation(kind, x)
+    codes, scales = export_activation(kind, act, cols, 9)
+    y = w.gemv(act, 9)
+    for b in range(9):
+        ref = orc.matvec_quantised(qt, wire, rows, cols, codes[b], scales[b])
+        same = (y[b].view(np.uint32) == ref.view(np.uint32)) | (np.isnan(y[b]) & np.isnan(ref))
+        assert same.all(), (name, b, np.nonzero(~same)[0][:5], y[b][~same][:5], ref[~same][:5])
+
+
 # The staged kernel's fused prologues: RMSNorm / plain / SwiGLU + quantiser + matvec in one launch
 # equals the three separate steps (same quantised codes, so the same result bit for bit).
 @pytest.mark.parametrize("name,rows,cols", [("Q8_0", 200, 2048), ("Q4_K", 200, 4096), ("Q6_K", 200, 4096), ("Q4_K", 72, 14336),
