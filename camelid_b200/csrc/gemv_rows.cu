@@ -26,14 +26,15 @@
 // with the rows as its 128-row operand A, whichever was the faster | here:
 //   rows                         3 to 8                16              32
 //   Q4_K 28672 x 4096          52 (3) | 19.6      64 | 23.3       67 | 35
-//   Q4_K  4096 x 4096          16 (3) |  8.0      20 |  9.6       20 | 12.8
-//   Q6_K  4096 x 14336         75 (3) | 27        79 | 38         81 | 56
+//   Q4_K  4096 x 4096          16 (3) |  7.9      20 |  9.4       20 | 11.7
+//   Q6_K  4096 x 14336         75 (3) | 24.6      79 | 33         81 | 48
 //   Q8_0 16384 x 2048          30 (3) | 11.2      34 | 13.3       35 | 19.5
 // What bounds it: neither memory (a launch whose weights lie in L2 is 1.3 us shorter) nor one unit of the SM: at eight rows a warp
 // spends 270 instructions on a Q4_K unit and 850 on a Q6_K one (340 of them unpacking, at two cycles each), three or four warps a
 // scheduler, half of the issue slots used; at 32 rows the MMAs (8 cycles each) and the multiply-adds behind them come to the same.
 // Tried and slower: warps that pass the running sums on from unit to unit instead of the terms (600 cycles a hand-over: Q6_K 27 -> 39
-// us), the teams' own warps adding the terms between two barriers (31 us), one bulk copy per weight row and unit in the whole form (the
+// us), the multiplying warps adding the terms themselves between two barriers (31 us) or fetching a
+// weight row each (29.5 us), one bulk copy per weight row and unit in the whole form (the
 // sixteen copies are issued one after another: 20 -> 28 us).
 #include "rows_record.cuh"
 
@@ -480,20 +481,23 @@ __device__ __forceinline__ void next_buf(const RowsArgs &a, Split &s) {
   if (++s.buf == a.bufs) s.buf = 0, s.buf_phase ^= 1;
 }
 
-// The next pass of this CTA's tiles into its stage: a lane per weight row.
+// The next pass of this CTA's tiles into its stage: each of the four adding warps four weight rows, a lane per row.  (A warp's copies are
+// issued one after another, about 60 cycles each: all of a pass by one warp kept the sums waiting.  Us per launch so | here: Q6_K
+// 4096 x 14336 27.1 | 24.6 at 8 rows, 55.8 | 47.7 at 32.)
 template <int QT>
-__device__ __forceinline__ void load_pass(const RowsArgs &a, Split &s, int lane) {
+__device__ __forceinline__ void load_pass(const RowsArgs &a, Split &s, int warp, int lane) {
   if (s.lk >= s.n_mine) return;
   const int tile = s.first + s.lk * s.step;
   const RowsJob &J = a.job[tile_job(a, tile)];
   const int row0 = (tile - J.first_tile) * 16, cnt = min(kWarps, J.units - s.lu);
   constexpr int UB = unit_bytes(QT);
   const int codes = cnt * UB, scales = QT == CMLD_Q4_K ? 0 : QT == CMLD_Q6_K ? (2 * cnt + 15) & ~15 : 8 * cnt;
-  if (lane == 0) bar_expect(&s.landed[s.ls], (uint32_t)(16 * (codes + scales)));
+  if (lane == 0) bar_expect(&s.landed[s.ls], (uint32_t)(4 * (codes + scales)));
   __syncwarp();
-  if (lane < 16) {
-    const uint8_t *row = J.w + (int64_t)min(row0 + lane, J.rows - 1) * J.stride;
-    const uint32_t dst = s32(s.smem + a.off_ring + s.ls * a.stage_bytes) + lane * pass_pitch(QT);
+  if (lane < 4) {
+    const int r = 4 * warp + lane;
+    const uint8_t *row = J.w + (int64_t)min(row0 + r, J.rows - 1) * J.stride;
+    const uint32_t dst = s32(s.smem + a.off_ring + s.ls * a.stage_bytes) + r * pass_pitch(QT);
     bulk_load(dst, row + (int64_t)s.lu * UB, (uint32_t)codes, &s.landed[s.ls]);
     if (scales) bulk_load(dst + kWarps * UB, row + (int64_t)J.units * UB + s.lu * (QT == CMLD_Q6_K ? 2 : 8), (uint32_t)scales, &s.landed[s.ls]);
   }
@@ -591,7 +595,7 @@ __device__ __forceinline__ void split_sums(const RowsArgs &a, const RowsJob &J, 
       if (lane == 0) bar_arrive(&s.empty[s.buf]);
       next_buf(a, s);
       // the pass's last terms were there: nobody reads its stage any more
-      if (x + 1 == HALVES * NT && idx < 32) load_pass<QT>(a, s, lane);
+      if (x + 1 == HALVES * NT) load_pass<QT>(a, s, idx >> 5, lane);
       sum_t v;
 #pragma unroll
       for (int l = 0; l < NL; ++l) reinterpret_cast<float *>(&v)[l] = acc[l];
@@ -627,8 +631,7 @@ __device__ __forceinline__ void split_multiply(const RowsArgs &a, int warp, int 
 }
 template <int QT, int NT>
 __device__ __forceinline__ void split_add(const RowsArgs &a, int warp, int lane, Split &s) {
-  if (warp == 0)
-    for (int i = 0; i < a.stages; ++i) load_pass<QT>(a, s, lane);
+  for (int i = 0; i < a.stages; ++i) load_pass<QT>(a, s, warp, lane);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int k = 0; k < s.n_mine; ++k) {
     const int tile = s.first + k * s.step;
@@ -645,7 +648,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) rows_split_kernel(const __gr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kMaxStages; ++i) {
-      bar_init(&bars[i], 1);
+      bar_init(&bars[i], kSplitWarps - kWarps);
       bar_init(&bars[kMaxStages + i], kWarps);
       bar_init(&bars[2 * kMaxStages + i], kSplitWarps - kWarps);
     }
