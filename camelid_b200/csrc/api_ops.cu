@@ -90,9 +90,12 @@ static int32_t gemv_launch(const cmld_weight *w, const uint8_t *act, int32_t bat
     const int64_t need = gemv_tc5_pack_bytes(w->cols, std::min(batch, kOpTc5Rows));
     uint8_t *pack = reinterpret_cast<uint8_t *>(op_scratch((need + 3) / 4));
     if (!pack) return fail(CMLD_ERR_OOM, "gemv: no room for %lld bytes of packed activations", (long long)need);
+    uint8_t *rec4 = w->qt == CMLD_Q4_K ? pack : nullptr, *rec6 = w->qt == CMLD_Q6_K ? pack : nullptr, *rec0 = w->qt == CMLD_Q8_0 ? pack : nullptr;
     for (int32_t b0 = 0; b0 < batch; b0 += kOpTc5Rows) {
+      const int32_t nb = std::min(batch - b0, kOpTc5Rows);
       const GemvJob j{w->data, w->qt, w->rows, w->cols, w->stride, y + (int64_t)b0 * w->rows, residual ? residual + (int64_t)b0 * w->rows : nullptr, w->rows};
-      CMLD_TRY(launch_gemv_tc5(&j, 1, act + (int64_t)b0 * act_row_stride(w->cols), std::min(batch - b0, kOpTc5Rows), pack, need, op_status(), stream, nullptr));
+      CMLD_TRY(launch_tc5_pack(act + (int64_t)b0 * act_row_stride(w->cols), w->cols, nb, rec4, rec6, rec0, stream));
+      CMLD_TRY(launch_gemv_tc5(&j, 1, nb, rec4, rec6, rec0, op_status(), stream, nullptr));
     }
     return CMLD_OK;
   }

@@ -285,7 +285,8 @@ int32_t launch_gemv_mma(const GemvJob *jobs, int n_jobs, const uint8_t *act, int
 // bit-identical to the one-row kernels (reference order of f32 operations in the epilogue)
 int64_t gemv_tc5_pack_bytes(int64_t cols, int32_t batch);
 bool gemv_tc5_fits(const GemvJob *jobs, int n_jobs, int32_t batch);
-int32_t launch_gemv_tc5(const GemvJob *jobs, int n_jobs, const uint8_t *act, int32_t batch, uint8_t *pack, int64_t pack_bytes,
+int32_t launch_tc5_pack(const uint8_t *act, int64_t cols, int32_t batch, uint8_t *rec4, uint8_t *rec6, uint8_t *rec0, cudaStream_t s);
+int32_t launch_gemv_tc5(const GemvJob *jobs, int n_jobs, int32_t batch, const uint8_t *rec4, const uint8_t *rec6, const uint8_t *rec0,
                         int32_t *status, cudaStream_t s, int64_t *launches);
 
 // gemv_rows.cu: up to 32 activation rows, weights unpacked in the operand registers of mma.sync, the one-row kernels' bits.  The
@@ -314,9 +315,11 @@ struct NormQuantArgs {
   uint8_t *act;         // quantised result or null
   int32_t act_q8_0, act_q8_k;  // which formats to emit; both allowed: Q8_K at act, Q8_0 at act2
   uint8_t *act2;
-  uint8_t *rec4, *rec6, *rec0;  // records of the row-batched matvec instead of (or beside) the rows above; null = not wanted
+  uint8_t *rec4, *rec6, *rec0;  // records of a batched matvec instead of (or beside) the rows above; null = not wanted
+  int32_t rec_tc5;              // they are the tcgen05 kernel's (else the row-batched kernel's)
   int32_t pdl;                 // launch with programmatic stream serialisation
   int32_t exact;               // RMSNorm: add the squares one after another like the CPU (slow)
+  int32_t vec;                 // the f32 operands are 16-byte aligned (set by launch_norm_quant)
 };
 int32_t launch_norm_quant(const NormQuantArgs &a, cudaStream_t s);
 int32_t launch_exact_sum_selftest(const float *terms, int32_t n, float *out, cudaStream_t s);

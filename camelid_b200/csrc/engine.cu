@@ -280,7 +280,7 @@ static int32_t engine_init(cmld_engine *e) {
     const int64_t widest = std::max<int64_t>(std::max<int64_t>(c.hidden, c.ffn_dim), e->q_width);
     const int64_t wide = (widest + 255) / 256 * 256;
     e->tc5_pack_bytes = gemv_tc5_pack_bytes(wide, (int32_t)R);
-    CMLD_TRY(dev_alloc(e, &e->tc5_pack, e->tc5_pack_bytes, false));
+    for (auto &pack : e->tc5_pack) CMLD_TRY(dev_alloc(e, &pack, e->tc5_pack_bytes, false));
     for (auto &rec : e->rows_rec) CMLD_TRY(dev_alloc(e, &rec, gemv_rows_rec_bytes(wide, kRowsMaxBatch), false));
   }
   if (const char *tp = getenv("CMLD_TRACE")) {
@@ -423,7 +423,7 @@ static int32_t run_gemv_group(cmld_engine *e, const Proj *p, int n, int32_t batc
 
 static int32_t run_norm_quant(cmld_engine *e, const float *x, const float *x2, const float *weight, int64_t cols,
                               int32_t batch, float *out, bool need_0, bool need_k, uint8_t *rec4 = nullptr, uint8_t *rec6 = nullptr,
-                              uint8_t *rec0 = nullptr) {
+                              uint8_t *rec0 = nullptr, bool rec_tc5 = false) {
   NormQuantArgs a{};
   a.x = x;
   a.x2 = x2;
@@ -439,6 +439,7 @@ static int32_t run_norm_quant(cmld_engine *e, const float *x, const float *x2, c
   a.rec4 = rec4;
   a.rec6 = rec6;
   a.rec0 = rec0;
+  a.rec_tc5 = rec_tc5;
   a.pdl = !(e->cfg.flags & CMLD_FLAG_NO_PDL);
   a.exact = (e->cfg.flags & CMLD_FLAG_EXACT_ORDER) != 0;
   CMLD_TRY(launch_norm_quant(a, e->stream));
@@ -494,16 +495,15 @@ static int32_t gemv_fused(cmld_engine *e, const Proj *p, int n, int32_t batch, i
       q4 = q4 || jobs[i].qt == CMLD_Q4_K;
       q6 = q6 || jobs[i].qt == CMLD_Q6_K;
     }
-    if (batch <= kRowsMaxBatch && gemv_rows_fits(jobs, n, batch)) {
-      uint8_t *rec4 = q4 ? e->rows_rec[0] : nullptr, *rec6 = q6 ? e->rows_rec[1] : nullptr, *rec0 = n0 ? e->rows_rec[0] : nullptr;
-      CMLD_TRY(run_norm_quant(e, x, mode == 3 ? x2 : nullptr, mode == 1 ? norm_w : nullptr, cols, batch, nullptr, false, false, rec4, rec6, rec0));
+    const bool few = batch <= kRowsMaxBatch;
+    if (few ? gemv_rows_fits(jobs, n, batch) : gemv_tc5_fits(jobs, n, batch) && gemv_tc5_pack_bytes(cols, batch) <= e->tc5_pack_bytes) {
+      uint8_t *const *rec = few ? e->rows_rec : e->tc5_pack;
+      uint8_t *rec4 = q4 ? rec[0] : nullptr, *rec6 = q6 ? rec[1] : nullptr, *rec0 = n0 ? rec[0] : nullptr;
+      CMLD_TRY(run_norm_quant(e, x, mode == 3 ? x2 : nullptr, mode == 1 ? norm_w : nullptr, cols, batch, nullptr, false, false, rec4, rec6, rec0, !few));
+      if (!few) return launch_gemv_tc5(jobs, n, batch, rec4, rec6, rec0, e->d_status, e->stream, &e->launches);
       CMLD_TRY(launch_gemv_rows(jobs, n, batch, rec4, rec6, rec0, e->d_status, e->stream, pdl));
       e->launches += 1;
       return CMLD_OK;
-    }
-    if (batch > kRowsMaxBatch && gemv_tc5_fits(jobs, n, batch) && gemv_tc5_pack_bytes(cols, batch) <= e->tc5_pack_bytes) {
-      CMLD_TRY(run_norm_quant(e, x, mode == 3 ? x2 : nullptr, mode == 1 ? norm_w : nullptr, cols, batch, nullptr, n0, nk));
-      return launch_gemv_tc5(jobs, n, n0 ? e->act_0 : e->act_k, batch, e->tc5_pack, e->tc5_pack_bytes, e->d_status, e->stream, &e->launches);
     }
   }
   if (!(e->cfg.flags & CMLD_FLAG_DIRECT_GEMV) && n <= 3 && batch > mma_min_rows(e) - 1 && !peer && !pair_swiglu && !(n0 && nk)) {

@@ -47,7 +47,7 @@ struct cmld_engine {
   int64_t kv_q8_bytes = 0;                 // bytes of one layer of one side
   uint32_t *tree_mask = nullptr;  // [kTreeMaxNodes] ancestor masks of a draft tree (one word: at most 32 nodes)
   std::vector<float> rope_freq;  // per-pair angular frequency of the engine-owned RoPE table (rope_pair_frequency)
-  uint8_t *tc5_pack = nullptr;   // packed activation records of the tcgen05 batched matvec
+  uint8_t *tc5_pack[2] = {nullptr, nullptr};  // activation records of the tcgen05 batched matvec: Q4_K or Q8_0, Q6_K
   int64_t tc5_pack_bytes = 0;
   uint8_t *rows_rec[2] = {nullptr, nullptr};  // activation records of the row-batched matvec: Q4_K or Q8_0, Q6_K
   int64_t mma_scratch_floats = 0;

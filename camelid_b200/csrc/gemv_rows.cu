@@ -22,20 +22,19 @@
 //                      to give every warp one (4096 rows: 1.7 tiles per SM).  Their operand B comes from L2, asked for one exchange
 //                      ahead.  A launch may hold Q4_K and Q6_K matrices, on CTAs of their own.
 //
-// Measured (us per launch, records from quantised rows included, 2.3; weights beyond L2), the staged kernel in passes or the tcgen05 one
-// with the rows as its 128-row operand A, whichever was the faster | here:
-//   rows                         3 to 8                16              32
-//   Q4_K 28672 x 4096          52 (3) | 19.6      64 | 23.3       67 | 35
-//   Q4_K  4096 x 4096          16 (3) |  7.9      20 |  9.4       20 | 11.7
-//   Q6_K  4096 x 14336         75 (3) | 24.6      79 | 33         81 | 48
-//   Q8_0 16384 x 2048          30 (3) | 11.2      34 | 13.3       35 | 19.5
+// Measured, us per launch (records from quantised rows included, 2.3; weights beyond L2): the staged kernel at 3 and 6 rows and the tcgen05
+// one (the rows four times over as its 128-row operand A) at 16 and 32 | here:
+//   rows                       3              6             16             32
+//   Q4_K 28672 x 4096     27.9 | 19.7    64.6 | 19.7    67.1 | 23.4    68.3 | 35.3
+//   Q4_K  4096 x 4096      8.4 |  7.9    16.3 |  7.9    20.4 |  9.4    20.5 | 11.7
+//   Q6_K  4096 x 14336    33.6 | 24.6    65.9 | 24.6    81.2 | 33.0    81.4 | 47.7
+//   Q8_0 16384 x 2048     26.0 | 11.3    48.3 | 11.3    35.2 | 13.4    35.3 | 19.6
 // What bounds it: neither memory (a launch whose weights lie in L2 is 1.3 us shorter) nor one unit of the SM: at eight rows a warp
 // spends 270 instructions on a Q4_K unit and 850 on a Q6_K one (340 of them unpacking, at two cycles each), three or four warps a
 // scheduler, half of the issue slots used; at 32 rows the MMAs (8 cycles each) and the multiply-adds behind them come to the same.
 // Tried and slower: warps that pass the running sums on from unit to unit instead of the terms (600 cycles a hand-over: Q6_K 27 -> 39
-// us), the multiplying warps adding the terms themselves between two barriers (31 us) or fetching a
-// weight row each (29.5 us), one bulk copy per weight row and unit in the whole form (the
-// sixteen copies are issued one after another: 20 -> 28 us).
+// us), the multiplying warps adding the terms themselves between two barriers (31 us) or fetching a weight row each (29.5 us), one bulk
+// copy per weight row and unit in the whole form (the sixteen copies are issued one after another: 20 -> 28 us).
 #include "rows_record.cuh"
 
 namespace cmld {

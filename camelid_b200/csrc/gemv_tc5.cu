@@ -33,7 +33,7 @@
 // unpacking, 401 with half of the MMAs; Q4_K 28672 x 4096: 276, 229, 227, 266).
 // Every wait is bounded: a wait that runs out sets the status word and an abort flag, all roles leave their loops, tensor
 // memory is freed and the kernel returns.
-#include "common.cuh"
+#include "tc5_record.cuh"
 
 namespace cmld {
 
@@ -42,15 +42,9 @@ namespace {
 constexpr int kTcMaxStages = 8;
 constexpr int kTcPrefetchAhead = 8;  // K steps by which a row's wire bytes are asked into L2 before they are copied
 constexpr uint32_t kTcSpin = 1u << 22;
-constexpr int kMR = 128;  // activation rows of a tile
+constexpr int kMR = kTc5Rows;  // activation rows of a tile
 
 __host__ __device__ constexpr int kq_bytes(int qt) { return qt == CMLD_Q4_K ? 144 : qt == CMLD_Q6_K ? 208 : 256; }  // of a row per K step
-
-// packed activation record of one K step and one tile of kMR rows: codes [row/8][k/16][row%8][16], (Q4_K) sums of 16 codes
-// as f16 [row/8][2][row%8][8], scales f32 [kMR] (Q8_0: [8 blocks][kMR])
-__host__ __device__ constexpr int rec_p(int qt) { return qt == CMLD_Q4_K ? kMR * 32 : 0; }
-__host__ __device__ constexpr int rec_scales(int qt) { return (qt == CMLD_Q8_0 ? 8 : 1) * kMR * 4; }
-__host__ __device__ constexpr int rec_bytes(int qt) { return kMR * 256 + rec_p(qt) + rec_scales(qt); }
 
 // shared memory of one stage of weights
 __host__ __device__ constexpr int b_planes(int qt) { return qt == CMLD_Q8_0 ? 1 : 2; }
@@ -217,51 +211,16 @@ __device__ __forceinline__ int tc_tile_job(const TcArgs &a, int t) {
 
 // ---------------------------------------------------------------- activation packing
 
-// One CTA per (K step, eight rows): the quantised activation rows (global layout: codes | f32 scales | i16 sums of 16)
-// rearranged into the records the matrix product's CTAs fetch with bulk copies.  Rows past `batch` are zero.
-template <int QT>
-__global__ void __launch_bounds__(128) tc5_pack_kernel(const uint8_t *act, int64_t cols, int batch, int m_tiles, uint8_t *pack) {
-  __shared__ uint4 codes[8][17];
-  const int ks = blockIdx.x, mt = blockIdx.y / (kMR / 8), g = blockIdx.y % (kMR / 8), tid = threadIdx.x;
-  const int64_t astride = act_row_stride(cols);
-  const int n0 = mt * kMR + g * 8;  // first row of the group
-  uint8_t *rec = pack + ((int64_t)ks * m_tiles + mt) * rec_bytes(QT);
-  {
-    const int i = tid >> 4, c = tid & 15;
-    codes[i][c] = n0 + i < batch ? *reinterpret_cast<const uint4 *>(act + (n0 + i) * astride + (int64_t)ks * 256 + 16 * c) : make_uint4(0, 0, 0, 0);
-  }
-  __syncthreads();
-  {
-    const int c = tid >> 3, i = tid & 7;
-    uint4 v;
-    if (QT == CMLD_Q6_K) {  // MMA l takes the values with index = l mod 8: chunk 2l + h holds the sixteen of half h
-      const uint8_t *src = reinterpret_cast<const uint8_t *>(codes[i]) + 128 * (c & 1) + (c >> 1);
-      uint32_t w[4];
-#pragma unroll
-      for (int x = 0; x < 4; ++x)
-        w[x] = (uint32_t)src[32 * x] | (uint32_t)src[32 * x + 8] << 8 | (uint32_t)src[32 * x + 16] << 16 | (uint32_t)src[32 * x + 24] << 24;
-      v = make_uint4(w[0], w[1], w[2], w[3]);
-    } else {
-      v = codes[i][c];
-    }
-    *reinterpret_cast<uint4 *>(rec + g * 2048 + c * 128 + i * 16) = v;
-  }
-  if (QT == CMLD_Q4_K && tid < 16) {
-    const int ch = tid >> 3, i = tid & 7;
-    __half2 s[4] = {};
-    if (n0 + i < batch) {
-      const int16_t *b16 = reinterpret_cast<const int16_t *>(act + (n0 + i) * astride + act_bsum_off(cols)) + ks * 16 + ch * 8;
-#pragma unroll
-      for (int x = 0; x < 4; ++x) s[x] = __halves2half2(__short2half_rn(b16[2 * x]), __short2half_rn(b16[2 * x + 1]));
-    }
-    *reinterpret_cast<uint4 *>(rec + kMR * 256 + g * 256 + ch * 128 + i * 16) = *reinterpret_cast<uint4 *>(s);
-  }
-  float *sc = reinterpret_cast<float *>(rec + kMR * 256 + rec_p(QT));
-  if (tid < (QT == CMLD_Q8_0 ? 64 : 8)) {
-    const int j = tid >> 3, i = tid & 7;
-    const float *src = reinterpret_cast<const float *>(act + (n0 + i) * astride + act_scale_off(cols));
-    sc[j * kMR + g * 8 + i] = n0 + i < batch ? src[QT == CMLD_Q8_0 ? ks * 8 + j : ks] : 0.0f;
-  }
+// Quantised rows in the global layout (codes | f32 scales | i16 sums of 16) rearranged into records: a warp per row and K step.
+__global__ void __launch_bounds__(256) tc5_pack_kernel(const uint8_t *act, int64_t cols, int tiles, uint8_t *rec4, uint8_t *rec6, uint8_t *rec0) {
+  const int lane = threadIdx.x & 31, b = blockIdx.y;
+  const int64_t ch = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (ch >= cols / 256) return;
+  const uint8_t *row = act + b * act_row_stride(cols);
+  const uint2 pk = *reinterpret_cast<const uint2 *>(row + ch * 256 + lane * 8);
+  const float *scales = reinterpret_cast<const float *>(row + act_scale_off(cols));
+  if (rec0) tc5_store_0(pk, scales[ch * 8 + (lane >> 2)], lane, b, ch, tiles, rec0);
+  else tc5_store_k(pk, scales[ch], lane, b, ch, tiles, rec4, rec6);
 }
 
 // ---------------------------------------------------------------- weight path
@@ -386,7 +345,7 @@ __global__ void __launch_bounds__(tc_threads(QT, NW), 1) gemv_tc5_kernel(const T
   constexpr int EG = epi_groups(QT, NW), EW = 4 * EG;   // epilogue warps
   constexpr int CW = NW / EG;                           // weight rows of one epilogue thread
   constexpr int MMA_WARP = EW + 4, ACT_WARP = MMA_WARP + 1;
-  constexpr int REC = rec_bytes(QT), BB = b_bytes(QT, NW), RB = raw_bytes(QT, NW);
+  constexpr int REC = tc5_rec(QT), BB = b_bytes(QT, NW), RB = raw_bytes(QT, NW);
   constexpr int G = acc_groups(QT), NS = acc_slots(QT), SC = slot_cols(QT, NW);
   constexpr uint32_t TCOLS = tmem_cols(QT, NW);
   constexpr int PL = b_planes(QT) * NW * 256;  // bytes of the operand planes
@@ -451,7 +410,7 @@ __global__ void __launch_bounds__(tc_threads(QT, NW), 1) gemv_tc5_kernel(const T
       for (int ks = 0; ks < nks; ++ks) {
         const uint8_t *as = a_ring + sa * REC;
         const uint8_t *bs = b_ring + sb * BB;
-        const float *xs = reinterpret_cast<const float *>(as + kMR * 256 + rec_p(QT)) + m;
+        const float *xs = reinterpret_cast<const float *>(as + kMR * 256 + tc5_rec_p(QT)) + m;
         const float *ws = reinterpret_cast<const float *>(bs + PL + b_p(QT, NW)) + col0;
         // the record's bytes arrive through the async proxy and the scales of the weights through other warps: each reader
         // observes their barriers itself (both phases completed before the step's MMAs were issued, and neither is re-armed
@@ -752,7 +711,7 @@ int g_tc_sms = 0;
 static bool tc5_qt_ok(int qt) { return qt == CMLD_Q4_K || qt == CMLD_Q6_K || qt == CMLD_Q8_0; }
 // Bytes of packed activation records a step of `batch` rows needs for `cols` columns of any type.
 int64_t gemv_tc5_pack_bytes(int64_t cols, int32_t batch) {
-  return cols / 256 * ((batch + kMR - 1) / kMR) * (int64_t)rec_bytes(CMLD_Q4_K);
+  return cols / 256 * ((batch + kMR - 1) / kMR) * (int64_t)tc5_rec(CMLD_Q4_K);
 }
 
 bool gemv_tc5_fits(const GemvJob *jobs, int n_jobs, int32_t batch) {
@@ -781,14 +740,14 @@ static int32_t launch_tc(TcArgs &a, const GemvJob *jobs, cudaStream_t s) {
   }
   a.w_tiles = tiles;
   constexpr int bar_bytes = 8 * (4 * kTcMaxStages + 8) + 16, a_stages = 3;
-  constexpr int left = 227 * 1024 - bar_bytes - a_stages * rec_bytes(QT) - ring_bytes(QT, NW);
+  constexpr int left = 227 * 1024 - bar_bytes - a_stages * tc5_rec(QT) - ring_bytes(QT, NW);
   constexpr int b_stages = std::min(kTcMaxStages, left / b_bytes(QT, NW));
   // Q8_0 loads go straight into the operand ring: it must hold more than the steps that are loaded ahead, or a load would
   // wait for a step that is not yet complete.
   static_assert(b_stages >= 2 && (QT != CMLD_Q8_0 || b_stages > kLoadAhead), "shared memory");
   a.a_stages = a_stages;
   a.b_stages = b_stages;
-  a.off_b = a_stages * rec_bytes(QT);
+  a.off_b = a_stages * tc5_rec(QT);
   a.off_raw = a.off_b + b_stages * b_bytes(QT, NW);
   a.off_bar = (a.off_raw + ring_bytes(QT, NW) + 15) & ~15;
   const int grid = std::min(tiles * a.m_tiles, g_tc_sms);
@@ -797,25 +756,16 @@ static int32_t launch_tc(TcArgs &a, const GemvJob *jobs, cudaStream_t s) {
   return CMLD_OK;
 }
 
-// Matrices of ONE type.  `pack`: room for gemv_tc5_pack_bytes(cols, batch).
-static int32_t launch_tc5_qt(const GemvJob *jobs, int n_jobs, const uint8_t *act, int32_t batch, uint8_t *pack, int32_t *status,
-                             cudaStream_t s, int64_t *launches) {
+// Matrices of ONE type; `pack`: their records.
+static int32_t launch_tc5_qt(const GemvJob *jobs, int n_jobs, int32_t batch, const uint8_t *pack, int32_t *status, cudaStream_t s) {
   const int qt = jobs[0].qt;
-  const int64_t cols = jobs[0].cols;
   TcArgs a{};
   a.n_jobs = n_jobs;
-  a.nks = (int32_t)(cols / 256);
+  a.nks = (int32_t)(jobs[0].cols / 256);
   a.batch = batch;
   a.m_tiles = (batch + kMR - 1) / kMR;
   a.pack = pack;
   a.status = status;
-  const dim3 pg((unsigned)a.nks, (unsigned)(a.m_tiles * (kMR / 8)));
-  switch (qt) {
-    case CMLD_Q4_K: tc5_pack_kernel<CMLD_Q4_K><<<pg, 128, 0, s>>>(act, cols, batch, a.m_tiles, pack); break;
-    case CMLD_Q6_K: tc5_pack_kernel<CMLD_Q6_K><<<pg, 128, 0, s>>>(act, cols, batch, a.m_tiles, pack); break;
-    default: tc5_pack_kernel<CMLD_Q8_0><<<pg, 128, 0, s>>>(act, cols, batch, a.m_tiles, pack); break;
-  }
-  CMLD_CUDA(cudaGetLastError());
   // Tiles of 64 weight rows, or of 32 where those leave the last wave of CTAs emptier.  A tile of 32 takes about 0.6 of the time of
   // one of 64 (it repeats the step's hand-offs for half of the rows), hence 3 rounds against 5.  Us with 32 | 64: Q4_K 28672 x 4096, 512
   // rows, 383 | 276; Q4_K 4096 x 4096 67 | 48, and at 128 rows, one round either way, 21.8 | 26.9; Q8_0 2048 x 8192 at 512 rows 110 | 85,
@@ -830,18 +780,21 @@ static int32_t launch_tc5_qt(const GemvJob *jobs, int n_jobs, const uint8_t *act
   if (qt == CMLD_Q4_K) rc = wide ? launch_tc<CMLD_Q4_K, 64>(a, jobs, s) : launch_tc<CMLD_Q4_K, 32>(a, jobs, s);
   else if (qt == CMLD_Q6_K) rc = launch_tc<CMLD_Q6_K, 32>(a, jobs, s);
   else rc = wide ? launch_tc<CMLD_Q8_0, 64>(a, jobs, s) : launch_tc<CMLD_Q8_0, 32>(a, jobs, s);
-  CMLD_TRY(rc);
-  if (launches) *launches += 2;
+  return rc;
+}
+
+int32_t launch_tc5_pack(const uint8_t *act, int64_t cols, int32_t batch, uint8_t *rec4, uint8_t *rec6, uint8_t *rec0, cudaStream_t s) {
+  // (grid.y, the rows, is at most 65535: the callers' passes are of 2048)
+  tc5_pack_kernel<<<dim3((unsigned)((cols / 256 + 7) / 8), (unsigned)batch), 256, 0, s>>>(act, cols, (batch + kMR - 1) / kMR, rec4, rec6, rec0);
+  CMLD_CUDA(cudaGetLastError());
   return CMLD_OK;
 }
 
-// `act`: the quantised activation rows in the global layout (Q8_0 rows for Q8_0 matrices, Q8_K rows otherwise).  `pack`:
-// scratch of gemv_tc5_pack_bytes(cols, batch) bytes, overwritten by every call.  Matrices of different types are served by
-// one launch per type.  CMLD_ERR_UNSUPPORTED (no message) when the shapes do not fit.
-int32_t launch_gemv_tc5(const GemvJob *jobs, int n_jobs, const uint8_t *act, int32_t batch, uint8_t *pack, int64_t pack_bytes,
+// The records: rec4 for Q4_K matrices, rec6 for Q6_K, rec0 for Q8_0 (those of the types that occur), gemv_tc5_pack_bytes(cols, batch)
+// each.  Matrices of different types are served by one launch per type.  CMLD_ERR_UNSUPPORTED (no message) when the shapes do not fit.
+int32_t launch_gemv_tc5(const GemvJob *jobs, int n_jobs, int32_t batch, const uint8_t *rec4, const uint8_t *rec6, const uint8_t *rec0,
                         int32_t *status, cudaStream_t s, int64_t *launches) {
   if (!gemv_tc5_fits(jobs, n_jobs, batch)) return CMLD_ERR_UNSUPPORTED;
-  if (!act || !pack || pack_bytes < gemv_tc5_pack_bytes(jobs[0].cols, batch)) return CMLD_ERR_UNSUPPORTED;
   if (g_tc_sms == 0) {
     int dev = 0;
     CMLD_CUDA(cudaGetDevice(&dev));
@@ -850,14 +803,18 @@ int32_t launch_gemv_tc5(const GemvJob *jobs, int n_jobs, const uint8_t *act, int
   bool done[3] = {false, false, false};
   for (int i = 0; i < n_jobs; ++i) {
     if (done[i]) continue;
+    const int qt = jobs[i].qt;
     GemvJob same[3];
     int n = 0;
     for (int k = i; k < n_jobs; ++k)
-      if (!done[k] && jobs[k].qt == jobs[i].qt) {
+      if (!done[k] && jobs[k].qt == qt) {
         same[n++] = jobs[k];
         done[k] = true;
       }
-    CMLD_TRY(launch_tc5_qt(same, n, act, batch, pack, status, s, launches));
+    const uint8_t *rec = qt == CMLD_Q4_K ? rec4 : qt == CMLD_Q6_K ? rec6 : rec0;
+    if (!rec) return fail(CMLD_ERR_INVALID, "gemv: activation records missing");
+    CMLD_TRY(launch_tc5_qt(same, n, batch, rec, status, s));
+    if (launches) *launches += 1;
   }
   return CMLD_OK;
 }

@@ -3,6 +3,7 @@
 #include "actquant.cuh"
 #include "exact_sum.cuh"
 #include "rows_record.cuh"
+#include "tc5_record.cuh"
 
 namespace cmld {
 
@@ -16,8 +17,23 @@ namespace cmld {
 //        its sign, iscale = -127/max, q = min(127, rne(iscale*v)), d = 1/iscale;
 //   Q8_0 (quantize_q8_0_block, src/inference.rs:22510-22528): d = amax/127 kept as its f16
 //        rounding, q = round-half-away(v * (1/d_unrounded)) clamped to [-128,127].
+// The quantised values go out as plain rows or straight as the records of a batched matvec (rows_record.cuh, tc5_record.cuh): the
+// kernel that rearranged rows into records took 3 to 4 us per product of a prompt step.  With 16-byte loads (a lane's eight values lie
+// together) SwiGLU of 512 x 14336 takes 29.4 us, 39.0 before; the norm of 512 x 4096, one CTA per row, 15.7, 18.4 before.
 constexpr int kNormThreads = 256;
+constexpr int kNormOneCta = 148;  // rows from which a row's norm is one CTA's work
 constexpr int kNormMaxExact = 8192;  // widest row whose squares are summed by all warps (exact_sum.cuh); wider rows by one thread
+
+// Eight consecutive values; vec: 16-byte aligned.
+__device__ __forceinline__ void load8(const float *p, bool vec, float (&v)[8]) {
+  if (vec) {
+    const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = p[i];
+  }
+}
 
 template <int MODE>  // 0 plain, 1 rmsnorm, 2 swiglu
 __global__ void __launch_bounds__(kNormThreads) norm_quant_kernel(NormQuantArgs a) {
@@ -51,27 +67,37 @@ __global__ void __launch_bounds__(kNormThreads) norm_quant_kernel(NormQuantArgs 
   // every CTA of a row repeats the mean-square (cheap) and quantises its own 256-value chunks
   for (int64_t ch = (int64_t)blockIdx.x * nwarps + warp; ch < n_chunks; ch += (int64_t)gridDim.x * nwarps) {
     const int64_t e0 = ch * 256 + lane * 8;
-    float v[8];
+    float v[8] = {};
+    if (e0 < a.cols) {  // (a width is a multiple of 32: all eight or none)
+      float u[8];
+      load8(x + e0, a.vec, v);
+      if (MODE == 1) load8(a.weight + e0, a.vec, u);
+      if (MODE == 2) load8(x2 + e0, a.vec, u);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int64_t e = e0 + i;
-      float t = 0.0f;
-      if (e < a.cols) {
-        if (MODE == 1) t = __fmul_rn(__fmul_rn(x[e], scale), a.weight[e]);
-        else if (MODE == 2) {
-          const float g = x[e];
-          t = swiglu_flat(g, x2[e]);
-        } else t = x[e];
-        if (a.out) a.out[(int64_t)b * a.cols + e] = t;
+      for (int i = 0; i < 8; ++i) {
+        if (MODE == 1) v[i] = __fmul_rn(__fmul_rn(v[i], scale), u[i]);
+        if (MODE == 2) v[i] = swiglu_flat(v[i], u[i]);
       }
-      v[i] = t;
+      if (a.out) {
+        float *o = a.out + (int64_t)b * a.cols + e0;
+        if (a.vec) {
+          reinterpret_cast<float4 *>(o)[0] = make_float4(v[0], v[1], v[2], v[3]);
+          reinterpret_cast<float4 *>(o)[1] = make_float4(v[4], v[5], v[6], v[7]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] = v[i];
+        }
+      }
     }
     if ((a.act_q8_k || a.rec4 || a.rec6) && e0 < a.cols) {
       int q[8];
       float d;
       q8k_quantise_chunk(v, lane, q, d);
       const uint2 packed = pack8(q);
-      if (a.rec4 || a.rec6) rows_store_k(packed, d, lane, b, ch, (a.batch + 7) >> 3, a.rec4, a.rec6);
+      if (a.rec4 || a.rec6) {
+        if (a.rec_tc5) tc5_store_k(packed, d, lane, b, ch, (a.batch + kTc5Rows - 1) / kTc5Rows, a.rec4, a.rec6);
+        else rows_store_k(packed, d, lane, b, ch, (a.batch + 7) >> 3, a.rec4, a.rec6);
+      }
       if (a.act_q8_k) {
         uint8_t *act = a.act + b * astride;
         *reinterpret_cast<uint2 *>(act + e0) = packed;
@@ -86,7 +112,10 @@ __global__ void __launch_bounds__(kNormThreads) norm_quant_kernel(NormQuantArgs 
       float scale;
       q80_quantise_chunk(v, q, scale);
       const uint2 packed = pack8(q);
-      if (a.rec0) rows_store_0(packed, scale, lane, b, ch, (a.batch + 7) >> 3, a.rec0);
+      if (a.rec0) {
+        if (a.rec_tc5) tc5_store_0(packed, scale, lane, b, ch, (a.batch + kTc5Rows - 1) / kTc5Rows, a.rec0);
+        else rows_store_0(packed, scale, lane, b, ch, (a.batch + 7) >> 3, a.rec0);
+      }
       if (a.act_q8_0 && e0 < a.cols) {
         uint8_t *act = (a.act_q8_k ? a.act2 : a.act) + b * astride;
         *reinterpret_cast<uint2 *>(act + e0) = packed;
@@ -96,7 +125,9 @@ __global__ void __launch_bounds__(kNormThreads) norm_quant_kernel(NormQuantArgs 
   }
 }
 
-int32_t launch_norm_quant(const NormQuantArgs &a, cudaStream_t s) {
+int32_t launch_norm_quant(const NormQuantArgs &args, cudaStream_t s) {
+  NormQuantArgs a = args;
+  a.vec = ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.x2) | reinterpret_cast<uintptr_t>(a.weight) | reinterpret_cast<uintptr_t>(a.out)) & 15) == 0;
   if (a.cols % 32 != 0) return fail(CMLD_ERR_SHAPE, "activation width %lld is not a multiple of 32", (long long)a.cols);
   if ((a.act_q8_k || a.rec4 || a.rec6 || a.rec0) && a.cols % 256 != 0)
     return fail(CMLD_ERR_SHAPE, "Q8_K activation width %lld is not a multiple of 256", (long long)a.cols);
@@ -104,7 +135,9 @@ int32_t launch_norm_quant(const NormQuantArgs &a, cudaStream_t s) {
   const int mode = a.x2 ? 2 : (a.weight ? 1 : 0);
   const int64_t n_chunks = (a.cols + 255) >> 8;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)((n_chunks + kNormThreads / 32 - 1) / (kNormThreads / 32)), (unsigned)a.batch);
+  // A norm's CTAs each repeat the row's sum, so many rows get one CTA each; a few share the machine better in more.
+  const int64_t row_ctas = mode == 1 && a.batch >= kNormOneCta ? 1 : (n_chunks + kNormThreads / 32 - 1) / (kNormThreads / 32);
+  cfg.gridDim = dim3((unsigned)row_ctas, (unsigned)a.batch);
   cfg.blockDim = dim3(kNormThreads);
   cfg.stream = s;
   if (mode == 1 && a.cols % 256 == 0 && a.cols <= kNormMaxExact) cfg.dynamicSmemBytes = (size_t)a.cols * 4 + xsum::workspace_bytes((int)a.cols);
