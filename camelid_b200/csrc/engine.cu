@@ -160,16 +160,18 @@ int32_t init_rows(cmld_engine *e, int64_t rows, int64_t logit_rows, int64_t voca
 }
 
 // Rows of one step of a prompt.  The batched matrix product shares an unpacked weight among 128 rows and reads it once for
-// all rows of a step, so a prompt goes in by steps of up to 512 rows where that product takes the shapes.  Four layers, 1024 tokens
-// of the 8B width (Q4_K_M), in steps of 128 | 256 | 384 | 512 | 1024 rows: 14.2 | 11.8 | 11.3 | 10.1 | 9.4 ms; 1500 tokens of the 1B
-// width (Q8_0): 13.4 | 9.7 | 8.7 | 8.0 | 7.7 ms: each doubling gives less, while the scratch rows, which every engine holds, double
-// too.  The experts of a Mixtral shape share an unpacked weight among a step's rows likewise.  Everything else: 32 rows, the rows of those modes' own products and attention (the
-// attention over a Q8_0 cache has a CTA for every row and head, the split-range one scratch for the rows of a listed step).
+// all rows of a step, so a prompt goes in by steps of up to 1024 rows where that product takes the shapes.  Four layers, in steps of
+// 512 | 768 | 1024 | 1536 rows, us: 1024 tokens of the 8B width (Q4_K_M) 9589 | 9799 | 8962 | 8964; 1000 of the 3B width 5963 | 5771 |
+// 5298 | 5295; 600 of it in Q8_0 4650 | 3779 | 3778 | 3773; 1500 of the 1B width (Q8_0) 7755 | 7992 | 7560 | 7538: longer steps only
+// add to the scratch rows, which every engine holds (1024 rows of the 8B width: 0.2 GB).  The experts of a Mixtral shape share an
+// unpacked weight among a step's rows likewise (600 tokens, two layers: 34.6 | 32.2 | 32.2 | 32.4 ms).  Everything else: 32 rows, the
+// rows of those modes' own products and attention (the attention over a Q8_0 cache has a CTA for every row and head, the split-range
+// one scratch for the rows of a listed step).
 static int32_t prompt_rows(const cmld_engine *e) {
   const cmld_config &c = e->cfg;
   const uint32_t other = CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV | CMLD_FLAG_TENSOR_BATCH | CMLD_FLAG_FAST_ORDER | CMLD_FLAG_KV_Q8_0;
   if (((uint32_t)c.flags & other) || c.hidden % 256 || c.ffn_dim % 256 || (c.n_heads * c.head_dim) % 256) return kShortRows;
-  return (int32_t)std::min<int64_t>(512, ((int64_t)c.max_pos + 31) / 32 * 32);
+  return (int32_t)std::min<int64_t>(1024, ((int64_t)c.max_pos + 31) / 32 * 32);
 }
 
 static int32_t engine_init(cmld_engine *e) {

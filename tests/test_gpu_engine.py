@@ -280,10 +280,10 @@ def test_moe_prompts_on_a_wide_shape(cm, orc, qt):
         assert token == orc.argmax(want[n - 1])
 
 
-@pytest.mark.parametrize("n", [150, 600])  # one long step; two, the first of 512 rows
+@pytest.mark.parametrize("n", [150, 600])  # one long step
 def test_logits_of_long_steps_by_row(cm, orc, n):
     """The rows of a long step whose logits are asked for are gathered 32 at a time: more of them than one pass takes, lists with
-    and without the last token (whose greedy token is returned either way), none at all, places in two steps; and the draw from
+    and without the last token (whose greedy token is returned either way), none at all; and the draw from
     the logits of the last token afterwards."""
     cfg = cm.EngineConfig(n_layers=2, n_heads=8, n_kv_heads=4, head_dim=64, hidden=256, ffn_dim=512, vocab=512, max_pos=640)
     pair = ModelPair(cfg, "q4_k_m", seed=61)
@@ -300,8 +300,25 @@ def test_logits_of_long_steps_by_row(cm, orc, n):
         assert eng.sample(1e-6, 7) == token, want  # so cold that the draw is the greedy token
 
 
+def test_prompt_of_two_long_steps(cm, orc):
+    """1100 tokens: steps of 1024 and 76 rows.  Logits at places in both, and the K/V rows, are the checker's."""
+    n = 1100
+    cfg = cm.EngineConfig(n_layers=2, n_heads=8, n_kv_heads=4, head_dim=64, hidden=256, ffn_dim=512, vocab=512, max_pos=1152)
+    pair = ModelPair(cfg, "q4_k_m", seed=63)
+    eng, ref = pair.engine, pair.oracle
+    prompt = orc.synth_tokens(9, 1, n, cfg.vocab)
+    all_logits = np.stack([ref.forward(ref.embedding(int(t)), pos)[0] for pos, t in enumerate(prompt)])
+    for want in ([0, 127, 128, 1023, 1024, 1099], [500], list(range(1000, 1060)), []):
+        token, logits = eng.extend(0, prompt, 0, want=want)
+        assert np.array_equal(logits.view(np.uint32), all_logits[want].view(np.uint32)), want
+        assert token == orc.argmax(all_logits[n - 1]), want
+    for layer in range(cfg.n_layers):
+        for got, kept in zip(eng.read_kv_layer(layer, n), ref.read_kv_layer(layer, n)):
+            assert np.array_equal(got, kept), layer
+
+
 def test_long_prefill_from_embeddings_leaves_the_serial_kv(cm, orc):
-    """Embedding rows in, long steps of 512 and 88 rows and a start past row 0: the K/V rows are the checker's."""
+    """Embedding rows in, a long step and a start past row 0: the K/V rows are the checker's."""
     cfg = cm.EngineConfig(n_layers=2, n_heads=8, n_kv_heads=4, head_dim=64, hidden=256, ffn_dim=512, vocab=512, max_pos=640)
     pair = ModelPair(cfg, "q4_k_m", seed=62)
     eng, ref = pair.engine, pair.oracle
