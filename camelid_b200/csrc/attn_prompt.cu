@@ -1,16 +1,18 @@
-// Reference-order attention for long steps of one sequence (prompts): a CTA serves R neighbouring rows x the G query heads of
-// one KV head, M = R * G queries, so that a key or value is read, widened to f32 and brought to shared memory once for all of
-// them.  The same f32 operations in the same order as the other reference-order kernels (attention_context_for_head,
-// src/inference.rs:30287-30466):
+// Reference-order attention for long steps of one sequence (prompts).  The same f32 operations in the same order as the other
+// reference-order kernels (attention_context_for_head, src/inference.rs:30287-30466):
 //   score_p = (sum over d, in order, of q_d * k_pd) * scale;  e_p = expf(score_p - max);  sum = e_0 + e_1 + ... in position
 //   order;  w_p = e_p * (1 / sum);  out_d = ((0 + w_0 * v_0d) + w_1 * v_1d) + ...
-// Both products are outer-product tiles, every output a chain of its own: scores 128 positions x M queries with the head
-// dimension running, outputs HD dimensions x M queries with the positions running; a thread holds W x A of them (W = 8 or 4
-// positions or dimensions) and multiplies and adds two at a time.  Bound by the FP32 units (a multiplication and an addition per term); keys and
-// values travel through registers into two buffers of 16 terms, one barrier per 16.
-// attn_rows_kernel, one CTA per row, reads a key from shared memory for every head and row and widens it each time.
-// Per layer and step of 512 rows: 8B width, prompt of 1024 tokens 503 -> 249 us (the FP32 units' share is 119 us), 1B width,
-// 1500 tokens 381 -> 254 us, 8B width from position 1500 on 2160 -> 1180 us, from 3500 on 5180 -> 3510 us.
+// A block of 64 queries is R neighbouring rows x the G query heads of a KV head.  Three kernels, the scores between them in memory
+// (a scratch of the engine's, most of it still in L2 when it is read):
+//   prompt_scores_kernel   64 queries x 128 positions per CTA, the head dimension running; a thread holds 8 x 8 scores
+//   prompt_weights_kernel  a CTA per block: maxima, exponentials in place, each query's sum by one thread in position order
+//   prompt_values_kernel   64 queries x 64 dimensions per CTA, the positions running; a thread holds 8 x 4 outputs
+// Both products are outer-product tiles, every output a chain of its own, multiplied and added two at a time; they are bound by the
+// FP32 units (a multiplication and an addition per term, and 64 or 32 of them per three or four loads from shared memory).
+// One kernel that kept a block's scores in shared memory instead (16 queries, two CTAs of four warps per SM) left the FP32 units idle
+// for half of the time.  Us of attention, that | this: 1024 tokens of the 8B width, 4 layers, 1992 | 1454 (scores 702, weights 163, values
+// 589; the FP32 units' share of the products is 956); 1500 tokens of the 1B width 3040 | 2007; 333 tokens of the 3B width from
+// position 700 on 1097 | 785.  What is left: the last CTAs of the scores (a CTA takes 26 us), the widening of keys and values.
 #include "common.cuh"
 #include "expf_exact.cuh"
 #include "packed_f32.cuh"
@@ -19,319 +21,354 @@ namespace cmld {
 
 namespace {
 
-constexpr int kPromptTile = 128;  // positions per tile of scores
-constexpr int kPromptK = 16;      // terms per buffer
+constexpr int kQ = 64;        // queries of a block
+constexpr int kTileP = 128;   // positions of a tile of scores
+constexpr int kStepP = 32;    // positions of a buffer of weights and values
+constexpr int kStepD = 32;    // dimensions of a buffer of keys
+constexpr int kThreads = 128;
 
-__host__ __device__ constexpr int prompt_pitch(int a) { return 8 * a + (a & 1 ? 1 : 2); }  // floats between positions (or dimensions) of the queries' values
+struct PromptArgs {
+  AttnArgs a;
+  float *scores;     // [block][n_alloc][kQ]: scores, then exponentials
+  float *tile_max;   // [block][n_alloc / 32][kQ]
+  float *inv;        // [block][kQ]
+  int64_t n_alloc;   // positions, a multiple of kTileP
+  int32_t group, rows, first, blocks;  // query heads per KV head; rows of a block; this launch's blocks of rows
+  float neg_zero;
+};
 
-template <int A>
-__device__ __forceinline__ void prompt_queries(const float *x, uint64_t (&xx)[A]) {
-  if (A == 2) {
-    const float2 v = *reinterpret_cast<const float2 *>(x);
-    xx[0] = both(v.x);
-    xx[A - 1] = both(v.y);
-  } else {
-#pragma unroll
-    for (int c = 0; c < A; ++c) xx[c] = both(x[c]);
+// The rows of a block: the longest contexts start first.
+struct Rows {
+  int b0, kvh, block;
+  __device__ __forceinline__ Rows(const PromptArgs &p, int y, int z) {
+    const int rb = p.blocks - 1 - y;
+    b0 = (p.first + rb) * p.rows;
+    kvh = z;
+    block = rb * p.a.n_kv_heads + z;
   }
-}
-
-template <int G, int HD, int A, int W>
-__global__ void __launch_bounds__(1024 / W) attn_prompt_kernel(AttnArgs a, float neg_zero) {
-  constexpr int M = 8 * A, R = M / G, PITCH = prompt_pitch(A), T = 1024 / W, PAIRS = W / 2;
-  constexpr int OPAIRS = W == 8 ? HD / 32 : 2;  // pairs of dimensions of a thread's outputs
-  extern __shared__ __align__(16) float prompt_smem[];
-  float *buf = prompt_smem;                        // [2][kPromptK][128]
-  float *q_s = buf + 2 * kPromptK * kPromptTile;   // [HD][PITCH]
-  float *sc = q_s + HD * PITCH;                    // [positions][PITCH]
-  __shared__ float s_max[8 / W][M], s_inv[M];
-  __shared__ int s_rows[R];  // context length of each row
-  const int kvh = blockIdx.x, tid = threadIdx.x, rg = (tid >> 1) & 15;
-  // neighbouring lanes share positions and differ in their queries: a 16-byte load whose lanes pair up so takes half the time.
-  // A thread's positions (dimensions): r0 .. r0 + 3 and, W = 8, 64 + the same; W = 4: warps 4..7 take the upper 64
-  const int half = tid >> 7, ag = ((tid >> 4) & 6) | (tid & 1), r0 = 64 * half + 4 * rg;
-  const int b0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * R;  // the longest contexts start first
-  const int slot = a.slots[b0];
-  const __half *kbase = a.k_cache + ((int64_t)slot * a.n_kv_heads + kvh) * a.max_pos * HD;
-  const __half *vbase = a.v_cache + ((int64_t)slot * a.n_kv_heads + kvh) * a.max_pos * HD;
-  if (tid < R) s_rows[tid] = a.positions[min(b0 + tid, a.batch - 1)] + 1;
-  for (int i = tid; i < M * HD; i += T) {
-    const int m = i / HD, d = i % HD, row = min(b0 + m / G, a.batch - 1);
-    q_s[d * PITCH + m] = a.q[(int64_t)row * a.q_stride + ((int64_t)kvh * G + m % G) * HD + d];
+  // context length of query m; 0: no such query
+  __device__ __forceinline__ int length(const PromptArgs &p, int m) const {
+    const int r = m / p.group, b = b0 + r;
+    return r < p.rows && b < p.a.batch ? p.a.positions[b] + 1 : 0;
   }
-  __syncthreads();
-  int n_min = s_rows[0], n_max = s_rows[0];
-#pragma unroll
-  for (int r = 1; r < R; ++r) n_min = min(n_min, s_rows[r]), n_max = max(n_max, s_rows[r]);
-  int len[A];  // context lengths of this thread's queries
-#pragma unroll
-  for (int c = 0; c < A; ++c) len[c] = s_rows[(ag * A + c) / G];
-  const uint64_t nz = both(neg_zero);
+  __device__ __forceinline__ int last_length(const PromptArgs &p) const { return p.a.positions[min(b0 + p.rows, p.a.batch) - 1] + 1; }
+};
 
-  // ---- scores
-  constexpr int KCH = HD / kPromptK;
-  const int steps = (n_max + kPromptTile - 1) / kPromptTile * KCH;
-  constexpr int KW = kPromptK * kPromptTile / T / 8;  // 16-byte pieces of a key per thread
-  uint4 raw[KW];
-  const int kp = tid & 127, kd = (tid >> 7) * (8 * KW);
-  auto load_k = [&](int s) {  // this thread's position and dimensions of a buffer
-    const int p = min(s / KCH * kPromptTile + kp, n_max - 1);
-    const uint4 *src = reinterpret_cast<const uint4 *>(kbase + (int64_t)p * HD + s % KCH * kPromptK + kd);
+template <int HD>
+__global__ void __launch_bounds__(kThreads) prompt_scores_kernel(const __grid_constant__ PromptArgs p) {
+  extern __shared__ __align__(16) float scores_smem[];
+  float *qs = scores_smem, *ks = qs + HD * kQ;  // [HD][kQ], [2][kStepD][kTileP]
+  const Rows R(p, blockIdx.y, blockIdx.z);
+  const int n_max = R.last_length(p), p0 = blockIdx.x * kTileP, tid = threadIdx.x, lane = tid & 31;
+  if (p0 >= n_max) return;
+  const AttnArgs &a = p.a;
+  const uint4 *src = reinterpret_cast<const uint4 *>(a.k_cache + (((int64_t)a.slots[R.b0] * a.n_kv_heads + R.kvh) * a.max_pos + min(p0 + tid, n_max - 1)) * HD);
+  uint4 raw[kStepD / 8];
+  auto load = [&](int s) {  // this thread's position
 #pragma unroll
-    for (int j = 0; j < KW; ++j) raw[j] = __ldg(src + j);
+    for (int j = 0; j < kStepD / 8; ++j) raw[j] = __ldg(src + s * (kStepD / 8) + j);
   };
-  auto store_k = [&](int s) {
-    float *dst = buf + (s & 1) * (kPromptK * kPromptTile) + kd * kPromptTile + kp;
+  auto store = [&](int s) {
+    float *dst = ks + (s & 1) * (kStepD * kTileP) + tid;
 #pragma unroll
-    for (int j = 0; j < KW; ++j) {
+    for (int j = 0; j < kStepD / 8; ++j) {
       const uint32_t w[4] = {raw[j].x, raw[j].y, raw[j].z, raw[j].w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[i]));
-        dst[(8 * j + 2 * i) * kPromptTile] = f.x;
-        dst[(8 * j + 2 * i + 1) * kPromptTile] = f.y;
+        dst[(8 * j + 2 * i) * kTileP] = f.x;
+        dst[(8 * j + 2 * i + 1) * kTileP] = f.y;
       }
     }
   };
-  float mx[A];
-#pragma unroll
-  for (int c = 0; c < A; ++c) mx[c] = -INFINITY;
-  uint64_t acc[A][PAIRS];
-  load_k(0);
-  store_k(0);
-  __syncthreads();
-  for (int s = 0; s < steps; ++s) {
-    if (s + 1 < steps) load_k(s + 1);
-    if (s % KCH == 0)
-#pragma unroll
-      for (int c = 0; c < A; ++c)
-#pragma unroll
-        for (int p = 0; p < PAIRS; ++p) acc[c][p] = 0;
-    const float *w = buf + (s & 1) * (kPromptK * kPromptTile) + r0, *x = q_s + s % KCH * kPromptK * PITCH + ag * A;
-#pragma unroll 8
-    for (int k = 0; k < kPromptK; ++k) {
-      uint64_t v[PAIRS], xx[A];
-#pragma unroll
-      for (int p = 0; p < PAIRS; p += 2) {
-        const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(w + k * kPromptTile + 32 * p);
-        v[p] = t.x;
-        v[p + 1] = t.y;
-      }
-      prompt_queries<A>(x + k * PITCH, xx);
-#pragma unroll
-      for (int c = 0; c < A; ++c)
-#pragma unroll
-        for (int p = 0; p < PAIRS; ++p) acc[c][p] = add2(acc[c][p], mul2(xx[c], v[p], nz));
+  load(0);
+  {
+    const int m = tid & (kQ - 1), row = min(R.b0 + min(m / p.group, p.rows - 1), a.batch - 1);
+    const float4 *q = reinterpret_cast<const float4 *>(a.q + (int64_t)row * a.q_stride + ((int64_t)R.kvh * p.group + m % p.group) * HD);
+#pragma unroll 4
+    for (int j = tid / kQ; j < HD / 4; j += kThreads / kQ) {
+      const float4 v = q[j];
+      qs[(4 * j) * kQ + m] = v.x, qs[(4 * j + 1) * kQ + m] = v.y, qs[(4 * j + 2) * kQ + m] = v.z, qs[(4 * j + 3) * kQ + m] = v.w;
     }
-    if (s % KCH == KCH - 1) {
-      const int p0 = s / KCH * kPromptTile + r0;
+  }
+  store(0);
+  __syncthreads();
+  // A warp has all queries and 32 positions (which, differs from CTA to CTA: the last tile's upper warps have nothing to do).
+  // Neighbouring lanes share positions, next but one queries: a 16-byte load whose lanes pair up so takes half the time.
+  const int pq = ((tid >> 5) + blockIdx.x + blockIdx.y) & 3, qg = (lane & 1) | ((lane >> 1) & 6), pg = ((lane >> 1) & 1) | ((lane >> 3) & 2);
+  const int r0 = 32 * pq + 4 * pg;
+  const bool any = p0 + 32 * pq < n_max;
+  const uint64_t nz = both(p.neg_zero);
+  uint64_t acc[8][4];  // [position r0 + i, r0 + 16 + i][pair of queries 4 qg, 4 qg + 2, 32 + the same]
 #pragma unroll
-      for (int i = 0; i < W; ++i) {
-        const int p = p0 + 64 * (i >> 2) + (i & 3);
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int c = 0; c < A; ++c) {
-          const float2 v = halves(acc[c][i >> 1]);
-          const float f = __fmul_rn(i & 1 ? v.y : v.x, a.scale);
-          if (p < n_max) sc[(int64_t)p * PITCH + ag * A + c] = f;
-          if (p < len[c]) mx[c] = fmaxf(mx[c], f);
+    for (int c = 0; c < 4; ++c) acc[i][c] = 0;
+#pragma unroll 1
+  for (int s = 0; s < HD / kStepD; ++s) {
+    if (s + 1 < HD / kStepD) load(s + 1);
+    const float *qp = qs + s * (kStepD * kQ) + 4 * qg, *kp = ks + (s & 1) * (kStepD * kTileP) + r0;
+    if (any) {
+#pragma unroll 4
+      for (int d = 0; d < kStepD; ++d) {
+        const ulonglong2 q0 = *reinterpret_cast<const ulonglong2 *>(qp + d * kQ), q1 = *reinterpret_cast<const ulonglong2 *>(qp + d * kQ + 32);
+        const float4 k0 = *reinterpret_cast<const float4 *>(kp + d * kTileP), k1 = *reinterpret_cast<const float4 *>(kp + d * kTileP + 16);
+        const float kv[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+        const uint64_t q[4] = {q0.x, q0.y, q1.x, q1.y};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint64_t k = both(kv[i]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[i][c] = add2(acc[i][c], mul2(q[c], k, nz));
         }
       }
     }
-    if (s + 1 < steps) store_k(s + 1);  // into the buffer that every thread left before the barrier below
+    if (s + 1 < HD / kStepD) store(s + 1);  // into the buffer that every thread left before the barrier below
     __syncthreads();
   }
-  // ---- maxima, exponentials, sums in position order, weights
+  if (!any) return;
+  float mx[8];
+  int len[8];
 #pragma unroll
-  for (int c = 0; c < A; ++c) {
+  for (int x = 0; x < 8; ++x) mx[x] = -INFINITY, len[x] = R.length(p, 4 * qg + 32 * (x >> 2) + (x & 3));
+  float *out = p.scores + ((int64_t)R.block * p.n_alloc + p0) * kQ + 4 * qg;
 #pragma unroll
-    for (int o = 16; o > 1; o >>= 1) mx[c] = fmaxf(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], o));
-    if (rg == 0) s_max[half][ag * A + c] = mx[c];
-  }
-  const int v_steps = (n_max + kPromptK - 1) / kPromptK;
-  constexpr int VPIECES = kPromptK * HD / 8, VLOADS = (VPIECES + T - 1) / T;  // 16-byte pieces of a buffer's values
-  uint4 vr[VLOADS];
-  auto load_v = [&](int s) {
+  for (int i = 0; i < 8; ++i) {
+    const int r = r0 + 16 * (i >> 2) + (i & 3);
+    float f[8];
 #pragma unroll
-    for (int j = 0; j < VLOADS; ++j) {
-      const int i = min(tid + j * T, VPIECES - 1), p = min(s * kPromptK + i / (HD / 8), n_max - 1);
-      vr[j] = __ldg(reinterpret_cast<const uint4 *>(vbase + (int64_t)p * HD) + i % (HD / 8));
+    for (int c = 0; c < 4; ++c) {
+      const float2 v = halves(acc[i][c]);
+      f[2 * c] = __fmul_rn(v.x, a.scale);
+      f[2 * c + 1] = __fmul_rn(v.y, a.scale);
     }
-  };
-  auto store_v = [&](int s) {
-    float *dst = buf + (s & 1) * (kPromptK * kPromptTile);
 #pragma unroll
-    for (int j = 0; j < VLOADS; ++j) {
-      const int i = tid + j * T;
-      if (i >= VPIECES) break;
+    for (int x = 0; x < 8; ++x)
+      if (p0 + r < len[x]) mx[x] = fmaxf(mx[x], f[x]);
+    *reinterpret_cast<float4 *>(out + (int64_t)r * kQ) = make_float4(f[0], f[1], f[2], f[3]);
+    *reinterpret_cast<float4 *>(out + (int64_t)r * kQ + 32) = make_float4(f[4], f[5], f[6], f[7]);
+  }
+#pragma unroll
+  for (int x = 0; x < 8; ++x) {
+    mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 2));
+    mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 16));
+  }
+  if (pg == 0) {
+    float *t = p.tile_max + ((int64_t)R.block * (p.n_alloc / 32) + p0 / 32 + pq) * kQ + 4 * qg;
+    *reinterpret_cast<float4 *>(t) = make_float4(mx[0], mx[1], mx[2], mx[3]);
+    *reinterpret_cast<float4 *>(t + 32) = make_float4(mx[4], mx[5], mx[6], mx[7]);
+  }
+}
+
+constexpr int kWeightThreads = 256, kWeightP = 64, kWeightN = kWeightP * kQ / kWeightThreads;
+
+__global__ void __launch_bounds__(kWeightThreads) prompt_weights_kernel(const __grid_constant__ PromptArgs p) {
+  __shared__ float e_s[2][kWeightP][kQ];
+  __shared__ float s_max[kWeightThreads / kQ][kQ];
+  constexpr int PARTS = kWeightThreads / kQ;
+  const Rows R(p, blockIdx.y, blockIdx.x);
+  const int n_max = R.last_length(p), tid = threadIdx.x, q = tid & (kQ - 1), part = tid / kQ, len = R.length(p, q);
+  const float *t = p.tile_max + (int64_t)R.block * (p.n_alloc / 32) * kQ + q;
+  float mx = -INFINITY;
+  for (int i = part; i < (n_max + 31) / 32; i += PARTS) mx = fmaxf(mx, t[(int64_t)i * kQ]);
+  s_max[part][q] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < PARTS; ++i) mx = fmaxf(mx, s_max[i][q]);
+  float *s = p.scores + (int64_t)R.block * p.n_alloc * kQ + q;
+  float sum = 0.0f, v[kWeightN];
+  // (positions beyond a query's context, up to n_alloc, hold some value; nothing of them is kept)
+#pragma unroll
+  for (int j = 0; j < kWeightN; ++j) v[j] = s[(int64_t)(part + PARTS * j) * kQ];
+  for (int t0 = 0, buf = 0; t0 < n_max; t0 += kWeightP, buf ^= 1) {
+#pragma unroll
+    for (int j = 0; j < kWeightN; ++j) {
+      const int r = part + PARTS * j;
+      const float e = expf_exact_flat(__fsub_rn(v[j], mx));
+      e_s[buf][r][q] = e;
+      if (t0 + r < len) s[(int64_t)(t0 + r) * kQ] = e;
+    }
+    if (t0 + kWeightP < n_max)
+#pragma unroll
+      for (int j = 0; j < kWeightN; ++j) v[j] = s[(int64_t)(t0 + kWeightP + part + PARTS * j) * kQ];
+    __syncthreads();
+    if (part == 0) {
+      const float *e = &e_s[buf][0][q];
+      const int n = min(kWeightP, len - t0);
+      if (n == kWeightP) {
+#pragma unroll
+        for (int i = 0; i < kWeightP; ++i) sum = __fadd_rn(sum, e[i * kQ]);
+      } else {
+        for (int i = 0; i < n; ++i) sum = __fadd_rn(sum, e[i * kQ]);
+      }
+    }
+  }
+  if (part == 0) p.inv[R.block * kQ + q] = __fdiv_rn(1.0f, sum);
+}
+
+template <int HD>
+__global__ void __launch_bounds__(kThreads) prompt_values_kernel(const __grid_constant__ PromptArgs p) {
+  __shared__ __align__(16) float ws[2][kStepP][kQ], vs[2][kStepP][64];
+  const Rows R(p, blockIdx.y, blockIdx.x / (HD / 64));
+  const int tid = threadIdx.x, lane = tid & 31, d0 = blockIdx.x % (HD / 64) * 64;
+  const AttnArgs &a = p.a;
+  const int n_max = R.last_length(p), n_min = a.positions[R.b0] + 1;
+  const __half *vbase = a.v_cache + ((int64_t)a.slots[R.b0] * a.n_kv_heads + R.kvh) * a.max_pos * HD + d0;
+  const float *wbase = p.scores + (int64_t)R.block * p.n_alloc * kQ + 4 * (tid & 15);
+  const float4 inv = *reinterpret_cast<const float4 *>(p.inv + R.block * kQ + 4 * (tid & 15));
+  uint4 vr[2];
+  float4 wr[4];
+  auto load = [&](int s) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      vr[j] = __ldg(reinterpret_cast<const uint4 *>(vbase + (int64_t)min(s * kStepP + 16 * j + (tid >> 3), n_max - 1) * HD) + (tid & 7));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) wr[j] = *reinterpret_cast<const float4 *>(wbase + (int64_t)(s * kStepP + 8 * j + (tid >> 4)) * kQ);
+  };
+  auto store = [&](int b) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
       const uint32_t w[4] = {vr[j].x, vr[j].y, vr[j].z, vr[j].w};
       float2 f[4];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) f[t] = __half22float2(*reinterpret_cast<const __half2 *>(&w[t]));
-      float4 *o = reinterpret_cast<float4 *>(dst + i * 8);  // [position][HD]
+      for (int i = 0; i < 4; ++i) f[i] = __half22float2(*reinterpret_cast<const __half2 *>(&w[i]));
+      float4 *o = reinterpret_cast<float4 *>(&vs[b][16 * j + (tid >> 3)][8 * (tid & 7)]);
       o[0] = make_float4(f[0].x, f[0].y, f[1].x, f[1].y);
       o[1] = make_float4(f[2].x, f[2].y, f[3].x, f[3].y);
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<float4 *>(&ws[b][8 * j + (tid >> 4)][4 * (tid & 15)]) =
+          make_float4(__fmul_rn(wr[j].x, inv.x), __fmul_rn(wr[j].y, inv.y), __fmul_rn(wr[j].z, inv.z), __fmul_rn(wr[j].w, inv.w));
   };
-  load_v(0);
+  // lanes paired as in the scores: neighbours share dimensions, next but one queries
+  const int qg = (lane & 1) | ((lane >> 1) & 6), dg = 4 * (tid >> 5) + (((lane >> 1) & 1) | ((lane >> 3) & 2));
+  const uint64_t nz = both(p.neg_zero);
+  uint64_t acc[4][4];  // [dimension 4 dg + i][pair of queries 4 qg, 4 qg + 2, 32 + the same]
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[i][c] = 0;
+  const int steps = (n_max + kStepP - 1) / kStepP;
+  load(0);
+  store(0);
   __syncthreads();
-  // thread: query m, every PS-th position, four at a time (the latencies of one hide behind the others)
-  constexpr int PS = T / M;
-  const int m = tid % M, own = tid < PS * M ? s_rows[m / G] : 0;
-  if (W == 4 && tid < M) s_max[0][tid] = fmaxf(s_max[0][tid], s_max[8 / W - 1][tid]);
-  if (W == 4) __syncthreads();
-  const float top = s_max[0][m];
-  for (int p = tid / M; p < own; p += 4 * PS) {
-    float e[4];
+  for (int s = 0; s < steps; ++s) {
+    if (s + 1 < steps) load(s + 1);
+    const float *w = &ws[s & 1][0][4 * qg], *v = &vs[s & 1][0][4 * dg];
+    if ((s + 1) * kStepP <= n_min) {
+#pragma unroll 4
+      for (int k = 0; k < kStepP; ++k) {
+        const ulonglong2 w0 = *reinterpret_cast<const ulonglong2 *>(w + k * kQ), w1 = *reinterpret_cast<const ulonglong2 *>(w + k * kQ + 32);
+        const float4 vv = *reinterpret_cast<const float4 *>(v + k * 64);
+        const float vd[4] = {vv.x, vv.y, vv.z, vv.w};
+        const uint64_t q[4] = {w0.x, w0.y, w1.x, w1.y};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) e[j] = sc[(int64_t)min(p + j * PS, own - 1) * PITCH + m];
+        for (int i = 0; i < 4; ++i) {
+          const uint64_t x = both(vd[i]);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) e[j] = expf_exact_flat(__fsub_rn(e[j], top));
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (p + j * PS < own) sc[(int64_t)(p + j * PS) * PITCH + m] = e[j];
-  }
-  store_v(0);
-  __syncthreads();
-  if (tid < M) {
-    const int n = s_rows[tid / G];
-    const float *e = sc + tid;
-    float sum = 0.0f, v[8];
-    if (n >= 8)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = e[j * PITCH];
-    int p = 0;
-    for (; p + 8 <= n; p += 8) {
-      float next[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) next[j] = e[(int64_t)min(p + 8 + j, n - 1) * PITCH];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) sum = __fadd_rn(sum, v[j]);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = next[j];
-    }
-    for (; p < n; ++p) sum = __fadd_rn(sum, e[(int64_t)p * PITCH]);
-    s_inv[tid] = __fdiv_rn(1.0f, sum);
-  }
-  __syncthreads();
-  const float inv = s_inv[m];
-  for (int p = tid / M; p < own; p += 4 * PS) {
-    float e[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) e[j] = sc[(int64_t)min(p + j * PS, own - 1) * PITCH + m];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (p + j * PS < own) sc[(int64_t)(p + j * PS) * PITCH + m] = __fmul_rn(e[j], inv);
-  }
-  __syncthreads();
-  // ---- weighted values: dimensions r0 .. r0 + 3 (and 64 + the same) of A queries per thread
-  const bool active = r0 < HD;
-  uint64_t out[A][OPAIRS];
-#pragma unroll
-  for (int c = 0; c < A; ++c)
-#pragma unroll
-    for (int p = 0; p < OPAIRS; ++p) out[c][p] = 0;
-  for (int s = 0; s < v_steps; ++s) {
-    if (s + 1 < v_steps) load_v(s + 1);
-    const float *w = buf + (s & 1) * (kPromptK * kPromptTile) + r0, *x = sc + (int64_t)s * kPromptK * PITCH + ag * A;
-    if (!active) {
-    } else if ((s + 1) * kPromptK <= n_min) {
-#pragma unroll 8
-      for (int k = 0; k < kPromptK; ++k) {
-        uint64_t v[OPAIRS], xx[A];
-#pragma unroll
-        for (int p = 0; p < OPAIRS; p += 2) {
-          const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(w + k * HD + 32 * p);
-          v[p] = t.x;
-          v[p + 1] = t.y;
+          for (int c = 0; c < 4; ++c) acc[i][c] = add2(acc[i][c], mul2(q[c], x, nz));
         }
-        prompt_queries<A>(x + k * PITCH, xx);
-#pragma unroll
-        for (int c = 0; c < A; ++c)
-#pragma unroll
-          for (int p = 0; p < OPAIRS; ++p) out[c][p] = add2(out[c][p], mul2(xx[c], v[p], nz));
       }
-    } else {  // the last positions: a row adds only what lies in its context
-      const int cnt = min(kPromptK, n_max - s * kPromptK);
+    } else {  // the last positions: a query adds only what lies in its context
+      int len[8];
+#pragma unroll
+      for (int x = 0; x < 8; ++x) len[x] = R.length(p, 4 * qg + 32 * (x >> 2) + (x & 3)) - s * kStepP;
+      const int cnt = min(kStepP, n_max - s * kStepP);
       for (int k = 0; k < cnt; ++k) {
-        uint64_t xx[A];
-        prompt_queries<A>(x + k * PITCH, xx);
+        const ulonglong2 w0 = *reinterpret_cast<const ulonglong2 *>(w + k * kQ), w1 = *reinterpret_cast<const ulonglong2 *>(w + k * kQ + 32);
+        const float4 vv = *reinterpret_cast<const float4 *>(v + k * 64);
+        const float vd[4] = {vv.x, vv.y, vv.z, vv.w};
+        const uint64_t q[4] = {w0.x, w0.y, w1.x, w1.y};
 #pragma unroll
-        for (int c = 0; c < A; ++c)
-          if (s * kPromptK + k < len[c])
+        for (int i = 0; i < 4; ++i) {
+          const uint64_t x = both(vd[i]);
 #pragma unroll
-            for (int p = 0; p < OPAIRS; ++p)
-              out[c][p] = add2(out[c][p], mul2(xx[c], *reinterpret_cast<const uint64_t *>(w + k * HD + 64 * (p >> 1) + 2 * (p & 1)), nz));
+          for (int c = 0; c < 4; ++c) {
+            const float2 o = halves(acc[i][c]), n = halves(add2(acc[i][c], mul2(q[c], x, nz)));
+            acc[i][c] = pair(k < len[2 * c] ? n.x : o.x, k < len[2 * c + 1] ? n.y : o.y);
+          }
+        }
       }
     }
-    if (s + 1 < v_steps) store_v(s + 1);
+    if (s + 1 < steps) store((s + 1) & 1);  // into the buffer that every thread left before the barrier below
     __syncthreads();
   }
 #pragma unroll
-  for (int c = 0; c < A; ++c) {
-    const int q = ag * A + c, row = b0 + q / G;
-    if (!active || row >= a.batch) continue;
-    float *o = a.out + (int64_t)row * a.q_stride + ((int64_t)kvh * G + q % G) * HD + r0;
+  for (int c = 0; c < 4; ++c) {
+    float2 v[4];
 #pragma unroll
-    for (int p = 0; p < OPAIRS; p += 2) {
-      const float2 lo = halves(out[c][p]), hi = halves(out[c][p + 1]);
-      *reinterpret_cast<float4 *>(o + 32 * p) = make_float4(lo.x, lo.y, hi.x, hi.y);
+    for (int i = 0; i < 4; ++i) v[i] = halves(acc[i][c]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int m = 4 * qg + 32 * (c >> 1) + 2 * (c & 1) + h;
+      if (R.length(p, m) == 0) continue;
+      float *o = a.out + (int64_t)(R.b0 + m / p.group) * a.q_stride + ((int64_t)R.kvh * p.group + m % p.group) * HD + d0 + 4 * dg;
+      *reinterpret_cast<float4 *>(o) = h ? make_float4(v[0].y, v[1].y, v[2].y, v[3].y) : make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
     }
   }
 }
 
-size_t prompt_smem_bytes(int HD, int A, int64_t n_pos) { return 4 * (size_t)(2 * kPromptK * kPromptTile + (HD + n_pos) * prompt_pitch(A)); }
-constexpr size_t kPromptTwo = 112 * 1024, kPromptOne = 220 * 1024;  // shared memory of which two CTAs, or one, fit an SM
+int64_t padded(int64_t n_pos) { return (n_pos + kTileP - 1) / kTileP * kTileP; }
+// floats of scratch for a block of rows: scores, maxima and inverse sums of every KV head's 64 queries
+int64_t block_floats(int n_kv_heads, int64_t n_pos) { return n_kv_heads * (padded(n_pos) * kQ + padded(n_pos) / 32 * kQ + kQ); }
 
-template <int G, int HD, int A, int W>
-int32_t launch_prompt(const AttnArgs &a, int64_t n_pos, cudaStream_t s) {
-  constexpr int R = 8 * A / G;
-  const size_t smem = prompt_smem_bytes(HD, A, n_pos);
+template <int HD>
+int32_t launch_prompt(PromptArgs &p, int64_t n_pos, int64_t scratch_floats, cudaStream_t s, int64_t *launches) {
+  const int kv = p.a.n_kv_heads, all = (p.a.batch + p.rows - 1) / p.rows;
+  const int per = (int)std::min<int64_t>(all, scratch_floats / block_floats(kv, n_pos));
+  const size_t smem = (size_t)(HD * kQ + 2 * kStepD * kTileP) * 4;
   static SmemLimit limit;
-  CMLD_TRY(allow_smem(limit, attn_prompt_kernel<G, HD, A, W>, smem));
-  dim3 grid((unsigned)a.n_kv_heads, (unsigned)((a.batch + R - 1) / R));
-  attn_prompt_kernel<G, HD, A, W><<<grid, 1024 / W, smem, s>>>(a, -0.0f);
-  CMLD_CUDA(cudaGetLastError());
-  return CMLD_OK;
-}
-
-// Eight threads side by side cover 8 * A queries, a multiple of G.  Contexts whose scores would leave room for one CTA per SM
-// only take half the queries, or (G = 3) twice the threads and half the outputs per thread.
-template <int G, int HD>
-int32_t launch_prompt(const AttnArgs &a, int64_t n_pos, cudaStream_t s) {
-  if constexpr (G == 3) {
-    return prompt_smem_bytes(HD, 3, n_pos) > kPromptTwo ? launch_prompt<G, HD, 3, 4>(a, n_pos, s) : launch_prompt<G, HD, 3, 8>(a, n_pos, s);
-  } else {
-    return prompt_smem_bytes(HD, 2, n_pos) > kPromptTwo ? launch_prompt<G, HD, 1, 8>(a, n_pos, s) : launch_prompt<G, HD, 2, 8>(a, n_pos, s);
+  CMLD_TRY(allow_smem(limit, prompt_scores_kernel<HD>, smem, true));
+  float *scratch = p.scores;
+  for (p.first = 0; p.first < all; p.first += per) {
+    p.blocks = std::min(per, all - p.first);
+    p.tile_max = scratch + (int64_t)p.blocks * kv * p.n_alloc * kQ;
+    p.inv = p.tile_max + (int64_t)p.blocks * kv * (p.n_alloc / 32) * kQ;
+    prompt_scores_kernel<HD><<<dim3((unsigned)(p.n_alloc / kTileP), (unsigned)p.blocks, (unsigned)kv), kThreads, smem, s>>>(p);
+    prompt_weights_kernel<<<dim3((unsigned)kv, (unsigned)p.blocks), kWeightThreads, 0, s>>>(p);
+    prompt_values_kernel<HD><<<dim3((unsigned)kv * (HD / 64), (unsigned)p.blocks), kThreads, 0, s>>>(p);
+    CMLD_CUDA(cudaGetLastError());
+    if (launches) *launches += 3;
   }
+  return CMLD_OK;
 }
 
 }  // namespace
 
-// n_pos: bound on positions[b] + 1 of every row; every row of the step belongs to one slot.
-bool attention_prompt_fits(int n_heads, int n_kv_heads, int head_dim, int batch, int64_t n_pos, int sms) {
-  if (n_kv_heads < 1 || n_heads % n_kv_heads) return false;
-  const int G = n_heads / n_kv_heads;
-  if (!(G == 1 || G == 2 || G == 3 || G == 4 || G == 8) || !(head_dim == 64 || head_dim == 128)) return false;
-  // a CTA for every SM, or the row kernel's many small ones are faster (8B width: 36 rows at 700 positions 73 us against about
-  // 50, 128 rows at 200 positions 47 us against 100)
-  const int R = 8 * (G == 3 ? 3 : 2) / G;
-  return (batch + R - 1) / R * n_kv_heads >= sms && n_pos > 0 && prompt_smem_bytes(head_dim, G == 3 ? 3 : 1, n_pos) <= kPromptOne;
+// Scratch of an engine whose prompt steps have up to `rows` rows and whose contexts up to `max_pos` positions: a whole step's, at most
+// half a GB (longer contexts then go by groups of rows).
+int64_t attention_prompt_scratch_floats(int n_heads, int n_kv_heads, int head_dim, int rows, int64_t max_pos) {
+  if (n_kv_heads < 1 || n_heads % n_kv_heads || n_heads / n_kv_heads > kQ || !(head_dim == 64 || head_dim == 128)) return 0;
+  const int R = kQ / (n_heads / n_kv_heads);
+  return std::min<int64_t>((int64_t)1 << 27, (rows + R - 1) / R * block_floats(n_kv_heads, max_pos));
 }
 
-int32_t launch_attention_prompt(const AttnArgs &a, int64_t n_pos, int sms, cudaStream_t s) {
-  if (!attention_prompt_fits(a.n_heads, a.n_kv_heads, a.head_dim, a.batch, n_pos, sms)) return CMLD_ERR_UNSUPPORTED;
+// n_pos: bound on positions[b] + 1 of every row; the rows of the step are neighbours in one slot.
+bool attention_prompt_fits(int n_heads, int n_kv_heads, int head_dim, int batch, int64_t n_pos, int sms, int64_t scratch_floats) {
+  if (n_kv_heads < 1 || n_heads % n_kv_heads || !(head_dim == 64 || head_dim == 128) || n_pos < 1) return false;
+  const int G = n_heads / n_kv_heads;
+  if (G > kQ) return false;
+  const int R = kQ / G, all = (batch + R - 1) / R;
+  const int per_block = n_kv_heads * (head_dim / 64), wanted = std::min(all, (sms + per_block - 1) / per_block);
+  // Half a machine of CTAs, or at long contexts a quarter: a CTA walks its positions alone, where the row kernel's many small CTAs share
+  // the machine.  Us per layer, row kernel | here: 8B width, 128 rows at 200 positions 74 | 62, 64 at 200 38 | 46, 36 at 700 53 | 78, 64 at
+  // 2000 325 | 205; 1B width, 100 rows at 200 35 | 47, 200 at 700 170 | 110; 3B width, 100 at 200 52 | 48, 40 at 200 26 | 42.
+  const int64_t ctas = (int64_t)all * per_block;
+  return (ctas * 2 >= sms || (ctas * 4 >= sms && n_pos >= 1024)) && scratch_floats >= wanted * block_floats(n_kv_heads, n_pos);
+}
+
+int32_t launch_attention_prompt(const AttnArgs &a, int64_t n_pos, int sms, float *scratch, int64_t scratch_floats, cudaStream_t s, int64_t *launches) {
+  if (!attention_prompt_fits(a.n_heads, a.n_kv_heads, a.head_dim, a.batch, n_pos, sms, scratch_floats)) return CMLD_ERR_UNSUPPORTED;
   if (a.tree_mask || a.fuse_rope) return fail(CMLD_ERR_INVALID, "attention (prompt): tree masks and fused RoPE are not supported here");
-#define CMLD_PROMPT(GG) \
-  case GG: return a.head_dim == 128 ? launch_prompt<GG, 128>(a, n_pos, s) : launch_prompt<GG, 64>(a, n_pos, s);
-  switch (a.n_heads / a.n_kv_heads) {
-    CMLD_PROMPT(1)
-    CMLD_PROMPT(2)
-    CMLD_PROMPT(3)
-    CMLD_PROMPT(4)
-    CMLD_PROMPT(8)
-  }
-#undef CMLD_PROMPT
-  return CMLD_ERR_UNSUPPORTED;
+  PromptArgs p{};
+  p.a = a;
+  p.scores = scratch;
+  p.n_alloc = padded(n_pos);
+  p.group = a.n_heads / a.n_kv_heads;
+  p.rows = kQ / p.group;
+  p.neg_zero = -0.0f;
+  return a.head_dim == 128 ? launch_prompt<128>(p, n_pos, scratch_floats, s, launches) : launch_prompt<64>(p, n_pos, scratch_floats, s, launches);
 }
 
 }  // namespace cmld

@@ -383,8 +383,9 @@ bool attention_rows_fits(int n_heads, int n_kv_heads, int head_dim, int64_t cap)
 int32_t launch_attention_rows(const AttnArgs &a, int64_t cap, cudaStream_t s);
 
 // attn_prompt.cu: the reference-order attention for long steps of one sequence (n_pos: positions after the last row)
-bool attention_prompt_fits(int n_heads, int n_kv_heads, int head_dim, int batch, int64_t n_pos, int sms);
-int32_t launch_attention_prompt(const AttnArgs &a, int64_t n_pos, int sms, cudaStream_t s);
+int64_t attention_prompt_scratch_floats(int n_heads, int n_kv_heads, int head_dim, int rows, int64_t max_pos);
+bool attention_prompt_fits(int n_heads, int n_kv_heads, int head_dim, int batch, int64_t n_pos, int sms, int64_t scratch_floats);
+int32_t launch_attention_prompt(const AttnArgs &a, int64_t n_pos, int sms, float *scratch, int64_t scratch_floats, cudaStream_t s, int64_t *launches);
 
 // comm.cu: NCCL collectives of the sharded engine
 int32_t comm_unique_id(uint8_t *out128);

@@ -282,6 +282,10 @@ static int32_t engine_init(cmld_engine *e) {
     const int64_t widest = std::max<int64_t>(std::max<int64_t>(c.hidden, c.ffn_dim), e->q_width);
     const int64_t wide = (widest + 255) / 256 * 256;
     e->tc5_pack_bytes = gemv_tc5_pack_bytes(wide, (int32_t)R);
+    if (e->chunk_rows > kShortRows) {
+      e->prompt_scratch_floats = attention_prompt_scratch_floats(c.n_heads, c.n_kv_heads, c.head_dim, e->chunk_rows, c.max_pos);
+      if (e->prompt_scratch_floats > 0) CMLD_TRY(dev_alloc(e, &e->prompt_scratch, e->prompt_scratch_floats, false));
+    }
     for (auto &pack : e->tc5_pack) CMLD_TRY(dev_alloc(e, &pack, e->tc5_pack_bytes, false));
     for (auto &rec : e->rows_rec) CMLD_TRY(dev_alloc(e, &rec, gemv_rows_rec_bytes(wide, kRowsMaxBatch), false));
   }
@@ -862,7 +866,7 @@ static int32_t engine_step(cmld_engine *e, const StepOpts &o) {
       const bool rows = !fast && !(c.flags & CMLD_FLAG_EXACT_ORDER) && B >= 3 && o.attn_cap > 0 && !o.tree_mask &&
                         attention_rows_fits(c.n_heads, c.n_kv_heads, c.head_dim, o.attn_cap);
       // a prompt's long steps (never captured: their context is exact): neighbouring rows share a CTA
-      const bool prompt = rows && o.prompt_end && attention_prompt_fits(c.n_heads, c.n_kv_heads, c.head_dim, B, o.prompt_end, e->sm_count);
+      const bool prompt = rows && o.prompt_end && attention_prompt_fits(c.n_heads, c.n_kv_heads, c.head_dim, B, o.prompt_end, e->sm_count, e->prompt_scratch_floats);
       const bool ordered = !rows && !fast && !(c.flags & CMLD_FLAG_EXACT_ORDER) && o.attn_cap > 0 && !o.tree_mask &&
                            attention_ordered_fits(c.n_heads, c.n_kv_heads, c.head_dim, o.attn_cap);
       const bool fuse = !o.shared_slots && (fast || ordered);
@@ -924,12 +928,12 @@ static int32_t engine_step(cmld_engine *e, const StepOpts &o) {
       a.tree_mask = o.tree_mask;
       a.tree_base = o.tree_base;
       a.tree_words = o.tree_words;
-      if (prompt) CMLD_TRY(launch_attention_prompt(a, o.prompt_end, e->sm_count, e->stream));
+      if (prompt) CMLD_TRY(launch_attention_prompt(a, o.prompt_end, e->sm_count, e->prompt_scratch, e->prompt_scratch_floats, e->stream, &e->launches));
       else if (rows) CMLD_TRY(launch_attention_rows(a, o.attn_cap, e->stream));
       else if (ordered) CMLD_TRY(launch_attention_ordered(a, o.attn_cap, e->stream));
       else if (fast) CMLD_TRY(launch_attention(a, e->stream));
       else CMLD_TRY(launch_attention_exact(a, e->stream));
-      e->launches += 1;
+      if (!prompt) e->launches += 1;
       }
     }
     {

@@ -49,6 +49,8 @@ struct cmld_engine {
   std::vector<float> rope_freq;  // per-pair angular frequency of the engine-owned RoPE table (rope_pair_frequency)
   uint8_t *tc5_pack[2] = {nullptr, nullptr};  // activation records of the tcgen05 batched matvec: Q4_K or Q8_0, Q6_K
   int64_t tc5_pack_bytes = 0;
+  float *prompt_scratch = nullptr;  // scores of the attention of long prompt steps
+  int64_t prompt_scratch_floats = 0;
   uint8_t *rows_rec[2] = {nullptr, nullptr};  // activation records of the row-batched matvec: Q4_K or Q8_0, Q6_K
   int64_t mma_scratch_floats = 0;
   unsigned long long *trace = nullptr;  // matvec timeline (environment CMLD_TRACE=<file>), dumped at destroy

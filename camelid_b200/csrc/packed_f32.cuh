@@ -25,6 +25,11 @@ __device__ __forceinline__ uint64_t both(float x) {
   asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
   return r;
 }
+__device__ __forceinline__ uint64_t pair(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
 __device__ __forceinline__ float2 halves(uint64_t v) {
   float2 r;
   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));

@@ -390,6 +390,21 @@ def test_long_prompt_steps_equal_the_serial_path(cm, orc, heads, kv, hd, first, 
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), hidden_gate(got, want)
 
 
+def test_long_prompt_steps_whose_scores_go_by_groups(cm, orc):
+    """64 heads without sharing at 2100 positions: the second and third step's scores do not fit the scratch at once.  Against the plain
+    reference-order kernels, bit for bit, at places in every step."""
+    from camelid_b200 import synth
+
+    def engine(flags):
+        cfg = cm.EngineConfig(n_layers=1, n_heads=64, n_kv_heads=64, head_dim=64, hidden=256, ffn_dim=512, vocab=512, max_pos=4096, flags=flags)
+        return synth.build_engine(cfg, "q4_k_m", 5)
+
+    prompt = orc.synth_tokens(4, 1, 2100, 512)
+    want = [5, 1023, 1024, 1500, 2040, 2047, 2048, 2099]
+    (t1, got), (t2, ref) = (engine(flags).extend(0, prompt, 0, want=want) for flags in (0, 16))
+    assert t1 == t2 and np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+
+
 @pytest.mark.parametrize("slots", [40, 64, 512])
 def test_prompts_take_the_same_steps_whatever_the_number_of_slots(cm, orc, slots):
     """A prompt's steps are chosen by its rows: an engine of many slots launches what an engine of one launches (no logits of
