@@ -500,6 +500,86 @@ __device__ __forceinline__ void rms_norm_cta(float *u, int n, const float *w, fl
   for (int i = threadIdx.x; i < n; i += blockDim.x) u[i] = u[i] * r * w[i];
 }
 
+// What the boundary of up to kMixStreams streams takes of the weights: the mixing matrix [s][t], then out[t], in[t]; zeros for absent streams.
+constexpr int kMixStreams = 4, kMixCoefs = kMixStreams * (kMixStreams + 2);
+__device__ __forceinline__ float mix_coef(const StreamMix &m, int i) {
+  const int s = i / kMixStreams, t = i % kMixStreams;
+  if (t >= m.streams || (s < kMixStreams && s >= m.streams)) return 0.0f;
+  if (s == kMixStreams) return m.out[t];
+  if (s > kMixStreams) return m.in ? m.in[t] : 1.0f;
+  return m.mix[s * m.streams + t];
+}
+// The boundary of mixed streams for widths that are a multiple of four and at most 4 V blockDim.x: everything a thread reads is asked for
+// at once and the row stays in registers (stream_mix_row goes through shared memory value by value, with one global latency after the
+// other).  put(i, v) takes values 4i .. 4i + 3 of the result.  `coef` (kMixCoefs, shared memory) is complete after a barrier.
+__device__ __forceinline__ bool mix_row_fits(const StreamMix &m, int v) {
+  return m.mix && !m.embed && m.streams <= kMixStreams && m.width % 4 == 0 && m.width <= 4 * v * (int)blockDim.x;
+}
+template <int V, typename Put>
+__device__ __forceinline__ void mix_row(const StreamMix &m, int64_t row, const float *coef, float *red, bool store, Put put) {
+  const int n4 = m.width / 4;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float4 u[V];
+  {
+    const float4 *x = reinterpret_cast<const float4 *>(m.x_in + row * m.streams * m.width), *y = reinterpret_cast<const float4 *>(m.y + row * m.width);
+    float4 *xo = store && m.x_out ? reinterpret_cast<float4 *>(m.x_out + row * m.streams * m.width) : nullptr;
+    float4 xv[V][kMixStreams], yv[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const int i = threadIdx.x + j * blockDim.x;
+      yv[j] = i < n4 ? y[i] : zero;
+#pragma unroll
+      for (int s = 0; s < kMixStreams; ++s) xv[j][s] = i < n4 && s < m.streams ? x[s * n4 + i] : zero;
+    }
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const int i = threadIdx.x + j * blockDim.x;
+      u[j] = zero;
+#pragma unroll
+      for (int t = 0; t < kMixStreams; ++t) {
+        const float o = coef[kMixStreams * kMixStreams + t], in = coef[kMixStreams * (kMixStreams + 1) + t];
+        float4 v = make_float4(o * yv[j].x, o * yv[j].y, o * yv[j].z, o * yv[j].w);
+#pragma unroll
+        for (int s = 0; s < kMixStreams; ++s) {
+          const float c = coef[s * kMixStreams + t];
+          v = make_float4(fmaf(c, xv[j][s].x, v.x), fmaf(c, xv[j][s].y, v.y), fmaf(c, xv[j][s].z, v.z), fmaf(c, xv[j][s].w, v.w));
+        }
+        if (xo && i < n4 && t < m.streams) xo[t * n4 + i] = v;
+        if (t < m.streams) u[j] = make_float4(fmaf(in, v.x, u[j].x), fmaf(in, v.y, u[j].y), fmaf(in, v.z, u[j].z), fmaf(in, v.w, u[j].w));
+      }
+    }
+  }
+  if (m.norm_w) {  // the formulas of layer_norm_cta and rms_norm_cta
+    const float4 *nw = reinterpret_cast<const float4 *>(m.norm_w), *nb = reinterpret_cast<const float4 *>(m.norm_b);
+    float4 w[V], b[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const int i = threadIdx.x + j * blockDim.x;
+      w[j] = i < n4 ? nw[i] : zero;
+      b[j] = nb && i < n4 ? nb[i] : zero;
+    }
+    if (nb) {
+      float s = 0.0f;
+#pragma unroll
+      for (int j = 0; j < V; ++j) s += (u[j].x + u[j].y) + (u[j].z + u[j].w);
+      const float mean = cta_total(s, red) / (float)m.width;
+#pragma unroll
+      for (int j = 0; j < V; ++j)
+        if ((int)threadIdx.x + j * (int)blockDim.x < n4) u[j] = make_float4(u[j].x - mean, u[j].y - mean, u[j].z - mean, u[j].w - mean);
+    }
+    float s = 0.0f;
+#pragma unroll
+    for (int j = 0; j < V; ++j) s += dot4(u[j], u[j]);
+    const float r = 1.0f / sqrtf(cta_total(s, red) / (float)m.width + m.eps);
+#pragma unroll
+    for (int j = 0; j < V; ++j)
+      u[j] = make_float4(fmaf(u[j].x * r, w[j].x, b[j].x), fmaf(u[j].y * r, w[j].y, b[j].y), fmaf(u[j].z * r, w[j].z, b[j].z), fmaf(u[j].w * r, w[j].w, b[j].w));
+  }
+#pragma unroll
+  for (int j = 0; j < V; ++j)
+    if ((int)threadIdx.x + j * (int)blockDim.x < n4) put((int)threadIdx.x + j * (int)blockDim.x, u[j]);
+}
+
 // The whole boundary for one row; the result is left in u[width] (shared memory, 16-byte aligned; each thread may read its
 // own stride).  `red` holds 2 * blockDim.x / 32 floats, 8-byte aligned.
 __device__ __forceinline__ void stream_mix_row(const StreamMix &m, int r, float *u, float *red, bool store) {

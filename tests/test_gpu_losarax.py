@@ -74,6 +74,17 @@ def test_linear_kernels(cm, shape):
         assert np.abs(linear(cm, 0, w, x[:n]) - ref[:n]).max() < 2e-5
 
 
+@pytest.mark.parametrize("shape", [(1, 14336), (5, 8200), (149, 2056), (593, 520), (1187, 264), (4099, 256), (9001, 1032)])
+def test_matrix_vector_rows_shared_by_warps(cm, shape):
+    """Warps that begin and end within a row, without work, with an odd last row; rows that end within a step."""
+    w, x = lin_case((*shape, 2), 9)
+    ref = x.astype(np.float64) @ w.astype(np.float64).T
+    # a chain of a lane's eighths of the columns, then five additions of lanes and at most sixteen of warps, each within half an ulp
+    bound = 2.0 ** -24 * (shape[1] / 32 + 8 + 5 + 16) * (np.abs(x) @ np.abs(w).T)
+    for n in (1, 2):
+        assert (np.abs(linear(cm, 0, w, x[:n]) - ref[:n]) <= bound[:n]).all()
+
+
 def test_linear_activations(cm):
     w, x = lin_case((200, 96, 40), 3)
     ref = x.astype(np.float64) @ w.astype(np.float64).T
