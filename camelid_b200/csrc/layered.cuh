@@ -511,9 +511,9 @@ __device__ __forceinline__ float mix_coef(const StreamMix &m, int i) {
 }
 // The boundary of mixed streams for widths that are a multiple of four and at most 4 V blockDim.x: everything a thread reads is asked for
 // at once and the row stays in registers (stream_mix_row goes through shared memory value by value, with one global latency after the
-// other).  put(i, v) takes values 4i .. 4i + 3 of the result.  `coef` (kMixCoefs, shared memory) is complete after a barrier.
-__device__ __forceinline__ bool mix_row_fits(const StreamMix &m, int v) {
-  return m.mix && !m.embed && m.streams <= kMixStreams && m.width % 4 == 0 && m.width <= 4 * v * (int)blockDim.x;
+// other).  put(i, v) takes values 4i .. 4i + 3 of the result.  `coef` (kMixCoefs, shared memory) is complete after a barrier, which is here.
+__host__ __device__ __forceinline__ bool mix_row_fits(const StreamMix &m, int v, int threads) {
+  return m.mix && !m.embed && m.streams <= kMixStreams && m.width % 4 == 0 && m.width <= 4 * v * threads;
 }
 template <int V, typename Put>
 __device__ __forceinline__ void mix_row(const StreamMix &m, int64_t row, const float *coef, float *red, bool store, Put put) {
@@ -531,6 +531,7 @@ __device__ __forceinline__ void mix_row(const StreamMix &m, int64_t row, const f
 #pragma unroll
       for (int s = 0; s < kMixStreams; ++s) xv[j][s] = i < n4 && s < m.streams ? x[s * n4 + i] : zero;
     }
+    __syncthreads();
 #pragma unroll
     for (int j = 0; j < V; ++j) {
       const int i = threadIdx.x + j * blockDim.x;

@@ -108,7 +108,7 @@ __device__ __forceinline__ void lin_mv_cta(const LinMvArgs &a, int cta, int ctas
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  const bool mixed = a.prologue == kProStreams && mix_row_fits(a.mix, 2);
+  const bool mixed = a.prologue == kProStreams && mix_row_fits(a.mix, 2, kMvThreads);
   if (mixed && tid < kMixCoefs) coef[tid] = mix_coef(a.mix, tid);
   pdl_wait();
 
@@ -124,7 +124,6 @@ __device__ __forceinline__ void lin_mv_cta(const LinMvArgs &a, int cta, int ctas
       __syncthreads();
     }
     if (mixed) {
-      if (r == 0) __syncthreads();  // coef
       mix_row<2>(a.mix, a.mix.row_map ? a.mix.row_map[r] : r, coef, red, cta == 0, [&](int i, float4 v) { x4[mv_unit(i)] = v; });
     } else if (quads && a.prologue == kProPlain) {
       const float4 *x = reinterpret_cast<const float4 *>(a.x + r * a.x_ld);

@@ -163,6 +163,22 @@ def test_portions_longer_than_a_step(dtype):
     eng.close()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width, streams", [(1028, 3), (4096, 4), (4100, 2), (8196, 2)])
+def test_wide_streams(width, streams, dtype):
+    """Rows that fill the threads of a boundary partly, wholly, and not at all in registers; long and short portions, single tokens."""
+    cfg = lc.config([lc.with_mlp(lc.latent(heads=2, dim=16, vdim=8, q_rank=24, kv_rank=32), 40), lc.lightning(heads=2, dim=16, vdim=8, decay=[0.9, 1.0])],
+                    width=width, vocab=64, streams=streams)
+    params = lc.random_params(cfg, 37)
+    n = 290
+    toks = lc.tokens(cfg, n, 38)
+    ref, _ = lc.plain(params, cfg, toks)
+    eng = lc.engine(cfg, params, max_pos=n, max_seqs=2, dtype=dtype)
+    for i, parts in enumerate(([260, 30], [255, 33, 1, 1])):
+        check(feed(eng, i, toks, parts), ref, dtype, parts)
+    eng.close()
+
+
 # ---------------------------------------------------------------- one key among many
 
 def latent_needle(seed):
