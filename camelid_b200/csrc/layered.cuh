@@ -105,7 +105,11 @@ struct LinArgs {
   int32_t act = kActNone, act_rows = 0;
   const float *bias = nullptr;
   float scale = 1.0f;
+  float *parts = nullptr;     // tcgen05: kTcLinPart floats per SM and kTcLinTiles zeros, kept between launches of one stream; null: whole tiles only
+  int32_t *counts = nullptr;
 };
+constexpr int kTcLinCtas = 192, kTcLinTiles = 4096;
+constexpr int64_t kTcLinPart = 2 * 128 * 256;
 int32_t launch_lin_tc5(const LinArgs &a, int32_t sm_count, int32_t *status, bool pdl, cudaStream_t s);
 int32_t launch_lin_f32(const LinArgs &a, cudaStream_t s);
 
@@ -260,6 +264,13 @@ __device__ __forceinline__ float ld_peer(uint32_t local_addr, uint32_t rank) {
   float v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_peer4(uint32_t local_addr, uint32_t rank) {
+  uint32_t addr;
+  float4 v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local_addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
 }
 __device__ __forceinline__ void cp16(void *dst, const void *src, bool live) {

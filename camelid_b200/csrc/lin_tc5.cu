@@ -1,14 +1,20 @@
 // Linear layers on the 5th-generation tensor cores: out[r][o] = act(scale * sum_k w[o][k] x[r][k] + bias[o]), bfloat16
 // operands, f32 accumulators in tensor memory.
 //
-// The weights are operand A (tiles of 128 output rows), the activation rows operand B (tiles of BN rows), both K-major
+// The weights are operand A (tiles of 128 output rows), the activation rows operand B (tiles of n_tile rows, 16 to 256), both K-major
 // and brought by TMA in 128-byte-swizzled boxes of 64 columns.  Persistent CTAs, one per SM; warp roles:
-//   warp 0      TMA: operand stages (one elected lane)
-//   warp 1      MMA issue (one elected lane), tensor-memory allocation
-//   warps 2-9   epilogue: tcgen05.ld, activation, stores, two warps for each quarter of the accumulator lanes (every
+//   warps 0, 1  TMA: every other operand stage each (one elected lane)
+//   warp 2      MMA issue (one elected lane), tensor-memory allocation
+//   warps 3-10  epilogue: tcgen05.ld, activation, stores, two warps for each quarter of the accumulator lanes (every
 //               other 16 columns); two accumulator slots, so that a tile's epilogue overlaps the next tile's products
-// Few rows leave few tiles: then `split` CTAs of a thread-block cluster share a tile's inner dimension, leave their
-// partial accumulators in shared memory, and each of them adds the partials of its share of the columns in rank order.
+// Many rows: bound by what an SM takes from L2, about 64 bytes a cycle for the 128 + n_tile rows of a step.  The tiles that read the same weights
+// are neighbours, on different SMs at the same time, so that the weights come from HBM once and are in L2 for the others (tile after tile of
+// weights first: 22544 x 4096 with 2048 rows 369 us, now 280; 32000 x 4096 511 -> 394), and the rows are cut into as few tiles as there can be,
+// of equal size (300 rows as 2 x 160 in place of 2 x 256 or 5 x 64: 22544 x 4096 92 -> 69 us, 4096 x 14336 79 -> 47).
+// Few rows: bound by HBM, as far as every SM has as much to do.  Few tiles: `split` CTAs of a thread-block cluster share a tile's inner
+// dimension, leave their partial accumulators in shared memory, and each of them adds the partials of its share of the columns in rank order.
+// More tiles than SMs, but no multiple: all CTAs get equal runs of the steps of all tiles; partial accumulators go through global memory, and
+// whoever brings a tile's last one adds them in the order of the inner columns (22544 x 4096, 177 tiles, 8 rows: 45.6 -> 35.3 us).
 // The first weight boxes are asked for before the kernel waits for its predecessor.
 // Every wait is bounded: one that runs out sets the status word and an abort flag, all roles leave their loops, tensor
 // memory is freed and the kernel returns.
@@ -20,17 +26,19 @@ namespace cmld {
 
 namespace {
 
-constexpr int kEpiWarps = 8, kThreads = (2 + kEpiWarps) * 32, kBM = 128, kBK = 64;
+constexpr int kEpiWarps = 8, kThreads = (3 + kEpiWarps) * 32, kBM = 128, kBK = 64, kMaxStages = 8;
 constexpr uint32_t kSpin = 1u << 22;
 constexpr int kABytes = kBM * kBK * 2;
+constexpr int kBarBytes = 256, kSmem = 226 * 1024;
 
-constexpr int b_bytes(int bn) { return bn * kBK * 2; }
-constexpr int stages(int bn) { return bn == 256 ? 4 : bn == 128 ? 6 : 8; }
-constexpr int off_bars(int bn) { return stages(bn) * (kABytes + b_bytes(bn)); }
-constexpr int smem_bytes(int bn) { return off_bars(bn) + 256 + 1024; }  // + slack to align the base to 1024
+__host__ __device__ constexpr int stage_bytes(int n_tile) { return kABytes + n_tile * kBK * 2; }
+constexpr int stages(int n_tile) { return std::min(kMaxStages, (kSmem - kBarBytes - 1024) / stage_bytes(n_tile)); }
+constexpr int smem_bytes(int n_tile) { return stages(n_tile) * stage_bytes(n_tile) + kBarBytes + 1024; }  // + slack to align the base to 1024
 
 struct TcLinArgs {
-  int32_t m_rows, n_rows, n_k, tiles_m, tiles, split;
+  int32_t m_rows, n_rows, n_k, tiles_n, tiles, n_tile, split, whole, stages, slot_cols;
+  float *parts;     // [CTA][2][n_tile][kBM]: sums of a tile that other CTAs share
+  int32_t *counts;  // [tile]: contributions that have arrived; zero between launches
   void *out;
   int64_t out_ld;
   int32_t act, act_rows;
@@ -94,26 +102,31 @@ __device__ __forceinline__ void tmem_ld16(uint32_t t, float (&r)[16]) {
 __device__ __forceinline__ void put(float *p, float v) { *p = v; }
 __device__ __forceinline__ void put(bf16 *p, float v) { *p = __float2bfloat16_rn(v); }
 
-template <int BN, typename OutT>
+template <typename OutT>
 __global__ void __launch_bounds__(kThreads, 1)
     lin_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const TcLinArgs a) {
-  constexpr int NS = stages(BN);
-  constexpr int TSLOT = BN < 32 ? 32 : BN;                 // tensor-memory columns of one accumulator slot
-  constexpr uint32_t TCOLS = 2 * TSLOT;
-  constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+  const int NS = a.stages, stage = stage_bytes(a.n_tile);
   extern __shared__ uint8_t raw[];
   uint8_t *smem = raw + ((1024u - (s32(raw) & 1023u)) & 1023u);
-  const uint32_t base = s32(smem), bars = base + off_bars(BN);
+  const uint32_t base = s32(smem), bars = base + NS * stage;
   auto full = [&](int i) { return bars + 8u * i; };
-  auto empty = [&](int i) { return bars + 8u * (NS + i); };
-  auto acc_full = [&](int i) { return bars + 8u * (2 * NS + i); };
-  auto acc_empty = [&](int i) { return bars + 8u * (2 * NS + 2 + i); };
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + off_bars(BN) + 8 * (2 * NS + 4));
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  auto empty = [&](int i) { return bars + 8u * (kMaxStages + i); };
+  auto acc_full = [&](int i) { return bars + 8u * (2 * kMaxStages + i); };
+  auto acc_empty = [&](int i) { return bars + 8u * (2 * kMaxStages + 2 + i); };
+  const uint32_t met = bars + 8u * (2 * kMaxStages + 4);  // the epilogue warps among themselves
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + NS * stage + 8 * (2 * kMaxStages + 5));
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1), *last_flag = abort_flag + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // a cluster of `split` CTAs works on one tile, each on its share of the inner dimension
-  const int rank = (int)blockIdx.x % a.split, first = (int)blockIdx.x / a.split, step = (int)gridDim.x / a.split;
-  const int per = (a.n_k + a.split - 1) / a.split, k_lo = min(rank * per, a.n_k), k_hi = min(k_lo + per, a.n_k), nk = k_hi - k_lo;
+  // Whole tiles: every gridDim.x-th.  Otherwise a run of steps, step s being inner columns s % n_k of tile s / n_k: a cluster's CTAs share the
+  // steps of one tile out among them, or all CTAs those of all tiles.  Tiles that read the same weights are neighbours.
+  const int rank = (int)blockIdx.x % a.split;
+  auto first_step = [&](int cta) {
+    return a.split > 1 ? cta / a.split * a.n_k + a.n_k * (cta % a.split) / a.split : (int)((int64_t)a.tiles * a.n_k * cta / gridDim.x);
+  };
+  const int s_lo = a.whole ? 0 : first_step(blockIdx.x);
+  const int total = a.whole ? (a.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x * a.n_k + a.n_k : first_step(blockIdx.x + 1) - s_lo;  // steps of this CTA
+  const int t_lo = a.whole ? (int)blockIdx.x : s_lo / a.n_k, k_lo = s_lo % a.n_k, t_step = a.whole ? (int)gridDim.x : 1;
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.n_tile >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 
   if (tid == 0) {
     for (int i = 0; i < NS; ++i) {
@@ -124,11 +137,12 @@ __global__ void __launch_bounds__(kThreads, 1)
       bar_init(acc_full(i), 1);
       bar_init(acc_empty(i), kEpiWarps);
     }
+    bar_init(met, kEpiWarps);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"(TCOLS) : "memory");
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"(2 * a.slot_cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -137,83 +151,83 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tbase = *tmem_slot;
   pdl_launch();
 
-  if (warp == 0) {
+  if (warp < 2) {
+    // every other step each: waiting for a stage and issuing its two copies takes one thread longer than the products of a step
     if (lane == 0) {
-      const int n_mine = first < a.tiles ? (a.tiles - first + step - 1) / step : 0;
-      const int total = n_mine * nk;
-      auto load_w = [&](int q) {
-        const int t = first + (q / nk) * step, kb = k_lo + q % nk, st = q % NS;
-        bar_expect(full(st), kABytes + b_bytes(BN));
-        tma_2d(base + st * (kABytes + b_bytes(BN)), &wmap, kb * kBK, (t % a.tiles_m) * kBM, full(st));
-      };
-      auto load_x = [&](int q) {
-        const int t = first + (q / nk) * step, kb = k_lo + q % nk, st = q % NS;
-        tma_2d(base + st * (kABytes + b_bytes(BN)) + kABytes, &xmap, kb * kBK, (t / a.tiles_m) * BN, full(st));
-      };
       const int early = min(total, NS);
-      for (int q = 0; q < early; ++q) load_w(q);
+      int q, kb, t;
+      auto begin = [&] {
+        q = warp, kb = k_lo + warp, t = t_lo;
+        while (kb >= a.n_k) kb -= a.n_k, t += t_step;
+      };
+      auto advance = [&] {
+        q += 2, kb += 2;
+        while (kb >= a.n_k) kb -= a.n_k, t += t_step;
+      };
+      auto load_w = [&](int st) {
+        bar_expect(full(st), stage);
+        tma_2d(base + st * stage, &wmap, kb * kBK, t / a.tiles_n * kBM, full(st));
+      };
+      auto load_x = [&](int st) { tma_2d(base + st * stage + kABytes, &xmap, kb * kBK, t % a.tiles_n * a.n_tile, full(st)); };
+      for (begin(); q < early; advance()) load_w(q);
       pdl_wait();
-      for (int q = 0; q < early; ++q) load_x(q);
-      for (int q = early; q < total; ++q) {
-        if (!bar_wait(empty(q % NS), (uint32_t)((q / NS - 1) & 1), abort_flag, a.status)) break;
-        load_w(q);
-        load_x(q);
+      for (begin(); q < early; advance()) load_x(q);
+      int st = q - NS;
+      for (uint32_t parity = 0; q < total; advance()) {
+        if (!bar_wait(empty(st), parity, abort_flag, a.status)) break;
+        load_w(st);
+        load_x(st);
+        st += 2;
+        if (st >= NS) st -= NS, parity ^= 1;
       }
       if (*abort_flag) __nanosleep(1000000);  // copies in flight land before the shared memory is given back
     }
-  } else if (warp == 1) {
-    if (lane == 0 && nk > 0) {
-      int q = 0, i = 0;
+  } else if (warp == 2) {
+    if (lane == 0) {
+      int i = 0, st = 0;
+      uint32_t parity = 0;
       bool ok = true;
-      for (int t = first; t < a.tiles && ok; t += step, ++i) {
-        const int slot = i & 1;
+      for (int q = 0; q < total && ok; ++i) {
+        const int slot = i & 1, end = min(((k_lo + q) / a.n_k + 1) * a.n_k - k_lo, total);  // of this tile's steps here
         if (i >= 2) ok = bar_wait(acc_empty(slot), (uint32_t)((i / 2 - 1) & 1), abort_flag, a.status);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int kb = 0; kb < nk && ok; ++kb, ++q) {
-          const int st = q % NS;
-          ok = bar_wait(full(st), (uint32_t)((q / NS) & 1), abort_flag, a.status);
+        for (bool more = false; q < end && ok; ++q) {
+          ok = bar_wait(full(st), parity, abort_flag, a.status);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint64_t da = smem_desc(base + st * (kABytes + b_bytes(BN))), db = smem_desc(base + st * (kABytes + b_bytes(BN)) + kABytes);
+          const uint64_t da = smem_desc(base + st * stage), db = smem_desc(base + st * stage + kABytes);
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) mma_bf16(tbase + slot * TSLOT, da + 2 * k, db + 2 * k, kIdesc, kb > 0 || k > 0);
+          for (int k = 0; k < kBK / 16; ++k) {
+            mma_bf16(tbase + slot * a.slot_cols, da + 2 * k, db + 2 * k, idesc, more);
+            more = true;
+          }
           mma_commit(empty(st));
+          if (++st == NS) st = 0, parity ^= 1;
         }
         if (ok) mma_commit(acc_full(slot));
       }
     }
     __syncwarp();
   } else {
-    const int quarter = warp & 3, half = (warp - 2) >> 2;  // the 32 accumulator lanes this warp may read; its column groups
+    const int quarter = warp & 3, half = (warp - 3) >> 2;  // the 32 accumulator lanes this warp may read; its column groups
     pdl_wait();                    // the output buffer may still be read by the predecessor
     int i = 0;
+    uint32_t meetings = 0;
     OutT *out = static_cast<OutT *>(a.out);
-    for (int t = first; t < a.tiles; t += step, ++i) {
-      const int slot = i & 1, o = (t % a.tiles_m) * kBM + quarter * 32 + lane, n0 = (t / a.tiles_m) * BN;
-      if (nk > 0) {
-        if (!bar_wait(acc_full(slot), (uint32_t)((i / 2) & 1), abort_flag, a.status)) break;
-      }
+    for (int q = 0, t = t_lo; q < total; ++i, t += t_step) {
+      const int end = min(((k_lo + q) / a.n_k + 1) * a.n_k - k_lo, total);
+      const bool all = end - q == a.n_k;  // else other CTAs add to this tile
+      q = end;
+      const int slot = i & 1, o = (t / a.tiles_n) * kBM + quarter * 32 + lane, n0 = (t % a.tiles_n) * a.n_tile;
+      if (!bar_wait(acc_full(slot), (uint32_t)((i / 2) & 1), abort_flag, a.status)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int n_live = min(BN, a.n_rows - n0);
-      float *part = reinterpret_cast<float *>(smem);  // [BN][128]: the operand stages are free by now
+      const int n_live = min(a.n_tile, a.n_rows - n0);
       const bool silu = a.act == kActSilu && o < a.act_rows, relu2 = a.act == kActRelu2, swiglu = a.act == kActSwiGlu;
       const float bias = a.bias && o < a.m_rows ? a.bias[o] : 0.0f;
       const bool odd = lane & 1;
-      OutT *p = out + (int64_t)(n0 + 16 * half) * a.out_ld + (swiglu ? o >> 1 : o);
-#pragma unroll 1
-      for (int c = 16 * half; c < n_live; c += 32, p += 32 * a.out_ld) {
-        float r[16];
-        if (nk > 0) {
-          tmem_ld16(tbase + slot * TSLOT + c + ((uint32_t)(quarter * 32) << 16), r);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) r[j] = 0.0f;
-        }
-        if (a.split > 1) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) part[(c + j) * kBM + quarter * 32 + lane] = r[j];
-          continue;
-        }
+      // columns c .. c + 15 of the tile
+      auto finish = [&](int c, float (&r)[16]) {
+        OutT *p = out + (int64_t)(n0 + c) * a.out_ld + (swiglu ? o >> 1 : o);
 #pragma unroll
         for (int j = 0; j < 16; ++j) r[j] = fmaf(r[j], a.scale, bias);
         if (swiglu) {
@@ -226,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const float v = odd ? silu_f(t) * r[j + 1] : silu_f(r[j]) * t;
             if (o < a.m_rows && c + j + (odd ? 1 : 0) < n_live) put(w, v);
           }
-          continue;
+          return;
         }
         if (silu) {
 #pragma unroll
@@ -249,35 +263,92 @@ __global__ void __launch_bounds__(kThreads, 1)
               if (c + j < n_live) put(w, r[j]);
           }
         }
+      };
+      auto part_of = [&](int cta) {
+        return a.parts + ((int64_t)cta * 2 + (t == first_step(cta) / a.n_k ? 0 : 1)) * a.n_tile * kBM + quarter * 32 + lane;
+      };
+      float *mine = all || a.split > 1 ? nullptr : part_of(blockIdx.x);
+#pragma unroll 1
+      for (int c = 16 * half; c < n_live; c += 32) {
+        float r[16];
+        tmem_ld16(tbase + slot * a.slot_cols + c + ((uint32_t)(quarter * 32) << 16), r);
+        if (all) {
+          finish(c, r);
+        } else if (a.split > 1) {
+          float *part = reinterpret_cast<float *>(smem);  // [n_tile][128]: the operand stages are free by now
+#pragma unroll
+          for (int j = 0; j < 16; ++j) part[(c + j) * kBM + quarter * 32 + lane] = r[j];
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) __stcg(mine + (c + j) * kBM, r[j]);
+        }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) bar_arrive(acc_empty(slot));
+      if (all || a.split > 1) continue;
+      // whoever brings the last contribution adds them all, in the order of the inner columns
+      const int64_t steps = (int64_t)a.tiles * a.n_k;
+      auto cta_of = [&](int64_t s) { return (int)(((s + 1) * gridDim.x - 1) / steps); };
+      const int c_lo = cta_of((int64_t)t * a.n_k), c_hi = cta_of((int64_t)(t + 1) * a.n_k - 1);
+      auto meet = [&] {
+        __syncwarp();
+        if (lane == 0) bar_arrive(met);
+        meetings ^= 1;
+        return bar_wait(met, meetings ^ 1, abort_flag, a.status);
+      };
+      __threadfence();
+      if (!meet()) break;
+      if (tid == 96) {
+        const int came = atomicAdd(a.counts + t, 1);
+        *last_flag = came == c_hi - c_lo;
+        if (came == c_hi - c_lo) a.counts[t] = 0;
+      }
+      if (!meet()) break;
+      if (!*last_flag) continue;
+      __threadfence();
+#pragma unroll 1
+      for (int c = 16 * half; c < n_live; c += 32) {
+        float r[16] = {};
+#pragma unroll 2
+        for (int cta = c_lo; cta <= c_hi; ++cta) {
+          const float *p = part_of(cta) + c * kBM;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) r[j] += __ldcg(p + j * kBM);
+        }
+        finish(c, r);
+      }
     }
   }
   __syncwarp();
   if (a.split > 1) {
     // one tile per cluster: add the partial accumulators, column by column, in rank order
     cluster_sync();
-    if (first < a.tiles && !*abort_flag) {
+    if (!*abort_flag) {
       OutT *out = static_cast<OutT *>(a.out);
-      const int m0 = (first % a.tiles_m) * kBM, n0 = (first / a.tiles_m) * BN, n_live = min(BN, a.n_rows - n0);
-      auto total = [&](int e, int o) {
-        float v = 0.0f;
-        for (int p = 0; p < a.split; ++p) v += ld_peer(base + 4u * e, p);
-        return fmaf(v, a.scale, a.bias && o < a.m_rows ? a.bias[o] : 0.0f);
-      };
-      if (a.act == kActSwiGlu) {
-        for (int e = 2 * (rank * kThreads + tid); e < n_live * kBM; e += 2 * a.split * kThreads) {
-          const int o = m0 + e % kBM, n = e / kBM;
-          const float v = silu_f(total(e, o)) * total(e + 1, o + 1);
-          if (o < a.m_rows) put(out + (int64_t)(n0 + n) * a.out_ld + (o >> 1), v);
-        }
-      } else {
-        for (int e = rank * kThreads + tid; e < n_live * kBM; e += a.split * kThreads) {
-          const int o = m0 + e % kBM, n = e / kBM;
-          const float v = total(e, o);
-          if (o < a.m_rows) put(out + (int64_t)(n0 + n) * a.out_ld + o, lin_activate(v, a.act, o < a.act_rows));
+      const int t = (int)blockIdx.x / a.split, m0 = (t / a.tiles_n) * kBM, n0 = (t % a.tiles_n) * a.n_tile, n_live = min(a.n_tile, a.n_rows - n0);
+      for (int e = 4 * (rank * kThreads + tid); e < n_live * kBM; e += 4 * a.split * kThreads) {  // four rows of a column
+        const int o = m0 + e % kBM;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float4 u[8];
+#pragma unroll
+        for (int p = 0; p < 8; ++p)
+          if (p < a.split) u[p] = ld_peer4(base + 4u * e, p);
+#pragma unroll
+        for (int p = 0; p < 8; ++p)
+          if (p < a.split) v = make_float4(v.x + u[p].x, v.y + u[p].y, v.z + u[p].z, v.w + u[p].w);
+        float r[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[j] = fmaf(r[j], a.scale, a.bias && o + j < a.m_rows ? a.bias[o + j] : 0.0f);
+        OutT *p = out + (int64_t)(n0 + e / kBM) * a.out_ld;
+        if (a.act == kActSwiGlu) {
+#pragma unroll
+          for (int j = 0; j < 4; j += 2)
+            if (o + j < a.m_rows) put(p + ((o + j) >> 1), silu_f(r[j]) * r[j + 1]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (o + j < a.m_rows) put(p + o + j, lin_activate(r[j], a.act, o + j < a.act_rows));
         }
       }
     }
@@ -286,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(TCOLS) : "memory");
+  if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(2 * a.slot_cols) : "memory");
 }
 
 typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
@@ -310,22 +381,33 @@ int32_t make_map(CUtensorMap *map, const void *p, int64_t cols, int64_t rows, in
   return CMLD_OK;
 }
 
-template <int BN, typename OutT>
-int32_t launch_bn(const LinArgs &L, int32_t sms, int32_t *status, bool pdl, cudaStream_t s) {
+template <typename OutT>
+int32_t launch_out(const LinArgs &L, int32_t sms, int32_t *status, bool pdl, cudaStream_t s) {
   static SmemLimit limit;
-  CMLD_TRY(allow_smem(limit, lin_tc5_kernel<BN, OutT>, smem_bytes(BN), true));
+  CMLD_TRY(allow_smem(limit, lin_tc5_kernel<OutT>, kSmem, true));
+  const int parts = (L.rows + 255) / 256, n_tile = ((L.rows + parts - 1) / parts + 15) & ~15;
   CUtensorMap wmap, xmap;
   CMLD_TRY(make_map(&wmap, L.w.w, L.w.cols, L.w.rows, L.w.ld, kBM));
-  CMLD_TRY(make_map(&xmap, L.x, L.w.cols, L.rows, L.x_ld, BN));
+  CMLD_TRY(make_map(&xmap, L.x, L.w.cols, L.rows, L.x_ld, n_tile));
   TcLinArgs a{};
   a.m_rows = L.w.rows;
   a.n_rows = L.rows;
   a.n_k = (L.w.cols + kBK - 1) / kBK;
-  a.tiles_m = (L.w.rows + kBM - 1) / kBM;
-  a.tiles = a.tiles_m * ((L.rows + BN - 1) / BN);
+  a.n_tile = n_tile;
+  a.stages = stages(n_tile);
+  a.slot_cols = 32;
+  while (a.slot_cols < n_tile) a.slot_cols *= 2;
+  a.tiles_n = (L.rows + n_tile - 1) / n_tile;
+  a.tiles = (L.w.rows + kBM - 1) / kBM * a.tiles_n;
   a.split = 1;
-  if (BN <= 64)  // few rows: spread a tile's inner dimension until the machine is full
-    while (a.split < 8 && a.tiles * a.split * 2 <= sms && a.n_k >= 4 * a.split) a.split *= 2;
+  // few tiles: spread a tile's inner dimension until the machine is full
+  while (a.split < 8 && a.tiles * a.split * 2 <= sms && a.n_k >= 4 * a.split) a.split *= 2;
+  // Whole tiles where they keep four fifths of the SMs busy (224 tiles, 8 rows: 46.1 us, as equal runs 42.6; 250 tiles: 46.4, 46.9) or the partial
+  // accumulators are large (224 tiles, 150 rows: 54 us, as equal runs 58).
+  const int rounds = (a.tiles + sms - 1) / sms;
+  a.whole = a.split == 1 && (!L.parts || n_tile > 64 || sms > kTcLinCtas || a.tiles <= sms || a.tiles > kTcLinTiles || a.tiles * 5 >= rounds * sms * 4);
+  a.parts = L.parts;
+  a.counts = L.counts;
   a.out = L.out;
   a.out_ld = L.out_ld;
   a.act = L.act;
@@ -336,7 +418,7 @@ int32_t launch_bn(const LinArgs &L, int32_t sms, int32_t *status, bool pdl, cuda
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(a.split > 1 ? a.tiles * a.split : std::min(a.tiles, sms)));
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem_bytes(BN);
+  cfg.dynamicSmemBytes = smem_bytes(n_tile);
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
   int n = 0;
@@ -352,18 +434,8 @@ int32_t launch_bn(const LinArgs &L, int32_t sms, int32_t *status, bool pdl, cuda
   }
   cfg.attrs = attr;
   cfg.numAttrs = n;
-  CMLD_CUDA(cudaLaunchKernelEx(&cfg, lin_tc5_kernel<BN, OutT>, wmap, xmap, a));
+  CMLD_CUDA(cudaLaunchKernelEx(&cfg, lin_tc5_kernel<OutT>, wmap, xmap, a));
   return CMLD_OK;
-}
-
-template <typename OutT>
-int32_t launch_out(const LinArgs &a, int32_t sms, int32_t *status, bool pdl, cudaStream_t s) {
-  if (a.rows <= 16) return launch_bn<16, OutT>(a, sms, status, pdl, s);
-  if (a.rows <= 32) return launch_bn<32, OutT>(a, sms, status, pdl, s);
-  const int64_t tm = (a.w.rows + kBM - 1) / kBM;
-  if (a.rows <= 64 || tm * ((a.rows + 127) / 128) * 2 <= sms) return launch_bn<64, OutT>(a, sms, status, pdl, s);
-  if (tm * ((a.rows + 255) / 256) <= sms / 2) return launch_bn<128, OutT>(a, sms, status, pdl, s);
-  return launch_bn<256, OutT>(a, sms, status, pdl, s);
 }
 
 }  // namespace

@@ -85,6 +85,25 @@ def test_matrix_vector_rows_shared_by_warps(cm, shape):
         assert (np.abs(linear(cm, 0, w, x[:n]) - ref[:n]) <= bound[:n]).all()
 
 
+@pytest.mark.parametrize("shape", [(19200, 72, 8), (19100, 520, 33), (22544, 136, 64), (40000, 200, 16), (1000, 392, 300), (260, 2056, 412), (19000, 64, 150),
+                                   (128, 4096, 350)])
+def test_linear_tiles_shared_out(cm, shape):
+    """Tiles that several CTAs add up, through global memory or a cluster, launch after launch; row tiles of every number of operand stages."""
+    import ctypes as C
+
+    from camelid_b200._lib import check as ok
+    from camelid_b200.engine import DeviceBuffer
+
+    w, x = lin_case(shape, 11)
+    v = lin_case(shape, 12)[0]
+    wd, xd, out, ms = device_rows(np.concatenate([w, v]), True), device_rows(x, True), DeviceBuffer(shape[0] * shape[2] * 4), C.c_float(0)
+    # the launches take w and v in turn; the last one takes v
+    ok(cm.lib().cmld_linear(1, wd.ptr, shape[0], shape[1], xd.ptr, shape[2], out.ptr, 0, 0, 0, None, 1.0, 2, 2, C.byref(ms)))
+    # a chain of all products, every addition within an ulp (the accumulator's own may truncate)
+    bound = 2.0 ** -23 * (shape[1] + 8) * (np.abs(x) @ np.abs(v).T)
+    assert (np.abs(out.to_numpy(np.float32).reshape(shape[2], shape[0]) - x.astype(np.float64) @ v.astype(np.float64).T) <= bound).all()
+
+
 def test_linear_activations(cm):
     w, x = lin_case((200, 96, 40), 3)
     ref = x.astype(np.float64) @ w.astype(np.float64).T
