@@ -1101,7 +1101,6 @@ int32_t finish(cmld_engine *e, const char *what) {
   if (ce != cudaSuccess) return fail(CMLD_ERR_CUDA, "%s: %s", what, cudaGetErrorString(ce));
   if (st != 0) {
     cudaMemsetAsync(e->d_status, 0, 4, e->stream);
-    if (e->lay) layered_clear(e);
     return fail(st, "%s: a bounded device-side wait gave up (status %d); results of this call are invalid", what, st);
   }
   return CMLD_OK;

@@ -180,7 +180,6 @@ int32_t init_rows(cmld_engine *e, int64_t rows, int64_t logit_rows, int64_t voca
 void layered_free(cmld_engine *e);
 int32_t layered_ready(const cmld_engine *e, bool report);  // 1: every tensor is set; `report`: leave an error message if not
 int32_t layered_step(cmld_engine *e, const StepOpts &o);
-void layered_clear(cmld_engine *e);  // after a device-side wait that gave up
 int32_t layered_claim(cmld_engine *e, int32_t n, const int32_t *seqs, const int64_t *positions);
 void layered_advance(cmld_engine *e, int32_t n, const int32_t *seqs, const int64_t *positions, int64_t steps);
 int32_t layered_extend(cmld_engine *e, int32_t seq, const int32_t *tokens, int64_t n, int64_t start, const int32_t *want, int32_t n_want,

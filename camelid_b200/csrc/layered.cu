@@ -87,8 +87,6 @@ struct LayeredModel {
   float *x[2] = {}, *y = nullptr, *proj = nullptr, *q = nullptr, *qa = nullptr, *part = nullptr, *taps = nullptr;
   void *act = nullptr, *wide = nullptr, *mixed = nullptr, *hidden = nullptr;  // bf16 or f32
   bf16 *kv = nullptr;
-  float *lin_parts = nullptr;  // see LinArgs
-  int32_t *lin_counts = nullptr;
   float *y2 = nullptr, *linear_out = nullptr;  // parallel: the second branch's result; what its recurrence gave
   uint8_t *chunks = nullptr;                   // parallel: scratch of the chunked recurrence
   int32_t *row_map = nullptr;
@@ -421,8 +419,6 @@ int32_t build(cmld_engine *e, LayeredModel *m) {
   CMLD_TRY(dev_alloc(e, &f, R * ff));
   m->hidden = f;
   if (kv > 0) CMLD_TRY(dev_alloc(e, &m->kv, c.max_pos * kv));
-  CMLD_TRY(dev_alloc(e, &m->lin_parts, m->f32 ? 1 : std::min(e->sm_count, kTcLinCtas) * kTcLinPart, false));
-  CMLD_TRY(dev_alloc(e, &m->lin_counts, kTcLinTiles));
   if (linear > 0) {
     CMLD_TRY(dev_alloc(e, &m->linear_out, R * linear));
     CMLD_TRY(dev_alloc(e, &m->y2, R * c.width));
@@ -535,8 +531,6 @@ struct Step {
     a.act_rows = act_rows;
     a.bias = bias;
     a.scale = scale;
-    a.parts = m->lin_parts;
-    a.counts = m->lin_counts;
     e->launches += 1;
     return x.half ? launch_lin_tc5(a, e->sm_count, e->d_status, pdl, e->stream) : launch_lin_f32(a, e->stream);
   }
@@ -856,8 +850,6 @@ bool all_fit_mv(const LayeredModel *m, int32_t R) {
 
 }  // namespace
 
-void layered_clear(cmld_engine *e) { cudaMemsetAsync(e->lay->lin_counts, 0, 4 * kTcLinTiles, e->stream); }
-
 int32_t layered_step(cmld_engine *e, const StepOpts &o) {
   LayeredModel *m = e->lay;
   const int32_t R = o.batch;
@@ -1162,13 +1154,6 @@ int32_t cmld_linear(int32_t kernel, const void *w_dev, int64_t rows, int64_t col
   auto cuda = [&](cudaError_t ce) {
     if (rc == CMLD_OK && ce != cudaSuccess) rc = fail(CMLD_ERR_CUDA, "linear: %s", cudaGetErrorString(ce));
   };
-  float *parts = nullptr;
-  int32_t *counts = nullptr;
-  if (kernel == 1) {
-    cuda(cudaMalloc(&parts, sizeof(float) * kTcLinCtas * kTcLinPart));
-    cuda(cudaMalloc(&counts, 4 * kTcLinTiles));
-    if (rc == CMLD_OK) cuda(cudaMemsetAsync(counts, 0, 4 * kTcLinTiles, s));
-  }
   cuda(cudaMalloc(&status, 4));
   if (rc == CMLD_OK) cuda(cudaMemsetAsync(status, 0, 4, s));
   int sms = 148, dev = 0;
@@ -1203,8 +1188,6 @@ int32_t cmld_linear(int32_t kernel, const void *w_dev, int64_t rows, int64_t col
     a.act_rows = act_rows;
     a.bias = bias_dev;
     a.scale = scale;
-    a.parts = parts;
-    a.counts = counts;
     return kernel == 1 ? launch_lin_tc5(a, sms, status, pdl, s) : launch_lin_f32(a, s);
   };
   if (rc == CMLD_OK) rc = once(0, false);
@@ -1237,8 +1220,6 @@ int32_t cmld_linear(int32_t kernel, const void *w_dev, int64_t rows, int64_t col
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   cudaFree(status);
-  cudaFree(parts);
-  cudaFree(counts);
   cudaStreamDestroy(s);
   return rc;
 }

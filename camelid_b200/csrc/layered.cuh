@@ -105,11 +105,7 @@ struct LinArgs {
   int32_t act = kActNone, act_rows = 0;
   const float *bias = nullptr;
   float scale = 1.0f;
-  float *parts = nullptr;     // tcgen05: kTcLinPart floats per SM and kTcLinTiles zeros, kept between launches of one stream; null: whole tiles only
-  int32_t *counts = nullptr;
 };
-constexpr int kTcLinCtas = 192, kTcLinTiles = 4096;
-constexpr int64_t kTcLinPart = 2 * 128 * 256;
 int32_t launch_lin_tc5(const LinArgs &a, int32_t sm_count, int32_t *status, bool pdl, cudaStream_t s);
 int32_t launch_lin_f32(const LinArgs &a, cudaStream_t s);
 
@@ -526,7 +522,7 @@ __device__ __forceinline__ float mix_coef(const StreamMix &m, int i) {
 __host__ __device__ __forceinline__ bool mix_row_fits(const StreamMix &m, int v, int threads) {
   return m.mix && !m.embed && m.streams <= kMixStreams && m.width % 4 == 0 && m.width <= 4 * v * threads;
 }
-template <int V, typename Put>
+template <int V, bool NORM = true, typename Put>
 __device__ __forceinline__ void mix_row(const StreamMix &m, int64_t row, const float *coef, float *red, bool store, Put put) {
   const int n4 = m.width / 4;
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -561,7 +557,7 @@ __device__ __forceinline__ void mix_row(const StreamMix &m, int64_t row, const f
       }
     }
   }
-  if (m.norm_w) {  // the formulas of layer_norm_cta and rms_norm_cta
+  if (NORM && m.norm_w) {  // the formulas of layer_norm_cta and rms_norm_cta
     const float4 *nw = reinterpret_cast<const float4 *>(m.norm_w), *nb = reinterpret_cast<const float4 *>(m.norm_b);
     float4 w[V], b[V];
 #pragma unroll

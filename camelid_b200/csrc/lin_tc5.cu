@@ -8,13 +8,12 @@
 //   warps 3-10  epilogue: tcgen05.ld, activation, stores, two warps for each quarter of the accumulator lanes (every
 //               other 16 columns); two accumulator slots, so that a tile's epilogue overlaps the next tile's products
 // Many rows: bound by what an SM takes from L2, about 64 bytes a cycle for the 128 + n_tile rows of a step.  The tiles that read the same weights
-// are neighbours, on different SMs at the same time, so that the weights come from HBM once and are in L2 for the others (tile after tile of
-// weights first: 22544 x 4096 with 2048 rows 369 us, now 280; 32000 x 4096 511 -> 394), and the rows are cut into as few tiles as there can be,
-// of equal size (300 rows as 2 x 160 in place of 2 x 256 or 5 x 64: 22544 x 4096 92 -> 69 us, 4096 x 14336 79 -> 47).
+// are neighbours, on different SMs at the same time, so that the weights come from HBM once and are in L2 for the others (all
+// weights for each tile of rows: 22544 x 4096 with 2048 rows 369 us, now 275; 32000 x 4096 511 -> 389), and the rows are cut into tiles that fill the SMs,
+// of equal size (300 rows as 2 x 160 in place of 2 x 256 or 4 x 80 in place of 5 x 64: 22544 x 4096 92 -> 63 us, 4096 x 14336 79 -> 66).
 // Few rows: bound by HBM, as far as every SM has as much to do.  Few tiles: `split` CTAs of a thread-block cluster share a tile's inner
 // dimension, leave their partial accumulators in shared memory, and each of them adds the partials of its share of the columns in rank order.
-// More tiles than SMs, but no multiple: all CTAs get equal runs of the steps of all tiles; partial accumulators go through global memory, and
-// whoever brings a tile's last one adds them in the order of the inner columns (22544 x 4096, 177 tiles, 8 rows: 45.6 -> 35.3 us).
+// (All CTAs with equal runs of the steps of all tiles took 22544 x 4096 with 8 rows from 45.6 to 35.3 us, but adds in another order.)
 // The first weight boxes are asked for before the kernel waits for its predecessor.
 // Every wait is bounded: one that runs out sets the status word and an abort flag, all roles leave their loops, tensor
 // memory is freed and the kernel returns.
@@ -36,9 +35,7 @@ constexpr int stages(int n_tile) { return std::min(kMaxStages, (kSmem - kBarByte
 constexpr int smem_bytes(int n_tile) { return stages(n_tile) * stage_bytes(n_tile) + kBarBytes + 1024; }  // + slack to align the base to 1024
 
 struct TcLinArgs {
-  int32_t m_rows, n_rows, n_k, tiles_n, tiles, n_tile, split, whole, stages, slot_cols;
-  float *parts;     // [CTA][2][n_tile][kBM]: sums of a tile that other CTAs share
-  int32_t *counts;  // [tile]: contributions that have arrived; zero between launches
+  int32_t m_rows, n_rows, n_k, tiles_n, tiles, n_tile, split, stages, slot_cols;
   void *out;
   int64_t out_ld;
   int32_t act, act_rows;
@@ -113,19 +110,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   auto empty = [&](int i) { return bars + 8u * (kMaxStages + i); };
   auto acc_full = [&](int i) { return bars + 8u * (2 * kMaxStages + i); };
   auto acc_empty = [&](int i) { return bars + 8u * (2 * kMaxStages + 2 + i); };
-  const uint32_t met = bars + 8u * (2 * kMaxStages + 4);  // the epilogue warps among themselves
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + NS * stage + 8 * (2 * kMaxStages + 5));
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1), *last_flag = abort_flag + 1;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + NS * stage + 8 * (2 * kMaxStages + 4));
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // Whole tiles: every gridDim.x-th.  Otherwise a run of steps, step s being inner columns s % n_k of tile s / n_k: a cluster's CTAs share the
-  // steps of one tile out among them, or all CTAs those of all tiles.  Tiles that read the same weights are neighbours.
-  const int rank = (int)blockIdx.x % a.split;
-  auto first_step = [&](int cta) {
-    return a.split > 1 ? cta / a.split * a.n_k + a.n_k * (cta % a.split) / a.split : (int)((int64_t)a.tiles * a.n_k * cta / gridDim.x);
-  };
-  const int s_lo = a.whole ? 0 : first_step(blockIdx.x);
-  const int total = a.whole ? (a.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x * a.n_k + a.n_k : first_step(blockIdx.x + 1) - s_lo;  // steps of this CTA
-  const int t_lo = a.whole ? (int)blockIdx.x : s_lo / a.n_k, k_lo = s_lo % a.n_k, t_step = a.whole ? (int)gridDim.x : 1;
+  // A cluster of `split` CTAs works on one tile, each on its share of the inner columns.  Tiles that read the same weights are neighbours.
+  const int rank = (int)blockIdx.x % a.split, per = (a.n_k + a.split - 1) / a.split, k_lo = min(rank * per, a.n_k), nk = min(k_lo + per, a.n_k) - k_lo;
+  const int t_lo = (int)blockIdx.x / a.split, t_step = (int)gridDim.x / a.split;
+  const int total = t_lo < a.tiles ? ((a.tiles - 1 - t_lo) / t_step + 1) * nk : 0;  // steps of this CTA
   const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.n_tile >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 
   if (tid == 0) {
@@ -137,7 +128,6 @@ __global__ void __launch_bounds__(kThreads, 1)
       bar_init(acc_full(i), 1);
       bar_init(acc_empty(i), kEpiWarps);
     }
-    bar_init(met, kEpiWarps);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -153,16 +143,16 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp < 2) {
     // every other step each: waiting for a stage and issuing its two copies takes one thread longer than the products of a step
-    if (lane == 0) {
+    if (lane == 0 && total > 0) {
       const int early = min(total, NS);
       int q, kb, t;
       auto begin = [&] {
         q = warp, kb = k_lo + warp, t = t_lo;
-        while (kb >= a.n_k) kb -= a.n_k, t += t_step;
+        while (kb >= k_lo + nk) kb -= nk, t += t_step;
       };
       auto advance = [&] {
         q += 2, kb += 2;
-        while (kb >= a.n_k) kb -= a.n_k, t += t_step;
+        while (kb >= k_lo + nk) kb -= nk, t += t_step;
       };
       auto load_w = [&](int st) {
         bar_expect(full(st), stage);
@@ -188,7 +178,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t parity = 0;
       bool ok = true;
       for (int q = 0; q < total && ok; ++i) {
-        const int slot = i & 1, end = min(((k_lo + q) / a.n_k + 1) * a.n_k - k_lo, total);  // of this tile's steps here
+        const int slot = i & 1, end = q + nk;
         if (i >= 2) ok = bar_wait(acc_empty(slot), (uint32_t)((i / 2 - 1) & 1), abort_flag, a.status);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (bool more = false; q < end && ok; ++q) {
@@ -212,12 +202,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int quarter = warp & 3, half = (warp - 3) >> 2;  // the 32 accumulator lanes this warp may read; its column groups
     pdl_wait();                    // the output buffer may still be read by the predecessor
     int i = 0;
-    uint32_t meetings = 0;
     OutT *out = static_cast<OutT *>(a.out);
-    for (int q = 0, t = t_lo; q < total; ++i, t += t_step) {
-      const int end = min(((k_lo + q) / a.n_k + 1) * a.n_k - k_lo, total);
-      const bool all = end - q == a.n_k;  // else other CTAs add to this tile
-      q = end;
+    for (int q = 0, t = t_lo; q < total; ++i, q += nk, t += t_step) {
       const int slot = i & 1, o = (t / a.tiles_n) * kBM + quarter * 32 + lane, n0 = (t % a.tiles_n) * a.n_tile;
       if (!bar_wait(acc_full(slot), (uint32_t)((i / 2) & 1), abort_flag, a.status)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -264,60 +250,21 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       };
-      auto part_of = [&](int cta) {
-        return a.parts + ((int64_t)cta * 2 + (t == first_step(cta) / a.n_k ? 0 : 1)) * a.n_tile * kBM + quarter * 32 + lane;
-      };
-      float *mine = all || a.split > 1 ? nullptr : part_of(blockIdx.x);
 #pragma unroll 1
       for (int c = 16 * half; c < n_live; c += 32) {
         float r[16];
         tmem_ld16(tbase + slot * a.slot_cols + c + ((uint32_t)(quarter * 32) << 16), r);
-        if (all) {
+        if (a.split == 1) {
           finish(c, r);
-        } else if (a.split > 1) {
+        } else {
           float *part = reinterpret_cast<float *>(smem);  // [n_tile][128]: the operand stages are free by now
 #pragma unroll
           for (int j = 0; j < 16; ++j) part[(c + j) * kBM + quarter * 32 + lane] = r[j];
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) __stcg(mine + (c + j) * kBM, r[j]);
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) bar_arrive(acc_empty(slot));
-      if (all || a.split > 1) continue;
-      // whoever brings the last contribution adds them all, in the order of the inner columns
-      const int64_t steps = (int64_t)a.tiles * a.n_k;
-      auto cta_of = [&](int64_t s) { return (int)(((s + 1) * gridDim.x - 1) / steps); };
-      const int c_lo = cta_of((int64_t)t * a.n_k), c_hi = cta_of((int64_t)(t + 1) * a.n_k - 1);
-      auto meet = [&] {
-        __syncwarp();
-        if (lane == 0) bar_arrive(met);
-        meetings ^= 1;
-        return bar_wait(met, meetings ^ 1, abort_flag, a.status);
-      };
-      __threadfence();
-      if (!meet()) break;
-      if (tid == 96) {
-        const int came = atomicAdd(a.counts + t, 1);
-        *last_flag = came == c_hi - c_lo;
-        if (came == c_hi - c_lo) a.counts[t] = 0;
-      }
-      if (!meet()) break;
-      if (!*last_flag) continue;
-      __threadfence();
-#pragma unroll 1
-      for (int c = 16 * half; c < n_live; c += 32) {
-        float r[16] = {};
-#pragma unroll 2
-        for (int cta = c_lo; cta <= c_hi; ++cta) {
-          const float *p = part_of(cta) + c * kBM;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) r[j] += __ldcg(p + j * kBM);
-        }
-        finish(c, r);
-      }
     }
   }
   __syncwarp();
@@ -333,10 +280,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         float4 u[8];
 #pragma unroll
         for (int p = 0; p < 8; ++p)
-          if (p < a.split) u[p] = ld_peer4(base + 4u * e, p);
+          if (p * per < a.n_k && p < a.split) u[p] = ld_peer4(base + 4u * e, p);
 #pragma unroll
         for (int p = 0; p < 8; ++p)
-          if (p < a.split) v = make_float4(v.x + u[p].x, v.y + u[p].y, v.z + u[p].z, v.w + u[p].w);
+          if (p * per < a.n_k && p < a.split) v = make_float4(v.x + u[p].x, v.y + u[p].y, v.z + u[p].z, v.w + u[p].w);
         float r[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) r[j] = fmaf(r[j], a.scale, a.bias && o + j < a.m_rows ? a.bias[o + j] : 0.0f);
@@ -385,29 +332,35 @@ template <typename OutT>
 int32_t launch_out(const LinArgs &L, int32_t sms, int32_t *status, bool pdl, cudaStream_t s) {
   static SmemLimit limit;
   CMLD_TRY(allow_smem(limit, lin_tc5_kernel<OutT>, kSmem, true));
-  const int parts = (L.rows + 255) / 256, n_tile = ((L.rows + parts - 1) / parts + 15) & ~15;
+  // Row tiles of equal size, as many as make (rounds over the SMs) x (rows of both operands that an SM takes in a step) least.
+  const int n_k = (L.w.cols + kBK - 1) / kBK, tiles_m = (L.w.rows + kBM - 1) / kBM;
+  int n_tile = 0;
+  int64_t least = 0;
+  for (int parts = (L.rows + 255) / 256; parts <= (L.rows + 63) / 64; ++parts) {
+    const int n = ((L.rows + parts - 1) / parts + 15) & ~15;
+    const int64_t rounds = ((int64_t)tiles_m * ((L.rows + n - 1) / n) + sms - 1) / sms, cost = rounds * (kBM + n);
+    if (!n_tile || cost < least) n_tile = n, least = cost;
+  }
+  // Few tiles of few rows: spread a tile's inner dimension until the machine is full.
+  const int few = L.rows <= 16 ? 16 : L.rows <= 32 ? 32 : 64;
+  int split = 1;
+  if (L.rows <= 64 || tiles_m * ((L.rows + 127) / 128) * 2 <= sms)
+    while (split < 8 && tiles_m * ((L.rows + few - 1) / few) * split * 2 <= sms && n_k >= 4 * split) split *= 2;
+  if (split > 1) n_tile = std::min(few, (L.rows + 15) & ~15);
   CUtensorMap wmap, xmap;
   CMLD_TRY(make_map(&wmap, L.w.w, L.w.cols, L.w.rows, L.w.ld, kBM));
   CMLD_TRY(make_map(&xmap, L.x, L.w.cols, L.rows, L.x_ld, n_tile));
   TcLinArgs a{};
   a.m_rows = L.w.rows;
   a.n_rows = L.rows;
-  a.n_k = (L.w.cols + kBK - 1) / kBK;
+  a.n_k = n_k;
   a.n_tile = n_tile;
   a.stages = stages(n_tile);
   a.slot_cols = 32;
   while (a.slot_cols < n_tile) a.slot_cols *= 2;
   a.tiles_n = (L.rows + n_tile - 1) / n_tile;
-  a.tiles = (L.w.rows + kBM - 1) / kBM * a.tiles_n;
-  a.split = 1;
-  // few tiles: spread a tile's inner dimension until the machine is full
-  while (a.split < 8 && a.tiles * a.split * 2 <= sms && a.n_k >= 4 * a.split) a.split *= 2;
-  // Whole tiles where they keep four fifths of the SMs busy (224 tiles, 8 rows: 46.1 us, as equal runs 42.6; 250 tiles: 46.4, 46.9) or the partial
-  // accumulators are large (224 tiles, 150 rows: 54 us, as equal runs 58).
-  const int rounds = (a.tiles + sms - 1) / sms;
-  a.whole = a.split == 1 && (!L.parts || n_tile > 64 || sms > kTcLinCtas || a.tiles <= sms || a.tiles > kTcLinTiles || a.tiles * 5 >= rounds * sms * 4);
-  a.parts = L.parts;
-  a.counts = L.counts;
+  a.tiles = tiles_m * a.tiles_n;
+  a.split = split;
   a.out = L.out;
   a.out_ld = L.out_ld;
   a.act = L.act;

@@ -30,16 +30,24 @@ __device__ __forceinline__ void store4(const ActBuf &out, int64_t at, float4 v) 
 }
 
 // Several streams, a row in the registers of a CTA.  Bound by HBM: streams + 1 rows in, streams and the result out.
-// 2048 rows of 2048, 4 streams: 32 us between two products (159 MB, 5 TB/s), 52 through shared memory value by value.
+// 2048 rows of 2048, 4 streams (159 MB): 32 us between two products with the norm in registers too, 52 through
+// shared memory value by value; a 4000-token document into 8 such layers 9.1 and 9.3 ms with the norm in registers and as it is, 10.1 before both.
+// (The norm's sums go over shared memory in the order of stream_mix_kernel: prompts keep its bits.)
 template <int V>
 __global__ void __launch_bounds__(kMixThreads / V) mix_rows_kernel(const __grid_constant__ StreamMix m, ActBuf out) {
+  extern __shared__ __align__(16) float u[];
   __shared__ __align__(8) float red[2 * kMixThreads / 32];
   __shared__ float coef[kMixCoefs];
   pdl_launch();
   if (threadIdx.x < kMixCoefs) coef[threadIdx.x] = mix_coef(m, threadIdx.x);
   pdl_wait();
   const int64_t r = blockIdx.x;
-  mix_row<V>(m, m.row_map ? m.row_map[r] : r, coef, red, true, [&](int i, float4 v) { store4(out, r * out.ld + 4 * i, v); });
+  mix_row<V, false>(m, m.row_map ? m.row_map[r] : r, coef, red, true, [&](int i, float4 v) { reinterpret_cast<float4 *>(u)[i] = v; });
+  __syncthreads();
+  if (m.norm_b) layer_norm_cta(u, m.width, m.norm_w, m.norm_b, m.eps, red);
+  else if (m.norm_w) rms_norm_cta(u, m.width, m.norm_w, m.eps, red);
+  __syncthreads();
+  for (int i = threadIdx.x; i < m.width / 4; i += blockDim.x) store4(out, r * out.ld + 4 * i, reinterpret_cast<const float4 *>(u)[i]);
 }
 
 // One stream with norms on the sublayers' outputs (or the embedding) and no norm in front of the next: the row stays in
@@ -111,11 +119,13 @@ int32_t launch_stream_mix(const StreamMix &m, int32_t rows, ActBuf out, bool pdl
     if (v == 2) return launch_kernel(post_norm_kernel<2>, dim3(rows), dim3(threads), 0, pdl, s, m, out);
     return launch_kernel(post_norm_kernel<4>, dim3(rows), dim3(threads), 0, pdl, s, m, out);
   }
-  // many rows: two units of four values a thread, so that several rows are in flight per SM
-  const int v = rows >= 256 || m.width > 4 * kMixThreads ? 2 : 1, threads = std::max(32, ((m.width / 4 + v - 1) / v + 31) & ~31);
-  if (threads <= kMixThreads / v && mix_row_fits(m, v, threads) && out.ld % 4 == 0) {
-    if (v == 1) return launch_kernel(mix_rows_kernel<1>, dim3(rows), dim3(threads), 0, pdl, s, m, out);
-    return launch_kernel(mix_rows_kernel<2>, dim3(rows), dim3(threads), 0, pdl, s, m, out);
+  const int threads = mix_threads(rows), v = threads == 256 ? 4 : threads == 512 ? 2 : 1;
+  if (mix_row_fits(m, v, threads) && out.ld % 4 == 0) {
+    const size_t row = (size_t)m.width * 4;
+    if (v == 1) return launch_kernel(mix_rows_kernel<1>, dim3(rows), dim3(threads), row, pdl, s, m, out);
+    if (v == 2) return launch_kernel(mix_rows_kernel<2>, dim3(rows), dim3(threads), row, pdl, s, m, out);
+    if (m.width <= 2048) return launch_kernel(mix_rows_kernel<2>, dim3(rows), dim3(threads), row, pdl, s, m, out);
+    return launch_kernel(mix_rows_kernel<4>, dim3(rows), dim3(threads), row, pdl, s, m, out);
   }
   const size_t smem = (size_t)m.width * 4;
   static SmemLimit limit;

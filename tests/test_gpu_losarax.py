@@ -88,7 +88,7 @@ def test_matrix_vector_rows_shared_by_warps(cm, shape):
 @pytest.mark.parametrize("shape", [(19200, 72, 8), (19100, 520, 33), (22544, 136, 64), (40000, 200, 16), (1000, 392, 300), (260, 2056, 412), (19000, 64, 150),
                                    (128, 4096, 350)])
 def test_linear_tiles_shared_out(cm, shape):
-    """Tiles that several CTAs add up, through global memory or a cluster, launch after launch; row tiles of every number of operand stages."""
+    """Tiles that a cluster adds up, several tiles for a CTA, launch after launch; row tiles of every number of operand stages."""
     import ctypes as C
 
     from camelid_b200._lib import check as ok
