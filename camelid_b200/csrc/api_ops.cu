@@ -2,6 +2,7 @@
 // Used by the microbenchmarks and the kernel-level parity tests; all work runs on the
 // calling thread's current device, default stream, and returns after completion.
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -20,51 +21,74 @@ static int32_t sync_ok(const char *what) {
   return CMLD_OK;
 }
 
-// Status word for the staged kernel's bounded waits, one per device, made on first use.
-static int32_t *op_status(void) {
-  static int32_t *words[64] = {nullptr};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  if (!words[dev]) {
-    if (cudaMalloc(&words[dev], 4) != cudaSuccess) return nullptr;
-    cudaMemset(words[dev], 0, 4);
+// What the operator-level calls of a device share: the status word of the bounded waits and the scratch of the batched matvecs, both made
+// on first use, the scratch grown on demand.  A call holds them, from before its first launch until it has waited for its last: two threads'
+// launches would otherwise take turns on the stream, one reading the records that the other has just written (and either could give back
+// the scratch that the other is about to launch on).
+class OpCall {
+  struct Device {
+    std::mutex busy;
+    int32_t *status = nullptr;
+    float *buf = nullptr;
+    int64_t cap = 0;
+  };
+  static Device *current() {
+    static Device devices[64];
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 ? &devices[dev] : nullptr;
   }
-  return words[dev];
-}
+  Device *d_;
+  std::unique_lock<std::mutex> hold_;
 
-// Partial-sum scratch of the batched matvec for the operator-level calls: one per device, grown on demand
-// (never inside a stream capture: a capture is preceded by warm-up launches of the same shape).
-static float *op_scratch(int64_t floats) {
-  static float *buf[64] = {nullptr};
-  static int64_t cap[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  if (cap[dev] < floats) {
-    if (buf[dev]) {
-      cudaDeviceSynchronize();
-      cudaFree(buf[dev]);
-    }
-    buf[dev] = nullptr;
-    cap[dev] = 0;
-    if (cudaMalloc(&buf[dev], (size_t)floats * 4) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    cap[dev] = floats;
+ public:
+  OpCall() : d_(current()) {
+    if (d_) hold_ = std::unique_lock<std::mutex>(d_->busy);
   }
-  return buf[dev];
-}
 
-static int32_t check_op_status(const char *what) {
-  int32_t *w = op_status(), st = 0;
-  if (!w) return CMLD_OK;
-  if (cudaMemcpy(&st, w, 4, cudaMemcpyDeviceToHost) != cudaSuccess) return fail(CMLD_ERR_CUDA, "%s: status read failed", what);
-  if (st != 0) {
-    cudaMemset(w, 0, 4);
-    return fail(st, "%s: a bounded device-side wait gave up (status %d)", what, st);
+  int32_t *status() {
+    if (!d_) return nullptr;
+    if (!d_->status) {
+      if (cudaMalloc(&d_->status, 4) != cudaSuccess) {
+        cudaGetLastError();
+        d_->status = nullptr;
+        return nullptr;
+      }
+      cudaMemset(d_->status, 0, 4);
+    }
+    return d_->status;
   }
-  return CMLD_OK;
-}
+
+  // (not inside a stream capture, unless as many were asked for before it)
+  float *scratch(int64_t floats) {
+    if (!d_) return nullptr;
+    if (d_->cap < floats) {
+      if (d_->buf) {
+        cudaDeviceSynchronize();
+        cudaFree(d_->buf);
+      }
+      d_->buf = nullptr;
+      d_->cap = 0;
+      if (cudaMalloc(&d_->buf, (size_t)floats * 4) != cudaSuccess) {
+        cudaGetLastError();
+        d_->buf = nullptr;
+        return nullptr;
+      }
+      d_->cap = floats;
+    }
+    return d_->buf;
+  }
+
+  int32_t check_status(const char *what) {
+    int32_t *w = status(), st = 0;
+    if (!w) return CMLD_OK;
+    if (cudaMemcpy(&st, w, 4, cudaMemcpyDeviceToHost) != cudaSuccess) return fail(CMLD_ERR_CUDA, "%s: status read failed", what);
+    if (st != 0) {
+      cudaMemset(w, 0, 4);
+      return fail(st, "%s: a bounded device-side wait gave up (status %d)", what, st);
+    }
+    return CMLD_OK;
+  }
+};
 
 static int g_gemv_pdl = 0;            // cmld_gemv_time: chain its launches with programmatic dependent launch
 static int g_gemv_kernel_choice = 0;  // 0 auto (staged when the shape fits), 1 generic kernel only
@@ -75,27 +99,27 @@ static int g_gemv_tc5_min_batch = 9;        // rows from which the tcgen05 kerne
 constexpr int32_t kOpTc5Rows = 2048;  // rows per pass of the tcgen05 kernel: bounds its scratch and its grids
 
 // One matvec launch on the default stream: staged kernel if it takes the shape, else the generic one.
-static int32_t gemv_launch(const cmld_weight *w, const uint8_t *act, int32_t batch, float *y, const float *residual,
+static int32_t gemv_launch(OpCall &op, const cmld_weight *w, const uint8_t *act, int32_t batch, float *y, const float *residual,
                            cudaStream_t stream = nullptr, bool pdl = false) {
   GemvJob probe{w->data, w->qt, w->rows, w->cols, w->stride, y, residual, w->rows};
   if (g_gemv_kernel_choice == 0 && batch >= g_gemv_rows_min_batch && batch <= kRowsMaxBatch && gemv_rows_fits(&probe, 1, batch)) {
-    uint8_t *rec = reinterpret_cast<uint8_t *>(op_scratch((gemv_rows_rec_bytes(w->cols, batch) + 3) / 4));
+    uint8_t *rec = reinterpret_cast<uint8_t *>(op.scratch((gemv_rows_rec_bytes(w->cols, batch) + 3) / 4));
     if (!rec) return fail(CMLD_ERR_OOM, "gemv: no room for %lld bytes of activation records", (long long)gemv_rows_rec_bytes(w->cols, batch));
     uint8_t *rec4 = w->qt == CMLD_Q4_K ? rec : nullptr, *rec6 = w->qt == CMLD_Q6_K ? rec : nullptr, *rec0 = w->qt == CMLD_Q8_0 ? rec : nullptr;
     CMLD_TRY(launch_rows_pack(act, w->cols, batch, rec4, rec6, rec0, stream));
-    return launch_gemv_rows(&probe, 1, batch, rec4, rec6, rec0, op_status(), stream, pdl);
+    return launch_gemv_rows(&probe, 1, batch, rec4, rec6, rec0, op.status(), stream, pdl);
   }
   if (g_gemv_kernel_choice == 0 && batch >= g_gemv_tc5_min_batch && batch < g_gemv_mma_min_batch && gemv_tc5_fits(&probe, 1, batch)) {
     // several rows: one pass over the weights per 2048 rows on the tcgen05 tensor cores, same bits as the one-row kernels
     const int64_t need = gemv_tc5_pack_bytes(w->cols, std::min(batch, kOpTc5Rows));
-    uint8_t *pack = reinterpret_cast<uint8_t *>(op_scratch((need + 3) / 4));
+    uint8_t *pack = reinterpret_cast<uint8_t *>(op.scratch((need + 3) / 4));
     if (!pack) return fail(CMLD_ERR_OOM, "gemv: no room for %lld bytes of packed activations", (long long)need);
     uint8_t *rec4 = w->qt == CMLD_Q4_K ? pack : nullptr, *rec6 = w->qt == CMLD_Q6_K ? pack : nullptr, *rec0 = w->qt == CMLD_Q8_0 ? pack : nullptr;
     for (int32_t b0 = 0; b0 < batch; b0 += kOpTc5Rows) {
       const int32_t nb = std::min(batch - b0, kOpTc5Rows);
       const GemvJob j{w->data, w->qt, w->rows, w->cols, w->stride, y + (int64_t)b0 * w->rows, residual ? residual + (int64_t)b0 * w->rows : nullptr, w->rows};
       CMLD_TRY(launch_tc5_pack(act + (int64_t)b0 * act_row_stride(w->cols), w->cols, nb, rec4, rec6, rec0, stream));
-      CMLD_TRY(launch_gemv_tc5(&j, 1, nb, rec4, rec6, rec0, op_status(), stream, nullptr));
+      CMLD_TRY(launch_gemv_tc5(&j, 1, nb, rec4, rec6, rec0, op.status(), stream, nullptr));
     }
     return CMLD_OK;
   }
@@ -103,9 +127,9 @@ static int32_t gemv_launch(const cmld_weight *w, const uint8_t *act, int32_t bat
     // more than 8 rows: one pass over the weights on the tensor cores
     const int64_t need = gemv_mma_scratch_floats(&probe, 1, batch);
     if (need >= 0) {
-      float *scratch = need > 0 ? op_scratch(need) : nullptr;
+      float *scratch = need > 0 ? op.scratch(need) : nullptr;
       if (need > 0 && !scratch) return fail(CMLD_ERR_OOM, "gemv: no room for %lld floats of partial sums", (long long)need);
-      const int32_t rc = launch_gemv_mma(&probe, 1, act, batch, scratch, need, op_status(), stream, pdl, nullptr);
+      const int32_t rc = launch_gemv_mma(&probe, 1, act, batch, scratch, need, op.status(), stream, pdl, nullptr);
       if (rc != CMLD_ERR_UNSUPPORTED) return rc;
     }
   }
@@ -120,7 +144,7 @@ static int32_t gemv_launch(const cmld_weight *w, const uint8_t *act, int32_t bat
       GemvPrologue pro{};
       pro.mode = 0;
       pro.act_k = pro.act_0 = a;
-      rc = launch_gemv_pipe(&j, 1, nb, pro, op_status(), stream, pdl);
+      rc = launch_gemv_pipe(&j, 1, nb, pro, op.status(), stream, pdl);
     }
     if (rc == CMLD_ERR_UNSUPPORTED) rc = launch_gemv(&j, 1, a, nb, stream);
     CMLD_TRY(rc);
@@ -301,9 +325,10 @@ int32_t cmld_gemv(const cmld_weight *w, const void *act_dev, int32_t batch, floa
   if (!w || !act_dev || !y_dev) return fail(CMLD_ERR_INVALID, "null buffer");
   if (w->qt == CMLD_F32) return fail(CMLD_ERR_UNSUPPORTED, "gemv over f32 weights is not part of this path");
   if (batch < 1) return fail(CMLD_ERR_INVALID, "batch %d", batch);
-  CMLD_TRY(gemv_launch(w, static_cast<const uint8_t *>(act_dev), batch, y_dev, residual_dev));
+  OpCall op;
+  const int32_t rc = gemv_launch(op, w, static_cast<const uint8_t *>(act_dev), batch, y_dev, residual_dev);
   CMLD_TRY(sync_ok("gemv"));
-  return check_op_status("gemv");
+  return rc == CMLD_OK ? op.check_status("gemv") : rc;
 }
 
 // The parallel evaluation of the sequential f32 sum on n device-resident non-negative terms: sums_host[0] by the
@@ -326,6 +351,7 @@ int32_t cmld_exact_sum_selftest(const float *terms_dev, int32_t n, float *sums_h
 int32_t cmld_peer_wait_selftest(int32_t timeout_ms) {
   if (timeout_ms < 1 || timeout_ms > 5000) return fail(CMLD_ERR_INVALID, "timeout_ms %d out of 1..=5000", timeout_ms);
   const int hidden = 256;
+  OpCall op;
   uint8_t *buf = nullptr;
   CMLD_CUDA(cudaMalloc(&buf, (size_t)(2 * kPeerRows * hidden + hidden) * 4 + 64));
   cudaMemset(buf, 0, (size_t)(2 * kPeerRows * hidden + hidden) * 4 + 64);
@@ -340,11 +366,11 @@ int32_t cmld_peer_wait_selftest(int32_t timeout_ms) {
   rx.rx_epoch = epoch;
   rx.rx_out = out;
   rx.timeout_ns = (unsigned long long)timeout_ms * 1000000ull;
-  int32_t rc = launch_peer_reduce(rx, 1, hidden, op_status(), false, nullptr);
+  int32_t rc = launch_peer_reduce(rx, 1, hidden, op.status(), false, nullptr);
   if (rc == CMLD_OK) rc = sync_ok("peer_wait_selftest");
   int32_t st = 0;
-  if (rc == CMLD_OK && cudaMemcpy(&st, op_status(), 4, cudaMemcpyDeviceToHost) != cudaSuccess) rc = fail(CMLD_ERR_CUDA, "status read failed");
-  cudaMemset(op_status(), 0, 4);
+  if (rc == CMLD_OK && cudaMemcpy(&st, op.status(), 4, cudaMemcpyDeviceToHost) != cudaSuccess) rc = fail(CMLD_ERR_CUDA, "status read failed");
+  cudaMemset(op.status(), 0, 4);
   cudaFree(buf);
   if (rc != CMLD_OK) return rc;
   if (st == CMLD_ERR_TIMEOUT) return fail(CMLD_ERR_TIMEOUT, "the wait ran out after %d ms as it should", timeout_ms);
@@ -360,21 +386,24 @@ static int32_t sample_fetch(uint32_t *dev, uint32_t *host, const char *what) {
 }
 int32_t cmld_sample_gumbel(const float *logits_dev, int32_t n, float inv_temp, uint64_t seed, uint32_t *token_out) {
   if (!logits_dev || !token_out || n < 1) return fail(CMLD_ERR_INVALID, "sample_gumbel: bad arguments");
-  uint32_t *d = reinterpret_cast<uint32_t *>(op_scratch(1));
+  OpCall op;
+  uint32_t *d = reinterpret_cast<uint32_t *>(op.scratch(1));
   if (!d) return fail(CMLD_ERR_OOM, "sample_gumbel: no scratch");
   CMLD_TRY(launch_sample_gumbel(logits_dev, n, inv_temp, seed, d, nullptr));
   return sample_fetch(d, token_out, "sample_gumbel");
 }
 int32_t cmld_sample_gumbel_filtered(const float *logits_dev, int32_t n, float temperature, float min_p, uint64_t seed, uint32_t *token_out) {
   if (!logits_dev || !token_out || n < 1) return fail(CMLD_ERR_INVALID, "sample_gumbel_filtered: bad arguments");
-  uint32_t *d = reinterpret_cast<uint32_t *>(op_scratch(1));
+  OpCall op;
+  uint32_t *d = reinterpret_cast<uint32_t *>(op.scratch(1));
   if (!d) return fail(CMLD_ERR_OOM, "sample_gumbel_filtered: no scratch");
   CMLD_TRY(launch_sample_gumbel_filtered(logits_dev, n, temperature, min_p, seed, d, nullptr));
   return sample_fetch(d, token_out, "sample_gumbel_filtered");
 }
 int32_t cmld_sample_min_p_mask(const float *logits_dev, int32_t n, float min_p, int32_t *mask_out) {
   if (!logits_dev || !mask_out || n < 1) return fail(CMLD_ERR_INVALID, "sample_min_p_mask: bad arguments");
-  int32_t *d = reinterpret_cast<int32_t *>(op_scratch(n));
+  OpCall op;
+  int32_t *d = reinterpret_cast<int32_t *>(op.scratch(n));
   if (!d) return fail(CMLD_ERR_OOM, "sample_min_p_mask: no scratch");
   CMLD_TRY(launch_min_p_mask(logits_dev, n, min_p, d, nullptr));
   CMLD_TRY(sync_ok("sample_min_p_mask"));
@@ -383,7 +412,8 @@ int32_t cmld_sample_min_p_mask(const float *logits_dev, int32_t n, float min_p, 
 }
 int32_t cmld_sample_uniforms(uint64_t seed, int32_t n, float *out) {
   if (!out || n < 1) return fail(CMLD_ERR_INVALID, "sample_uniforms: bad arguments");
-  float *d = op_scratch(n);
+  OpCall op;
+  float *d = op.scratch(n);
   if (!d) return fail(CMLD_ERR_OOM, "sample_uniforms: no scratch");
   CMLD_TRY(launch_sample_uniforms(seed, n, d, nullptr));
   CMLD_TRY(sync_ok("sample_uniforms"));
@@ -416,11 +446,12 @@ int32_t cmld_gemv_fused(const cmld_weight *w, int32_t mode, const float *x_dev, 
   pro.norm_w = norm_w_dev;
   pro.x_stride = w->cols;
   pro.eps = eps;
-  const int32_t rc = launch_gemv_pipe(&j, 1, batch, pro, op_status(), nullptr, false);
+  OpCall op;
+  const int32_t rc = launch_gemv_pipe(&j, 1, batch, pro, op.status(), nullptr, false);
   if (rc == CMLD_ERR_UNSUPPORTED) return fail(rc, "the staged kernel does not take a %lld x %lld matrix at batch %d", (long long)w->rows, (long long)w->cols, batch);
   CMLD_TRY(rc);
   CMLD_TRY(sync_ok("gemv_fused"));
-  return check_op_status("gemv_fused");
+  return op.check_status("gemv_fused");
 }
 
 int32_t cmld_gemv_time(cmld_weight *const *copies, int32_t n_copies, const void *act_dev, int32_t batch, float *y_dev,
@@ -437,13 +468,14 @@ int32_t cmld_gemv_time(cmld_weight *const *copies, int32_t n_copies, const void 
   CMLD_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   CMLD_CUDA(cudaEventCreate(&e0));
   CMLD_CUDA(cudaEventCreate(&e1));
-  op_status();  // make the status word before capture
+  OpCall op;
+  op.status();  // make the status word before capture
   int32_t rc = CMLD_OK;
   const uint8_t *act = static_cast<const uint8_t *>(act_dev);
-  for (int it = 0; it < warmup && rc == CMLD_OK; ++it) rc = gemv_launch(copies[it % n_copies], act, batch, y_dev, nullptr, st, false);
+  for (int it = 0; it < warmup && rc == CMLD_OK; ++it) rc = gemv_launch(op, copies[it % n_copies], act, batch, y_dev, nullptr, st, false);
   if (rc == CMLD_OK && cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) rc = fail(CMLD_ERR_CUDA, "graph capture failed to start");
   if (rc == CMLD_OK) {
-    for (int it = 0; it < iters && rc == CMLD_OK; ++it) rc = gemv_launch(copies[it % n_copies], act, batch, y_dev, nullptr, st, g_gemv_pdl != 0);
+    for (int it = 0; it < iters && rc == CMLD_OK; ++it) rc = gemv_launch(op, copies[it % n_copies], act, batch, y_dev, nullptr, st, g_gemv_pdl != 0);
     cudaError_t ce = cudaStreamEndCapture(st, &graph);
     if (rc == CMLD_OK && ce != cudaSuccess) rc = fail(CMLD_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(ce));
   }
@@ -455,7 +487,8 @@ int32_t cmld_gemv_time(cmld_weight *const *copies, int32_t n_copies, const void 
     cudaEventRecord(e1, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) rc = fail(CMLD_ERR_CUDA, "gemv_time: %s", cudaGetErrorString(cudaGetLastError()));
   }
-  if (rc == CMLD_OK) rc = check_op_status("gemv_time");
+  if (rc != CMLD_OK) cudaStreamSynchronize(st);  // what was launched still uses the scratch
+  if (rc == CMLD_OK) rc = op.check_status("gemv_time");
   float ms = 0.0f;
   if (rc == CMLD_OK) cudaEventElapsedTime(&ms, e0, e1);
   if (exec) cudaGraphExecDestroy(exec);

@@ -209,6 +209,30 @@ def test_gemv_rows_largest_sums(cm, orc, name):
         assert same.all(), (name, b, np.nonzero(~same)[0][:5], y[b][~same][:5], ref[~same][:5])
 
 
+@pytest.mark.parametrize("batch", [3, 8, 9, 32])
+def test_gemv_of_several_threads(cm, batch):
+    """Threads with matrices, activations and outputs of their own, of several widths: each has the results it has alone."""
+    from concurrent.futures import ThreadPoolExecutor
+    from threading import Barrier
+
+    from camelid_b200.engine import quantize_activation
+
+    cases = []
+    for i, (qt, rows, cols) in enumerate([(12, 700, 1024), (14, 300, 3072), (12, 2000, 14336), (14, 64, 512)]):
+        w = cm.Weight.synth(qt, 3, 70 + i, rows, cols, 0.02)
+        act = quantize_activation(cm.ACT_Q8_K, np.random.default_rng(i).standard_normal((batch, cols)).astype(np.float32))
+        cases.append((w, act, w.gemv(act, batch)))
+    start = Barrier(len(cases))
+
+    def calls(case):
+        w, act, alone = case
+        start.wait()
+        return [np.array_equal(w.gemv(act, batch).view(np.uint32), alone.view(np.uint32)) for _ in range(50)]
+
+    with ThreadPoolExecutor(len(cases)) as pool:
+        assert all(all(same) for same in pool.map(calls, cases))
+
+
 # The staged kernel's fused prologues: RMSNorm / plain / SwiGLU + quantiser + matvec in one launch
 # equals the three separate steps (same quantised codes, so the same result bit for bit).
 @pytest.mark.parametrize("name,rows,cols", [("Q8_0", 200, 2048), ("Q4_K", 200, 4096), ("Q6_K", 200, 4096), ("Q4_K", 72, 14336),
