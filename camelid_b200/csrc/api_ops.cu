@@ -377,6 +377,25 @@ int32_t cmld_peer_wait_selftest(int32_t timeout_ms) {
   return fail(CMLD_ERR_STATE, "the wait did not report a timeout (status %d)", st);
 }
 
+// A row-batched matvec whose device-side waits run out at once, with copies of weights in flight: every role has to leave, the copies have
+// to land and the status word has to say so.  Returns what it said (CMLD_ERR_TIMEOUT when the bound works); the context stays usable.
+int32_t cmld_gemv_rows_wait_selftest(const cmld_weight *w, const void *act_dev, int32_t batch, float *y_dev) {
+  if (!w || !act_dev || !y_dev || batch < 1) return fail(CMLD_ERR_INVALID, "gemv_rows_wait_selftest: bad arguments");
+  const GemvJob j{w->data, w->qt, w->rows, w->cols, w->stride, y_dev, nullptr, w->rows};
+  if (!gemv_rows_fits(&j, 1, batch)) return fail(CMLD_ERR_UNSUPPORTED, "gemv_rows_wait_selftest: the row-batched kernel does not take this");
+  OpCall op;
+  uint8_t *rec = reinterpret_cast<uint8_t *>(op.scratch((gemv_rows_rec_bytes(w->cols, batch) + 3) / 4));
+  if (!rec || !op.status()) return fail(CMLD_ERR_OOM, "gemv_rows_wait_selftest: no scratch");
+  uint8_t *rec4 = w->qt == CMLD_Q4_K ? rec : nullptr, *rec6 = w->qt == CMLD_Q6_K ? rec : nullptr, *rec0 = w->qt == CMLD_Q8_0 ? rec : nullptr;
+  int32_t rc = launch_rows_pack(static_cast<const uint8_t *>(act_dev), w->cols, batch, rec4, rec6, rec0, nullptr);
+  if (rc == CMLD_OK) rc = launch_gemv_rows(&j, 1, batch, rec4, rec6, rec0, op.status(), nullptr, false, true);
+  CMLD_TRY(sync_ok("gemv_rows_wait_selftest"));
+  if (rc == CMLD_ERR_UNSUPPORTED) return fail(rc, "gemv_rows_wait_selftest: the form that takes this shape has no waits");
+  CMLD_TRY(rc);
+  CMLD_TRY(op.check_status("gemv_rows_wait_selftest"));
+  return fail(CMLD_ERR_STATE, "the waits did not report a timeout");
+}
+
 // Sampling over a logits row on the device (sample_gumbel, sample_gumbel_filtered, sample_min_p_mask and the uniform
 // generator of src/cuda_resident/sampling.cuh), results returned to the host.
 static int32_t sample_fetch(uint32_t *dev, uint32_t *host, const char *what) {

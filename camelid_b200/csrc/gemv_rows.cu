@@ -49,6 +49,7 @@ constexpr int kMagicBits = 0x4B400000;
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23, the number with these bits
 constexpr int kSmemMax = 226 * 1024;
 constexpr int kMaxStages = 4;
+constexpr uint32_t kRowsSpin = 1u << 22;  // polls after which a wait gives up
 
 // a weight row of one unit in the ring: the wire bytes, padded to an odd multiple of 32 (Q6_K: with the word that holds the f16
 // scale), so that the eight rows x four lanes of a load meet distinct banks
@@ -73,6 +74,7 @@ struct RowsArgs {
   int32_t stages, stage_bytes;  // of the CTA's ring (split form), of a warp's (whole form)
   int32_t bufs;                 // split form: exchange buffers
   int32_t off_ring, off_sums;
+  uint32_t spin;                // split form: polls of a wait
   int32_t *status;
 };
 
@@ -446,17 +448,13 @@ __device__ __forceinline__ void bar_arrive(uint64_t *bar) {
 __device__ __forceinline__ void bar_expect(uint64_t *bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(s32(bar)), "r"(bytes) : "memory");
 }
-// Bounded: a wait that runs out records the status and carries on (the results are then invalid, the host reports the error).
-__device__ __forceinline__ void bar_wait(uint64_t *bar, uint32_t parity, int32_t *status) {
-  for (uint32_t i = 0; i < (1u << 22); ++i) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok)
-                 : "r"(s32(bar)), "r"(parity)
-                 : "memory");
-    if (ok) return;
-  }
-  if (status) atomicExch(status, (int32_t)CMLD_ERR_TIMEOUT);
+__device__ __forceinline__ bool bar_try(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok)
+               : "r"(s32(bar)), "r"(parity)
+               : "memory");
+  return ok;
 }
 __device__ __forceinline__ void bulk_load(uint32_t dst, const uint8_t *src, uint32_t bytes, uint64_t *bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),
@@ -470,9 +468,25 @@ struct Split {
   int stage, stage_phase;    // ring stage of the next pass
   int buf, buf_phase;        // buffer of the next exchange
   int lk, lu, ls;            // the next load: tile of this CTA's list, first unit, ring stage
+  int loads;                 // passes whose copies this warp has issued
   uint8_t *smem;
   uint64_t *landed, *full, *empty;  // mbarriers of the stages; of the exchange buffers
+  volatile int *gave_up;            // a wait of this CTA ran out
 };
+// Bounded, for a whole warp: where a lane's wait runs out, the status word and the CTA's flag are set, every role leaves its loops and the
+// host reports the error.
+__device__ __forceinline__ bool warp_wait(const RowsArgs &a, const Split &s, uint64_t *bar, uint32_t parity) {
+  bool ok = false;
+  for (uint32_t i = 0; i < a.spin && !ok; ++i) {
+    ok = bar_try(bar, parity);
+    if (!ok && (i & 255u) == 255u && *s.gave_up) break;
+  }
+  if (!ok) {
+    *s.gave_up = 1;
+    if (a.status) atomicExch(a.status, (int32_t)CMLD_ERR_TIMEOUT);
+  }
+  return __all_sync(0xffffffffu, ok);
+}
 __device__ __forceinline__ void next_stage(const RowsArgs &a, Split &s) {
   if (++s.stage == a.stages) s.stage = 0, s.stage_phase ^= 1;
 }
@@ -500,6 +514,7 @@ __device__ __forceinline__ void load_pass(const RowsArgs &a, Split &s, int warp,
     bulk_load(dst, row + (int64_t)s.lu * UB, (uint32_t)codes, &s.landed[s.ls]);
     if (scales) bulk_load(dst + kWarps * UB, row + (int64_t)J.units * UB + s.lu * (QT == CMLD_Q6_K ? 2 : 8), (uint32_t)scales, &s.landed[s.ls]);
   }
+  ++s.loads;
   if (++s.ls == a.stages) s.ls = 0;
   s.lu += kWarps;
   if (s.lu >= J.units) s.lu = 0, ++s.lk;
@@ -517,9 +532,9 @@ __device__ __forceinline__ void add_terms(float *s, const float4 &v) {
   }
 }
 
-// The products of one tile: warp `warp` takes one unit of each pass, `first` of the first.
+// The products of one tile: warp `warp` takes one unit of each pass, `first` of the first.  False: a wait ran out.
 template <int QT, int NT>
-__device__ __forceinline__ void split_products(const RowsArgs &a, const RowsJob &J, int first, int lane, Split &s) {
+__device__ __forceinline__ bool split_products(const RowsArgs &a, const RowsJob &J, int first, int lane, Split &s) {
   constexpr int HALVES = QT == CMLD_Q6_K ? 2 : 1, P = pass_pitch(QT), UB = unit_bytes(QT);
   const int g = lane >> 2, t = lane & 3, units = J.units;
   const uint8_t *rec = J.rec + (int64_t)first * NT * rows_rec(QT);
@@ -528,8 +543,7 @@ __device__ __forceinline__ void split_products(const RowsArgs &a, const RowsJob 
   for (int u = first; u < units + kWarps - 1; u += kWarps, rec += kWarps * NT * rows_rec(QT)) {
     if (u - first >= units) break;  // no such pass
     const bool mine = u < units;
-    bar_wait(&s.landed[s.stage], (uint32_t)s.stage_phase, a.status);
-    __syncwarp();
+    if (!warp_wait(a, s, &s.landed[s.stage], (uint32_t)s.stage_phase)) return false;
     const uint8_t *raw = s.smem + a.off_ring + s.stage * a.stage_bytes + first * UB;
     const uint8_t *scales = raw + (kWarps - first) * UB + first * (QT == CMLD_Q6_K ? 2 : 8);
     next_stage(a, s);
@@ -540,7 +554,7 @@ __device__ __forceinline__ void split_products(const RowsArgs &a, const RowsJob 
       if (mine) unpack_codes<P>(w, raw, g, t, e);
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
-        bar_wait(&s.empty[s.buf], (uint32_t)(s.buf_phase ^ 1), a.status);
+        if (!warp_wait(a, s, &s.empty[s.buf], (uint32_t)(s.buf_phase ^ 1))) return false;
         if (mine) {
           float4 *dst = reinterpret_cast<float4 *>(s.smem + s.buf * (kWarps * kSlice) + first * kSlice) + lane;
           product(w, o, [&](int i, const float4 &f) { dst[i == 0 ? 0 : i == 1 ? 64 : i == 2 ? 32 : 96] = f; });
@@ -555,12 +569,13 @@ __device__ __forceinline__ void split_products(const RowsArgs &a, const RowsJob 
       }
     }
   }
+  return true;
 }
 
 // The sums of one tile: four warps, a thread per output of a row group (its place in a slice: idx).  Between passes the running sums
-// lie in shared memory, a float (Q6_K: two float4, the halves' classes) per row group.
+// lie in shared memory, a float (Q6_K: two float4, the halves' classes) per row group.  False: a wait ran out.
 template <int QT, int NT>
-__device__ __forceinline__ void split_sums(const RowsArgs &a, const RowsJob &J, int row0, int idx, Split &s) {
+__device__ __forceinline__ bool split_sums(const RowsArgs &a, const RowsJob &J, int row0, int idx, Split &s) {
   constexpr int HALVES = QT == CMLD_Q6_K ? 2 : 1, NL = QT == CMLD_Q6_K ? 4 : 1;
   typedef typename Sums<QT>::type sum_t;
   const int lane = idx & 31;
@@ -578,8 +593,7 @@ __device__ __forceinline__ void split_sums(const RowsArgs &a, const RowsJob &J, 
 #pragma unroll
         for (int l = 0; l < NL; ++l) acc[l] = 0.0f;
       }
-      bar_wait(&s.full[s.buf], (uint32_t)s.buf_phase, a.status);
-      __syncwarp();
+      if (!warp_wait(a, s, &s.full[s.buf], (uint32_t)s.buf_phase)) return false;
       const float4 *p = reinterpret_cast<const float4 *>(s.smem + s.buf * (kWarps * kSlice)) + idx;
       if (cnt == kWarps) {
         float4 v[kWarps];
@@ -618,6 +632,27 @@ __device__ __forceinline__ void split_sums(const RowsArgs &a, const RowsJob &J, 
       J.y[at] = J.residual ? __fadd_rn(__ldcg(J.residual + at), v) : v;
     }
   }
+  return true;
+}
+
+// Behind the adding warps' loops: where one of them gave up, copies may still be on their way into this CTA's shared memory, and nobody has
+// waited for them.  A warp that issued fewer passes than another arrives for those it left out, so that every stage's last phase can end.
+__device__ __forceinline__ void drain(const RowsArgs &a, Split &s, bool ok, int warp, int lane, int *loads) {
+  uint32_t gave_up;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.or.pred p, 1, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(gave_up)
+               : "r"(ok ? 0u : 1u)
+               : "memory");
+  if (!gave_up) return;  // (every pass was used up)
+  if (lane == 0) loads[warp] = s.loads;
+  asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+  const int most = max(max(loads[0], loads[1]), max(loads[2], loads[3]));
+  if (lane == 0) {
+    for (int i = s.loads; i < most; ++i) bar_arrive(&s.landed[i % a.stages]);
+    for (int i = max(0, most - a.stages); i < most; ++i)
+      for (uint32_t n = 0; n < kRowsSpin && !bar_try(&s.landed[i % a.stages], (uint32_t)(i / a.stages & 1)); ++n) {
+      }
+  }
 }
 
 // The two roles over all tiles of this CTA.
@@ -625,24 +660,27 @@ template <int QT, int NT>
 __device__ __forceinline__ void split_multiply(const RowsArgs &a, int warp, int lane, Split &s) {
   for (int k = 0; k < s.n_mine; ++k) {
     const RowsJob &J = a.job[tile_job(a, s.first + k * s.step)];
-    split_products<QT, NT>(a, J, (warp - k * J.units) & (kWarps - 1), lane, s);  // (who has no unit in a short pass differs from tile to tile)
+    // (who has no unit in a short pass differs from tile to tile)
+    if (!split_products<QT, NT>(a, J, (warp - k * J.units) & (kWarps - 1), lane, s)) break;
   }
 }
 template <int QT, int NT>
-__device__ __forceinline__ void split_add(const RowsArgs &a, int warp, int lane, Split &s) {
+__device__ __forceinline__ bool split_add(const RowsArgs &a, int warp, int lane, Split &s) {
   for (int i = 0; i < a.stages; ++i) load_pass<QT>(a, s, warp, lane);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int k = 0; k < s.n_mine; ++k) {
     const int tile = s.first + k * s.step;
     const RowsJob &J = a.job[tile_job(a, tile)];
-    split_sums<QT, NT>(a, J, (tile - J.first_tile) * 16, warp * 32 + lane, s);
+    if (!split_sums<QT, NT>(a, J, (tile - J.first_tile) * 16, warp * 32 + lane, s)) return false;
   }
+  return true;
 }
 
 template <int NT>
 __global__ void __launch_bounds__(kSplitThreads, 1) rows_split_kernel(const __grid_constant__ RowsArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];  // exchange buffers [buffer][unit of the pass][kSlice], then the stages
   __shared__ __align__(8) uint64_t bars[3 * kMaxStages];
+  __shared__ int gave_up, loads[kSplitWarps - kWarps];
   asm volatile("griddepcontrol.launch_dependents;");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -651,6 +689,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) rows_split_kernel(const __gr
       bar_init(&bars[kMaxStages + i], kWarps);
       bar_init(&bars[2 * kMaxStages + i], kSplitWarps - kWarps);
     }
+    gave_up = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -662,7 +701,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) rows_split_kernel(const __gr
   s.n_mine = ((second ? a.tiles : a.tiles0) - s.first + s.step - 1) / s.step;
   s.smem = smem;
   s.landed = bars, s.full = bars + kMaxStages, s.empty = bars + 2 * kMaxStages;
-  // the adding warps hold few values: they leave registers to the others (512 x 112 + 128 x 32 = the 640 x 96 of the launch)
+  s.gave_up = &gave_up;
+  // the adding warps hold few values: they leave registers to the others
   const int qt = a.job[tile_job(a, s.first)].qt;
   if (warp < kWarps) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");  // 512 x 104 + 128 x 64 = the 640 x 96 of the launch
@@ -672,9 +712,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) rows_split_kernel(const __gr
     else split_multiply<CMLD_Q8_0, NT>(a, warp, lane, s);
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-    if (qt == CMLD_Q4_K) split_add<CMLD_Q4_K, NT>(a, warp - kWarps, lane, s);
-    else if (qt == CMLD_Q6_K) split_add<CMLD_Q6_K, NT>(a, warp - kWarps, lane, s);
-    else split_add<CMLD_Q8_0, NT>(a, warp - kWarps, lane, s);
+    bool ok;
+    if (qt == CMLD_Q4_K) ok = split_add<CMLD_Q4_K, NT>(a, warp - kWarps, lane, s);
+    else if (qt == CMLD_Q6_K) ok = split_add<CMLD_Q6_K, NT>(a, warp - kWarps, lane, s);
+    else ok = split_add<CMLD_Q8_0, NT>(a, warp - kWarps, lane, s);
+    drain(a, s, ok, warp - kWarps, lane, loads);
   }
 }
 
@@ -857,9 +899,10 @@ int32_t launch_rows_pack(const uint8_t *act, int64_t cols, int32_t batch, uint8_
   return CMLD_OK;
 }
 
-// The records: rec4 for Q4_K matrices, rec6 for Q6_K, rec0 for Q8_0 (those of the types that occur).
+// The records: rec4 for Q4_K matrices, rec6 for Q6_K, rec0 for Q8_0 (those of the types that occur).  no_wait (a self-test): the waits of
+// the split form run out at once; shapes that take the other form, which has none, are refused.
 int32_t launch_gemv_rows(const GemvJob *jobs, int n_jobs, int32_t batch, const uint8_t *rec4, const uint8_t *rec6, const uint8_t *rec0,
-                         int32_t *status, cudaStream_t s, bool pdl) {
+                         int32_t *status, cudaStream_t s, bool pdl, bool no_wait) {
   if (!gemv_rows_fits(jobs, n_jobs, batch)) return CMLD_ERR_UNSUPPORTED;
   const int sms = sm_count(), nt = (batch + 7) / 8;
   if (sms < 1) return fail(CMLD_ERR_CUDA, "gemv: no device");
@@ -867,6 +910,7 @@ int32_t launch_gemv_rows(const GemvJob *jobs, int n_jobs, int32_t batch, const u
   a.n_jobs = n_jobs;
   a.batch = batch;
   a.status = status;
+  a.spin = no_wait ? 0 : kRowsSpin;
   for (int pass = 0, k = 0; pass < 2; ++pass)  // Q6_K last
     for (int i = 0; i < n_jobs; ++i) {
       const int qt = jobs[i].qt;
@@ -884,6 +928,7 @@ int32_t launch_gemv_rows(const GemvJob *jobs, int n_jobs, int32_t batch, const u
   const int warps = std::min(kWarps, per_cta), rec = a.job[0].units * nt * rows_rec(qt);
   const int fit = warps > 0 ? (kSmemMax - rec) / (warps * raw_bytes(qt)) : 0;
   if (same && per_cta >= 5 && fit >= 2 && (qt != CMLD_Q6_K || nt == 1)) {
+    if (no_wait) return CMLD_ERR_UNSUPPORTED;
     a.stages = std::min(kMaxStages, fit);
     a.off_ring = rec;
     const int smem = rec + warps * a.stages * raw_bytes(qt);

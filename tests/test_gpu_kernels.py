@@ -209,6 +209,22 @@ def test_gemv_rows_largest_sums(cm, orc, name):
         assert same.all(), (name, b, np.nonzero(~same)[0][:5], y[b][~same][:5], ref[~same][:5])
 
 
+@pytest.mark.parametrize("name,rows,cols", [("Q4_K", 4096, 14336), ("Q6_K", 300, 1792), ("Q8_0", 70, 4352)])
+@pytest.mark.parametrize("batch", [3, 32])
+def test_gemv_rows_waits_that_run_out(cm, name, rows, cols, batch):
+    """Every role leaves while copies are in flight, the status says why, and the next call has the results of the one before."""
+    from camelid_b200.engine import DeviceBuffer, quantize_activation
+
+    qt = QT[name]
+    w = cm.Weight.synth(qt, 5, 80, rows, cols, 0.02)
+    x = np.random.default_rng(batch).standard_normal((batch, cols)).astype(np.float32)
+    act = quantize_activation(cm.ACT_Q8_0 if qt == 8 else cm.ACT_Q8_K, x)
+    before = w.gemv(act, batch)
+    y = DeviceBuffer(batch * rows * 4)
+    assert cm.lib().cmld_gemv_rows_wait_selftest(w._h, act.ptr, batch, y.ptr) == 6  # CMLD_ERR_TIMEOUT
+    assert np.array_equal(w.gemv(act, batch).view(np.uint32), before.view(np.uint32))
+
+
 @pytest.mark.parametrize("batch", [3, 8, 9, 32])
 def test_gemv_of_several_threads(cm, batch):
     """Threads with matrices, activations and outputs of their own, of several widths: each has the results it has alone."""
