@@ -102,6 +102,21 @@ def test_activation_quantisers_bit_exact(cm, orc, cols, batch):
             assert np.array_equal(codes[b], rq) and np.array_equal(scales[b].view(np.uint32), rd.view(np.uint32))
 
 
+@pytest.mark.parametrize("largest", [1e-45, 1e-38, 3.7e-37, 3.8e-37])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_q8_k_codes_of_values_near_zero(cm, orc, largest, sign):
+    """Chunks whose -127 / max overflows (and the first that does not): the CPU's codes and scales, bit for bit."""
+    from camelid_b200.engine import quantize_activation, export_activation
+
+    x = np.random.default_rng(3).uniform(-1, 1, (2, 512)).astype(np.float32)
+    x = (x / np.abs(x).max() * np.float32(largest) * np.float32(sign)).astype(np.float32)
+    x[1, 256:] = 1.5  # beside an ordinary chunk
+    codes, scales = export_activation(cm.ACT_Q8_K, quantize_activation(cm.ACT_Q8_K, x), 512, 2)
+    for b in range(2):
+        rq, rd = orc.quantize_act_q8_k(x[b])
+        assert np.array_equal(codes[b], rq) and np.array_equal(scales[b].view(np.uint32), rd.view(np.uint32))
+
+
 # q4k_gemv_matches_oracle / q6k_gemv_matches_oracle / q8 (src/cuda_resident/tests.rs:7749,
 # :10302): same wire bytes, same quantised activation, CPU row dot as the oracle.
 @pytest.mark.parametrize("name,rows,cols", [
