@@ -377,8 +377,8 @@ int32_t cmld_peer_wait_selftest(int32_t timeout_ms) {
   return fail(CMLD_ERR_STATE, "the wait did not report a timeout (status %d)", st);
 }
 
-// A row-batched matvec whose device-side waits run out at once, with copies of weights in flight: every role has to leave, the copies have
-// to land and the status word has to say so.  Returns what it said (CMLD_ERR_TIMEOUT when the bound works); the context stays usable.
+// A row-batched matvec whose adding warps wait for an arrival that never comes, with copies of weights in flight: every role has to end, the
+// copies have to land and the status word has to say so.  Returns what it said (CMLD_ERR_TIMEOUT when the bound works); the context stays usable.
 int32_t cmld_gemv_rows_wait_selftest(const cmld_weight *w, const void *act_dev, int32_t batch, float *y_dev) {
   if (!w || !act_dev || !y_dev || batch < 1) return fail(CMLD_ERR_INVALID, "gemv_rows_wait_selftest: bad arguments");
   const GemvJob j{w->data, w->qt, w->rows, w->cols, w->stride, y_dev, nullptr, w->rows};

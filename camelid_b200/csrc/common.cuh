@@ -296,7 +296,7 @@ int64_t gemv_rows_rec_bytes(int64_t cols, int32_t batch);
 bool gemv_rows_fits(const GemvJob *jobs, int n_jobs, int32_t batch);
 int32_t launch_rows_pack(const uint8_t *act, int64_t cols, int32_t batch, uint8_t *rec4, uint8_t *rec6, uint8_t *rec0, cudaStream_t s);
 int32_t launch_gemv_rows(const GemvJob *jobs, int n_jobs, int32_t batch, const uint8_t *rec4, const uint8_t *rec6, const uint8_t *rec0,
-                         int32_t *status, cudaStream_t s, bool pdl, bool no_wait = false);
+                         int32_t *status, cudaStream_t s, bool pdl, bool lose_one = false);
 
 int64_t gemv_mma_expert_scratch_floats(const GemvJob *jobs, int n_jobs, int nt, int n_experts, int n_pass);
 int32_t launch_gemv_mma_experts(const GemvJob *jobs, int n_jobs, const uint8_t *act, int nt, int n_experts, int n_pass,

@@ -74,7 +74,7 @@ struct RowsArgs {
   int32_t stages, stage_bytes;  // of the CTA's ring (split form), of a warp's (whole form)
   int32_t bufs;                 // split form: exchange buffers
   int32_t off_ring, off_sums;
-  uint32_t spin;                // split form: polls of a wait
+  int32_t lose_one;             // split form, a self-test: the terms' barriers expect an arrival that never comes
   int32_t *status;
 };
 
@@ -468,24 +468,23 @@ struct Split {
   int stage, stage_phase;    // ring stage of the next pass
   int buf, buf_phase;        // buffer of the next exchange
   int lk, lu, ls;            // the next load: tile of this CTA's list, first unit, ring stage
-  int loads;                 // passes whose copies this warp has issued
   uint8_t *smem;
   uint64_t *landed, *full, *empty;  // mbarriers of the stages; of the exchange buffers
   volatile int *gave_up;            // a wait of this CTA ran out
 };
-// Bounded, for a whole warp: where a lane's wait runs out, the status word and the CTA's flag are set, every role leaves its loops and the
-// host reports the error.
-__device__ __forceinline__ bool warp_wait(const RowsArgs &a, const Split &s, uint64_t *bar, uint32_t parity) {
-  bool ok = false;
-  for (uint32_t i = 0; i < a.spin && !ok; ++i) {
-    ok = bar_try(bar, parity);
-    if (!ok && (i & 255u) == 255u && *s.gave_up) break;
+__device__ __forceinline__ void give_up(const RowsArgs &a, const Split &s) {
+  *s.gave_up = 1;
+  if (a.status) atomicExch(a.status, (int32_t)CMLD_ERR_TIMEOUT);
+}
+// Bounded.  Once a wait of the CTA has run out, the others give up after a few polls and no more weights are fetched: the roles run through
+// their loops without a result, and the host reports the error.  (Roles that leave their loops instead need the verdict of all lanes of a
+// warp: 1 % of a launch.)
+__device__ __forceinline__ void bar_wait(const RowsArgs &a, const Split &s, uint64_t *bar, uint32_t parity) {
+  for (uint32_t i = 0; i < kRowsSpin; ++i) {
+    if (bar_try(bar, parity)) return;
+    if ((i & 7u) == 7u && *s.gave_up) return;
   }
-  if (!ok) {
-    *s.gave_up = 1;
-    if (a.status) atomicExch(a.status, (int32_t)CMLD_ERR_TIMEOUT);
-  }
-  return __all_sync(0xffffffffu, ok);
+  give_up(a, s);
 }
 __device__ __forceinline__ void next_stage(const RowsArgs &a, Split &s) {
   if (++s.stage == a.stages) s.stage = 0, s.stage_phase ^= 1;
@@ -505,16 +504,19 @@ __device__ __forceinline__ void load_pass(const RowsArgs &a, Split &s, int warp,
   const int row0 = (tile - J.first_tile) * 16, cnt = min(kWarps, J.units - s.lu);
   constexpr int UB = unit_bytes(QT);
   const int codes = cnt * UB, scales = QT == CMLD_Q4_K ? 0 : QT == CMLD_Q6_K ? (2 * cnt + 15) & ~15 : 8 * cnt;
-  if (lane == 0) bar_expect(&s.landed[s.ls], (uint32_t)(4 * (codes + scales)));
+  const bool stop = __shfl_sync(0xffffffffu, *s.gave_up, 0);
+  if (lane == 0) {
+    if (stop) bar_arrive(&s.landed[s.ls]);
+    else bar_expect(&s.landed[s.ls], (uint32_t)(4 * (codes + scales)));
+  }
   __syncwarp();
-  if (lane < 4) {
+  if (lane < 4 && !stop) {
     const int r = 4 * warp + lane;
     const uint8_t *row = J.w + (int64_t)min(row0 + r, J.rows - 1) * J.stride;
     const uint32_t dst = s32(s.smem + a.off_ring + s.ls * a.stage_bytes) + r * pass_pitch(QT);
     bulk_load(dst, row + (int64_t)s.lu * UB, (uint32_t)codes, &s.landed[s.ls]);
     if (scales) bulk_load(dst + kWarps * UB, row + (int64_t)J.units * UB + s.lu * (QT == CMLD_Q6_K ? 2 : 8), (uint32_t)scales, &s.landed[s.ls]);
   }
-  ++s.loads;
   if (++s.ls == a.stages) s.ls = 0;
   s.lu += kWarps;
   if (s.lu >= J.units) s.lu = 0, ++s.lk;
@@ -532,9 +534,9 @@ __device__ __forceinline__ void add_terms(float *s, const float4 &v) {
   }
 }
 
-// The products of one tile: warp `warp` takes one unit of each pass, `first` of the first.  False: a wait ran out.
+// The products of one tile: warp `warp` takes one unit of each pass, `first` of the first.
 template <int QT, int NT>
-__device__ __forceinline__ bool split_products(const RowsArgs &a, const RowsJob &J, int first, int lane, Split &s) {
+__device__ __forceinline__ void split_products(const RowsArgs &a, const RowsJob &J, int first, int lane, Split &s) {
   constexpr int HALVES = QT == CMLD_Q6_K ? 2 : 1, P = pass_pitch(QT), UB = unit_bytes(QT);
   const int g = lane >> 2, t = lane & 3, units = J.units;
   const uint8_t *rec = J.rec + (int64_t)first * NT * rows_rec(QT);
@@ -543,7 +545,8 @@ __device__ __forceinline__ bool split_products(const RowsArgs &a, const RowsJob 
   for (int u = first; u < units + kWarps - 1; u += kWarps, rec += kWarps * NT * rows_rec(QT)) {
     if (u - first >= units) break;  // no such pass
     const bool mine = u < units;
-    if (!warp_wait(a, s, &s.landed[s.stage], (uint32_t)s.stage_phase)) return false;
+    bar_wait(a, s, &s.landed[s.stage], (uint32_t)s.stage_phase);
+    __syncwarp();
     const uint8_t *raw = s.smem + a.off_ring + s.stage * a.stage_bytes + first * UB;
     const uint8_t *scales = raw + (kWarps - first) * UB + first * (QT == CMLD_Q6_K ? 2 : 8);
     next_stage(a, s);
@@ -554,7 +557,7 @@ __device__ __forceinline__ bool split_products(const RowsArgs &a, const RowsJob 
       if (mine) unpack_codes<P>(w, raw, g, t, e);
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
-        if (!warp_wait(a, s, &s.empty[s.buf], (uint32_t)(s.buf_phase ^ 1))) return false;
+        bar_wait(a, s, &s.empty[s.buf], (uint32_t)(s.buf_phase ^ 1));
         if (mine) {
           float4 *dst = reinterpret_cast<float4 *>(s.smem + s.buf * (kWarps * kSlice) + first * kSlice) + lane;
           product(w, o, [&](int i, const float4 &f) { dst[i == 0 ? 0 : i == 1 ? 64 : i == 2 ? 32 : 96] = f; });
@@ -569,13 +572,12 @@ __device__ __forceinline__ bool split_products(const RowsArgs &a, const RowsJob 
       }
     }
   }
-  return true;
 }
 
 // The sums of one tile: four warps, a thread per output of a row group (its place in a slice: idx).  Between passes the running sums
-// lie in shared memory, a float (Q6_K: two float4, the halves' classes) per row group.  False: a wait ran out.
+// lie in shared memory, a float (Q6_K: two float4, the halves' classes) per row group.
 template <int QT, int NT>
-__device__ __forceinline__ bool split_sums(const RowsArgs &a, const RowsJob &J, int row0, int idx, Split &s) {
+__device__ __forceinline__ void split_sums(const RowsArgs &a, const RowsJob &J, int row0, int idx, Split &s) {
   constexpr int HALVES = QT == CMLD_Q6_K ? 2 : 1, NL = QT == CMLD_Q6_K ? 4 : 1;
   typedef typename Sums<QT>::type sum_t;
   const int lane = idx & 31;
@@ -593,7 +595,8 @@ __device__ __forceinline__ bool split_sums(const RowsArgs &a, const RowsJob &J, 
 #pragma unroll
         for (int l = 0; l < NL; ++l) acc[l] = 0.0f;
       }
-      if (!warp_wait(a, s, &s.full[s.buf], (uint32_t)s.buf_phase)) return false;
+      bar_wait(a, s, &s.full[s.buf], (uint32_t)s.buf_phase);
+      __syncwarp();
       const float4 *p = reinterpret_cast<const float4 *>(s.smem + s.buf * (kWarps * kSlice)) + idx;
       if (cnt == kWarps) {
         float4 v[kWarps];
@@ -632,27 +635,17 @@ __device__ __forceinline__ bool split_sums(const RowsArgs &a, const RowsJob &J, 
       J.y[at] = J.residual ? __fadd_rn(__ldcg(J.residual + at), v) : v;
     }
   }
-  return true;
 }
 
-// Behind the adding warps' loops: where one of them gave up, copies may still be on their way into this CTA's shared memory, and nobody has
-// waited for them.  A warp that issued fewer passes than another arrives for those it left out, so that every stage's last phase can end.
-__device__ __forceinline__ void drain(const RowsArgs &a, Split &s, bool ok, int warp, int lane, int *loads) {
-  uint32_t gave_up;
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.or.pred p, 1, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(gave_up)
-               : "r"(ok ? 0u : 1u)
-               : "memory");
-  if (!gave_up) return;  // (every pass was used up)
-  if (lane == 0) loads[warp] = s.loads;
-  asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
-  const int most = max(max(loads[0], loads[1]), max(loads[2], loads[3]));
-  if (lane == 0) {
-    for (int i = s.loads; i < most; ++i) bar_arrive(&s.landed[i % a.stages]);
-    for (int i = max(0, most - a.stages); i < most; ++i)
-      for (uint32_t n = 0; n < kRowsSpin && !bar_try(&s.landed[i % a.stages], (uint32_t)(i / a.stages & 1)); ++n) {
-      }
-  }
+// After a wait that ran out, what was fetched may still be on its way into this CTA's shared memory: the adding warps stay until it is there.
+// (All of them have arrived for every pass by the time the last of them is here.)
+__device__ __forceinline__ void drain(const RowsArgs &a, const Split &s, int lane) {
+  if (!*s.gave_up || lane != 0) return;
+  int loads = 0;
+  for (int k = 0; k < s.n_mine; ++k) loads += (a.job[tile_job(a, s.first + k * s.step)].units + kWarps - 1) / kWarps;
+  for (int i = max(0, loads - a.stages); i < loads; ++i)
+    for (uint32_t n = 0; n < kRowsSpin && !bar_try(&s.landed[i % a.stages], (uint32_t)(i / a.stages & 1)); ++n) {
+    }
 }
 
 // The two roles over all tiles of this CTA.
@@ -660,33 +653,31 @@ template <int QT, int NT>
 __device__ __forceinline__ void split_multiply(const RowsArgs &a, int warp, int lane, Split &s) {
   for (int k = 0; k < s.n_mine; ++k) {
     const RowsJob &J = a.job[tile_job(a, s.first + k * s.step)];
-    // (who has no unit in a short pass differs from tile to tile)
-    if (!split_products<QT, NT>(a, J, (warp - k * J.units) & (kWarps - 1), lane, s)) break;
+    split_products<QT, NT>(a, J, (warp - k * J.units) & (kWarps - 1), lane, s);  // (who has no unit in a short pass differs from tile to tile)
   }
 }
 template <int QT, int NT>
-__device__ __forceinline__ bool split_add(const RowsArgs &a, int warp, int lane, Split &s) {
+__device__ __forceinline__ void split_add(const RowsArgs &a, int warp, int lane, Split &s) {
   for (int i = 0; i < a.stages; ++i) load_pass<QT>(a, s, warp, lane);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int k = 0; k < s.n_mine; ++k) {
     const int tile = s.first + k * s.step;
     const RowsJob &J = a.job[tile_job(a, tile)];
-    if (!split_sums<QT, NT>(a, J, (tile - J.first_tile) * 16, warp * 32 + lane, s)) return false;
+    split_sums<QT, NT>(a, J, (tile - J.first_tile) * 16, warp * 32 + lane, s);
   }
-  return true;
 }
 
 template <int NT>
 __global__ void __launch_bounds__(kSplitThreads, 1) rows_split_kernel(const __grid_constant__ RowsArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];  // exchange buffers [buffer][unit of the pass][kSlice], then the stages
   __shared__ __align__(8) uint64_t bars[3 * kMaxStages];
-  __shared__ int gave_up, loads[kSplitWarps - kWarps];
+  __shared__ int gave_up;
   asm volatile("griddepcontrol.launch_dependents;");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kMaxStages; ++i) {
       bar_init(&bars[i], kSplitWarps - kWarps);
-      bar_init(&bars[kMaxStages + i], kWarps);
+      bar_init(&bars[kMaxStages + i], kWarps + a.lose_one);
       bar_init(&bars[2 * kMaxStages + i], kSplitWarps - kWarps);
     }
     gave_up = 0;
@@ -707,16 +698,16 @@ __global__ void __launch_bounds__(kSplitThreads, 1) rows_split_kernel(const __gr
   if (warp < kWarps) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");  // 512 x 104 + 128 x 64 = the 640 x 96 of the launch
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (a.lose_one && threadIdx.x == 0) give_up(a, s);
     if (qt == CMLD_Q4_K) split_multiply<CMLD_Q4_K, NT>(a, warp, lane, s);
     else if (qt == CMLD_Q6_K) split_multiply<CMLD_Q6_K, NT>(a, warp, lane, s);
     else split_multiply<CMLD_Q8_0, NT>(a, warp, lane, s);
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-    bool ok;
-    if (qt == CMLD_Q4_K) ok = split_add<CMLD_Q4_K, NT>(a, warp - kWarps, lane, s);
-    else if (qt == CMLD_Q6_K) ok = split_add<CMLD_Q6_K, NT>(a, warp - kWarps, lane, s);
-    else ok = split_add<CMLD_Q8_0, NT>(a, warp - kWarps, lane, s);
-    drain(a, s, ok, warp - kWarps, lane, loads);
+    if (qt == CMLD_Q4_K) split_add<CMLD_Q4_K, NT>(a, warp - kWarps, lane, s);
+    else if (qt == CMLD_Q6_K) split_add<CMLD_Q6_K, NT>(a, warp - kWarps, lane, s);
+    else split_add<CMLD_Q8_0, NT>(a, warp - kWarps, lane, s);
+    drain(a, s, lane);
   }
 }
 
@@ -899,10 +890,10 @@ int32_t launch_rows_pack(const uint8_t *act, int64_t cols, int32_t batch, uint8_
   return CMLD_OK;
 }
 
-// The records: rec4 for Q4_K matrices, rec6 for Q6_K, rec0 for Q8_0 (those of the types that occur).  no_wait (a self-test): the waits of
-// the split form run out at once; shapes that take the other form, which has none, are refused.
+// The records: rec4 for Q4_K matrices, rec6 for Q6_K, rec0 for Q8_0 (those of the types that occur).  lose_one (a self-test): an arrival of
+// the split form never comes and a wait counts as run out; shapes that take the other form, which has no such waits, are refused.
 int32_t launch_gemv_rows(const GemvJob *jobs, int n_jobs, int32_t batch, const uint8_t *rec4, const uint8_t *rec6, const uint8_t *rec0,
-                         int32_t *status, cudaStream_t s, bool pdl, bool no_wait) {
+                         int32_t *status, cudaStream_t s, bool pdl, bool lose_one) {
   if (!gemv_rows_fits(jobs, n_jobs, batch)) return CMLD_ERR_UNSUPPORTED;
   const int sms = sm_count(), nt = (batch + 7) / 8;
   if (sms < 1) return fail(CMLD_ERR_CUDA, "gemv: no device");
@@ -910,7 +901,7 @@ int32_t launch_gemv_rows(const GemvJob *jobs, int n_jobs, int32_t batch, const u
   a.n_jobs = n_jobs;
   a.batch = batch;
   a.status = status;
-  a.spin = no_wait ? 0 : kRowsSpin;
+  a.lose_one = lose_one;
   for (int pass = 0, k = 0; pass < 2; ++pass)  // Q6_K last
     for (int i = 0; i < n_jobs; ++i) {
       const int qt = jobs[i].qt;
@@ -928,7 +919,7 @@ int32_t launch_gemv_rows(const GemvJob *jobs, int n_jobs, int32_t batch, const u
   const int warps = std::min(kWarps, per_cta), rec = a.job[0].units * nt * rows_rec(qt);
   const int fit = warps > 0 ? (kSmemMax - rec) / (warps * raw_bytes(qt)) : 0;
   if (same && per_cta >= 5 && fit >= 2 && (qt != CMLD_Q6_K || nt == 1)) {
-    if (no_wait) return CMLD_ERR_UNSUPPORTED;
+    if (lose_one) return CMLD_ERR_UNSUPPORTED;
     a.stages = std::min(kMaxStages, fit);
     a.off_ring = rec;
     const int smem = rec + warps * a.stages * raw_bytes(qt);

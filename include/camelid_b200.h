@@ -407,8 +407,8 @@ CMLD_API int32_t cmld_gemv_select_kernel(int32_t choice);
  * arrival word that nobody raises; returns CMLD_ERR_TIMEOUT after timeout_ms (1..5000) when the bound works,
  * CMLD_ERR_STATE otherwise.  One GPU; nothing faults or hangs. */
 CMLD_API int32_t cmld_peer_wait_selftest(int32_t timeout_ms);
-/* Self-test of the bounded waits inside the row-batched matvec (no reference counterpart): the product of cmld_gemv with
- * waits that run out at once.  Returns CMLD_ERR_TIMEOUT when every role leaves and the status word says so; y_dev is
+/* Self-test of the bounded waits inside the row-batched matvec (no reference counterpart): the product of cmld_gemv
+ * with an arrival that never comes.  Returns CMLD_ERR_TIMEOUT when every role ends and the status word says so; y_dev is
  * overwritten with no meaning, the context stays usable.  CMLD_ERR_UNSUPPORTED for shapes whose kernel has no such waits. */
 CMLD_API int32_t cmld_gemv_rows_wait_selftest(const cmld_weight *w, const void *act_dev, int32_t batch, float *y_dev);
 /* Self-test of the parallel evaluation of the sequential f32 sum that RMSNorm (rms_norm_into,

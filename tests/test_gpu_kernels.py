@@ -227,7 +227,7 @@ def test_gemv_rows_largest_sums(cm, orc, name):
 @pytest.mark.parametrize("name,rows,cols", [("Q4_K", 4096, 14336), ("Q6_K", 300, 1792), ("Q8_0", 70, 4352)])
 @pytest.mark.parametrize("batch", [3, 32])
 def test_gemv_rows_waits_that_run_out(cm, name, rows, cols, batch):
-    """Every role leaves while copies are in flight, the status says why, and the next call has the results of the one before."""
+    """Every role ends while copies are in flight, the status says why, and the next call has the results of the one before."""
     from camelid_b200.engine import DeviceBuffer, quantize_activation
 
     qt = QT[name]
