@@ -332,12 +332,12 @@ static void dump_trace(cmld_engine *e) {
   FILE *f = fopen(e->trace_path.c_str(), "w");
   if (!f) return;
   const size_t n = std::min<size_t>(host[0], kTraceRecords);
-  fprintf(f, "start_ns,visible,arrived,prologue,rows,ticket,jobs,tx,rx,cols\n");
+  fprintf(f, "start_ns,visible,arrived,prologue,rows,ticket,jobs,tx,rx,paired,cols\n");
   for (size_t i = 0; i < n; ++i) {
     const unsigned long long *r = host.data() + 1 + i * 8;
-    fprintf(f, "%llu,%lld,%lld,%lld,%lld,%lld,%llu,%llu,%llu,%llu,%lld\n", r[0], (long long)(r[1] - r[0]), (long long)(r[2] - r[0]),
+    fprintf(f, "%llu,%lld,%lld,%lld,%lld,%lld,%llu,%llu,%llu,%llu,%llu,%lld\n", r[0], (long long)(r[1] - r[0]), (long long)(r[2] - r[0]),
             (long long)(r[3] - r[0]), (long long)(r[4] - r[0]), r[5] ? (long long)(r[5] - r[0]) : -1, r[6] & 0xff, (r[6] >> 8) & 0xff,
-            (r[6] >> 16) & 0xff, r[6] >> 32, r[7] ? (long long)(r[7] - r[0]) : -1);
+            (r[6] >> 16) & 0xff, (r[6] >> 24) & 0xff, r[6] >> 32, r[7] ? (long long)(r[7] - r[0]) : -1);
   }
   fclose(f);
   // per-CTA stamps: one line per (CTA, launch) of the last kTraceCtaRecords launches, absolute nanoseconds
@@ -474,6 +474,15 @@ static int rows_min_rows(const cmld_engine *e, int32_t qt) {
   return (e->cfg.flags & (CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV | CMLD_FLAG_TENSOR_BATCH)) ? (1 << 30) : qt == CMLD_Q8_0 ? 1 : 2;
 }
 
+// Whether that is how these matrices of one activation run in a step of `batch` rows.
+static bool batched_takes(const cmld_engine *e, const GemvJob *jobs, int n, int32_t batch) {
+  if (batch < rows_min_rows(e, jobs[0].qt)) return false;
+  if (batch <= kRowsMaxBatch) return gemv_rows_fits(jobs, n, batch);
+  for (int i = 1; i < n; ++i)
+    if ((jobs[i].qt == CMLD_Q8_0) != (jobs[0].qt == CMLD_Q8_0)) return false;
+  return gemv_tc5_fits(jobs, n, batch) && gemv_tc5_pack_bytes(jobs[0].cols, batch) <= e->tc5_pack_bytes;
+}
+
 static int32_t gemv_fused(cmld_engine *e, const Proj *p, int n, int32_t batch, int mode, const float *x, const float *x2,
                           const float *norm_w, int64_t cols, const GemvPeer *peer = nullptr, bool pair_swiglu = false,
                           const KvPrefetch *pf = nullptr) {
@@ -493,7 +502,7 @@ static int32_t gemv_fused(cmld_engine *e, const Proj *p, int n, int32_t batch, i
     }
     return CMLD_OK;
   }
-  if (batch >= rows_min_rows(e, p[0].w->qt) && n <= 3 && !peer && !pair_swiglu && !(n0 && nk)) {
+  if (n <= 3 && !peer && !pair_swiglu) {
     GemvJob jobs[3];
     bool q4 = false, q6 = false;
     for (int i = 0; i < n; ++i) {
@@ -501,8 +510,8 @@ static int32_t gemv_fused(cmld_engine *e, const Proj *p, int n, int32_t batch, i
       q4 = q4 || jobs[i].qt == CMLD_Q4_K;
       q6 = q6 || jobs[i].qt == CMLD_Q6_K;
     }
-    const bool few = batch <= kRowsMaxBatch;
-    if (few ? gemv_rows_fits(jobs, n, batch) : gemv_tc5_fits(jobs, n, batch) && gemv_tc5_pack_bytes(cols, batch) <= e->tc5_pack_bytes) {
+    if (batched_takes(e, jobs, n, batch)) {
+      const bool few = batch <= kRowsMaxBatch;
       uint8_t *const *rec = few ? e->rows_rec : e->tc5_pack;
       uint8_t *rec4 = q4 ? rec[0] : nullptr, *rec6 = q6 ? rec[1] : nullptr, *rec0 = n0 ? rec[0] : nullptr;
       CMLD_TRY(run_norm_quant(e, x, mode == 3 ? x2 : nullptr, mode == 1 ? norm_w : nullptr, cols, batch, nullptr, false, false, rec4, rec6, rec0, !few));
@@ -955,13 +964,18 @@ static int32_t engine_step(cmld_engine *e, const StepOpts &o) {
       const Proj p[2] = {{&L.proj[4], e->gate, nullptr, c.ffn_dim}, {&L.proj[5], e->up, nullptr, c.ffn_dim}};
       GemvPeer g{};
       take_pending(g);
-      // gate and up of equal type: the staged kernel pairs their tiles and writes SwiGLU(gate, up) itself,
-      // so the down projection's operand is a plain quantisation of one vector
-      bool pair = !(c.flags & (CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV)) && L.proj[4].qt == L.proj[5].qt && B < mma_min_rows(e) && (use_peer || B < rows_min_rows(e, L.proj[4].qt));
+      // Gate and up of equal type: the staged kernel, where they run on it, pairs their tiles and writes SwiGLU(gate, up)
+      // itself, so the down projection's operand is a plain quantisation of one vector.  At one row they also go that way if the down
+      // projection does: SwiGLU in the prologue of its CTAs costs more than the row-batched product of gate and up saves (hidden 2048, feed-forward
+      // 5472, Q8_0: 264 | 241 us a step of 4 layers; two rows 313 | 330).  From three rows on a kernel of its own forms the operand once
+      // (hidden 896, 4 rows: 407 us a step, paired 435).
+      bool pair = !(c.flags & (CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV)) && L.proj[4].qt == L.proj[5].qt && B < mma_min_rows(e) &&
+                  (use_peer || B <= kFusedPrologueMaxBatch || B < rows_min_rows(e, L.proj[4].qt));
       if (pair) {
         const GemvJob pj[2] = {{L.proj[4].data, L.proj[4].qt, L.proj[4].rows, L.proj[4].cols, L.proj[4].stride, nullptr, nullptr, 0},
                                {L.proj[5].data, L.proj[5].qt, L.proj[5].rows, L.proj[5].cols, L.proj[5].stride, nullptr, nullptr, 0}};
-        pair = gemv_pipe_fit_batch(pj, 2, true, true) >= 1;
+        const GemvJob dj{L.proj[6].data, L.proj[6].qt, L.proj[6].rows, L.proj[6].cols, L.proj[6].stride, nullptr, nullptr, 0};
+        pair = (use_peer || !batched_takes(e, pj, 2, B) || (B == 1 && !batched_takes(e, &dj, 1, B))) && gemv_pipe_fit_batch(pj, 2, true, true) >= 1;
       }
       CMLD_TRY(gemv_fused(e, p, 2, B, 1, e->h, nullptr, L.ffn_norm, c.hidden, use_peer ? &g : nullptr, pair));
       const Proj pd[1] = {{&L.proj[6], e->h, (e->tp == 1 || lead) ? e->h : nullptr, c.hidden}};

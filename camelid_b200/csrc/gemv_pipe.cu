@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) gemv_pipe_kernel(const PipeAr
       tr = a.peer.trace + 1 + idx * 8;
       tr[0] = global_ns();
       tr[6] = (unsigned long long)a.n_jobs | ((unsigned long long)a.peer.tx_n << 8) | ((unsigned long long)a.peer.rx_n << 16) |
-              ((unsigned long long)a.cols << 32);
+              ((unsigned long long)a.paired << 24) | ((unsigned long long)a.cols << 32);
     }
   }
 

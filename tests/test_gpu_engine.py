@@ -139,6 +139,29 @@ def test_batched_rows_equal_serial_bitwise(pair, orc):
     assert np.array_equal(k0, k2) and np.array_equal(v0, v2)
 
 
+def staged_launches(monkeypatch, tmp_path, cm, orc, hidden, ffn, rows):
+    """(matrices, paired) of every launch of the staged matvec in one Q8_0 step of `rows` rows, whose logits are the checker's."""
+    import csv
+
+    cfg = cm.EngineConfig(n_layers=1, n_heads=4, n_kv_heads=2, head_dim=64, hidden=hidden, ffn_dim=ffn, vocab=512, max_pos=32, max_seqs=4)
+    monkeypatch.setenv("CMLD_TRACE", str(tmp_path / "trace"))
+    pair = ModelPair(cfg, "q8_0", seed=64)
+    tokens = orc.synth_tokens(5, 1, rows, cfg.vocab)
+    _, logits, _ = pair.engine.step_batch(list(range(rows)), tokens, [0] * rows, want_logits=True)
+    for b in range(rows):
+        want = pair.oracle.forward(pair.oracle.embedding(int(tokens[b])), 0)[0]
+        assert np.array_equal(logits[b].view(np.uint32), want.view(np.uint32)), b
+    pair.engine.close()
+    with open(tmp_path / "trace.0") as f:
+        return [(int(r["jobs"]), int(r["paired"])) for r in csv.DictReader(f)]
+
+
+@pytest.mark.parametrize("hidden, ffn, rows, paired", [(288, 576, 1, 1), (288, 576, 2, 1), (288, 576, 3, 0), (1024, 1056, 1, 1)])
+def test_gate_and_up_pair_where_the_staged_kernel_runs_them(monkeypatch, tmp_path, cm, orc, hidden, ffn, rows, paired):
+    """Widths that the row-batched kernel does not take."""
+    assert (2, paired) in staged_launches(monkeypatch, tmp_path, cm, orc, hidden, ffn, rows)
+
+
 def test_seed_layer_round_trip_and_continue(pair, orc):
     eng, cfg = pair.engine, pair.cfg
     prompt = orc.synth_tokens(4, 1, 10, cfg.vocab)
