@@ -470,8 +470,15 @@ static int mma_min_rows(const cmld_engine *e) { return (e->cfg.flags & CMLD_FLAG
 // they are.  Eight steps of 4 layers, us, staged | here:
 //   1 row: Q8_0 1B 2177 | 2023, 8B 4036 | 3557; Q4_K_M 1B 1844 | 2117, 8B 2843 | 3355
 //   2 rows: Q8_0 1B 2974 | 2269, 3B 3973 | 3183, 8B 5693 | 3947; Q4_K_M 1B 2514 | 2278, 3B 3260 | 2931, 8B 4096 | 3779
+// The staged kernel's launches fetch the KV rows of the attention behind them into L2 and these do not; the order of the two stays
+// at long contexts.  A step at contexts of 40 | 1024 | 8000, staged and here: 1 row of Q8_0, 1B 260 | 282 | 477 and 230 | 261 | 450, 8B 479 | 504
+// | 758 and 377 | 407 | 653; 2 rows of Q4_K_M, 1B 298 | 346 | 752 and 270 | 326 | 681, 8B 479 | 532 | 1027 and 408 | 466 | 937.
+// One row of a narrow Q8_0 model has too few weights to pay for the launches that the fused prologue and the pairing of gate and up
+// spare: hidden 256 124 | 149 a step, 512 135 | 150, 768 161 | 163 (wider feed-forward 169 | 167), 1024 174 | 159.
+constexpr int kRowsOneRowHidden = 768;
 static int rows_min_rows(const cmld_engine *e, int32_t qt) {
-  return (e->cfg.flags & (CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV | CMLD_FLAG_TENSOR_BATCH)) ? (1 << 30) : qt == CMLD_Q8_0 ? 1 : 2;
+  if (e->cfg.flags & (CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV | CMLD_FLAG_TENSOR_BATCH)) return 1 << 30;
+  return qt == CMLD_Q8_0 && e->cfg.hidden >= kRowsOneRowHidden ? 1 : 2;
 }
 
 // Whether that is how these matrices of one activation run in a step of `batch` rows.

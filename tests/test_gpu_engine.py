@@ -162,6 +162,12 @@ def test_gate_and_up_pair_where_the_staged_kernel_runs_them(monkeypatch, tmp_pat
     assert (2, paired) in staged_launches(monkeypatch, tmp_path, cm, orc, hidden, ffn, rows)
 
 
+@pytest.mark.parametrize("hidden, rows, staged", [(512, 1, True), (512, 2, False), (768, 1, False)])
+def test_one_row_of_a_narrow_model_runs_on_the_staged_kernel(monkeypatch, tmp_path, cm, orc, hidden, rows, staged):
+    launches = staged_launches(monkeypatch, tmp_path, cm, orc, hidden, 1024, rows)
+    assert ((3, 0) in launches and (2, 1) in launches) if staged else not any(n > 1 for n, _ in launches)
+
+
 def test_seed_layer_round_trip_and_continue(pair, orc):
     eng, cfg = pair.engine, pair.cfg
     prompt = orc.synth_tokens(4, 1, 10, cfg.vocab)
