@@ -98,22 +98,39 @@ static int g_gemv_tc5_min_batch = 9;        // rows from which the tcgen05 kerne
 
 constexpr int32_t kOpTc5Rows = 2048;  // rows per pass of the tcgen05 kernel: bounds its scratch and its grids
 
+// The kernel of a matvec and the floats of scratch that it needs.
+struct GemvRoute {
+  enum Kernel { kRows, kTc5, kMma, kOneRow } kernel;
+  int64_t scratch;
+};
+static GemvRoute gemv_route(const GemvJob &job, int32_t batch) {
+  if (g_gemv_kernel_choice == 0 && batch >= g_gemv_rows_min_batch && batch <= kRowsMaxBatch && gemv_rows_fits(&job, 1, batch))
+    return {GemvRoute::kRows, (gemv_rows_rec_bytes(job.cols, batch) + 3) / 4};
+  if (g_gemv_kernel_choice == 0 && batch >= g_gemv_tc5_min_batch && batch < g_gemv_mma_min_batch && gemv_tc5_fits(&job, 1, batch))
+    return {GemvRoute::kTc5, (gemv_tc5_pack_bytes(job.cols, std::min(batch, kOpTc5Rows)) + 3) / 4};
+  if (g_gemv_kernel_choice == 0 && batch >= g_gemv_mma_min_batch && batch <= 32) {
+    const int64_t need = gemv_mma_scratch_floats(&job, 1, batch);
+    if (need >= 0) return {GemvRoute::kMma, need};
+  }
+  return {GemvRoute::kOneRow, 0};
+}
+
 // One matvec launch on the default stream: staged kernel if it takes the shape, else the generic one.
 static int32_t gemv_launch(OpCall &op, const cmld_weight *w, const uint8_t *act, int32_t batch, float *y, const float *residual,
                            cudaStream_t stream = nullptr, bool pdl = false) {
   GemvJob probe{w->data, w->qt, w->rows, w->cols, w->stride, y, residual, w->rows};
-  if (g_gemv_kernel_choice == 0 && batch >= g_gemv_rows_min_batch && batch <= kRowsMaxBatch && gemv_rows_fits(&probe, 1, batch)) {
-    uint8_t *rec = reinterpret_cast<uint8_t *>(op.scratch((gemv_rows_rec_bytes(w->cols, batch) + 3) / 4));
-    if (!rec) return fail(CMLD_ERR_OOM, "gemv: no room for %lld bytes of activation records", (long long)gemv_rows_rec_bytes(w->cols, batch));
+  const GemvRoute route = gemv_route(probe, batch);
+  float *scratch = route.scratch > 0 ? op.scratch(route.scratch) : nullptr;
+  if (route.scratch > 0 && !scratch) return fail(CMLD_ERR_OOM, "gemv: no room for %lld bytes of scratch", (long long)route.scratch * 4);
+  if (route.kernel == GemvRoute::kRows) {
+    uint8_t *rec = reinterpret_cast<uint8_t *>(scratch);
     uint8_t *rec4 = w->qt == CMLD_Q4_K ? rec : nullptr, *rec6 = w->qt == CMLD_Q6_K ? rec : nullptr, *rec0 = w->qt == CMLD_Q8_0 ? rec : nullptr;
     CMLD_TRY(launch_rows_pack(act, w->cols, batch, rec4, rec6, rec0, stream));
     return launch_gemv_rows(&probe, 1, batch, rec4, rec6, rec0, op.status(), stream, pdl);
   }
-  if (g_gemv_kernel_choice == 0 && batch >= g_gemv_tc5_min_batch && batch < g_gemv_mma_min_batch && gemv_tc5_fits(&probe, 1, batch)) {
+  if (route.kernel == GemvRoute::kTc5) {
     // several rows: one pass over the weights per 2048 rows on the tcgen05 tensor cores, same bits as the one-row kernels
-    const int64_t need = gemv_tc5_pack_bytes(w->cols, std::min(batch, kOpTc5Rows));
-    uint8_t *pack = reinterpret_cast<uint8_t *>(op.scratch((need + 3) / 4));
-    if (!pack) return fail(CMLD_ERR_OOM, "gemv: no room for %lld bytes of packed activations", (long long)need);
+    uint8_t *pack = reinterpret_cast<uint8_t *>(scratch);
     uint8_t *rec4 = w->qt == CMLD_Q4_K ? pack : nullptr, *rec6 = w->qt == CMLD_Q6_K ? pack : nullptr, *rec0 = w->qt == CMLD_Q8_0 ? pack : nullptr;
     for (int32_t b0 = 0; b0 < batch; b0 += kOpTc5Rows) {
       const int32_t nb = std::min(batch - b0, kOpTc5Rows);
@@ -123,15 +140,10 @@ static int32_t gemv_launch(OpCall &op, const cmld_weight *w, const uint8_t *act,
     }
     return CMLD_OK;
   }
-  if (g_gemv_kernel_choice == 0 && batch >= g_gemv_mma_min_batch && batch <= 32) {
+  if (route.kernel == GemvRoute::kMma) {
     // more than 8 rows: one pass over the weights on the tensor cores
-    const int64_t need = gemv_mma_scratch_floats(&probe, 1, batch);
-    if (need >= 0) {
-      float *scratch = need > 0 ? op.scratch(need) : nullptr;
-      if (need > 0 && !scratch) return fail(CMLD_ERR_OOM, "gemv: no room for %lld floats of partial sums", (long long)need);
-      const int32_t rc = launch_gemv_mma(&probe, 1, act, batch, scratch, need, op.status(), stream, pdl, nullptr);
-      if (rc != CMLD_ERR_UNSUPPORTED) return rc;
-    }
+    const int32_t rc = launch_gemv_mma(&probe, 1, act, batch, scratch, route.scratch, op.status(), stream, pdl, nullptr);
+    if (rc != CMLD_ERR_UNSUPPORTED) return rc;
   }
   const int fit = g_gemv_kernel_choice == 0 ? gemv_pipe_fit_batch(&probe, 1) : 0;
   const int pass = fit > 0 ? fit : 8;
@@ -488,8 +500,14 @@ int32_t cmld_gemv_time(cmld_weight *const *copies, int32_t n_copies, const void 
   CMLD_CUDA(cudaEventCreate(&e0));
   CMLD_CUDA(cudaEventCreate(&e1));
   OpCall op;
-  op.status();  // make the status word before capture
+  op.status();  // the status word and the scratch are made before the capture, whatever the number of warm-up launches
+  int64_t scratch = 0;
+  for (int i = 0; i < n_copies; ++i) {
+    const GemvJob j{copies[i]->data, copies[i]->qt, copies[i]->rows, copies[i]->cols, copies[i]->stride, y_dev, nullptr, copies[i]->rows};
+    scratch = std::max(scratch, gemv_route(j, batch).scratch);
+  }
   int32_t rc = CMLD_OK;
+  if (scratch > 0 && !op.scratch(scratch)) rc = fail(CMLD_ERR_OOM, "gemv_time: no room for %lld bytes of scratch", (long long)scratch * 4);
   const uint8_t *act = static_cast<const uint8_t *>(act_dev);
   for (int it = 0; it < warmup && rc == CMLD_OK; ++it) rc = gemv_launch(op, copies[it % n_copies], act, batch, y_dev, nullptr, st, false);
   if (rc == CMLD_OK && cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) rc = fail(CMLD_ERR_CUDA, "graph capture failed to start");

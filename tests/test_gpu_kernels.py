@@ -240,6 +240,28 @@ def test_gemv_rows_waits_that_run_out(cm, name, rows, cols, batch):
     assert np.array_equal(w.gemv(act, batch).view(np.uint32), before.view(np.uint32))
 
 
+@pytest.mark.parametrize("batch", [3, 32, 33])
+def test_gemv_time_without_warm_up(batch):
+    """The first call of a process captures its launches at once: the scratch has to be there before."""
+    import subprocess
+    import sys
+
+    program = f"""if True:
+        import ctypes as C
+        import numpy as np
+        import camelid_b200 as cm
+        from camelid_b200.engine import DeviceBuffer, quantize_activation
+
+        w = cm.Weight.synth(cm.Q4_K, 1, 2, 64, 4096, 0.02)
+        act = quantize_activation(cm.ACT_Q8_K, np.ones(({batch}, 4096), np.float32))
+        y, ms, copies = DeviceBuffer({batch} * 64 * 4), C.c_float(0), (C.c_void_p * 1)(w._h)
+        rc = cm.lib().cmld_gemv_time(copies, 1, act.ptr, {batch}, y.ptr, 0, 4, C.byref(ms))
+        assert rc == 0 and ms.value > 0, cm.lib().cmld_last_error()
+        """
+    done = subprocess.run([sys.executable, "-c", program], cwd=GOLDEN.parent.parent, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr
+
+
 @pytest.mark.parametrize("batch", [3, 8, 9, 32])
 def test_gemv_of_several_threads(cm, batch):
     """Threads with matrices, activations and outputs of their own, of several widths: each has the results it has alone."""
