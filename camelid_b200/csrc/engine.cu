@@ -163,15 +163,32 @@ int32_t init_rows(cmld_engine *e, int64_t rows, int64_t logit_rows, int64_t voca
 // all rows of a step, so a prompt goes in by steps of up to 1024 rows where that product takes the shapes.  Four layers, in steps of
 // 512 | 768 | 1024 | 1536 rows, us: 1024 tokens of the 8B width (Q4_K_M) 9589 | 9799 | 8962 | 8964; 1000 of the 3B width 5963 | 5771 |
 // 5298 | 5295; 600 of it in Q8_0 4650 | 3779 | 3778 | 3773; 1500 of the 1B width (Q8_0) 7755 | 7992 | 7560 | 7538: longer steps only
-// add to the scratch rows, which every engine holds (1024 rows of the 8B width: 0.2 GB).  The experts of a Mixtral shape share an
+// add to the scratch rows, which every engine holds (1024 rows of the 8B width: 0.27 GB, and 0.3 GB for the scores of contexts of 2048
+// positions, at most 0.54).  The experts of a Mixtral shape share an
 // unpacked weight among a step's rows likewise (600 tokens, two layers: 34.6 | 32.2 | 32.2 | 32.4 ms).  Everything else: 32 rows, the
 // rows of those modes' own products and attention (the attention over a Q8_0 cache has a CTA for every row and head, the split-range
 // one scratch for the rows of a listed step).
+constexpr int32_t kLongRows = 1024;  // (half of them where an engine's rows do not fit the card otherwise)
 static int32_t prompt_rows(const cmld_engine *e) {
   const cmld_config &c = e->cfg;
   const uint32_t other = CMLD_FLAG_EXACT_ORDER | CMLD_FLAG_DIRECT_GEMV | CMLD_FLAG_TENSOR_BATCH | CMLD_FLAG_FAST_ORDER | CMLD_FLAG_KV_Q8_0;
   if (((uint32_t)c.flags & other) || c.hidden % 256 || c.ffn_dim % 256 || (c.n_heads * c.head_dim) % 256) return kShortRows;
-  return (int32_t)std::min<int64_t>(1024, ((int64_t)c.max_pos + 31) / 32 * 32);
+  return (int32_t)std::min<int64_t>(e->chunk_rows, ((int64_t)c.max_pos + 31) / 32 * 32);
+}
+
+// The scratch of the attention of long prompt steps, up to half a GB: made once the weights are in, or by the first long step.  An engine
+// for which there is no room keeps to the row kernel.  Returns the floats there are.
+static int64_t hold_prompt_scratch(cmld_engine *e) {
+  if (e->prompt_scratch_floats > 0 && !e->prompt_scratch) {
+    if (cudaMalloc(&e->prompt_scratch, (size_t)e->prompt_scratch_floats * sizeof(float)) == cudaSuccess) {
+      e->allocs.push_back(e->prompt_scratch);
+    } else {
+      cudaGetLastError();
+      e->prompt_scratch = nullptr;
+      e->prompt_scratch_floats = 0;
+    }
+  }
+  return e->prompt_scratch_floats;
 }
 
 static int32_t engine_init(cmld_engine *e) {
@@ -282,10 +299,7 @@ static int32_t engine_init(cmld_engine *e) {
     const int64_t widest = std::max<int64_t>(std::max<int64_t>(c.hidden, c.ffn_dim), e->q_width);
     const int64_t wide = (widest + 255) / 256 * 256;
     e->tc5_pack_bytes = gemv_tc5_pack_bytes(wide, (int32_t)R);
-    if (e->chunk_rows > kShortRows) {
-      e->prompt_scratch_floats = attention_prompt_scratch_floats(c.n_heads, c.n_kv_heads, c.head_dim, e->chunk_rows, c.max_pos);
-      if (e->prompt_scratch_floats > 0) CMLD_TRY(dev_alloc(e, &e->prompt_scratch, e->prompt_scratch_floats, false));
-    }
+    if (e->chunk_rows > kShortRows) e->prompt_scratch_floats = attention_prompt_scratch_floats(c.n_heads, c.n_kv_heads, c.head_dim, e->chunk_rows, c.max_pos);
     for (auto &pack : e->tc5_pack) CMLD_TRY(dev_alloc(e, &pack, e->tc5_pack_bytes, false));
     for (auto &rec : e->rows_rec) CMLD_TRY(dev_alloc(e, &rec, gemv_rows_rec_bytes(wide, kRowsMaxBatch), false));
   }
@@ -882,7 +896,7 @@ static int32_t engine_step(cmld_engine *e, const StepOpts &o) {
       const bool rows = !fast && !(c.flags & CMLD_FLAG_EXACT_ORDER) && B >= 3 && o.attn_cap > 0 && !o.tree_mask &&
                         attention_rows_fits(c.n_heads, c.n_kv_heads, c.head_dim, o.attn_cap);
       // a prompt's long steps (never captured: their context is exact): neighbouring rows share a CTA
-      const bool prompt = rows && o.prompt_end && attention_prompt_fits(c.n_heads, c.n_kv_heads, c.head_dim, B, o.prompt_end, e->sm_count, e->prompt_scratch_floats);
+      const bool prompt = rows && o.prompt_end && attention_prompt_fits(c.n_heads, c.n_kv_heads, c.head_dim, B, o.prompt_end, e->sm_count, hold_prompt_scratch(e));
       const bool ordered = !rows && !fast && !(c.flags & CMLD_FLAG_EXACT_ORDER) && o.attn_cap > 0 && !o.tree_mask &&
                            attention_ordered_fits(c.n_heads, c.n_kv_heads, c.head_dim, o.attn_cap);
       const bool fuse = !o.shared_slots && (fast || ordered);
@@ -1291,22 +1305,27 @@ int32_t cmld_engine_create(const cmld_config *cfg_in, cmld_engine **out) {
   CMLD_CUDA(cudaMemGetInfo(&free_b, &total_b));
   if (kv_bytes > 0.95 * (double)free_b)
     return fail(CMLD_ERR_OOM, "KV cache of %.1f GiB does not fit in %.1f GiB free", kv_bytes / (1 << 30), (double)free_b / (1 << 30));
-  cmld_engine *e = new cmld_engine();
-  e->cfg = local;
-  e->full = *cfg_in;
-  e->tp = tp;
-  e->ep = ep;
-  e->shard_rank = shard_rank;
-  e->vocab_local = local.vocab / tp;
-  e->device = dev;
-  int32_t rc = engine_init(e);
-  if (rc != CMLD_OK) {
+  for (int32_t rows = kLongRows;; rows /= 2) {
+    cmld_engine *e = new cmld_engine();
+    e->cfg = local;
+    e->full = *cfg_in;
+    e->tp = tp;
+    e->ep = ep;
+    e->shard_rank = shard_rank;
+    e->vocab_local = local.vocab / tp;
+    e->device = dev;
+    e->chunk_rows = rows;
+    const int32_t rc = engine_init(e);
+    if (rc == CMLD_OK) {
+      *out = e;
+      return CMLD_OK;
+    }
+    const bool shorter = rc == CMLD_ERR_OOM && e->chunk_rows == kLongRows;  // there may be room for the rows of shorter prompt steps
+    cudaGetLastError();
     engine_free(e);
     delete e;
-    return rc;
+    if (!shorter) return rc;
   }
-  *out = e;
-  return CMLD_OK;
 }
 
 int32_t cmld_engine_destroy(cmld_engine *e) {
@@ -1457,6 +1476,7 @@ int32_t cmld_engine_set_output(cmld_engine *e, const float *final_norm, const cm
   if (e->output.qt == CMLD_F32) return fail(CMLD_ERR_UNSUPPORTED, "set_output: f32 output weights are not supported");
   CMLD_TRY(upload_f32(&e->final_norm, final_norm, e->cfg.hidden, e->stream));
   e->has_output = true;
+  if (e->has_embd) hold_prompt_scratch(e);
   return CMLD_OK;
 }
 
@@ -1467,6 +1487,7 @@ int32_t cmld_engine_set_token_embd(cmld_engine *e, const cmld_tensor *t) {
   if (!t) return fail(CMLD_ERR_INVALID, "set_token_embd: tensor is null");
   CMLD_TRY(weight_upload(e->token_embd, t->qtype, e->cfg.vocab, e->cfg.hidden, t->data, t->nbytes, e->stream));
   e->has_embd = true;
+  if (e->has_output) hold_prompt_scratch(e);
   return CMLD_OK;
 }
 
@@ -1556,6 +1577,7 @@ int32_t cmld_engine_adopt_output(cmld_engine *e, const float *final_norm, cmld_w
   CMLD_TRY(adopt(e->output, output, e->vocab_local, e->cfg.hidden, "adopt_output"));
   CMLD_TRY(upload_f32(&e->final_norm, final_norm, e->cfg.hidden, e->stream));
   e->has_output = true;
+  if (e->has_embd) hold_prompt_scratch(e);
   return CMLD_OK;
 }
 
@@ -1566,6 +1588,7 @@ int32_t cmld_engine_adopt_token_embd(cmld_engine *e, cmld_weight *token_embd) {
   if (!token_embd) return fail(CMLD_ERR_INVALID, "adopt_token_embd: weight is null");
   CMLD_TRY(adopt(e->token_embd, token_embd, e->cfg.vocab, e->cfg.hidden, "adopt_token_embd", true));
   e->has_embd = true;
+  if (e->has_output) hold_prompt_scratch(e);
   return CMLD_OK;
 }
 

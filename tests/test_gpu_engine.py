@@ -434,6 +434,44 @@ def test_long_prompt_steps_whose_scores_go_by_groups(cm, orc):
     assert t1 == t2 and np.array_equal(got.view(np.uint32), ref.view(np.uint32))
 
 
+def test_engines_open_on_a_nearly_full_card(monkeypatch, cm, orc):
+    """Without room for the prompt attention's scratch, and without room for the rows of the longest steps: the same logits."""
+    import torch
+
+    from camelid_b200 import synth
+    from camelid_b200.engine import DeviceBuffer
+
+    cfg = cm.EngineConfig(n_layers=1, n_heads=64, n_kv_heads=64, head_dim=64, hidden=4096, ffn_dim=14336, vocab=512, max_pos=4096)
+    prompt, want = orc.synth_tokens(4, 1, 1100, 512), [5, 511, 1023, 1024, 1099]
+    free = lambda: torch.cuda.mem_get_info()[0]
+
+    def run(eng):
+        token, logits = eng.extend(0, prompt, 0, want=want)
+        launches = eng.last_timing()[1]
+        eng.close()
+        return token, logits.view(np.uint32), launches
+
+    run(synth.build_engine(cfg, "q4_k_m", 5))  # (what the library itself loads is in place)
+    before = free()
+    eng = cm.ResidentDecode(cfg)
+    opened = before - free()
+    eng.close()
+    eng = synth.build_engine(cfg, "q4_k_m", 5)
+    held = before - free()
+    token, logits, launches = run(eng)
+    full = DeviceBuffer(free() - held + (256 << 20))  # half of the scratch is missing
+    eng = synth.build_engine(cfg, "q4_k_m", 5)
+    del full
+    fewer = run(eng)
+    assert fewer[0] == token and np.array_equal(fewer[1], logits) and fewer[2] < launches  # one kernel of attention a step in place of three
+    full = DeviceBuffer(free() - opened + (64 << 20))
+    eng = cm.ResidentDecode(cfg)
+    del full
+    monkeypatch.setattr(synth, "ResidentDecode", lambda cfg: eng)
+    shorter = run(synth.build_engine(cfg, "q4_k_m", 5))
+    assert shorter[0] == token and np.array_equal(shorter[1], logits) and shorter[2] > launches  # three steps in place of two
+
+
 @pytest.mark.parametrize("slots", [40, 64, 512])
 def test_prompts_take_the_same_steps_whatever_the_number_of_slots(cm, orc, slots):
     """A prompt's steps are chosen by its rows: an engine of many slots launches what an engine of one launches (no logits of
