@@ -104,6 +104,18 @@ def test_linear_tiles_shared_out(cm, shape):
     assert (np.abs(out.to_numpy(np.float32).reshape(shape[2], shape[0]) - x.astype(np.float64) @ v.astype(np.float64).T) <= bound).all()
 
 
+@pytest.mark.parametrize("cols", [320, 576, 1088])  # 2, 4 and 8 CTAs a tile, of the last two some without a share of the columns
+@pytest.mark.parametrize("rows", [3, 16, 64])
+def test_linear_tiles_of_a_cluster(cm, cols, rows):
+    w, x = lin_case((130, cols, rows), 14)
+    ref = x.astype(np.float64) @ w.astype(np.float64).T
+    # a chain of all products, every addition within an ulp (the accumulator's own may truncate), and the eight partials
+    bound = 2.0 ** -23 * (cols + 16) * (np.abs(x) @ np.abs(w).T)
+    y = linear(cm, 1, w, x)
+    assert (np.abs(y - ref) <= bound).all()
+    assert np.abs(linear(cm, 1, w, x, act=3) - pl.silu(y[:, 0::2].astype(np.float64)) * y[:, 1::2]).max() < 1e-5 * np.abs(y).max() ** 2
+
+
 def test_linear_activations(cm):
     w, x = lin_case((200, 96, 40), 3)
     ref = x.astype(np.float64) @ w.astype(np.float64).T
