@@ -8,8 +8,12 @@
 // the boundary between sublayers, an RMS norm (with a sigmoid gate, or over groups of columns with a SiLU gate), or a plain copy, with all
 // its loads in flight at once.  Two products that do not depend on each other can share a launch: the first `n_first` CTAs work on one.
 // One row, one after the other in a graph, before (whole rows per warp, weights in registers, fetched when the last were used up) and now:
-// 14336 x 4096 25.4 -> 19.7 us, 4096 x 14336 24.3 -> 20.6, 32000 x 4096 47.1 -> 41.7 (6.3 TB/s), 6144 x 1536 6.7 -> 5.5; two rows 29.4 -> 22.7,
-// 30.1 -> 23.5, 52.8 -> 45.0, 8.4 -> 6.9.  What is left is 4 to 5 us a launch: the wait, the operand, the last CTA.  Rings of 48, 96 and 160 KB
+// 14336 x 4096 25.4 -> 19.7 us, 4096 x 14336 24.3 -> 20.6, 32000 x 4096 47.1 -> 41.7 (6.3 TB/s), 6144 x 1536 6.7 -> 5.4; two rows 29.4 -> 20.8,
+// 29.9 -> 21.7 and, of the last, 8.3 -> 6.3.  The operand of two rows is asked for together (14336 x 4096 23.0 -> 20.8), and so are a group's values,
+// gate and weights (two rows of a pair of products with groups of 128, 25.0 us before, cold; a model's step of two rows 395 -> 337).
+// Narrow matrices have too few steps to pay for rows that lie in several warps: up to kMvWholeCols columns and as many rows as there are
+// warps, a row goes whole to a warp (1024 x 1024 2.8 -> 2.4 us, two rows 3.7 -> 2.5; at 2048 columns, 768 rows, 3.1 -> 3.3: not there).
+// What is left is 4 to 5 us a launch: the wait, the operand, the last CTA.  Rings of 48, 96 and 160 KB
 // measured 21.1, 20.1 and 19.7 us for 14336 x 4096 and 16.6, 16.4 and 16.9 ms for a request that 64 KB serve in 16.1 (4 layers, 32 tokens).
 // Registers keep it at one CTA per SM: where two fit, the CTAs of the next launch pile up on some SMs (42 us in place of 23).
 #include "layered.cuh"
@@ -20,6 +24,7 @@ namespace {
 
 constexpr int kMvThreads = 512, kMvWarps = kMvThreads / 32;
 constexpr int kMvRing = 64 * 1024;  // bytes
+constexpr int kMvWholeCols = 1024;  // rows of up to so many columns go whole to a warp where every warp has at most one
 constexpr size_t kMvMaxCols = 220 * 1024, kMvMaxSmem = 224 * 1024;  // (kMvRing + two thirds of kMvMaxCols is less)
 
 __host__ __device__ constexpr int mv_kpad(int cols) { return (cols + 255) & ~255; }
@@ -44,6 +49,22 @@ __device__ __noinline__ void mv_prologue(const LinMvArgs &a, int r, float *xr, f
     const float *gate = a.gate + r * a.gate_ld;
     for (int c0 = warp * a.group; c0 < K; c0 += kMvWarps * a.group) {
       float s = 0.0f;
+      if (a.group <= 128) {  // everything asked for at once
+        float xv[4], gv[4], nw[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int i = lane + 32 * j;
+          const bool in = i < a.group;
+          xv[j] = in ? x[c0 + i] : 0.0f, gv[j] = in ? gate[c0 + i] : 0.0f, nw[j] = in ? a.norm_w[i] : 0.0f;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s = fmaf(xv[j], xv[j], s);
+        const float inv = 1.0f / sqrtf(warp_sum(s) / (float)a.group + a.eps);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (lane + 32 * j < a.group) xr[c0 + lane + 32 * j] = xv[j] * inv * nw[j] * silu_f(gv[j]);
+        continue;
+      }
       for (int i = lane; i < a.group; i += 32) s = fmaf(x[c0 + i], x[c0 + i], s);
       const float inv = 1.0f / sqrtf(warp_sum(s) / (float)a.group + a.eps);
       for (int i = lane; i < a.group; i += 32) xr[c0 + i] = x[c0 + i] * inv * a.norm_w[i] * silu_f(gate[c0 + i]);
@@ -78,8 +99,13 @@ __device__ __forceinline__ void lin_mv_cta(const LinMvArgs &a, int cta, int ctas
   uint4 *ring = reinterpret_cast<uint4 *>(smem) + tid;  // [stage][ROWS][thread]
   float *xs = smem + kMvRing / 4;                       // [R][kp]
   const int groups = (a.w.rows + ROWS - 1) / ROWS;
-  const int g0 = (int)((int64_t)groups * cta / ctas), steps = ((int)((int64_t)groups * (cta + 1) / ctas) - g0) * nit;
-  const int lo = (int)((int64_t)steps * warp / kMvWarps), hi = (int)((int64_t)steps * (warp + 1) / kMvWarps);
+  // groups * c / ctas and steps * w / kMvWarps, rounded down, without 64-bit divisions
+  const unsigned whole = (unsigned)groups / (unsigned)ctas, rest = (unsigned)groups - whole * ctas;
+  auto group_of = [&](int c) { return (int)(whole * c + rest * c / (unsigned)ctas); };
+  const int g0 = group_of(cta), mine = group_of(cta + 1) - g0, steps = mine * nit;
+  auto run_of = [&](int w) { return steps / kMvWarps * w + steps % kMvWarps * w / kMvWarps; };
+  const bool rows_whole = ROWS == 1 && mine <= kMvWarps && K <= kMvWholeCols;  // a row per warp, all of it asked for at once
+  const int lo = rows_whole ? min(warp, mine) * nit : run_of(warp), hi = rows_whole ? min(warp + 1, mine) * nit : run_of(warp + 1);
 
   // Step s of the CTA: columns s % nit * 256 .. of the ROWS rows s / nit; a lane copies what it will use itself.
   const uint32_t ring_at = (uint32_t)__cvta_generic_to_shared(ring);
@@ -99,12 +125,16 @@ __device__ __forceinline__ void lin_mv_cta(const LinMvArgs &a, int cta, int ctas
     src += 256;
   };
   pdl_launch();
-  if (lo < hi) rows_at(lo);
+  if (rows_whole) {
+    src = a.w.w + (int64_t)(g0 + warp) * a.w.ld + lane * 8, below = 0, left = nit;
+  } else if (lo < hi) {
+    rows_at(lo);
+  }
 #pragma unroll
   for (int i = 0; i < kStages - 1; ++i) {
     if (lo + i < hi) {
       copy(i);
-      if (--left == 0) rows_at(lo + i + 1);
+      if (--left == 0 && lo + i + 1 < hi) rows_at(lo + i + 1);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
@@ -115,27 +145,32 @@ __device__ __forceinline__ void lin_mv_cta(const LinMvArgs &a, int cta, int ctas
   const auto aligned = [](const float *p, int64_t ld) { return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)(4 * ld)) & 15) == 0; };
   const bool quads = K % 4 == 0 && aligned(a.x, a.x_ld) && aligned(a.gate, a.gate_ld) && aligned(a.norm_w, 0);
   const int n4 = K / 4;
+  if (K < kp) {  // zeros behind the rows, in place before anything of them is
+    for (int i = tid; i < 64 * R; i += kMvThreads) reinterpret_cast<float4 *>(xs + (i / 64 + 1) * kp)[i % 64 - 64] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    __syncthreads();
+  }
+  if (quads && a.prologue == kProPlain) {
+    constexpr int N = 8 / R;
+    for (int i0 = tid; i0 < n4; i0 += N * kMvThreads) {
+      float4 v[R][N];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+          if (i0 + j * kMvThreads < n4) v[r][j] = reinterpret_cast<const float4 *>(a.x + r * a.x_ld)[i0 + j * kMvThreads];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+          if (i0 + j * kMvThreads < n4) reinterpret_cast<float4 *>(xs + r * kp)[mv_unit(i0 + j * kMvThreads)] = v[r][j];
+    }
+  } else
 #pragma unroll 1
   for (int r = 0; r < R; ++r) {
     float *xr = xs + r * kp;
     float4 *x4 = reinterpret_cast<float4 *>(xr);
-    if (K < kp) {  // zeros behind the row, in place before anything of it is
-      for (int i = kp / 4 - 64 + tid; i < kp / 4; i += kMvThreads) x4[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      __syncthreads();
-    }
     if (mixed) {
       mix_row<2>(a.mix, a.mix.row_map ? a.mix.row_map[r] : r, coef, red, cta == 0, [&](int i, float4 v) { x4[mv_unit(i)] = v; });
-    } else if (quads && a.prologue == kProPlain) {
-      const float4 *x = reinterpret_cast<const float4 *>(a.x + r * a.x_ld);
-      for (int i0 = tid; i0 < n4; i0 += 8 * kMvThreads) {
-        float4 v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (i0 + j * kMvThreads < n4) v[j] = x[i0 + j * kMvThreads];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (i0 + j * kMvThreads < n4) x4[mv_unit(i0 + j * kMvThreads)] = v[j];
-      }
     } else if (quads && (a.prologue == kProRms || a.prologue == kProRmsGate) && n4 <= 2 * kMvThreads) {
       const float4 *x = reinterpret_cast<const float4 *>(a.x + r * a.x_ld), *gate = reinterpret_cast<const float4 *>(a.gate + r * a.gate_ld);
       const float4 *nw = reinterpret_cast<const float4 *>(a.norm_w);
@@ -188,7 +223,7 @@ __device__ __forceinline__ void lin_mv_cta(const LinMvArgs &a, int cta, int ctas
       if (ROWS == 2 && a.act == kActSwiGlu) a.y[r * a.y_ld + g] = silu_f(v[0]) * v[ROWS - 1];
     }
   };
-  int g = g0 + lo / nit, it = lo % nit;
+  int g = rows_whole ? g0 + warp : g0 + lo / nit, it = rows_whole ? 0 : lo - (g - g0) * nit;
   const bool joins = it != 0 && lo < hi;  // the warp's first row began in another warp
   bool head = joins;
   const float *x = xs + it * 256 + lane * 8;
@@ -198,7 +233,7 @@ __device__ __forceinline__ void lin_mv_cta(const LinMvArgs &a, int cta, int ctas
   for (int i = 0; i < ROWS; ++i)
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[i][r] = 0.0f;
-  if (lo + kStages - 1 < hi) rows_at(lo + kStages - 1);
+  if (!rows_whole && lo + kStages - 1 < hi) rows_at(lo + kStages - 1);
   for (int s0 = lo; s0 < hi; s0 += kStages) {
 #pragma unroll
     for (int j = 0; j < kStages; ++j) {
@@ -206,7 +241,7 @@ __device__ __forceinline__ void lin_mv_cta(const LinMvArgs &a, int cta, int ctas
       if (s >= hi) break;
       if (s + kStages - 1 < hi) {  // into the stage of step s - 1, whose bytes this thread has used
         copy((j + kStages - 1) % kStages);
-        if (--left == 0) rows_at(s + kStages);
+        if (--left == 0 && s + kStages < hi) rows_at(s + kStages);
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
       asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
@@ -256,6 +291,7 @@ __device__ __forceinline__ void lin_mv_cta(const LinMvArgs &a, int cta, int ctas
       }
     }
   }
+  if (rows_whole) return;
   __syncthreads();
   // a row that begins in this warp and ends in another: `it` of its steps were done here
   if (lane == 0 && lo < hi && it != 0 && (!joins || g > g0 + lo / nit)) {
@@ -266,7 +302,7 @@ __device__ __forceinline__ void lin_mv_cta(const LinMvArgs &a, int cta, int ctas
       for (int r = 0; r < R; ++r) sum[i][r] = part[warp][1][i][r];
     const int end = (g - g0 + 1) * nit;
     for (int w = warp + 1, at = hi; at < end; ++w) {
-      const int upto = (int)((int64_t)steps * (w + 1) / kMvWarps);
+      const int upto = run_of(w + 1);
       if (upto > at) {
 #pragma unroll
         for (int i = 0; i < ROWS; ++i)
@@ -286,8 +322,8 @@ __global__ void __launch_bounds__(kMvThreads, 1) lin_mv_kernel(const __grid_cons
 
 template <int R, int ROWS>
 __global__ void __launch_bounds__(kMvThreads, 1) lin_mv_pair_kernel(const __grid_constant__ LinMvArgs a, const __grid_constant__ LinMvArgs b, int n_first) {
-  if ((int)blockIdx.x < n_first) lin_mv_cta<R, ROWS>(a, blockIdx.x, n_first);
-  else lin_mv_cta<R, ROWS>(b, blockIdx.x - n_first, gridDim.x - n_first);
+  const bool first = (int)blockIdx.x < n_first;
+  lin_mv_cta<R, ROWS>(first ? a : b, first ? blockIdx.x : blockIdx.x - n_first, first ? n_first : gridDim.x - n_first);
 }
 
 size_t mv_smem(int cols, int batch) { return kMvRing + (size_t)batch * mv_kpad(cols) * 4; }
@@ -328,8 +364,8 @@ int32_t launch_lin_mv(const LinMvArgs &a, bool pdl, cudaStream_t s) {
     return a.batch == 1 ? mv_launch<1, 2>(a, pdl, s) : mv_launch<2, 2>(a, pdl, s);
   }
   // single rows only where pairs would leave SMs without work or with one more than others (576 x 4096: 3.2 us, in pairs 3.4; 1536 x 4096: 4.8
-  // and 4.5, 4096 x 4096: 8.0 and 7.6)
-  const bool single = a.w.rows <= 4 * mv_sms();
+  // and 4.5, 4096 x 4096: 8.0 and 7.6), and where rows go whole to warps
+  const bool single = a.w.rows <= 4 * mv_sms() || (a.w.rows <= kMvWarps * mv_sms() && a.w.cols <= kMvWholeCols);
   if (a.batch == 1) return single ? mv_launch<1, 1>(a, pdl, s) : mv_launch<1, 2>(a, pdl, s);
   return single ? mv_launch<2, 1>(a, pdl, s) : mv_launch<2, 2>(a, pdl, s);
 }

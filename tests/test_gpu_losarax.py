@@ -85,6 +85,17 @@ def test_matrix_vector_rows_shared_by_warps(cm, shape):
         assert (np.abs(linear(cm, 0, w, x[:n]) - ref[:n]) <= bound[:n]).all()
 
 
+@pytest.mark.parametrize("shape", [(593, 1024), (2368, 1024), (2369, 1024), (2368, 1032), (1000, 72), (700, 257), (2368, 515)])
+def test_matrix_vector_rows_whole_to_warps(cm, shape):
+    """Narrow matrices at the ends of the rule: all warps with a row, one more row, one more column; widths within a step and over several."""
+    w, x = lin_case((*shape, 2), 15)
+    ref = x.astype(np.float64) @ w.astype(np.float64).T
+    # a chain of a lane's share of the columns, then five additions of lanes and at most sixteen of warps, each within half an ulp
+    bound = 2.0 ** -24 * (shape[1] / 32 + 8 + 5 + 16) * (np.abs(x) @ np.abs(w).T)
+    for n in (1, 2):
+        assert (np.abs(linear(cm, 0, w, x[:n]) - ref[:n]) <= bound[:n]).all()
+
+
 @pytest.mark.parametrize("shape", [(19200, 72, 8), (19100, 520, 33), (22544, 136, 64), (40000, 200, 16), (1000, 392, 300), (260, 2056, 412), (19000, 64, 150),
                                    (128, 4096, 350)])
 def test_linear_tiles_shared_out(cm, shape):
