@@ -3,8 +3,9 @@
 //
 //   Q8_K (quantize_q8_k_blocks, src/inference.rs:23121-23152 in the Camelid tree): the first
 //        largest |v| of the 256 keeps its sign; iscale = -127/max; q = min(127, rne(iscale*v));
-//        d = 1/iscale; an all-zero chunk gives d = 0, and codes
-//        are 0 where iscale overflows.
+//        d = 1/iscale; an all-zero chunk gives d = 0.  Where iscale
+//        overflows d is a zero too: the codes then count for nothing in a dot, but a kernel that hands
+//        them out has to write the CPU's (its rounding by a magic number leaves 0).
 //   Q8_0 (quantize_q8_0_block, src/inference.rs:22510-22528): per 32 values d = amax/127 kept
 //        as its f16 rounding; q = round-half-away(v * (1/d_unrounded)) clamped to [-128,127].
 #pragma once
@@ -35,9 +36,8 @@ __device__ __forceinline__ void q8k_quantise_chunk(const float (&v)[8], int lane
     for (int i = 0; i < 8; ++i) q[i] = 0;
   } else {
     const float iscale = __fdiv_rn(-127.0f, mx);
-    const bool none = isinf(iscale);  // |mx| below 2^-121: the CPU's rounding by a magic number leaves no code but 0
 #pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = none ? 0 : min(127, __float2int_rn(__fmul_rn(iscale, v[i])));
+    for (int i = 0; i < 8; ++i) q[i] = min(127, __float2int_rn(__fmul_rn(iscale, v[i])));
     d = __fdiv_rn(1.0f, iscale);
   }
 }

@@ -93,6 +93,8 @@ __global__ void __launch_bounds__(kNormThreads) norm_quant_kernel(NormQuantArgs 
       int q[8];
       float d;
       q8k_quantise_chunk(v, lane, q, d);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) q[i] = d == 0.0f ? 0 : q[i];
       const uint2 packed = pack8(q);
       if (a.rec4 || a.rec6) {
         if (a.rec_tc5) tc5_store_k(packed, d, lane, b, ch, (a.batch + kTc5Rows - 1) / kTc5Rows, a.rec4, a.rec6);
