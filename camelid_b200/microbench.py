@@ -19,6 +19,17 @@ SHAPES = [(4096, 4096), (14336, 4096), (4096, 14336), (128256, 4096)]
 BPW = {"Q8_0": 34 / 32, "Q4_K": 144 / 256, "Q6_K": 210 / 256}
 
 
+# What cmld_gemv_select_kernel takes for each kernel, and the batches that it then serves with it.
+KERNELS = {"staged": (16, 1, 1 << 30), "direct": (1, 1, 1 << 30), "rows": (0, 3, 32), "tcgen05": (32, 1, 1 << 30), "mma": (4, 1, 32)}
+
+
+def kernel_choice(kernel: str, batch: int) -> int:
+    choice, least, most = KERNELS[kernel]
+    if not least <= batch <= most:
+        raise ValueError(f"the {kernel} kernel takes batches of {least} to {most} rows, not {batch}")
+    return choice
+
+
 def peak_gbs() -> tuple[float, str]:
     p = Path(__file__).resolve().parent.parent / "MEASURED_PEAKS.json"
     if p.exists():
@@ -88,8 +99,9 @@ def main():
     ap.add_argument("--batch", type=int, default=0)
     ap.add_argument("--iters", type=int, default=200)
     ap.add_argument("--warmup", type=int, default=20)
-    ap.add_argument("--kernel", default="staged", choices=["staged", "direct", "mma", "tcgen05"],
-                    help="staged = bulk-copy pipelined kernel when the shape fits (default); direct = direct-load kernel")
+    ap.add_argument("--kernel", default="staged", choices=sorted(KERNELS),
+                    help="staged = bulk-copy pipelined kernel where the shape fits, in passes of up to 8 rows (default); direct = direct-load kernel; "
+                         "rows = row-batched kernel (3 to 32 rows; with the rearranging of the activations); tcgen05, mma = tensor-core kernels")
     ap.add_argument("--pdl", action="store_true", help="chain the timed launches with programmatic dependent launch")
     a = ap.parse_args()
     if a.attention:
@@ -98,16 +110,13 @@ def main():
     import camelid_b200 as cm
     from camelid_b200._lib import check
 
-    sel = {"direct": 1, "mma": 4, "tcgen05": 32}.get(a.kernel, 0)
-    check(cm.lib().cmld_gemv_select_kernel(sel))
-    if a.pdl:
-        check(cm.lib().cmld_gemv_select_kernel(sel | 2))
     qts = [a.qt] if a.qt else sorted(BPW)
     shapes = [(a.rows, a.cols)] if a.rows and a.cols else SHAPES
-    batches = [a.batch] if a.batch else [1, 4, 8]
+    batches = [a.batch] if a.batch else [b for b in (1, 4, 8) if KERNELS[a.kernel][1] <= b <= KERNELS[a.kernel][2]]
     for qt in qts:
         for rows, cols in shapes:
             for b in batches:
+                check(cm.lib().cmld_gemv_select_kernel(kernel_choice(a.kernel, b) | (2 if a.pdl else 0)))
                 res = run_case(qt, rows, cols, b, a.iters, a.warmup)
                 res["kernel"] = a.kernel
                 res["pdl"] = bool(a.pdl)
