@@ -347,19 +347,20 @@ def test_prompt_of_two_long_steps(cm, orc):
 
 
 def test_long_prefill_from_embeddings_leaves_the_serial_kv(cm, orc):
-    """Embedding rows in, a long step and a start past row 0: the K/V rows are the checker's."""
-    cfg = cm.EngineConfig(n_layers=2, n_heads=8, n_kv_heads=4, head_dim=64, hidden=256, ffn_dim=512, vocab=512, max_pos=640)
+    """Embedding rows in, long steps of 1024 and 76 rows and a start past row 0: the K/V rows are the checker's."""
+    n = 1100
+    cfg = cm.EngineConfig(n_layers=2, n_heads=8, n_kv_heads=4, head_dim=64, hidden=256, ffn_dim=512, vocab=512, max_pos=1152)
     pair = ModelPair(cfg, "q4_k_m", seed=62)
     eng, ref = pair.engine, pair.oracle
-    prompt = orc.synth_tokens(9, 1, 600, cfg.vocab)
+    prompt = orc.synth_tokens(9, 1, n, cfg.vocab)
     embs = np.stack([ref.embedding(int(t)) for t in prompt])
-    for pos in range(600):
+    for pos in range(n):
         ref.forward(embs[pos], pos, want_logits=False)
-    cos, sin = (np.stack(t) for t in zip(*[pair.rope(pos) for pos in range(600)]))
+    cos, sin = (np.stack(t) for t in zip(*[pair.rope(pos) for pos in range(n)]))
     for start in (0, 3):
-        eng.prefill_from(embs, cos, sin, 600, pair.scale, start)
+        eng.prefill_from(embs, cos, sin, n, pair.scale, start)
         for layer in range(cfg.n_layers):
-            for got, want in zip(eng.read_kv_layer(layer, 600), ref.read_kv_layer(layer, 600)):
+            for got, want in zip(eng.read_kv_layer(layer, n), ref.read_kv_layer(layer, n)):
                 assert np.array_equal(got, want), (start, layer)
 
 
@@ -479,11 +480,11 @@ def test_prompts_take_the_same_steps_whatever_the_number_of_slots(cm, orc, slots
     from camelid_b200 import synth
 
     def engine(n_slots):
-        cfg = cm.EngineConfig(n_layers=2, n_heads=8, n_kv_heads=4, head_dim=64, hidden=512, ffn_dim=512, vocab=512, max_pos=704, max_seqs=n_slots)
+        cfg = cm.EngineConfig(n_layers=2, n_heads=8, n_kv_heads=4, head_dim=64, hidden=512, ffn_dim=512, vocab=512, max_pos=1152, max_seqs=n_slots)
         return synth.build_engine(cfg, "q4_k_m", 5)
 
     one, many = engine(1), engine(slots)
-    for n in (40, 200, 600):
+    for n in (40, 200, 600, 1100):
         prompt = orc.synth_tokens(3, 1, n, 512)
         for want in ([], [], [], [0, n // 2, n - 2]):  # a step was captured at its second call and replayed from the third on
             t1, l1 = one.extend(0, prompt, 0, want=want)
