@@ -476,7 +476,7 @@ def run_ours(args):
                           "frac_of_measured_copy_peak": gbs / (hbm_peak * peaks), "frac_of_8tbs_nominal": gbs / (8000.0 * peaks)},
     }
     if r["prefill_ms"] is not None:
-        # not part of the metric: the prompts are ingested up to 512 rows at a time through the batched matvec
+        # not part of the metric: the prompts are ingested up to 1024 rows at a time through the batched matvec
         line["prefill"] = {"prompt_tokens": n_prompt * batch, "ms": r["prefill_ms"], "tokens_per_s": n_prompt * batch / (r["prefill_ms"] * 1e-3)}
     if e2e:
         line["e2e"] = e2e

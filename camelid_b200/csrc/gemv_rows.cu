@@ -16,11 +16,13 @@
 //
 // Two forms share this:
 //   rows_whole_kernel  a warp walks a tile of 16 weight rows, its sums stay in its registers; the step's records lie in shared
-//                      memory.  For matrices with five tiles per SM or more.
+//                      memory.  For matrices of one type with five tiles per SM or more whose records leave room for two ring stages
+//                      of every warp; of Q6_K, whose sums take the registers, at most eight activation rows.  (At the 128 registers of
+//                      512 threads Q6_K and 25 to 32 rows of Q4_K spill 88 and 48 bytes.)
 //   rows_split_kernel  sixteen warps share a tile, a warp per unit, and hand the f32 terms of a pass (sixteen units) through shared
 //                      memory to four warps that add them in block order, a thread per output.  For matrices whose tiles are too few
 //                      to give every warp one (4096 rows: 1.7 tiles per SM).  Their operand B comes from L2, asked for one exchange
-//                      ahead.  A launch may hold Q4_K and Q6_K matrices, on CTAs of their own.
+//                      ahead.  A launch may hold Q4_K and Q6_K matrices, on CTAs of their own.  All that the other form does not take.
 //
 // Measured, us per launch (records from quantised rows included, 2.3; weights beyond L2): the staged kernel at 3 and 6 rows and the tcgen05
 // one (the rows four times over as its 128-row operand A) at 16 and 32 | here:

@@ -21,7 +21,7 @@ namespace cmld {
 // kernel that rearranged rows into records took 3 to 4 us per product of a prompt step.  With 16-byte loads (a lane's eight values lie
 // together) SwiGLU of 512 x 14336 takes 29.4 us, 39.0 before; the norm of 512 x 4096, one CTA per row, 15.7, 18.4 before.
 constexpr int kNormThreads = 256;
-constexpr int kNormOneCta = 148;  // rows from which a row's norm is one CTA's work
+constexpr int kNormOneCta = 148;  // rows from which a row's norm is one CTA's work: a row for every SM of a B200
 constexpr int kNormMaxExact = 8192;  // widest row whose squares are summed by all warps (exact_sum.cuh); wider rows by one thread
 
 // Eight consecutive values; vec: 16-byte aligned.
@@ -132,7 +132,7 @@ int32_t launch_norm_quant(const NormQuantArgs &args, cudaStream_t s) {
   a.vec = ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.x2) | reinterpret_cast<uintptr_t>(a.weight) | reinterpret_cast<uintptr_t>(a.out)) & 15) == 0;
   if (a.cols % 32 != 0) return fail(CMLD_ERR_SHAPE, "activation width %lld is not a multiple of 32", (long long)a.cols);
   if ((a.act_q8_k || a.rec4 || a.rec6 || a.rec0) && a.cols % 256 != 0)
-    return fail(CMLD_ERR_SHAPE, "Q8_K activation width %lld is not a multiple of 256", (long long)a.cols);
+    return fail(CMLD_ERR_SHAPE, "activation width %lld of Q8_K rows or of a batched product's records is not a multiple of 256", (long long)a.cols);
   if (a.batch <= 0) return CMLD_OK;
   const int mode = a.x2 ? 2 : (a.weight ? 1 : 0);
   const int64_t n_chunks = (a.cols + 255) >> 8;
