@@ -99,24 +99,53 @@ __device__ __forceinline__ void tmem_ld16(uint32_t t, float (&r)[16]) {
 __device__ __forceinline__ void put(float *p, float v) { *p = v; }
 __device__ __forceinline__ void put(bf16 *p, float v) { *p = __float2bfloat16_rn(v); }
 
-// The tile of a cluster of S CTAs, whose partial accumulators [n_tile][128] lie at `base` of each: the elements are shared out over the
-// CTAs' threads, neighbours side by side, and their partials added in rank order, all of them asked for first.  (Four neighbours per thread
-// in 16-byte loads left whole warps without any at few rows and stored quarters of a line.  Us, that | this: 2048 x 2048 with
-// 16 rows 10.3 | 9.3, 768 x 2048 with 16 4.7 | 4.2, 1536 x 4096 with 8 7.0 | 6.5, 4096 x 4096 with 8 9.9 | 9.6.)
-template <int S, typename OutT>
+// The tile of a cluster, whose partial accumulators [n_tile][128] lie at `base` of each CTA: the elements are shared out over all threads and
+// their partials, all of them asked for first, added in rank order.  Few rows: an element per thread, neighbours side by side (four to a
+// thread in 16-byte loads leave whole warps without any and store quarters of a line).  Many rows, from four rounds of all threads on: four
+// to a thread.  Us, four | one: 2048 x 2048 with 16 rows 10.3 | 9.1, 768 x 2048 with 16 4.7 | 4.0, 1536 x 4096 with 8 7.0 | 6.6, 4096 x 4096 with 100
+// 14.7 | 16.1.  One loop per number of CTAs, four elements of a thread at once, did as well with every launch alike (9.3, 4.2, 6.5, 14.5) and was
+// slower among other kernels, where its code is fetched anew: a step of the 2k Tokovik at 12 rows 410 us, here 406, 421 with four to a thread.
+template <typename OutT>
 __device__ __forceinline__ void add_parts(const TcLinArgs &a, uint32_t base, int rank) {
   OutT *out = static_cast<OutT *>(a.out);
-  const int t = (int)blockIdx.x / S, m0 = (t / a.tiles_n) * kBM, n0 = (t % a.tiles_n) * a.n_tile;
-  const int n_el = min(a.n_tile, a.n_rows - n0) * kBM, per = (a.n_k + S - 1) / S, parts = (a.n_k + per - 1) / per;  // (the last may have none)
-  constexpr int kStep = S * kThreads, N = 4;
-  auto load = [&](int e, float (&u)[S]) {
+  const int t = (int)blockIdx.x / a.split, m0 = (t / a.tiles_n) * kBM, n0 = (t % a.tiles_n) * a.n_tile;
+  const int n_el = min(a.n_tile, a.n_rows - n0) * kBM, step = a.split * kThreads;
+  const int per = (a.n_k + a.split - 1) / a.split, parts = (a.n_k + per - 1) / per;  // (the last CTAs may have none)
+  if (n_el > 4 * step) {
+    for (int e = 4 * (rank * kThreads + (int)threadIdx.x); e < n_el; e += 4 * step) {
+      const int o = m0 + e % kBM;
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f), u[8];
 #pragma unroll
-    for (int p = 0; p < S; ++p) u[p] = ld_peer(base + 4u * e, p);
-  };
-  auto finish = [&](int e, const float (&u)[S]) {
-    float v = 0.0f;
+      for (int p = 0; p < 8; ++p)
+        if (p < parts) u[p] = ld_peer4(base + 4u * e, p);
 #pragma unroll
-    for (int p = 0; p < S; ++p) v = p < parts ? v + u[p] : v;
+      for (int p = 0; p < 8; ++p)
+        if (p < parts) v = make_float4(v.x + u[p].x, v.y + u[p].y, v.z + u[p].z, v.w + u[p].w);
+      float r[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) r[j] = fmaf(r[j], a.scale, a.bias && o + j < a.m_rows ? a.bias[o + j] : 0.0f);
+      OutT *p = out + (int64_t)(n0 + e / kBM) * a.out_ld;
+      if (a.act == kActSwiGlu) {
+#pragma unroll
+        for (int j = 0; j < 4; j += 2)
+          if (o + j < a.m_rows) put(p + ((o + j) >> 1), silu_f(r[j]) * r[j + 1]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (o + j < a.m_rows) put(p + o + j, lin_activate(r[j], a.act, o + j < a.act_rows));
+      }
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int e = rank * kThreads + (int)threadIdx.x; e < n_el; e += step) {  // (all counts are multiples of 32: a warp's lanes agree on what is there)
+    float u[8], v = 0.0f;
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+      if (p < parts) u[p] = ld_peer(base + 4u * e, p);
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+      if (p < parts) v += u[p];
     const int o = m0 + e % kBM;
     v = fmaf(v, a.scale, a.bias && o < a.m_rows ? a.bias[o] : 0.0f);
     OutT *q = out + (int64_t)(n0 + e / kBM) * a.out_ld;
@@ -126,19 +155,6 @@ __device__ __forceinline__ void add_parts(const TcLinArgs &a, uint32_t base, int
     } else if (o < a.m_rows) {
       put(q + o, lin_activate(v, a.act, o < a.act_rows));
     }
-  };
-  int e = rank * kThreads + (int)threadIdx.x;  // (all counts are multiples of 32: a warp's lanes agree on what is there)
-  for (; e + (N - 1) * kStep < n_el; e += N * kStep) {
-    float u[N][S];
-#pragma unroll
-    for (int j = 0; j < N; ++j) load(e + j * kStep, u[j]);
-#pragma unroll
-    for (int j = 0; j < N; ++j) finish(e + j * kStep, u[j]);
-  }
-  for (; e < n_el; e += kStep) {
-    float u[S];
-    load(e, u);
-    finish(e, u);
   }
 }
 
@@ -314,11 +330,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (a.split > 1) {
     // one tile per cluster: add the partial accumulators in rank order
     cluster_sync();
-    if (!*abort_flag) {
-      if (a.split == 2) add_parts<2, OutT>(a, base, rank);
-      else if (a.split == 4) add_parts<4, OutT>(a, base, rank);
-      else add_parts<8, OutT>(a, base, rank);
-    }
+    if (!*abort_flag) add_parts<OutT>(a, base, rank);
     cluster_sync();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
