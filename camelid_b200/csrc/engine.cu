@@ -191,6 +191,16 @@ static int64_t hold_prompt_scratch(cmld_engine *e) {
   return e->prompt_scratch_floats;
 }
 
+// Rows of the next step of a prompt with `left` rows to come.  Up to eight rows beyond 512 go by themselves: with them the batched product has a
+// fifth tile of 128 rows, which takes as long as a full one, where a short step reads the weights once more.  In one step | as 512 and
+// the rest, two layers, us, at 513 and 520 tokens: 1B Q8_0 1316 | 1127 and 1322 | 1135, 8B Q8_0 3305 | 2805 and 3306 | 2857, 8B Q4_K_M 2631 | 2374 and
+// 2629 | 2410, 3B 1539 | 1480 and 1541 | 1521.  Beyond 640, 768 and 896 it depends on the width (at 897: 8B 4083 | 3931, 1B 1650 | 1704): one step.
+constexpr int kEvenRows = 512, kRestRows = 8;
+static int step_rows(int chunk, int64_t left) {
+  const int rows = (int)std::min<int64_t>(chunk, left);
+  return rows > kEvenRows && rows <= kEvenRows + kRestRows ? kEvenRows : rows;
+}
+
 static int32_t engine_init(cmld_engine *e) {
   const cmld_config &c = e->cfg;
   CMLD_TRY(engine_open(e, e->device));
@@ -1715,9 +1725,9 @@ int32_t cmld_engine_prefill_from(cmld_engine *e, const float *embeddings, const 
   const int half = e->cfg.rope_dim / 2;
   // up to 8 rows are one short step; longer prompts go in chunk_rows at a time
   const int chunk = (n - start > 8 && !(e->cfg.flags & CMLD_FLAG_EXACT_ORDER)) ? e->chunk_rows : 8;
-  for (int64_t i = start; i < n; i += chunk) {
-    const int rows = (int)std::min<int64_t>(chunk, n - i);
-    CMLD_TRY(forward_embedding_rows(e, embeddings + i * e->cfg.hidden, cos_all + i * half, sin_all + i * half, i, rows, scale,
+  for (int64_t i = start, rows; i < n; i += rows) {
+    rows = step_rows(chunk, n - i);
+    CMLD_TRY(forward_embedding_rows(e, embeddings + i * e->cfg.hidden, cos_all + i * half, sin_all + i * half, i, (int32_t)rows, scale,
                                     false, false, false, 0, -1, true));
   }
   return finish(e, "prefill");
@@ -1953,8 +1963,9 @@ static int32_t llama_extend(cmld_engine *e, int32_t seq, const int32_t *tokens, 
                             float *logits_out) {
   const int chunk = (n > 8 && !(e->cfg.flags & CMLD_FLAG_EXACT_ORDER)) ? e->chunk_rows : 8;
   int32_t w = 0;
-  for (int64_t i = 0; i < n; i += chunk) {
-    const int rows = (int)std::min<int64_t>(chunk, n - i);
+  for (int64_t i = 0, next; i < n; i = next) {
+    const int rows = step_rows(chunk, n - i);
+    next = i + rows;
     std::vector<int32_t> seqs(rows, seq), pos32;
     std::vector<int64_t> pos(rows);
     for (int r = 0; r < rows; ++r) pos[r] = start_pos + i + r;
@@ -1965,7 +1976,7 @@ static int32_t llama_extend(cmld_engine *e, int32_t seq, const int32_t *tokens, 
       pos32.insert(pos32.end(), part.begin(), part.end());
     }
     CMLD_TRY(stage_rows(e, rows, tokens + i, pos32.data(), seqs.data()));
-    const bool wanted = w < n_want && want[w] < i + rows, last = i + chunk >= n;
+    const bool wanted = w < n_want && want[w] < i + rows, last = next >= n;
     const bool by_row = rows > kShortRows;  // a long step: logits of the rows that are asked for only
     StepOpts o;
     o.batch = rows;

@@ -473,6 +473,27 @@ def test_engines_open_on_a_nearly_full_card(monkeypatch, cm, orc):
     assert shorter[0] == token and np.array_equal(shorter[1], logits) and shorter[2] > launches  # three steps in place of two
 
 
+@pytest.mark.parametrize("n", [513, 520, 521])  # 512 and a rest of its own, and the first that is one step
+def test_prompts_just_beyond_512_rows(cm, orc, n):
+    cfg = cm.EngineConfig(n_layers=2, n_heads=8, n_kv_heads=4, head_dim=64, hidden=256, ffn_dim=512, vocab=512, max_pos=640)
+    pair = ModelPair(cfg, "q4_k_m", seed=65)
+    eng, ref = pair.engine, pair.oracle
+    prompt = orc.synth_tokens(9, 1, n, cfg.vocab)
+    all_logits = np.stack([ref.forward(ref.embedding(int(t)), pos)[0] for pos, t in enumerate(prompt)])
+    launches = {}
+    for want in (sorted({0, 511, 512, n - 1}), [511], [512], []):
+        token, logits = eng.extend(0, prompt, 0, want=want)
+        launches[n] = eng.last_timing()[1]
+        assert np.array_equal(logits.view(np.uint32), all_logits[want].view(np.uint32)), want
+        assert token == orc.argmax(all_logits[n - 1]), want
+    eng.extend(0, prompt[:512], 0)
+    assert (launches[n] > eng.last_timing()[1]) == (n <= 520)  # (no logits but the last token's)
+    for layer in range(cfg.n_layers):
+        eng.extend(0, prompt, 0)
+        for got, kept in zip(eng.read_kv_layer(layer, n), ref.read_kv_layer(layer, n)):
+            assert np.array_equal(got, kept), layer
+
+
 @pytest.mark.parametrize("slots", [40, 64, 512])
 def test_prompts_take_the_same_steps_whatever_the_number_of_slots(cm, orc, slots):
     """A prompt's steps are chosen by its rows: an engine of many slots launches what an engine of one launches (no logits of
