@@ -351,11 +351,18 @@ bool attention_prompt_fits(int n_heads, int n_kv_heads, int head_dim, int batch,
   if (G > kQ) return false;
   const int R = kQ / G, all = (batch + R - 1) / R;
   const int per_block = n_kv_heads * (head_dim / 64), wanted = std::min(all, (sms + per_block - 1) / per_block);
-  // Half a machine of CTAs, or at long contexts a quarter: a CTA walks its positions alone, where the row kernel's many small CTAs share
-  // the machine.  Us per layer, row kernel | here: 8B width, 128 rows at 200 positions 74 | 62, 64 at 200 38 | 46, 36 at 700 53 | 78, 64 at
-  // 2000 325 | 205; 1B width, 100 rows at 200 35 | 47, 200 at 700 170 | 110; 3B width, 100 at 200 52 | 48, 40 at 200 26 | 42.
+  // Half a machine of CTAs: a CTA walks its positions alone, where the row kernel's many small CTAs share the machine.  Us per layer, row
+  // kernel | here: 8B width, 128 rows at 200 positions 74 | 62, 64 at 200 38 | 46, 36 at 700 53 | 78, 64 at 2000 325 | 205; 1B width, 100 rows at
+  // 200 35 | 47, 200 at 700 170 | 110; 3B width, 100 at 200 52 | 48, 40 at 200 26 | 42.
+  if (scratch_floats < wanted * block_floats(n_kv_heads, n_pos)) return false;
   const int64_t ctas = (int64_t)all * per_block;
-  return (ctas * 2 >= sms || (ctas * 4 >= sms && n_pos >= 1024)) && scratch_floats >= wanted * block_floats(n_kv_heads, n_pos);
+  if (ctas * 2 >= sms) return true;
+  // Down to a quarter at long contexts, where the row kernel is not done in few rounds of the machine: per 1000 positions a round takes it 41, 35
+  // and 25 us at the 8B, 3B and 1B widths (10 us and 0.06 per query head of a group and dimension), a CTA here 83 us, and 50 to 70 more
+  // whatever the context.  Two layers, us, row kernel | here, rows from position p on: 8B 36 from 2000 937 | 1054, 33 from 6000 1586 | 1718, 40 from 1000
+  // 888 | 899; 1B 72 from 2000 731 | 796, 80 from 1000 616 | 637, 96 from 1000 662 | 647; 3B 48 from 2000 799 | 839, 56 from 1000 686 | 676.
+  const double rounds = (double)(((int64_t)batch * n_kv_heads + sms - 1) / sms);
+  return ctas * 4 >= sms && n_pos >= 1024 && (double)n_pos * (rounds * (10.0 + 0.06 * G * head_dim) - 83.0) > 50000.0;
 }
 
 int32_t launch_attention_prompt(const AttnArgs &a, int64_t n_pos, int sms, float *scratch, int64_t scratch_floats, cudaStream_t s, int64_t *launches) {

@@ -494,6 +494,29 @@ def test_prompts_just_beyond_512_rows(cm, orc, n):
             assert np.array_equal(got, kept), layer
 
 
+@pytest.mark.parametrize("rows, first, kernels", [(36, 2000, 1), (40, 2000, 3), (40, 1000, 1), (36, 6000, 1), (80, 100, 3)])
+def test_attention_of_some_rows_at_long_contexts(cm, rows, first, kernels):
+    """The row kernel where it is done in two rounds of the machine, the three prompt kernels beyond: as many launches a layer more than with one
+    kernel, the same logits as from the plain reference-order kernels."""
+    from camelid_b200 import synth
+
+    def engine(layers, flags):
+        cfg = cm.EngineConfig(n_layers=layers, n_heads=32, n_kv_heads=8, head_dim=128, hidden=256, ffn_dim=512, vocab=512, max_pos=8192, flags=flags)
+        return synth.build_engine(cfg, "q4_k_m", 5)
+
+    def run(eng, tokens, start):
+        token, logits = eng.extend(0, tokens, start, want=[0, len(tokens) - 1])
+        return token, logits.view(np.uint32), eng.last_timing()[1]
+
+    prompt = np.arange(rows, dtype=np.int32)
+    per_layer = run(engine(2, 0), prompt, first)[2] - run(engine(1, 0), prompt, first)[2]
+    short = np.arange(36, dtype=np.int32)  # (at a short context always one kernel)
+    base = run(engine(2, 0), short, 100)[2] - run(engine(1, 0), short, 100)[2]
+    assert per_layer - base == kernels - 1
+    got, ref = run(engine(1, 0), prompt, first), run(engine(1, 16), prompt, first)
+    assert got[0] == ref[0] and np.array_equal(got[1], ref[1])
+
+
 @pytest.mark.parametrize("slots", [40, 64, 512])
 def test_prompts_take_the_same_steps_whatever_the_number_of_slots(cm, orc, slots):
     """A prompt's steps are chosen by its rows: an engine of many slots launches what an engine of one launches (no logits of
